@@ -87,7 +87,7 @@ struct ListRef {
 
 struct opb_batch_plan {
     int f16 = 0;
-    int mode = 0, nlat = 0, nmat = 0, nK = 0, ldk = 64, maxn = 0, cfg = 0, grid = 0;
+    int mode = 0, nlat = 0, nmat = 0, nK = 0, ldk = 64, maxn = 0, cfg = 0, grid = 0, dmax = 0;
     long long total_rows = 0;
     int ell_width = 0;
     const int *cols = nullptr;
@@ -102,15 +102,15 @@ struct opb_batch_plan {
     double period = 0.0;
     // device tables
     opb::BatchLattice *lats = nullptr;
-    // the squaring and chain problems and maps come in two sets, [0] reading the parts in
-    // the A buffers and [1] those in the other buffer (squarings: B; chains: the pair carved
-    // from the FP32 chain buffer), each product writing its output's parts into the other
-    opb::TcProblem *sq[2] = {nullptr, nullptr}, *chain[2] = {nullptr, nullptr}, *price = nullptr;
+    // the squaring problems and maps come in two sets, [0] reading the parts in the A buffers
+    // and [1] those in the B buffers, each product writing its output's parts into the other
+    opb::TcProblem *sq[2] = {nullptr, nullptr}, *price = nullptr;
+    opb::RowChainLat *rows = nullptr;  // the quoted row of each lattice's chain
     opb::RenormProblem *rn_sq = nullptr;
     // 4 maps per lattice (Ahi, Alo, Bhi, Blo), the same for every tile width: squaring (B =
-    // E's row-major parts, MN-major), chain (B = P1's row-major parts), pricing (K-major
-    // payoff parts), per part set
-    CUtensorMap *maps_sq[2] = {nullptr, nullptr}, *maps_ch[2] = {nullptr, nullptr}, *maps_price[2] = {nullptr, nullptr};
+    // E's row-major parts, MN-major; set 1's B is P1 after the squarings, which the chained
+    // rows read), pricing (A = the rows' parts, B = K-major payoff parts)
+    CUtensorMap *maps_sq[2] = {nullptr, nullptr}, *maps_price = nullptr;
     __nv_bfloat16 *B_hi = nullptr, *B_lo = nullptr;  // the B part buffers of all lattices
     size_t B_bytes = 0;                                 // of each
     // backward induction: A = P1's parts, B = the option values' parts read d x ldk row-major
@@ -120,10 +120,10 @@ struct opb_batch_plan {
     size_t E_bytes = 0;
     // work lists (offsets into `work`)
     std::vector<ListRef> gemm_level[NCFG];
-    ListRef gemm_chain[NCFG];
     std::vector<ListRef> gemm_level_rest[NCFG];  // pair configurations: the 128 x 256 items
-    ListRef gemm_chain_rest[NCFG];
-    ListRef gemm_price;
+    ListRef gemm_price;                // every 128-row tile (the induction's products)
+    ListRef gemm_rows;                 // one tile per lattice (the priced rows)
+    ListRef row_items;                 // the chained rows' 64-column items
     std::vector<ListRef> rn_level;     // per level: the lattices whose last level it is (P1)
     std::vector<char> level_inter;     // per level: some lattice squares on after it
     ListRef rn_init;
@@ -228,12 +228,11 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     const int ldk = 64;
     auto lats = c.take<opb::BatchLattice>(n);
     auto sq = c.take<opb::TcProblem>(2 * (size_t)n);
-    auto ch = c.take<opb::TcProblem>(2 * (size_t)n);
+    auto rw = c.take<opb::RowChainLat>(n);
     auto pr = c.take<opb::TcProblem>(n);
     auto rs = c.take<opb::RenormProblem>(n);
     auto msq = c.take<CUtensorMap>(8 * (size_t)n);
-    auto mch = c.take<CUtensorMap>(8 * (size_t)n);
-    auto mp = c.take<CUtensorMap>(8 * (size_t)n);
+    auto mp = c.take<CUtensorMap>(4 * (size_t)n);
     size_t Etot = 0;
     for (int i = 0; i < n; i++) Etot += (size_t)b->d[i] * b->d[i];
     float *E = c.take<float>(Etot);
@@ -261,18 +260,18 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     // sel: 0 every lattice, 1 only sizes that are multiples of 256, 2 only the others.  A
     // size that is not a multiple of bn gets a last column tile that overhangs the matrix:
     // its B columns beyond d load as zeros and its output groups beyond d are not stored.
-    auto gemm_list = [&](const std::vector<int> &order, int bn, int level, bool chain_or_all, int sel = 0,
-                         int tile_m = 128, bool by_work = false) {
+    auto gemm_list = [&](const std::vector<int> &order, int bn, int level, int sel = 0, int tile_m = 128,
+                         bool by_work = false) {
         ListRef r{W.size(), 0};
         for (int i : order) {
-            if (!chain_or_all && b->niter[i] <= level) continue;
+            if (b->niter[i] <= level) continue;
             if ((sel == 1 && b->d[i] % 256) || (sel == 2 && b->d[i] % 256 == 0)) continue;
             const int mt = b->d[i] / tile_m, nt = (b->d[i] + bn - 1) / bn;
             for (int a = 0; a < mt; a++)
                 for (int bb = 0; bb < nt; bb++) W.push_back(((uint32_t)i << 16) | ((uint32_t)a << 8) | (uint32_t)bb);
         }
         r.n = (int)(W.size() - r.off);
-        if (by_work && bands && !chain_or_all) {
+        if (by_work && bands) {
             auto kb = [&](uint32_t w) {
                 const int i = (int)(w >> 16);
                 return host_band_kblocks((*bands)[i], level, (int)((w >> 8) & 255u) * tile_m, tile_m,
@@ -283,7 +282,6 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
         return r;
     };
     std::vector<ListRef> gl[NCFG], glr[NCFG];
-    ListRef gch[NCFG], gchr[NCFG];
     for (int cfg = 0; cfg < NCFG; cfg++) {
         const bool longest = cfg < 2 || cfg == 4 || cfg == 6;
         const auto &order = longest ? lpt : nat;
@@ -291,24 +289,27 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
             // 256 x 256 pair items for the multiples of 256, then 128 x 256 items (column
             // overhang) for the other sizes
             for (int lv = 0; lv < maxn; lv++) {
-                gl[cfg].push_back(gemm_list(order, 256, lv, false, 1, 256, longest));
-                glr[cfg].push_back(gemm_list(order, 256, lv, false, 2, 128, longest));
+                gl[cfg].push_back(gemm_list(order, 256, lv, 1, 256, longest));
+                glr[cfg].push_back(gemm_list(order, 256, lv, 2, 128, longest));
             }
-            gch[cfg] = gemm_list(order, 256, 0, true, 1, 256);
-            gchr[cfg] = gemm_list(order, 256, 0, true, 2, 128);
         } else {
             for (int lv = 0; lv < maxn; lv++) {
-                gl[cfg].push_back(gemm_list(order, CFG_BN[cfg], lv, false, 0, 128, longest));
+                gl[cfg].push_back(gemm_list(order, CFG_BN[cfg], lv, 0, 128, longest));
                 glr[cfg].push_back(ListRef{W.size(), 0});
             }
-            gch[cfg] = gemm_list(order, CFG_BN[cfg], 0, true);
-            gchr[cfg] = ListRef{W.size(), 0};
         }
     }
     ListRef gpr{W.size(), 0};
     for (int i : lpt)
         for (int a = 0; a < b->d[i] / 128; a++) W.push_back(((uint32_t)i << 16) | ((uint32_t)a << 8));
     gpr.n = (int)(W.size() - gpr.off);
+    ListRef grw{W.size(), 0};
+    for (int i : lpt) W.push_back((uint32_t)i << 16);
+    grw.n = (int)(W.size() - grw.off);
+    ListRef gri{W.size(), 0};
+    for (int i : lpt)
+        for (int a = 0; a < b->d[i] / 64; a++) W.push_back(((uint32_t)i << 16) | (uint32_t)a);
+    gri.n = (int)(W.size() - gri.off);
     auto rn_list = [&](int level, int kind) {  // kind: 0 init split, 1 the lattices ending at `level`
         ListRef r{W.size(), 0};
         for (int i : lpt) {
@@ -347,26 +348,21 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     P->cols_pad = cols_pad; P->vals_pad = vals_pad; P->x_pad = x_pad;
 
     // ---- fill the plan and host copies of the tables
-    P->nlat = n; P->nmat = b->nmat; P->nK = b->nK; P->ldk = ldk; P->maxn = maxn;
+    P->nlat = n; P->nmat = b->nmat; P->nK = b->nK; P->ldk = ldk; P->maxn = maxn; P->dmax = b->d[lpt[0]];
     P->total_rows = off[n]; P->ell_width = b->ell_width; P->cols = b->gen_cols; P->vals = b->gen_vals;
     P->x = b->x; P->strikes = b->strikes; P->period = b->period;
-    P->lats = lats; P->sq[0] = sq; P->sq[1] = sq + n; P->chain[0] = ch; P->chain[1] = ch + n; P->price = pr;
+    P->lats = lats; P->sq[0] = sq; P->sq[1] = sq + n; P->rows = rw; P->price = pr;
     P->rn_sq = rs;
-    for (int k = 0; k < 2; k++) {
-        P->maps_sq[k] = msq + 4 * (size_t)n * k;
-        P->maps_ch[k] = mch + 4 * (size_t)n * k;
-        P->maps_price[k] = mp + 4 * (size_t)n * k;
-    }
+    for (int k = 0; k < 2; k++) P->maps_sq[k] = msq + 4 * (size_t)n * k;
+    P->maps_price = mp;
     P->maps_berm = mbm; P->work = work;
     P->B_hi = Bh; P->B_lo = Bl; P->B_bytes = sizeof(__nv_bfloat16) * Etot;
     P->E_base = E; P->E_bytes = Etot * sizeof(float);
     for (int cfg = 0; cfg < NCFG; cfg++) {
         P->gemm_level[cfg] = gl[cfg];
-        P->gemm_chain[cfg] = gch[cfg];
         P->gemm_level_rest[cfg] = glr[cfg];
-        P->gemm_chain_rest[cfg] = gchr[cfg];
     }
-    P->gemm_price = gpr; P->rn_level = rl; P->level_inter = inter; P->rn_init = rinit;
+    P->gemm_price = gpr; P->gemm_rows = grw; P->row_items = gri; P->rn_level = rl; P->level_inter = inter; P->rn_init = rinit;
     if (work_out) *work_out = W;
     return total;
 }
@@ -449,14 +445,15 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
     }
     // host images of the device tables
     std::vector<opb::BatchLattice> lats(n);
-    std::vector<opb::TcProblem> sq(2 * (size_t)n), ch(2 * (size_t)n), pr(n);
+    std::vector<opb::TcProblem> sq(2 * (size_t)n), pr(n);
+    std::vector<opb::RowChainLat> rw(n);
     std::vector<opb::RenormProblem> rs(n);
-    std::vector<CUtensorMap> msq(8 * (size_t)n), mch(8 * (size_t)n), mp(8 * (size_t)n), mbm(4 * (size_t)n);
+    std::vector<CUtensorMap> msq(8 * (size_t)n), mp(4 * (size_t)n), mbm(4 * (size_t)n);
     // recompute buffer pointers exactly as layout() carved them
     Carve cv{base, 0};
-    cv.take<opb::BatchLattice>(n); cv.take<opb::TcProblem>(2 * (size_t)n); cv.take<opb::TcProblem>(2 * (size_t)n);
+    cv.take<opb::BatchLattice>(n); cv.take<opb::TcProblem>(2 * (size_t)n); cv.take<opb::RowChainLat>(n);
     cv.take<opb::TcProblem>(n); cv.take<opb::RenormProblem>(n);
-    cv.take<CUtensorMap>(8 * (size_t)n); cv.take<CUtensorMap>(8 * (size_t)n); cv.take<CUtensorMap>(8 * (size_t)n);
+    cv.take<CUtensorMap>(8 * (size_t)n); cv.take<CUtensorMap>(4 * (size_t)n);
     size_t Etot = 0;
     for (int i = 0; i < n; i++) Etot += (size_t)b->d[i] * b->d[i];
     float *E = cv.take<float>(Etot), *Pa = cv.take<float>(Etot);
@@ -491,29 +488,28 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
         L.Vd = vd + (size_t)ro * P->ldk;
         double *pi = part + po;
         L.niter = b->niter[i]; L.partial = pi; L.fix = fix + ro;
-        // part sets: squarings between A and B, chains between A and a pair carved from the
-        // FP32 chain buffer (2 d^2 BF16 values in its d^2 floats)
+        // part sets: squarings between A and B
         __nv_bfloat16 *sh[2] = {Ah + eo, Bh + eo}, *sl[2] = {Al + eo, Bl + eo};
-        __nv_bfloat16 *c2 = reinterpret_cast<__nv_bfloat16 *>(Pa + eo);
-        __nv_bfloat16 *chh[2] = {Ah + eo, c2}, *chl[2] = {Al + eo, c2 + dd};
         for (int k = 0; k < 2 && rc_status == OPB_OK; k++) {
             // squaring: E' = 2E + E.E in place of E (as the previous level's GEMM left it, its
             // normalisation deferred into this epilogue through the row fixes), the output's
             // parts into the other set
             sq[k * n + i] = opb::TcProblem{d, d, d, bands[i], L.E, L.E, pi, d, un2, 2.f, fix + ro, sh[k ^ 1],
                                            sl[k ^ 1]};
-            // chain: parts only, P_{m-1}'s row fix applied in the epilogue
-            ch[k * n + i] = opb::TcProblem{d, d, d, 0, nullptr, nullptr, pi, d, un2, 0.f, fix + ro, chh[k ^ 1],
-                                           chl[k ^ 1]};
             rc_status = opb::tc_make_maps(&msq[4 * ((size_t)k * n + i)], sh[k], sl[k], d, d, sh[k], sl[k], d, d, d,
                                           64, f16, 1);
-            if (rc_status == OPB_OK)
-                rc_status = opb::tc_make_maps(&mch[4 * ((size_t)k * n + i)], chh[k], chl[k], d, d, Bh + eo, Bl + eo, d,
-                                              d, d, 64, f16, 1);
-            if (rc_status == OPB_OK)
-                rc_status = opb::tc_make_maps(&mp[4 * ((size_t)k * n + i)], chh[k], chl[k], d, d, L.GThi, L.GTlo,
-                                              P->ldk, d, d, 64, f16);
         }
+        // the quoted row of the chained kernels: FP32 rows in E (done with after the
+        // squarings), the parts to be priced in Pa, their row scales in the row-sum partials
+        opb::RowChainLat &R = rw[i];
+        R.d = d;
+        R.hi = Ah + eo + (size_t)L.y0 * d; R.lo = Al + eo + (size_t)L.y0 * d;
+        R.C[0] = L.E; R.C[1] = L.E + d;
+        R.Qhi = reinterpret_cast<__nv_bfloat16 *>(Pa + eo); R.Qlo = R.Qhi + (size_t)opb::kRowSlots * d;
+        R.qinv = pi;
+        if (rc_status == OPB_OK)
+            rc_status = opb::tc_make_maps(&mp[4 * (size_t)i], R.Qhi, R.Qlo, opb::kRowSlots, d, L.GThi, L.GTlo, P->ldk,
+                                          d, d, 64, f16);
         pr[i] = opb::TcProblem{d, P->ldk, d, 0, L.V, nullptr, nullptr, P->ldk, un1, 0.f, nullptr};
         rs[i] = opb::RenormProblem{d, 0, L.E, pi, Ah + eo, Al + eo, Bh + eo, Bl + eo, fix + ro};
         if (rc_status == OPB_OK)  // the same buffers, the value parts read d x ldk row-major
@@ -536,12 +532,11 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = up(P->lats, lats.data(), sizeof(opb::BatchLattice) * n);
     if (e == cudaSuccess) e = up(P->sq[0], sq.data(), sizeof(opb::TcProblem) * 2 * (size_t)n);
-    if (e == cudaSuccess) e = up(P->chain[0], ch.data(), sizeof(opb::TcProblem) * 2 * (size_t)n);
+    if (e == cudaSuccess) e = up(P->rows, rw.data(), sizeof(opb::RowChainLat) * n);
     if (e == cudaSuccess) e = up(P->price, pr.data(), sizeof(opb::TcProblem) * n);
     if (e == cudaSuccess) e = up(P->rn_sq, rs.data(), sizeof(opb::RenormProblem) * n);
     if (e == cudaSuccess) e = up(P->maps_sq[0], msq.data(), sizeof(CUtensorMap) * 8 * (size_t)n);
-    if (e == cudaSuccess) e = up(P->maps_ch[0], mch.data(), sizeof(CUtensorMap) * 8 * (size_t)n);
-    if (e == cudaSuccess) e = up(P->maps_price[0], mp.data(), sizeof(CUtensorMap) * 8 * (size_t)n);
+    if (e == cudaSuccess) e = up(P->maps_price, mp.data(), sizeof(CUtensorMap) * 4 * (size_t)n);
     if (e == cudaSuccess) e = up(P->maps_berm, mbm.data(), sizeof(CUtensorMap) * 4 * (size_t)n);
     if (e == cudaSuccess) e = up(P->work, W.data(), sizeof(uint32_t) * W.size());
     const cudaError_t es = cudaStreamSynchronize(ls);
@@ -578,20 +573,22 @@ OPB_API int opb_batch_set_config(opb_batch_plan *P, int cfg, int grid) {
 
 namespace {
 
-// One squaring level (or the chain product) under configuration cfg: one launch, or two
-// for the pair configurations (256 x 256 pair items, then 128 x 256 ones).  maps: the
-// squaring or the chain table (MN-major B); fixmode: how the problems' row fixes apply.
-int cfg_gemm(opb_batch_plan *P, int cfg, const CUtensorMap *maps, const opb::TcProblem *probs, const ListRef &l,
-             const ListRef &rest, cudaStream_t s, int level, int lolo, int skip, int fixmode, int fuse) {
-    const int bn = CFG_BN[cfg];
+// One squaring level under configuration cfg: one launch, or two for the pair configurations
+// (256 x 256 pair items, then 128 x 256 ones).  The level reads the part set level % 2;
+// fixmode: how the problems' row fixes apply.
+int cfg_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s, int lolo, int skip, int fixmode) {
+    const int bn = CFG_BN[cfg], k = level & 1;
     const float ss = P->f16 ? F16S : 0.f;
+    const CUtensorMap *maps = P->maps_sq[k];
+    const opb::TcProblem *probs = P->sq[k];
+    const ListRef &l = P->gemm_level[cfg][level], &rest = P->gemm_level_rest[cfg][level];
     int r = CFG_PAIR[cfg] ? opb::launch_tc_gemm_batched_pair(maps, probs, P->work + l.off, l.n, s, P->f16, 1, level,
-                                                             lolo, skip, fixmode, ss, fuse)
+                                                             lolo, skip, fixmode, ss, 1)
                           : opb::launch_tc_gemm_batched(bn, maps, probs, P->work + l.off, l.n, P->grid, s, P->f16, 1,
-                                                        level, lolo, skip, fixmode, ss, fuse);
+                                                        level, lolo, skip, fixmode, ss, 1);
     if (r == 0 && rest.n > 0)
         r = opb::launch_tc_gemm_batched(256, maps, probs, P->work + rest.off, rest.n, P->grid, s, P->f16, 1, level,
-                                        lolo, skip, fixmode, ss, fuse);
+                                        lolo, skip, fixmode, ss, 1);
     return r;
 }
 
@@ -602,17 +599,12 @@ int cfg_gemm(opb_batch_plan *P, int cfg, const CUtensorMap *maps, const opb::TcP
 // is deferred into this epilogue.
 int level_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s) {
     const int lolo = (!P->f16 && level < opb::g_lolo_levels) ? 1 : 0;
-    const int k = level & 1;
-    return cfg_gemm(P, cfg, P->maps_sq[k], P->sq[k], P->gemm_level[cfg][level], P->gemm_level_rest[cfg][level], s,
-                    level, lolo, opb::g_band_skip, level > 0 ? opb::OPB_FIX_SQUARE : opb::OPB_FIX_NONE, 1);
+    return cfg_gemm(P, cfg, level, s, lolo, opb::g_band_skip, level > 0 ? opb::OPB_FIX_SQUARE : opb::OPB_FIX_NONE);
 }
 
-// The chain product of every lattice (dense, all lattices active): what the autotuner times.
-// set: the part set holding P_{m-1}; scaled: apply P_{m-1}'s row fixes (every chain but the
-// first, whose A is the normalised P1).
-int chain_gemm(opb_batch_plan *P, int cfg, cudaStream_t s, int set = 0, bool scaled = false) {
-    return cfg_gemm(P, cfg, P->maps_ch[set], P->chain[set], P->gemm_chain[cfg], P->gemm_chain_rest[cfg], s, 0, 0, 0,
-                    scaled ? opb::OPB_FIX_ROWSCALE : opb::OPB_FIX_NONE, 2);
+// What the autotuner times: the first level's squaring of every lattice, without its band.
+int dense_gemm(opb_batch_plan *P, int cfg, cudaStream_t s) {
+    return cfg_gemm(P, cfg, 0, s, 0, 0, opb::OPB_FIX_NONE);
 }
 
 // E0 build and every squaring level: P1 of every lattice as row-major parts in its A and B
@@ -637,7 +629,7 @@ int batch_square(opb_batch_plan *P, cudaStream_t s) {
     for (int lv = 0; lv < P->maxn && r == 0; lv++) {
         r = level_gemm(P, cfg, lv, s);
         if (r == 0 && P->level_inter[lv])
-            r = opb::launch_rowfix_batched(P->lats, P->nlat, P->total_rows, pdiv, lv, 1, s);
+            r = opb::launch_rowfix_batched(P->lats, P->nlat, P->total_rows, pdiv, lv, s);
         if (r == 0 && P->rn_level[lv].n > 0)
             r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_level[lv].off, P->rn_level[lv].n, pdiv, s, ss);
     }
@@ -665,21 +657,25 @@ OPB_API int opb_batch_execute(opb_batch_plan *P, double *quotes) {
                                  P->fp32_ws_bytes, quotes + (size_t)i * P->nmat * P->nK, nullptr));
         return set_status(OPB_OK);
     }
-    const int cfg = P->cfg, bn = CFG_BN[cfg], pdiv = bn < 128 ? bn : 128;
     BT(batch_square(P, s));
     BT(opb::launch_payoff_batched(P->lats, P->nlat, P->total_rows, P->nK, P->ldk, P->x, P->strikes, s, P->f16));
-    // chains: P_m = P_{m-1} . P1 writes only its parts (into the other part set) and its row
-    // sums; its row fixes scale the next chain's epilogue and this maturity's quotes
-    int set = 0;
+    // chains: the quoted row of P_m = P_{m-1} . P1 for every lattice (row_chain.cuh), its
+    // normalisation deferred into the next step and into the quotes; one product prices up
+    // to kRowSlots maturities
+    const float ss = P->f16 ? F16S : 0.f, un2 = P->f16 ? 1.f / (F16S * F16S) : 1.f;
     for (int m = 1; m <= P->nmat; m++) {
-        if (m > 1) {
-            BT(chain_gemm(P, cfg, s, set, m > 2));
-            BT(opb::launch_rowfix_batched(P->lats, P->nlat, P->total_rows, pdiv, -1, 0, s));
-            set ^= 1;
-        }
-        BT(opb::launch_tc_gemm_batched(64, P->maps_price[set], P->price, P->work + P->gemm_price.off,
-                                       P->gemm_price.n, P->grid, s, P->f16, 0));
-        BT(opb::launch_quotes_batched(P->lats, P->nlat, P->nK, P->ldk, m, P->nmat, quotes, s, P->f16, m > 1));
+        const bool last = m == P->nmat, full = m % opb::kRowSlots == 0;
+        if (last)
+            BT(opb::launch_row_finish_batched(P->rows, P->nlat, m, ss, s));
+        else
+            BT(opb::launch_row_step_batched(P->rows, P->maps_sq[1], P->work + P->row_items.off, P->row_items.n, P->dmax,
+                                            m + 1, P->f16, un2, ss, s));
+        if (!last && !full) continue;
+        const int m0 = (m - 1) / opb::kRowSlots * opb::kRowSlots;
+        BT(opb::launch_tc_gemm_batched(64, P->maps_price, P->price, P->work + P->gemm_rows.off, P->gemm_rows.n,
+                                       P->grid, s, P->f16, 0));
+        BT(opb::launch_row_quotes_batched(P->lats, P->rows, P->nlat, m - m0, m0, P->nK, P->ldk, P->nmat, quotes, s,
+                                          P->f16));
     }
 #undef BT
     return set_status(OPB_OK);
@@ -721,8 +717,8 @@ OPB_API int opb_batch_execute_bermudan(opb_batch_plan *P, int put, int exercise,
     return set_status(OPB_OK);
 }
 
-// Times the chain product (dense, all lattices active: the shape of every squaring level
-// once the operands have filled in) for every configuration with CUDA events and keeps the
+// Times a dense squaring (all lattices active: the shape of every squaring level once the
+// operands have filled in) for every configuration with CUDA events and keeps the
 // fastest; ms[cfg] (optional, opb_batch_num_configs() entries) receives the times.
 // Blocking; leaves the plan's buffers in an arbitrary state (run execute afterwards).
 OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *best_cfg) {
@@ -739,11 +735,11 @@ OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *
     float best = 1e30f;
     int bc = 0;
     for (int cfg = 0; cfg < NCFG; cfg++) {
-        int r = chain_gemm(P, cfg, s);  // warm-up (also sets the smem attribute)
+        int r = dense_gemm(P, cfg, s);  // warm-up (also sets the smem attribute)
         if (r) return set_status(r);
         OPB_TRY(cudaEventRecord(e0, s));
         for (int i = 0; i < reps; i++) {
-            r = chain_gemm(P, cfg, s);
+            r = dense_gemm(P, cfg, s);
             if (r) return set_status(r);
         }
         OPB_TRY(cudaEventRecord(e1, s));
@@ -765,11 +761,12 @@ OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *
 OPB_API int opb_batch_launches(const opb_batch_plan *P) {
     if (!P) return 0;
     if (!tc_mode_b(P->mode)) return -1;
-    int extra = 0;  // the pair configurations' second GEMM launch per level / chain
+    int extra = 0;  // the pair configurations' second GEMM launch per level
     for (int lv = 0; lv < P->maxn; lv++) extra += P->gemm_level_rest[P->cfg][lv].n > 0 ? 1 : 0;
-    if (P->gemm_chain_rest[P->cfg].n > 0) extra += P->nmat - 1;
     int per_level = 0;  // GEMM, row fixes (some lattice squares on), renormalisation (some ends)
     for (int lv = 0; lv < P->maxn; lv++)
         per_level += 1 + (P->level_inter[lv] ? 1 : 0) + (P->rn_level[lv].n > 0 ? 1 : 0);
-    return 5 + (P->padded ? 1 : 0) + per_level + 1 + (P->f16 ? 1 : 0) + 2 * P->nmat + 2 * (P->nmat - 1) + extra;
+    // a row launch per maturity; a product and a quote launch per group of priced maturities
+    const int groups = (P->nmat + opb::kRowSlots - 1) / opb::kRowSlots;
+    return 5 + (P->padded ? 1 : 0) + per_level + 1 + (P->f16 ? 1 : 0) + P->nmat + 2 * groups + extra;
 }

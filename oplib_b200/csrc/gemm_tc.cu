@@ -1321,8 +1321,8 @@ int launch_tc_gemm_batched_pair(const CUtensorMap *maps, const TcProblem *probs,
     if (nwork <= 0) return OPB_OK;
     if (!b_kn) return OPB_E_UNSUPPORTED;
     if (fuse == 1) return batched_pair_fused<1>(maps, probs, work, nwork, s, f16, level, lolo, band_skip, fixmode, sscale);
-    if (fuse == 2) return batched_pair_fused<2>(maps, probs, work, nwork, s, f16, level, lolo, band_skip, fixmode, sscale);
-    return batched_pair_fused<0>(maps, probs, work, nwork, s, f16, level, lolo, band_skip, fixmode, sscale);
+    return fuse ? OPB_E_UNSUPPORTED
+                : batched_pair_fused<0>(maps, probs, work, nwork, s, f16, level, lolo, band_skip, fixmode, sscale);
 }
 
 // MN-major B (b_kn) in every tile width and epilogue form; K-major B (pricing) 64-wide only.
@@ -1361,8 +1361,7 @@ int launch_tc_gemm_batched(int bn, const CUtensorMap *maps, const TcProblem *pro
     if (b_kn) {
         if (fuse == 1)
             return batched_kn<1>(bn, maps, probs, work, nwork, grid, s, f16, level, lolo, band_skip, fixmode, sscale);
-        if (fuse == 2)
-            return batched_kn<2>(bn, maps, probs, work, nwork, grid, s, f16, level, lolo, band_skip, fixmode, sscale);
+        if (fuse) return OPB_E_UNSUPPORTED;
         return batched_kn<0>(bn, maps, probs, work, nwork, grid, s, f16, level, lolo, band_skip, fixmode, sscale);
     }
     if (bn != 64 || fuse) return OPB_E_UNSUPPORTED;
@@ -1744,6 +1743,8 @@ int launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s) {
         default: return OPB_E_UNSUPPORTED;
     }
 }
+
+#include "row_chain.cuh"
 
 }  // namespace opb
 

@@ -310,6 +310,34 @@ int solve_tc(const opb_lattice_desc &L, Bufs &b, double *quotes, double *V_all, 
     // K-slices fill the GPU with this small-N product's tiles; the discount sums them
     pg.ksplit = opb::tc_gemm_split_for(d, nKp, d);
     pg.c_slice = (long long)d * nKp;
+    // Without the all-state values the quotes are one row of each P_m G, and that row of P_m
+    // needs the same row of P_{m-1} and P1: one pass over P1 per maturity instead of a d^3
+    // product, then one product prices up to kRowSlots maturities' rows together.  The quotes
+    // are the full products' bit for bit (row_chain.cuh).  The rows lie in X (P1's FP32 form,
+    // done with), their parts in the FP32 chain buffer.  Larger lattices than the row kernel's
+    // shared memory takes, and the K-sliced accumulation knob, go through the full products.
+    if (!V_all && opb::row_chain_fits(d) && g_ksplit <= 1) {
+        opb::RowChainLat R{};
+        R.d = d;
+        R.hi = b.Ahi + (size_t)L.y0 * d; R.lo = b.Alo + (size_t)L.y0 * d;
+        R.C[0] = b.X; R.C[1] = b.X + d;
+        R.Qhi = reinterpret_cast<__nv_bfloat16 *>(b.Pa); R.Qlo = R.Qhi + (size_t)opb::kRowSlots * d;
+        R.qinv = b.Vd;
+        const int fz = opb::fused_single(d) ? 1 : 0;
+        pg.M = opb::kRowSlots; pg.Ahi = R.Qhi; pg.Alo = R.Qlo;
+        pg.c_slice = (long long)opb::kRowSlots * nKp;
+        for (int m = 1; m <= L.nmat; m++) {
+            const bool last = m == L.nmat, full = m % opb::kRowSlots == 0;
+            if (last) LT(opb::launch_row_finish(R, m, fz, ss, s));
+            else LT(opb::launch_row_step(R, b.Bhi, b.Blo, m + 1, fz, f16 ? 1 : 0, unscale, ss, s));
+            if (!last && !full) continue;
+            const int m0 = (m - 1) / opb::kRowSlots * opb::kRowSlots;
+            LT(tc_gemm_ksplit(pg, s));
+            LT(opb::launch_row_quotes(m - m0, m0, nK, nKp, b.V, L.rate, L.period, R.qinv, gs, pg.ksplit, pg.c_slice,
+                                      quotes, s));
+        }
+        return 0;
+    }
     // The chain products write only the parts of their output, ping-ponging between the A
     // part buffers and a second pair carved from the FP32 chain buffer (unused in the split
     // modes); each output's row normalisation is deferred into the next chain product's

@@ -172,14 +172,14 @@ int launch_ek_batched(const BatchLattice *lats, int nlat, long long total_rows, 
                       const double *vals, cudaStream_t s);
 int launch_payoff_batched(const BatchLattice *lats, int nlat, long long total_rows, int nK, int ldk, const double *x,
                           const double *strikes, cudaStream_t s, int f16 = 0);
-// rowfix: scale each lattice's V row y0 by its fix (P-form products with deferred normalisation)
-int launch_quotes_batched(const BatchLattice *lats, int nlat, int nK, int ldk, int m, int nmat, double *quotes,
-                          cudaStream_t s, int f16 = 0, int rowfix = 0);
+// Quotes of nm priced rows of every lattice (row slot i: maturity m0 + i + 1)
+struct RowChainLat;
+int launch_row_quotes_batched(const BatchLattice *lats, const RowChainLat *rows, int nlat, int nm, int m0, int nK,
+                              int ldk, int nmat, double *quotes, cudaStream_t s, int f16 = 0);
 // BatchLattice::fix from BatchLattice::partial (parts_div columns per partial) for every
-// lattice still squaring after `level` (eform, niter > level + 1), or for all (P-form,
-// level < 0)
+// lattice still squaring after `level` (niter > level + 1)
 int launch_rowfix_batched(const BatchLattice *lats, int nlat, long long total_rows, int parts_div, int level,
-                          int eform, cudaStream_t s);
+                          cudaStream_t s);
 
 // gemm_tc.cu -- split-BF16 tensor-core GEMM.
 //   C[M,N] = alpha * (Ahi.Bhi^T + Ahi.Blo^T + Alo.Bhi^T) + beta * Cin[M,N]
@@ -308,6 +308,33 @@ int launch_tc_gemm_batched(int bn, const CUtensorMap *maps, const TcProblem *pro
 int launch_tc_gemm_batched_pair(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
                                 cudaStream_t s, int f16, int b_kn, int level = 0,
                                 int lolo = 0, int band_skip = 0, int fixmode = 0, float sscale = 0.f, int fuse = 0);
+
+// row_chain.cuh (in gemm_tc.cu) -- the quoted row of the chained kernels.
+// The quoted row of one lattice.
+struct RowChainLat {
+    int d, pad;
+    const __nv_bfloat16 *hi, *lo;  // row y0 of P1's parts
+    float *C[2];                   // the row of P_m as the product leaves it (index m & 1), d floats each
+    __nv_bfloat16 *Qhi, *Qlo;      // parts of the rows of P_1, P_2, ... (slot (m - 1) % kRowSlots, d each)
+    double *qinv;                  // per slot: what the priced row is still to be multiplied by
+};
+constexpr int kRowSlots = 128;  // maturities priced by one product
+bool row_chain_fits(int d);     // d % 128 == 0 and the row's operand fits shared memory (d <= 30336)
+// Row of P_m = P_{m-1} . P1 (m >= 2) into L.C[m & 1], and P_{m-1}'s parts into its pricing slot.
+// Bhi / Blo: P1's parts, row-major.  fused: as opb::fused_single (the batched form always is).
+int launch_row_step(const RowChainLat &L, const __nv_bfloat16 *Bhi, const __nv_bfloat16 *Blo, int m, int fused, int f16,
+                    float alpha, float sscale, cudaStream_t s);
+// P_m's row into its slot, after the last step.
+int launch_row_finish(const RowChainLat &L, int m, int fused, float sscale, cudaStream_t s);
+// All lattices of a plan: work items lattice << 16 | 64-column tile, maps 4 per lattice (the
+// last two P1's parts, MN-major), dmax the largest size.
+int launch_row_step_batched(const RowChainLat *lats, const CUtensorMap *maps, const uint32_t *work, int nwork, int dmax,
+                            int m, int f16, float alpha, float sscale, cudaStream_t s);
+int launch_row_finish_batched(const RowChainLat *lats, int nlat, int m, float sscale, cudaStream_t s);
+// quotes[(m0 + i) * nK + k] = exp(-rate * period * (m0 + i + 1)) * (the slices' sum of V[i][k]) * qinv[i]
+// / *dscale for the nm priced slots (lattice_kernels.cu)
+int launch_row_quotes(int nm, int m0, int nK, int ldk, const float *V, double rate, double period, const double *qinv,
+                      const float *dscale, int nslice, long long slice_stride, double *quotes, cudaStream_t s);
 
 // sck.cu
 int launch_sck_rm(int d, int nrows, const float *P, float *C, cudaStream_t s);

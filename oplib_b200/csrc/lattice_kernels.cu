@@ -455,17 +455,21 @@ __global__ void k_payoff_batched(const BatchLattice *__restrict__ lats, int nlat
     L.GTlo[(long long)k * L.d + z] = l;
 }
 
-// quotes[(i*nmat + m-1)*nK + k] = exp(-r_i T_m) * V_i[y0_i, k]
-__global__ void k_quotes_batched(const BatchLattice *__restrict__ lats, int nlat, int nK, int ldk, int m, int nmat,
-                                 double *__restrict__ quotes, int f16, int rowfix) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nlat * nK) return;
-    int i = t / nK, k = t - i * nK;
-    const BatchLattice &L = lats[i];
-    double disc = exp(-L.rate * L.period * m);
+// Quotes of nm priced rows of every lattice (slot i of lattice l holds maturity m0 + i + 1):
+// quotes[(l*nmat + m0 + i)*nK + k] = exp(-r_l T) * V_l[i, k], times what the row's deferred
+// normalisation still owes (qinv).
+__global__ void k_row_quotes_batched(const BatchLattice *__restrict__ lats, const RowChainLat *__restrict__ rows,
+                                     int nlat, int nm, int m0, int nK, int ldk, int nmat, double *__restrict__ quotes,
+                                     int f16) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= (long long)nlat * nm * nK) return;
+    const int l = (int)(t / ((long long)nm * nK)), r = (int)(t - (long long)l * nm * nK);
+    const int i = r / nK, k = r - i * nK;
+    const BatchLattice &L = lats[l];
+    double disc = exp(-L.rate * L.period * (m0 + i + 1));
     if (f16) disc /= (double)L.gscale[0];
-    if (rowfix) disc *= L.fix[L.y0].y;  // the deferred normalisation of the priced row
-    quotes[((long long)i * nmat + (m - 1)) * nK + k] = disc * (double)L.V[(long long)L.y0 * ldk + k];
+    disc *= rows[l].qinv[i];
+    quotes[((long long)l * nmat + m0 + i) * nK + k] = disc * (double)L.V[(long long)i * ldk + k];
 }
 
 // Row fixes from FP64 row-sum partials, with the arithmetic of the renormalisation
@@ -492,11 +496,10 @@ __global__ void k_rowfix(int d, const double *__restrict__ partial, int nparts, 
     if (r < d) fix[r] = row_fix(partial, d, nparts, r, eform);
 }
 
-// Thread per global row of all lattices (rows concatenated); level >= 0: only the lattices
-// whose next level is an intermediate squaring (niter > level + 1), E-form; level < 0: all,
-// P-form.
+// Thread per global row of all lattices (rows concatenated), for the lattices whose next
+// level is an intermediate squaring (niter > level + 1).
 __global__ void k_rowfix_batched(const BatchLattice *__restrict__ lats, int nlat, long long total_rows, int parts_div,
-                                 int level, int eform) {
+                                 int level) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= total_rows) return;
     int lo = 0, hi = nlat - 1;
@@ -505,9 +508,9 @@ __global__ void k_rowfix_batched(const BatchLattice *__restrict__ lats, int nlat
         if (lats[mid].row_off <= t) lo = mid; else hi = mid - 1;
     }
     const BatchLattice &L = lats[lo];
-    if (level >= 0 && L.niter <= level + 1) return;
+    if (L.niter <= level + 1) return;
     const int row = (int)(t - L.row_off);
-    L.fix[row] = row_fix(L.partial, L.d, L.d / parts_div, row, eform);
+    L.fix[row] = row_fix(L.partial, L.d, L.d / parts_div, row, 1);
 }
 
 // E-form -> P-form: P = I + E (in place), FP32.
@@ -560,6 +563,19 @@ __global__ void k_discount(int d, int nK, int ldk, const float *__restrict__ V32
     if (rowfix) v *= rowfix[y].y;  // the deferred row normalisation of the priced product
     if (V64) V64[t] = v;
     if (quotes && y == y0) quotes[k] = v;
+}
+
+// Quotes of nm priced rows (slot i: maturity m0 + i + 1) of one lattice.
+__global__ void k_row_quotes(int nm, int m0, int nK, int ldk, const float *__restrict__ V, double rate, double period,
+                             const double *__restrict__ qinv, const float *__restrict__ dscale, int nslice,
+                             long long slice_stride, double *__restrict__ quotes) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nm * nK) return;
+    const int i = t / nK, k = t - i * nK;
+    double disc = exp(-rate * period * (m0 + i + 1));
+    if (dscale) disc /= (double)*dscale;
+    const double v = disc * sum_slices(V, (long long)i * ldk + k, nslice, slice_stride);
+    quotes[(long long)(m0 + i) * nK + k] = v * qinv[i];
 }
 
 // ------------------------------------------------------------------ backward induction
@@ -955,10 +971,17 @@ int launch_payoff_batched(const BatchLattice *lats, int nlat, long long total_ro
     return (int)cudaGetLastError();
 }
 
-int launch_quotes_batched(const BatchLattice *lats, int nlat, int nK, int ldk, int m, int nmat, double *quotes,
-                          cudaStream_t s, int f16, int rowfix) {
-    int n = nlat * nK;
-    k_quotes_batched<<<(n + 255) / 256, 256, 0, s>>>(lats, nlat, nK, ldk, m, nmat, quotes, f16, rowfix);
+int launch_row_quotes_batched(const BatchLattice *lats, const RowChainLat *rows, int nlat, int nm, int m0, int nK,
+                              int ldk, int nmat, double *quotes, cudaStream_t s, int f16) {
+    const long long n = (long long)nlat * nm * nK;
+    k_row_quotes_batched<<<blocks_for(n, 256), 256, 0, s>>>(lats, rows, nlat, nm, m0, nK, ldk, nmat, quotes, f16);
+    return (int)cudaGetLastError();
+}
+
+int launch_row_quotes(int nm, int m0, int nK, int ldk, const float *V, double rate, double period, const double *qinv,
+                      const float *dscale, int nslice, long long slice_stride, double *quotes, cudaStream_t s) {
+    k_row_quotes<<<blocks_for((long long)nm * nK, 256), 256, 0, s>>>(nm, m0, nK, ldk, V, rate, period, qinv, dscale,
+                                                                    nslice > 1 ? nslice : 1, slice_stride, quotes);
     return (int)cudaGetLastError();
 }
 
@@ -968,9 +991,9 @@ int launch_rowfix(int d, const double *partial, int nparts, int eform, double2 *
 }
 
 int launch_rowfix_batched(const BatchLattice *lats, int nlat, long long total_rows, int parts_div, int level,
-                          int eform, cudaStream_t s) {
+                          cudaStream_t s) {
     if (parts_div <= 0) return OPB_E_ARG;
-    k_rowfix_batched<<<blocks_for(total_rows, 256), 256, 0, s>>>(lats, nlat, total_rows, parts_div, level, eform);
+    k_rowfix_batched<<<blocks_for(total_rows, 256), 256, 0, s>>>(lats, nlat, total_rows, parts_div, level);
     return (int)cudaGetLastError();
 }
 
