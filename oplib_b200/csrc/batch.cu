@@ -111,11 +111,14 @@ struct opb_batch_plan {
     // E's row-major parts, MN-major; set 1's B is P1 after the squarings, which the chained
     // rows read), pricing (A = the rows' parts, B = K-major payoff parts)
     CUtensorMap *maps_sq[2] = {nullptr, nullptr}, *maps_price = nullptr;
-    __nv_bfloat16 *B_hi = nullptr, *B_lo = nullptr;  // the B part buffers of all lattices
-    size_t B_bytes = 0;                                 // of each
     // backward induction: A = P1's parts, B = the option values' parts read d x ldk row-major
     CUtensorMap *maps_berm = nullptr;
     uint32_t *work = nullptr;
+    // tile plans of a level's two launches, and the marks of the two part sets (all lattices,
+    // each set occ_bytes; the plans' counter lies behind set 1)
+    opb::TilePlan plan[2];
+    uint8_t *occ[2] = {nullptr, nullptr};
+    size_t occ_bytes = 0;
     float *E_base = nullptr;
     size_t E_bytes = 0;
     // work lists (offsets into `work`)
@@ -125,7 +128,6 @@ struct opb_batch_plan {
     ListRef gemm_rows;                 // one tile per lattice (the priced rows)
     ListRef row_items;                 // the chained rows' 64-column items
     std::vector<ListRef> rn_level;     // per level: the lattices whose last level it is (P1)
-    std::vector<char> level_inter;     // per level: some lattice squares on after it
     ListRef rn_init;
     // FP32 path
     std::vector<LatticeDescMirror> fp32_desc;
@@ -247,6 +249,22 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     (void)c.take<float>(n);          // per-lattice FP16 payoff scales
     (void)c.take<double2>(off[n]);   // per-row fixes of the deferred E-form renormalisation
     auto mbm = c.take<CUtensorMap>(4 * (size_t)n);  // backward-induction maps
+    size_t marks = 0, tiles = 0;  // tiles of the narrowest configuration
+    int nw = 1;
+    for (int i = 0; i < n; i++) {
+        marks += opb::tile_plan_marks(b->d[i]);
+        tiles += (size_t)(b->d[i] / 128) * (b->d[i] / 64);
+        nw = std::max(nw, opb::tile_plan_words(b->d[i]));
+    }
+    uint8_t *occ0 = c.take<uint8_t>(marks), *occ1 = c.take<uint8_t>(marks + 64);
+    opb::TilePlan plan[2];
+    for (auto &pl : plan) {
+        pl.order = c.take<uint32_t>(tiles);
+        pl.kmask = c.take<uint32_t>(tiles * nw);
+        pl.count = c.take<uint16_t>(tiles);
+        pl.nw = nw;
+        pl.done = reinterpret_cast<unsigned *>(occ1 + marks);
+    }
     (void)c.take<double>((size_t)off[n] * ldk);     // FP64 option values of the backward induction
 
     // ---- work lists (host), appended into one blob
@@ -328,11 +346,7 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     };
     ListRef rinit = rn_list(0, 0);
     std::vector<ListRef> rl;
-    std::vector<char> inter(maxn, 0);
-    for (int lv = 0; lv < maxn; lv++) {
-        rl.push_back(rn_list(lv, 1));
-        for (int i = 0; i < n; i++) inter[lv] |= b->niter[i] > lv + 1 ? 1 : 0;
-    }
+    for (int lv = 0; lv < maxn; lv++) rl.push_back(rn_list(lv, 1));
     uint32_t *work = c.take<uint32_t>(W.size());
     // padded copies of the generator and spot values (lattices off the 128 grid)
     int *cols_pad = nullptr;
@@ -356,13 +370,14 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     for (int k = 0; k < 2; k++) P->maps_sq[k] = msq + 4 * (size_t)n * k;
     P->maps_price = mp;
     P->maps_berm = mbm; P->work = work;
-    P->B_hi = Bh; P->B_lo = Bl; P->B_bytes = sizeof(__nv_bfloat16) * Etot;
+    P->plan[0] = plan[0]; P->plan[1] = plan[1];
+    P->occ[0] = occ0; P->occ[1] = occ1; P->occ_bytes = marks;
     P->E_base = E; P->E_bytes = Etot * sizeof(float);
     for (int cfg = 0; cfg < NCFG; cfg++) {
         P->gemm_level[cfg] = gl[cfg];
         P->gemm_level_rest[cfg] = glr[cfg];
     }
-    P->gemm_price = gpr; P->gemm_rows = grw; P->row_items = gri; P->rn_level = rl; P->level_inter = inter; P->rn_init = rinit;
+    P->gemm_price = gpr; P->gemm_rows = grw; P->row_items = gri; P->rn_level = rl; P->rn_init = rinit;
     if (work_out) *work_out = W;
     return total;
 }
@@ -472,7 +487,7 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
     const int f16 = mode == OPB_FP16X3_B ? 1 : 0;
     P->f16 = f16;
     const float un2 = f16 ? 1.f / (F16S * F16S) : 1.f, un1 = f16 ? 1.f / F16S : 1.f;
-    size_t eo = 0, po = 0;
+    size_t eo = 0, po = 0, mo = 0;
     long long ro = 0, so = 0;
     int rc_status = OPB_OK;
     for (int i = 0; i < n && rc_status == OPB_OK; i++) {
@@ -495,7 +510,7 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
             // normalisation deferred into this epilogue through the row fixes), the output's
             // parts into the other set
             sq[k * n + i] = opb::TcProblem{d, d, d, bands[i], L.E, L.E, pi, d, un2, 2.f, fix + ro, sh[k ^ 1],
-                                           sl[k ^ 1]};
+                                           sl[k ^ 1], P->occ[k ^ 1] + mo, P->occ[k] + mo};
             rc_status = opb::tc_make_maps(&msq[4 * ((size_t)k * n + i)], sh[k], sl[k], d, d, sh[k], sl[k], d, d, d,
                                           64, f16, 1);
         }
@@ -516,6 +531,7 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
             rc_status = opb::tc_make_maps(&mbm[4 * (size_t)i], Ah + eo, Al + eo, d, d, L.GThi, L.GTlo, P->ldk,
                                           P->ldk, d, 64, f16, 1);
         eo += dd;
+        mo += opb::tile_plan_marks(d);
         po += (size_t)(d / 64) * d;
         ro += d;
     }
@@ -576,19 +592,21 @@ namespace {
 // One squaring level under configuration cfg: one launch, or two for the pair configurations
 // (256 x 256 pair items, then 128 x 256 ones).  The level reads the part set level % 2;
 // fixmode: how the problems' row fixes apply.
-int cfg_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s, int lolo, int skip, int fixmode) {
+int cfg_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s, int lolo, int skip, int fixmode, bool planned) {
     const int bn = CFG_BN[cfg], k = level & 1;
-    const float ss = P->f16 ? F16S : 0.f;
     const CUtensorMap *maps = P->maps_sq[k];
     const opb::TcProblem *probs = P->sq[k];
     const ListRef &l = P->gemm_level[cfg][level], &rest = P->gemm_level_rest[cfg][level];
-    int r = CFG_PAIR[cfg] ? opb::launch_tc_gemm_batched_pair(maps, probs, P->work + l.off, l.n, s, P->f16, 1, level,
-                                                             lolo, skip, fixmode, ss, 1)
-                          : opb::launch_tc_gemm_batched(bn, maps, probs, P->work + l.off, l.n, P->grid, s, P->f16, 1,
-                                                        level, lolo, skip, fixmode, ss, 1);
+    opb::TcBatchArgs a{P->f16, 1, level, lolo, skip, fixmode, P->f16 ? F16S : 0.f, 1, nullptr, nullptr, 0};
+    auto use = [&](const opb::TilePlan &pl) {
+        if (planned) { a.order = pl.order; a.kmask = pl.kmask; a.nw = pl.nw; }
+    };
+    use(P->plan[0]);
+    int r = CFG_PAIR[cfg] ? opb::launch_tc_gemm_batched_pair(maps, probs, P->work + l.off, l.n, s, a)
+                          : opb::launch_tc_gemm_batched(bn, maps, probs, P->work + l.off, l.n, P->grid, s, a);
+    use(P->plan[1]);
     if (r == 0 && rest.n > 0)
-        r = opb::launch_tc_gemm_batched(256, maps, probs, P->work + rest.off, rest.n, P->grid, s, P->f16, 1, level,
-                                        lolo, skip, fixmode, ss, 1);
+        r = opb::launch_tc_gemm_batched(256, maps, probs, P->work + rest.off, rest.n, P->grid, s, a);
     return r;
 }
 
@@ -599,17 +617,29 @@ int cfg_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s, int lolo, in
 // is deferred into this epilogue.
 int level_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s) {
     const int lolo = (!P->f16 && level < opb::g_lolo_levels) ? 1 : 0;
-    return cfg_gemm(P, cfg, level, s, lolo, opb::g_band_skip, level > 0 ? opb::OPB_FIX_SQUARE : opb::OPB_FIX_NONE);
+    return cfg_gemm(P, cfg, level, s, lolo, opb::g_band_skip, level > 0 ? opb::OPB_FIX_SQUARE : opb::OPB_FIX_NONE,
+                    level > 0 && opb::g_band_skip);
+}
+
+// The tile plans of level `level` >= 1 under configuration cfg (which K-blocks each item
+// issues, from the marks that the previous level left), and its row fixes.
+int level_plan(opb_batch_plan *P, int cfg, int level, cudaStream_t s) {
+    const int bn = CFG_BN[cfg], k = level & 1;
+    const ListRef &l = P->gemm_level[cfg][level], &rest = P->gemm_level_rest[cfg][level];
+    const uint32_t *work[2] = {P->work + l.off, P->work + rest.off};
+    const int n[2] = {l.n, rest.n}, tm[2] = {CFG_PAIR[cfg] ? 256 : 128, 128}, tn[2] = {CFG_PAIR[cfg] ? 256 : bn, 256};
+    return opb::launch_tile_plan_batched(P->plan, work, n, tm, tn, P->sq[k], P->sq[k ^ 1], level, P->occ[k ^ 1],
+                                         (long long)P->occ_bytes, P->lats, P->nlat, bn < 128 ? bn : 128, P->total_rows, s);
 }
 
 // What the autotuner times: the first level's squaring of every lattice, without its band.
 int dense_gemm(opb_batch_plan *P, int cfg, cudaStream_t s) {
-    return cfg_gemm(P, cfg, 0, s, 0, 0, opb::OPB_FIX_NONE);
+    return cfg_gemm(P, cfg, 0, s, 0, 0, opb::OPB_FIX_NONE, false);
 }
 
 // E0 build and every squaring level: P1 of every lattice as row-major parts in its A and B
-// buffers.  Per level one GEMM, then the row fixes of the lattices that square on and the
-// renormalisation (to P1) of those whose last level it was.
+// buffers.  Per level the tile plan with the row fixes of the level before, one GEMM, and the
+// renormalisation (to P1) of the lattices whose last level it was.
 int batch_square(opb_batch_plan *P, cudaStream_t s) {
     const int cfg = P->cfg, bn = CFG_BN[cfg], pdiv = bn < 128 ? bn : 128;
     const float ss = P->f16 ? F16S : 0.f;
@@ -620,16 +650,17 @@ int batch_square(opb_batch_plan *P, cudaStream_t s) {
         r = opb::launch_pad_batched(P->lats, P->nlat, P->total_rows, P->ell_width, P->cols_src, P->vals_src,
                                     P->x_src, P->cols_pad, P->vals_pad, P->x_pad, s);
     if (r == 0) r = (int)cudaMemsetAsync(P->E_base, 0, P->E_bytes, s);
-    // the B part set starts zeroed: a level skips the output tiles outside its operands'
-    // band, which must read as zeros when the next level issues their K-blocks
-    if (r == 0) r = (int)cudaMemsetAsync(P->B_hi, 0, P->B_bytes, s);
-    if (r == 0) r = (int)cudaMemsetAsync(P->B_lo, 0, P->B_bytes, s);
+    // Under the tile plans no block is read that its level did not write.  Without them (band
+    // skipping off) every level writes every tile.
+    const bool planned = opb::g_band_skip != 0;
+    if (r == 0 && planned) r = (int)cudaMemsetAsync(P->occ[1], 0, P->occ_bytes + 64, s);
     if (r == 0) r = opb::launch_ek_batched(P->lats, P->nlat, P->total_rows, P->ell_width, P->cols, P->vals, s);
     if (r == 0) r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_init.off, P->rn_init.n, 0, s, ss);
     for (int lv = 0; lv < P->maxn && r == 0; lv++) {
-        r = level_gemm(P, cfg, lv, s);
-        if (r == 0 && P->level_inter[lv])
-            r = opb::launch_rowfix_batched(P->lats, P->nlat, P->total_rows, pdiv, lv, s);
+        if (lv > 0)
+            r = planned ? level_plan(P, cfg, lv, s)
+                        : opb::launch_rowfix_batched(P->lats, P->nlat, P->total_rows, pdiv, lv - 1, s);
+        if (r == 0) r = level_gemm(P, cfg, lv, s);
         if (r == 0 && P->rn_level[lv].n > 0)
             r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_level[lv].off, P->rn_level[lv].n, pdiv, s, ss);
     }
@@ -673,7 +704,7 @@ OPB_API int opb_batch_execute(opb_batch_plan *P, double *quotes) {
         if (!last && !full) continue;
         const int m0 = (m - 1) / opb::kRowSlots * opb::kRowSlots;
         BT(opb::launch_tc_gemm_batched(64, P->maps_price, P->price, P->work + P->gemm_rows.off, P->gemm_rows.n,
-                                       P->grid, s, P->f16, 0));
+                                       P->grid, s, opb::TcBatchArgs{P->f16, 0}));
         BT(opb::launch_row_quotes_batched(P->lats, P->rows, P->nlat, m - m0, m0, P->nK, P->ldk, P->nmat, quotes, s,
                                           P->f16));
     }
@@ -709,7 +740,7 @@ OPB_API int opb_batch_execute_bermudan(opb_batch_plan *P, int put, int exercise,
                                      P->f16, s));
     for (int m = P->nmat - 1; m >= 0; m--) {
         BT(opb::launch_tc_gemm_batched(64, P->maps_berm, P->price, P->work + P->gemm_price.off, P->gemm_price.n,
-                                       P->grid, s, P->f16, 1));
+                                       P->grid, s, opb::TcBatchArgs{P->f16, 1}));
         BT(opb::launch_berm_batched_step(P->lats, P->nlat, P->total_rows, P->nK, P->ldk, P->x, P->strikes, put,
                                          barrier, exercise, m == 0, P->f16, quotes, s));
     }
@@ -763,10 +794,9 @@ OPB_API int opb_batch_launches(const opb_batch_plan *P) {
     if (!tc_mode_b(P->mode)) return -1;
     int extra = 0;  // the pair configurations' second GEMM launch per level
     for (int lv = 0; lv < P->maxn; lv++) extra += P->gemm_level_rest[P->cfg][lv].n > 0 ? 1 : 0;
-    int per_level = 0;  // GEMM, row fixes (some lattice squares on), renormalisation (some ends)
-    for (int lv = 0; lv < P->maxn; lv++)
-        per_level += 1 + (P->level_inter[lv] ? 1 : 0) + (P->rn_level[lv].n > 0 ? 1 : 0);
+    int per_level = 0;  // plan with row fixes (from the second level on), GEMM, renormalisation (some end)
+    for (int lv = 0; lv < P->maxn; lv++) per_level += 1 + (lv > 0 ? 1 : 0) + (P->rn_level[lv].n > 0 ? 1 : 0);
     // a row launch per maturity; a product and a quote launch per group of priced maturities
     const int groups = (P->nmat + opb::kRowSlots - 1) / opb::kRowSlots;
-    return 5 + (P->padded ? 1 : 0) + per_level + 1 + (P->f16 ? 1 : 0) + P->nmat + 2 * groups + extra;
+    return 4 + (P->padded ? 1 : 0) + per_level + 1 + (P->f16 ? 1 : 0) + P->nmat + 2 * groups + extra;
 }

@@ -40,6 +40,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -279,16 +280,23 @@ struct TcCfg {
     static constexpr int CPT = BN < CPT_MAX ? BN : CPT_MAX;  // accumulator columns per epilogue thread
     static constexpr int HALVES = BN / CPT;                 // column groups per TMEM lane
     static constexpr int EPI_WARPS = 4 * HALVES;            // epilogue warps (4 lane quadrants x groups)
-    // FP32 output: each epilogue warp transposes 32 x 32 blocks through shared memory
-    // (row stride 33 words) so that Cin loads and C stores are whole 128-byte lines.
+    // FP32 output: each epilogue warp transposes 32 x 32 blocks through shared memory so that
+    // Cin loads and C stores are whole 128-byte lines.
     // Network layers (EPIMODE 1): each warp stages its 32 rows x CPT/2 BF16 activations
     // (row stride CPT + 16 bytes) so that its global stores cover 64-byte row segments
     static constexpr int OUT_BYTES =
-        EPIMODE == 0 ? EPI_WARPS * 32 * 33 * 4 : EPIMODE == 1 ? EPI_WARPS * 32 * (CPT + 16) : 0;
+        EPIMODE == 0 ? EPI_WARPS * 32 * 32 * 4 : EPIMODE == 1 ? EPI_WARPS * 32 * (CPT + 16) : 0;
     // network layers: the tile's bias (and output weights) staged in shared memory once
     static constexpr int VEC_BYTES = EPIMODE ? 2 * BN * 4 : 0;
     static constexpr int SMEM = RING_BYTES + 1024 /*align*/ + 256 /*barriers*/ + OUT_BYTES + VEC_BYTES;
-    static constexpr int THREADS = 32 * (EPI_WARPS + 2);    // + TMA producer warp + MMA warp
+    // eight epilogue warps with 128 sums a thread: whole warpgroups, so that the registers can be
+    // split (224 an epilogue thread, 56 for the TMA and MMA warps' group: 2 x 128 x 224 + 128 x 56
+    // = 384 x 168, what the block is launched with); with an even share of 168 the output phase
+    // spilled 0.5 KB a thread
+    static constexpr bool REGSPLIT = EPIMODE == 0 && EPI_WARPS == 8;
+    static constexpr int REGS_LAUNCH = 168, REGS_EPI = 224, REGS_REST = 56;
+    static_assert(!REGSPLIT || 256 * REGS_EPI + 128 * REGS_REST <= 384 * REGS_LAUNCH, "register split");
+    static constexpr int THREADS = REGSPLIT ? 384 : 32 * (EPI_WARPS + 2);  // + TMA producer warp + MMA warp
     static constexpr int TMEM_COLS = 2 * BN;                // two accumulators (ping-pong chunks)
     // K-blocks accumulated in TMEM per chunk: K = 128 for the split products (bounds the
     // tensor cores' truncation); the whole K for single BF16 products (network layers,
@@ -322,6 +330,10 @@ struct TcParams {
     int fixmode;             // as TcGemmArgs::fixmode
     __nv_bfloat16 *Shi, *Slo;  // as TcGemmArgs::Shi / Slo (single products; batched: TcProblem)
     float sscale;            // as TcGemmArgs::sscale
+    const uint32_t *order, *kmask;  // as TcGemmArgs::plan (order and masks of this launch's items)
+    int nw;
+    uint8_t *occ;            // as TcGemmArgs::occ, occ_in (single products; batched: TcProblem)
+    const uint8_t *occ_in;
 };
 
 // K-blocks [kb_lo, kb_lo + nkb) that can contribute to the output tile rows [m0, m0 + tm),
@@ -360,6 +372,8 @@ __device__ __forceinline__ long long level_band(int h0, int level) {
     return (long long)h0 << level;
 }
 
+#include "tile_plan.cuh"
+
 // Batched launches read per-problem tensor maps (4 per problem: Ahi, Alo, Bhi, Blo) and
 // parameters from device tables and walk a work list of packed items
 // (problem << 16 | m-tile << 8 | n-tile).
@@ -391,6 +405,8 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     using Cfg = TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>;
     constexpr int EPI = Cfg::EPI_WARPS;
     constexpr int CPT = Cfg::CPT;
+    constexpr bool PLANNED = NPROD == 3 && BK == 64;  // launches that may carry a tile plan
+    constexpr bool OCC = PLANNED && EPIMODE == 0 && FUSE != 2;  // and marks of their blocks
     static_assert(!BMN || (NPROD == 3 && Cfg::B_ROWS % 64 == 0), "MN-major B: split products");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -420,7 +436,14 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     const int istep = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     // item t -> (problem, m0, n0, K-blocks, first K-block, K-slice); a single product split
     // into nsplit K-slices has nsplit consecutive items per output tile
-    auto get_item = [&](int t, int &prob, int &m0, int &n0, int &nkb, int &kb0, int &slice) {
+    // mk: the item's K-block mask when the launch has a plan (kmask); its chunks keep their
+    // K-blocks, and those whose operand parts are zero are left out
+    auto get_item = [&](int t, int &prob, int &m0, int &n0, int &nkb, int &kb0, int &slice, const uint32_t *&mk) {
+        mk = nullptr;
+        if (PLANNED && p.kmask) {
+            t = (int)p.order[t];
+            mk = p.kmask + (long long)t * p.nw;
+        }
         if constexpr (BATCHED) {
             const uint32_t w = bt.work[t];
             prob = (int)(w >> 16);
@@ -448,6 +471,14 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                 const int h0 = *p.band;
                 band_kblocks(h0 > 0 ? level_band(h0, p.level) : -1, m0, Cfg::TILE_M, n0, BN, p.K, BK, Cfg::CHUNK,
                              kb0, nkb);
+            }
+        }
+        if (PLANNED && mk) {
+            if (nkb == 0) mk = nullptr;  // outside twice the band: nothing to issue, nothing to write
+            else {
+                if constexpr (BATCHED) nkb = bt.probs[prob].K / BK;
+                else nkb = p.K / BK;
+                kb0 = 0;
             }
         }
     };
@@ -512,8 +543,9 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == EPI) {
-        if (lane == 0) {
+    if (warp >= EPI) {
+        if constexpr (Cfg::REGSPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_REST));
+        if (warp == EPI && lane == 0) {
             // ---------------- TMA producer
             long kbg = 0;  // K-blocks issued over the CTA's lifetime (stage ring position)
             bool ok = true;
@@ -528,14 +560,20 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
             }
             for (int t = item0; t < nitems && ok; t += istep) {
                 int prob, m0, n0, nkb, kb0, slice;
-                get_item(t, prob, m0, n0, nkb, kb0, slice);
+                const uint32_t *mk;
+                get_item(t, prob, m0, n0, nkb, kb0, slice, mk);
+                uint32_t mw = 0;
                 const int ma = m0 + (int)rank * TC_BM;          // this CTA's A rows
                 const int nb = n0 + (int)rank * Cfg::B_ROWS;    // this CTA's B rows
                 const CUtensorMap *mp[4] = {&mAhi, &mAlo, &mBhi, &mBlo};
                 if constexpr (BATCHED) {
                     for (int i = 0; i < 4; i++) mp[i] = bt.maps + 4 * prob + i;
                 }
-                for (int kb = 0; kb < nkb; kb++, kbg++) {
+                for (int kb = 0; kb < nkb; kb++) {
+                    if (PLANNED && mk) {
+                        if ((kb & 31) == 0) mw = mk[kb >> 5];
+                        if (!((mw >> (kb & 31)) & 1u)) continue;
+                    }
                     const int s = (int)(kbg % STAGES);
                     if (kbg >= STAGES &&
                         !mbar_wait(empty_bar(s), (uint32_t)(((kbg / STAGES) + 1) & 1), abort_flag, TC_WAIT_NS)) {
@@ -584,6 +622,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                             }
                         }
                     }
+                    kbg++;
                 }
             }
             if (!ok) {
@@ -599,9 +638,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                                         100000000ull);
             }
         }
-        __syncwarp();
-    } else if (warp == EPI + 1) {
-        if (lane == 0 && rank == 0) {
+        if (warp == EPI + 1 && lane == 0 && rank == 0) {
             // ---------------- MMA issuer (pair mode: the even CTA issues for both)
             const uint32_t idesc = umma_idesc_16(BN, F16, Cfg::TILE_M, BMN);
             long kbg = 0, g = 0;  // K-blocks consumed, chunks issued
@@ -614,10 +651,18 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
             }
             for (int t = item0; t < nitems && ok; t += istep) {
                 int prob, m0, n0, nkb, kb0, slice;
-                get_item(t, prob, m0, n0, nkb, kb0, slice);
+                const uint32_t *mk;
+                get_item(t, prob, m0, n0, nkb, kb0, slice, mk);
+                uint32_t mw = 0;
                 const bool lolo = item_lolo(prob);
                 const int nch = (nkb + Cfg::CHUNK - 1) / Cfg::CHUNK;
-                for (int c = 0; c < nch && ok; c++, g++) {
+                for (int c = 0; c < nch && ok; c++) {
+                    uint32_t bits = ~0u;  // which of the chunk's K-blocks are issued
+                    if (PLANNED && mk) {
+                        if ((c & 15) == 0) mw = mk[c >> 4];
+                        bits = (mw >> (2 * c & 31)) & 3u;
+                        if (!bits) continue;
+                    }
                     const int a = (int)(g & 1);
                     if (g >= 2 && !mbar_wait(acce_bar(a), (uint32_t)(((g >> 1) + 1) & 1), abort_flag, TC_WAIT_NS)) {
                         ok = false;
@@ -626,7 +671,9 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     tc_fence_after();
                     const uint32_t dacc = tmem + (uint32_t)(a * BN);
                     const int kb_end = min(nkb, (c + 1) * Cfg::CHUNK);
-                    for (int kb = c * Cfg::CHUNK; kb < kb_end; kb++, kbg++) {
+                    uint32_t fresh = 0u;  // 0: the chunk's first MMA, which starts the accumulator
+                    for (int kb = c * Cfg::CHUNK; kb < kb_end; kb++) {
+                        if (PLANNED && mk && !((bits >> (kb - c * Cfg::CHUNK)) & 1u)) continue;
                         const int s = (int)(kbg % STAGES);
                         if (!mbar_wait(full_bar(s), (uint32_t)((kbg / STAGES) & 1), abort_flag, TC_WAIT_NS)) {
                             ok = false;
@@ -646,7 +693,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                             const uint64_t adv = (uint64_t)((k16 * 32) >> 4);  // +32 bytes along K
                             // MN-major B: +16 rows of 128 bytes along K
                             const uint64_t advb = BMN ? (uint64_t)((k16 * 16 * 128) >> 4) : adv;
-                            const uint32_t acc0 = (kb > c * Cfg::CHUNK || k16 > 0) ? 1u : 0u;
+                            const uint32_t acc0 = k16 > 0 ? 1u : fresh;
                             if constexpr (PAIR) {
                                 umma_bf16_pair(dacc, dAh + adv, dBh + advb, idesc, acc0);
                                 umma_bf16_pair(dacc, dAh + adv, dBl + advb, idesc, 1u);
@@ -661,13 +708,16 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                                 }
                             }
                         }
+                        fresh = 1u;
                         if constexpr (PAIR) umma_commit_pair(empty_bar(s));
                         else umma_commit(empty_bar(s));
+                        kbg++;
                     }
                     if (ok) {
                         if constexpr (PAIR) umma_commit_pair(accf_bar(a));
                         else umma_commit(accf_bar(a));
                     }
+                    g++;
                 }
             }
             if (!ok) {
@@ -682,6 +732,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
         __syncwarp();
     } else {
         // ---------------- epilogue warps: lane quadrant q, column group h
+        if constexpr (Cfg::REGSPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_EPI));
         const int q = warp & 3, h = warp >> 2;
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
         float sum[CPT];
@@ -689,34 +740,88 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
         bool ok = true;
         for (int t = item0; t < nitems && ok; t += istep) {
             int prob, m0, n0, nkb, kb0, slice;
-            get_item(t, prob, m0, n0, nkb, kb0, slice);
-            const int nch = (nkb + Cfg::CHUNK - 1) / Cfg::CHUNK;
+            const uint32_t *mk;
+            get_item(t, prob, m0, n0, nkb, kb0, slice, mk);
+            const bool reached = nkb > 0;
+            int nch = (nkb + Cfg::CHUNK - 1) / Cfg::CHUNK;
+            if (PLANNED && mk) {  // the chunks with a K-block to issue
+                static_assert(!PLANNED || Cfg::CHUNK == 2, "two mask bits per chunk");
+                nch = 0;
+                for (int i = 0; i < p.nw; i++) nch += __popc((mk[i] | (mk[i] >> 1)) & 0x55555555u);
+            }
             if constexpr (NPROD != 1) {  // single products have one chunk: its values are the sums
 #pragma unroll
                 for (int j = 0; j < CPT; j++) sum[j] = 0.f;
             }
-            // this thread's Cin row segment is prefetched into L2 about three chunks before
-            // the output needs it
-            const float *pf = nullptr;
-            long long pf_ld = 0;
             // a batched item's last column tile may overhang its matrix (zero B columns
             // beyond N): this thread's column group then has nothing to store
             const bool group_in = !BATCHED || n0 + h * CPT < bt.probs[prob].N;
+            const int rbase = m0 + (int)rank * TC_BM + q * 32, col0 = n0 + h * CPT;
+            // this thread's Cin row segment is prefetched into L2 about three chunks before
+            // the output needs it (the live 64-column blocks); the row and column fixes are
+            // loaded here, while the MMAs run
+            const float *pf = nullptr;
+            long long pf_ld = 0;
+            const double2 *fix = nullptr;
+            const uint8_t *mi = nullptr;  // marks of the operand's blocks (E before this level)
+            // 64-column blocks that are not zero, or on the diagonal; the second level still
+            // writes every block of its tiles, so that both part sets hold what the marks say
+            uint32_t had = 0, live = ~0u;
+            bool fill = false;            // a zero block's parts are still to be written as zeros
+            double2 rfix = make_double2(0.0, 0.0);
+            float scol[CPT / 32];
             if constexpr (EPIMODE == 0) {
+                int h0 = 0;
                 if constexpr (BATCHED) {
-                    pf = group_in ? bt.probs[prob].Cin : nullptr;
-                    pf_ld = bt.probs[prob].ldc;
+                    const TcProblem &pr = bt.probs[prob];
+                    pf = group_in ? pr.Cin : nullptr;
+                    pf_ld = pr.ldc;
+                    fix = pr.cin_fix;
+                    if (OCC && p.kmask && group_in) {
+                        mi = pr.occ_in;
+                        h0 = pr.band;
+                    }
                 } else {
                     pf = p.Cin;
                     pf_ld = p.ldc;
+                    fix = p.cin_fix;
+                    if (OCC && p.kmask) {
+                        mi = p.occ_in;
+                        h0 = p.band ? *p.band : 0;
+                    }
+                }
+                if (!reached) mi = nullptr;
+                if (OCC && mi) {
+#pragma unroll
+                    for (int b = 0; b < CPT / 64; b++) {
+                        const int c = col0 + 64 * b;
+                        if ((mi[(long long)(rbase >> 5) * (pf_ld >> 6) + (c >> 6)] & 2) || (rbase < c + 64 && c < rbase + 32))
+                            had |= 1u << b;
+                    }
+                    if (p.level >= 2) live = had;
+                    if (FUSE == 1 && h0 > 0 && p.level >= 2) {
+                        const int K = BATCHED ? bt.probs[prob].K : p.K;
+                        int lo, cnt;
+                        band_kblocks(level_band(h0, p.level - 2), m0, Cfg::TILE_M, n0, BN, K, BK, Cfg::CHUNK, lo, cnt);
+                        fill = cnt == 0;
+                    }
+                }
+                if (fix && group_in && (FUSE == 0 || p.fixmode != OPB_FIX_NONE)) {
+                    rfix = fix[rbase + lane];
+                    if constexpr (FUSE == 1) {
+#pragma unroll
+                        for (int j = 0; j < CPT / 32; j++) scol[j] = (float)fix[col0 + 32 * j + lane].x;
+                    }
                 }
             }
             const int pf_chunk = nch > 3 ? nch - 3 : 0;
             for (int c = 0; c < nch; c++, g++) {
                 const int a = (int)(g & 1);
-                if (pf && c == pf_chunk)
-                    prefetch_l2(pf + (long long)(m0 + (int)rank * TC_BM + q * 32 + lane) * pf_ld + n0 + h * CPT,
-                                CPT * 4);
+                if (pf && c == pf_chunk) {
+#pragma unroll
+                    for (int b = 0; b < CPT / 64; b++)
+                        if ((live >> b) & 1u) prefetch_l2(pf + (long long)(rbase + lane) * pf_ld + col0 + 64 * b, 256);
+                }
                 if (!mbar_wait(accf_bar(a), (uint32_t)((g >> 1) & 1), abort_flag, TC_WAIT_NS)) {
                     ok = false;
                     break;
@@ -750,23 +855,22 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
             long long ldc;
             float alpha, beta;
             double *rowsum;
-            const double2 *fix;
             __nv_bfloat16 *Shi, *Slo;  // optional 16-bit parts of the stored values
+            uint8_t *occ;              // optional: which blocks of those parts are not zero
             int M;
             if constexpr (BATCHED) {
                 const TcProblem &pr = bt.probs[prob];
                 C = pr.C; Cin = pr.Cin; ldc = pr.ldc; alpha = pr.alpha; beta = pr.beta; rowsum = pr.rowsum; M = pr.M;
-                fix = pr.cin_fix; Shi = pr.Shi; Slo = pr.Slo;
+                Shi = pr.Shi; Slo = pr.Slo; occ = pr.occ;
             } else {
                 C = p.C ? p.C + (long long)slice * p.c_slice : nullptr;  // K-slices write separate partials
                 Cin = p.Cin; ldc = p.ldc; alpha = p.alpha; beta = p.beta; rowsum = p.rowsum; M = p.M;
-                fix = p.cin_fix; Shi = p.Shi; Slo = p.Slo;
+                Shi = p.Shi; Slo = p.Slo; occ = p.occ;
             }
             const int fm = fix ? (p.fixmode ? p.fixmode : OPB_FIX_CIN) : OPB_FIX_NONE;
-            const int row = m0 + (int)rank * TC_BM + q * 32 + lane;
-            const int col0 = n0 + h * CPT;
+            const int row = rbase + lane;
             if constexpr (EPIMODE == 0) {
-                if (nch == 0 && C && Cin == C) {
+                if (!reached && C && Cin == C) {
                     // a tile that no K-block reaches (outside twice the operands' band): the
                     // product is zero there, and C, updated in place, is zero there too and
                     // keeps its values; only the row-sum partial is written
@@ -785,7 +889,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                 constexpr int HC = CPT / 2, RS = HC * 2 + 16;
                 static_assert(HC == 32, "four 16-byte chunks per staged row segment");
                 uint8_t *stg = gbase + Cfg::RING_BYTES + 256 + warp * (32 * RS);
-                const int rb = m0 + (int)rank * TC_BM + q * 32;
+                const int rb = rbase;
 #pragma unroll
                 for (int hh = 0; hh < 2; hh++) {
 #pragma unroll
@@ -839,46 +943,83 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
             // FP32 output in 32 x 32 blocks: the warp's rows (lane = row while the values are
             // in the accumulator layout) are staged in shared memory and read back so that
             // lane l handles row 4i + l/8, columns 4(l%8)..+3 of the block: every Cin load and
-            // C store of the warp covers four whole 128-byte lines.  The FP64 row sum keeps
-            // its order (float4 groups in column order): each group sum is parked in the
-            // first two words of its group's slots (read by this lane alone) and the row's
-            // lane adds them up.
-            float *st = reinterpret_cast<float *>(gbase + Cfg::RING_BYTES + 256) + warp * (32 * 33);
-            const int rbase = m0 + (int)rank * TC_BM + q * 32;
-            const int tr = lane >> 3, tc4 = (lane & 7) * 4;
-            double rs = 0.0;
+            // C store of the warp covers four whole 128-byte lines.  Rows are 32 words, their
+            // 16-byte chunks at c ^ (row % 8): both sides move 16 bytes a lane without conflicts.
+            // The row sums of the stored values stay with the lanes (FP64, one per row a lane
+            // handles) and are added over a row's eight lanes at the end.
+            //
+            // What bounds this phase: the latency of the Cin loads and the instructions between
+            // them, with two warps a scheduler (ncu, a banded squaring at d = 4096 before these
+            // measures: 0.18 instructions a cycle and scheduler, 47% of the stalls on loads, about
+            // 30 us a tile, as long as 18 chunks of MMAs).  So the next half block's loads are
+            // issued before the current one's arithmetic, the row and column fixes are loaded
+            // while the MMAs run and passed by shuffles, and 32 x 64 blocks that are zero before
+            // and after (off the generator's spread band) are left as they are.
+            float4 *st = reinterpret_cast<float4 *>(gbase + Cfg::RING_BYTES + 256) + warp * (32 * 8);
+            const int tr = lane >> 3, tc = lane & 7;
+            const float rsi = (float)rfix.x, rinv = (float)rfix.y;
+            double acc[8];
 #pragma unroll
-            for (int j = 0; j < CPT / 32; j++) {
+            for (int i = 0; i < 8; i++) acc[i] = 0.0;
+            // half block hb (16 rows) of the 32 columns at block j
+            auto load_cin = [&](float4 (&cv)[4], int j, int hb) {
 #pragma unroll
-                for (int c = 0; c < 32; c++) st[lane * 33 + c] = sum[32 * j + c];
-                // deferred squaring: the column terms s_j of this lane's four columns
-                float sj[4] = {0.f, 0.f, 0.f, 0.f};
-                if constexpr (FUSE == 1) {
-                    if (fm == OPB_FIX_SQUARE) {
+                for (int i = 0; i < 4; i++)
+                    cv[i] = *reinterpret_cast<const float4 *>(Cin + (long long)(rbase + 4 * (4 * hb + i) + tr) * ldc + col0 +
+                                                             32 * j + 4 * tc);
+            };
 #pragma unroll
-                        for (int u = 0; u < 4; u++) sj[u] = (float)fix[col0 + 32 * j + tc4 + u].x;
+            for (int b = 0; b < CPT / 64; b++) {
+                float4 cv[2][4];
+                const bool alive = (live >> b) & 1u;
+                if (FUSE != 2 && Cin && alive) load_cin(cv[0], 2 * b, 0);
+                if (OCC && !alive) {
+                    uint32_t any = 0;
+#pragma unroll
+                    for (int i = 0; i < 64; i++) any |= __float_as_uint(sum[64 * b + i]);
+                    if (!__any_sync(0xffffffffu, any != 0)) {
+                        // zero before, nothing added: E, updated in place, is zero already, and so
+                        // are its parts in this set unless the tile is new to it
+                        if (FUSE == 1 && Shi && fill) {
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                const long long so = (long long)(rbase + 4 * i + tr) * ldc + col0 + 64 * b + 8 * tc;
+                                *reinterpret_cast<uint4 *>(Shi + so) = make_uint4(0, 0, 0, 0);
+                                *reinterpret_cast<uint4 *>(Slo + so) = make_uint4(0, 0, 0, 0);
+                            }
+                        }
+                        continue;
                     }
+                    if (FUSE != 2 && Cin) load_cin(cv[0], 2 * b, 0);
                 }
-                __syncwarp();
-                // each half block's Cin loads are issued before any of its stores (with Cin = C
-                // each element is read and then written by this lane alone), so that four
-                // line-sized loads per warp are in flight at once
+                uint32_t nzp = 0, nze = 0;  // any bit of this block's hi parts, of its values
 #pragma unroll
-                for (int hb = 0; hb < 2; hb++) {
-                    float4 cv[4];
-                    if (FUSE != 2 && Cin) {
+                for (int hf = 0; hf < 4; hf++) {
+                    const int j = 2 * b + (hf >> 1), hb = hf & 1;
+                    if (hb == 0) {
+                        if (hf) __syncwarp();  // the previous block has been read
 #pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            cv[i] = *reinterpret_cast<const float4 *>(
-                                Cin + (long long)(rbase + 4 * (4 * hb + i) + tr) * ldc + col0 + 32 * j + tc4);
+                        for (int c = 0; c < 8; c++)
+                            st[lane * 8 + (c ^ (lane & 7))] = make_float4(sum[32 * j + 4 * c], sum[32 * j + 4 * c + 1],
+                                                                         sum[32 * j + 4 * c + 2], sum[32 * j + 4 * c + 3]);
+                        __syncwarp();
+                    }
+                    if (FUSE != 2 && Cin && hf < 3) load_cin(cv[(hf + 1) & 1], 2 * b + ((hf + 1) >> 1), (hf + 1) & 1);
+                    // deferred squaring: the column terms s_j of this lane's four columns
+                    float sj[4] = {0.f, 0.f, 0.f, 0.f};
+                    if constexpr (FUSE == 1) {
+                        if (fm == OPB_FIX_SQUARE) {
+#pragma unroll
+                            for (int u = 0; u < 4; u++) sj[u] = __shfl_sync(0xffffffffu, scol[j], 4 * tc + u);
+                        }
                     }
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const int rr = 4 * (4 * hb + i) + tr;
-                        const int grow = rbase + rr, gcol = col0 + 32 * j + tc4;
-                        float o[4];
-#pragma unroll
-                        for (int u = 0; u < 4; u++) o[u] = alpha * st[rr * 33 + tc4 + u];
+                        const int grow = rbase + rr, gcol = col0 + 32 * j + 4 * tc;
+                        const float4 sv = st[rr * 8 + (tc ^ (rr & 7))];
+                        float o[4] = {alpha * sv.x, alpha * sv.y, alpha * sv.z, alpha * sv.w};
+                        const float4 &cf = cv[hf & 1][i];
                         if constexpr (FUSE == 1) {
                             // squaring with the parts of its output: alpha acc + beta E', and with
                             // the previous level's normalisation deferred here (OPB_FIX_SQUARE):
@@ -886,10 +1027,10 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                             // in FP32 (s ~ 1e-5: the products with s are far below an ulp of the
                             // result's terms' rounding; inv's own rounding scales a whole row, which
                             // the next level's row sums renormalise)
-                            const float c4[4] = {cv[i].x, cv[i].y, cv[i].z, cv[i].w};
+                            const float c4[4] = {cf.x, cf.y, cf.z, cf.w};
                             if (fm == OPB_FIX_SQUARE) {
-                                const double2 fx = fix[grow];
-                                const float si = (float)fx.x, inv = (float)fx.y, bi = beta - si;
+                                const float si = __shfl_sync(0xffffffffu, rsi, rr);
+                                const float inv = __shfl_sync(0xffffffffu, rinv, rr), bi = beta - si;
 #pragma unroll
                                 for (int u = 0; u < 4; u++) {
                                     float x = fmaf(bi - sj[u], c4[u], o[u]);
@@ -904,22 +1045,23 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                             // parts only, A's rows normalised here (OPB_FIX_ROWSCALE; FP32 inv:
                             // its rounding scales the whole row, renormalised by the next row sums)
                             if (fm == OPB_FIX_ROWSCALE) {
-                                const float inv = (float)fix[grow].y;
+                                const float inv = __shfl_sync(0xffffffffu, rinv, rr);
 #pragma unroll
                                 for (int u = 0; u < 4; u++) o[u] *= inv;
                             }
                         } else if (Cin) {
-                            float c4[4] = {cv[i].x, cv[i].y, cv[i].z, cv[i].w};
+                            float c4[4] = {cf.x, cf.y, cf.z, cf.w};
                             if (fm == OPB_FIX_CIN) {
                                 // deferred renormalisation of Cin (the arithmetic of the
                                 // E-form renormalisation kernel, so Cin reads exactly as if
                                 // that kernel had stored it)
-                                const double2 fx = fix[grow];
+                                const double fs = __shfl_sync(0xffffffffu, rfix.x, rr);
+                                const double fi = __shfl_sync(0xffffffffu, rfix.y, rr);
 #pragma unroll
                                 for (int u = 0; u < 4; u++) {
                                     double x = (double)c4[u];
-                                    if (grow == gcol + u) x -= fx.x;
-                                    c4[u] = (float)(x * fx.y);
+                                    if (grow == gcol + u) x -= fs;
+                                    c4[u] = (float)(x * fi);
                                 }
                             }
 #pragma unroll
@@ -934,21 +1076,41 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                                 const long long so = (long long)grow * ldc + gcol;
                                 *reinterpret_cast<uint2 *>(Shi + so) = make_uint2(hh[0], hh[1]);
                                 *reinterpret_cast<uint2 *>(Slo + so) = make_uint2(ll[0], ll[1]);
+                                if constexpr (OCC) {
+                                    nzp |= hh[0] | hh[1];
+                                    nze |= __float_as_uint(o[0]) | __float_as_uint(o[1]) | __float_as_uint(o[2]) |
+                                           __float_as_uint(o[3]);
+                                }
                             }
                         }
-                        const double g = (double)o[0] + (double)o[1] + (double)o[2] + (double)o[3];
-                        st[rr * 33 + tc4] = __int_as_float(__double2loint(g));
-                        st[rr * 33 + tc4 + 1] = __int_as_float(__double2hiint(g));
+                        if (rowsum) acc[4 * hb + i] += (double)o[0] + (double)o[1] + (double)o[2] + (double)o[3];
                     }
                 }
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < 8; k++)
-                    rs += __hiloint2double(__float_as_int(st[lane * 33 + 4 * k + 1]),
-                                           __float_as_int(st[lane * 33 + 4 * k]));
                 __syncwarp();  // before the next block overwrites the buffer
+                if constexpr (OCC && FUSE == 1) {
+                    if (occ) {
+                        const bool np = __any_sync(0xffffffffu, nzp != 0), ne = __any_sync(0xffffffffu, nze != 0);
+                        // (a block once non-zero keeps its mark: its parts stay in the other set)
+                        if (lane == 0)
+                            occ[(long long)(rbase >> 5) * (ldc >> 6) + ((col0 + 64 * b) >> 6)] =
+                                (uint8_t)((np ? 1u : 0u) | (ne || ((had >> b) & 1u) ? 2u : 0u));
+                    }
+                }
             }
-            if (rowsum) rowsum[(long long)(col0 / CPT) * M + row] = rs;
+            if (rowsum) {
+                // lane (tr, tc) holds its columns' sums of the rows 4i + tr: after exchanging halves
+                // three times it holds the whole sum of row 4 tc + tr
+#pragma unroll
+                for (int w = 4; w >= 1; w >>= 1) {
+                    const bool up = (tc & w) != 0;
+#pragma unroll
+                    for (int i = 0; i < w; i++) {
+                        const double send = up ? acc[i] : acc[i + w], keep = up ? acc[i + w] : acc[i];
+                        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+                    }
+                }
+                rowsum[(long long)(col0 / CPT) * M + rbase + 4 * tc + tr] = acc[0];
+            }
         }
         if (!ok) atomicExch(&g_tc_error, 3);
     }
@@ -1126,6 +1288,14 @@ static int set_smem_attr() {
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              Cfg::SMEM);
         if (e != cudaSuccess) return (int)e;
+        if (Cfg::REGSPLIT) {
+            // the split's shares must add up to what the block is launched with: a build that
+            // gave the kernel fewer registers would wait for the rest
+            cudaFuncAttributes fa;
+            e = cudaFuncGetAttributes(&fa, k_tc_gemm<BN, STAGES, BATCHED, F16, NPROD, EPIMODE, BK, PAIR, BMN, FUSE>);
+            if (e != cudaSuccess) return (int)e;
+            if (fa.numRegs < Cfg::REGS_LAUNCH) return OPB_E_UNSUPPORTED;
+        }
         attr_set[dev] = true;
     }
     return 0;
@@ -1154,6 +1324,11 @@ static int launch_tc_impl(const TcGemmArgs &a, cudaStream_t s) {
     p.Shi = a.Shi;
     p.Slo = a.Slo;
     p.sscale = a.sscale;
+    p.order = a.order;
+    p.kmask = a.kmask;
+    p.nw = a.nw;
+    p.occ = a.occ;
+    p.occ_in = a.occ_in;
     const int ntiles = (a.M / TC_BM) * (a.N / BN) * p.ksplit;
     const int grid = ntiles < num_sms() ? ntiles : num_sms();
     TcBatch none{nullptr, nullptr, nullptr, 0};
@@ -1188,6 +1363,11 @@ static int launch_tc_pair(const TcGemmArgs &a, cudaStream_t s) {
     p.Shi = a.Shi;
     p.Slo = a.Slo;
     p.sscale = a.sscale;
+    p.order = a.order;
+    p.kmask = a.kmask;
+    p.nw = a.nw;
+    p.occ = a.occ;
+    p.occ_in = a.occ_in;
     TcBatch none{nullptr, nullptr, nullptr, 0};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1236,19 +1416,21 @@ int tc_make_maps(CUtensorMap *out4, const __nv_bfloat16 *Ahi, const __nv_bfloat1
 
 template <int BN, int STAGES, bool F16, bool BMN, int FUSE>
 static int launch_batched_impl(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
-                               int grid, cudaStream_t s, int level, int lolo, int band_skip, int fixmode,
-                               float sscale) {
+                               int grid, cudaStream_t s, const TcBatchArgs &b) {
     using Cfg = TcCfg<BN, STAGES>;
     int e0 = set_smem_attr<BN, STAGES, true, F16, 3, 0, TC_BK, false, BMN, FUSE>();
     if (e0) return e0;
     CUtensorMap dummy;
     std::memset(&dummy, 0, sizeof(dummy));
     TcParams p{};
-    p.level = level;
-    p.lolo = lolo;
-    p.band_skip = band_skip;
-    p.fixmode = fixmode;
-    p.sscale = sscale;
+    p.level = b.level;
+    p.lolo = b.lolo;
+    p.band_skip = b.band_skip;
+    p.fixmode = b.fixmode;
+    p.sscale = b.sscale;
+    p.order = b.order;
+    p.kmask = b.kmask;
+    p.nw = b.nw;
     TcBatch bt{maps, probs, work, nwork};
     k_tc_gemm<BN, STAGES, true, F16, 3, 0, TC_BK, false, BMN, FUSE><<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(
         dummy, dummy, dummy, dummy, p, bt);
@@ -1260,7 +1442,7 @@ static int launch_batched_impl(const CUtensorMap *maps, const TcProblem *probs, 
 // loads its own half), problems with M % 256 == 0 and N % 256 == 0.
 template <bool F16, bool BMN, int FUSE>
 static int launch_batched_pair_impl(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
-                                    cudaStream_t s, int level, int lolo, int band_skip, int fixmode, float sscale) {
+                                    cudaStream_t s, const TcBatchArgs &b) {
     constexpr int BN = 256, STAGES = 3;
     using Cfg = TcCfg<BN, STAGES, 3, TC_BK, true>;
     auto kern = k_tc_gemm<BN, STAGES, true, F16, 3, 0, TC_BK, true, BMN, FUSE>;
@@ -1294,81 +1476,52 @@ static int launch_batched_pair_impl(const CUtensorMap *maps, const TcProblem *pr
     CUtensorMap dummy;
     std::memset(&dummy, 0, sizeof(dummy));
     TcParams p{};
-    p.level = level;
-    p.lolo = lolo;
-    p.band_skip = band_skip;
-    p.fixmode = fixmode;
-    p.sscale = sscale;
+    p.level = b.level;
+    p.lolo = b.lolo;
+    p.band_skip = b.band_skip;
+    p.fixmode = b.fixmode;
+    p.sscale = b.sscale;
+    p.order = b.order;
+    p.kmask = b.kmask;
+    p.nw = b.nw;
     TcBatch bt{maps, probs, work, nwork};
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, dummy, dummy, dummy, dummy, p, bt);
     return e == cudaSuccess ? (int)cudaGetLastError() : (int)e;
 }
 
-// Batched squaring and chain products take MN-major B maps (b_kn = 1): pair and 256/128
-// tiles exist only in that form; 64-wide tiles in both (pricing is K-major).
-template <int FUSE>
-static int batched_pair_fused(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
-                              cudaStream_t s, int f16, int level, int lolo, int band_skip, int fixmode, float sscale) {
-    return f16 ? launch_batched_pair_impl<true, true, FUSE>(maps, probs, work, nwork, s, level, lolo, band_skip,
-                                                            fixmode, sscale)
-               : launch_batched_pair_impl<false, true, FUSE>(maps, probs, work, nwork, s, level, lolo, band_skip,
-                                                             fixmode, sscale);
-}
-
+// Batched squarings take MN-major B maps (b_kn = 1): pair and 256/128 tiles exist only in that
+// form; 64-wide tiles in both (pricing is K-major).
 int launch_tc_gemm_batched_pair(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
-                                cudaStream_t s, int f16, int b_kn, int level, int lolo, int band_skip, int fixmode,
-                                float sscale, int fuse) {
+                                cudaStream_t s, const TcBatchArgs &b) {
     if (nwork <= 0) return OPB_OK;
-    if (!b_kn) return OPB_E_UNSUPPORTED;
-    if (fuse == 1) return batched_pair_fused<1>(maps, probs, work, nwork, s, f16, level, lolo, band_skip, fixmode, sscale);
-    return fuse ? OPB_E_UNSUPPORTED
-                : batched_pair_fused<0>(maps, probs, work, nwork, s, f16, level, lolo, band_skip, fixmode, sscale);
+    if (!b.b_kn || !b.fuse) return OPB_E_UNSUPPORTED;
+    return b.f16 ? launch_batched_pair_impl<true, true, 1>(maps, probs, work, nwork, s, b)
+                 : launch_batched_pair_impl<false, true, 1>(maps, probs, work, nwork, s, b);
 }
 
-// MN-major B (b_kn) in every tile width and epilogue form; K-major B (pricing) 64-wide only.
-template <int FUSE>
-static int batched_kn(int bn, const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
-                      int grid, cudaStream_t s, int f16, int level, int lolo, int band_skip, int fixmode,
-                      float sscale) {
-    switch (bn * 2 + (f16 ? 1 : 0)) {
-        case 512:
-            return launch_batched_impl<256, 2, false, true, FUSE>(maps, probs, work, nwork, grid, s, level, lolo,
-                                                                  band_skip, fixmode, sscale);
-        case 513:
-            return launch_batched_impl<256, 2, true, true, FUSE>(maps, probs, work, nwork, grid, s, level, lolo,
-                                                                 band_skip, fixmode, sscale);
-        case 256:
-            return launch_batched_impl<128, 3, false, true, FUSE>(maps, probs, work, nwork, grid, s, level, lolo,
-                                                                  band_skip, fixmode, sscale);
-        case 257:
-            return launch_batched_impl<128, 3, true, true, FUSE>(maps, probs, work, nwork, grid, s, level, lolo,
-                                                                 band_skip, fixmode, sscale);
-        case 128:
-            return launch_batched_impl<64, 4, false, true, FUSE>(maps, probs, work, nwork, grid, s, level, lolo,
-                                                                 band_skip, fixmode, sscale);
-        case 129:
-            return launch_batched_impl<64, 4, true, true, FUSE>(maps, probs, work, nwork, grid, s, level, lolo,
-                                                                band_skip, fixmode, sscale);
-        default: return OPB_E_UNSUPPORTED;
-    }
-}
-
+// MN-major B (b_kn): squarings in every tile width, FP32 output 64-wide only; K-major B 64-wide.
 int launch_tc_gemm_batched(int bn, const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
-                           int grid, cudaStream_t s, int f16, int b_kn, int level, int lolo, int band_skip, int fixmode,
-                           float sscale, int fuse) {
+                           int grid, cudaStream_t s, const TcBatchArgs &b) {
     if (nwork <= 0) return OPB_OK;
     if (grid <= 0 || grid > nwork) grid = nwork < num_sms() ? nwork : num_sms();
-    if (b_kn) {
-        if (fuse == 1)
-            return batched_kn<1>(bn, maps, probs, work, nwork, grid, s, f16, level, lolo, band_skip, fixmode, sscale);
-        if (fuse) return OPB_E_UNSUPPORTED;
-        return batched_kn<0>(bn, maps, probs, work, nwork, grid, s, f16, level, lolo, band_skip, fixmode, sscale);
+    if (b.fuse) {
+        if (!b.b_kn) return OPB_E_UNSUPPORTED;
+        switch (bn * 2 + (b.f16 ? 1 : 0)) {
+            case 512: return launch_batched_impl<256, 2, false, true, 1>(maps, probs, work, nwork, grid, s, b);
+            case 513: return launch_batched_impl<256, 2, true, true, 1>(maps, probs, work, nwork, grid, s, b);
+            case 256: return launch_batched_impl<128, 3, false, true, 1>(maps, probs, work, nwork, grid, s, b);
+            case 257: return launch_batched_impl<128, 3, true, true, 1>(maps, probs, work, nwork, grid, s, b);
+            case 128: return launch_batched_impl<64, 4, false, true, 1>(maps, probs, work, nwork, grid, s, b);
+            case 129: return launch_batched_impl<64, 4, true, true, 1>(maps, probs, work, nwork, grid, s, b);
+            default: return OPB_E_UNSUPPORTED;
+        }
     }
-    if (bn != 64 || fuse) return OPB_E_UNSUPPORTED;
-    return f16 ? launch_batched_impl<64, 4, true, false, 0>(maps, probs, work, nwork, grid, s, level, lolo, band_skip,
-                                                            fixmode, sscale)
-               : launch_batched_impl<64, 4, false, false, 0>(maps, probs, work, nwork, grid, s, level, lolo, band_skip,
-                                                             fixmode, sscale);
+    if (bn != 64) return OPB_E_UNSUPPORTED;
+    if (b.b_kn)
+        return b.f16 ? launch_batched_impl<64, 4, true, true, 0>(maps, probs, work, nwork, grid, s, b)
+                     : launch_batched_impl<64, 4, false, true, 0>(maps, probs, work, nwork, grid, s, b);
+    return b.f16 ? launch_batched_impl<64, 4, true, false, 0>(maps, probs, work, nwork, grid, s, b)
+                 : launch_batched_impl<64, 4, false, false, 0>(maps, probs, work, nwork, grid, s, b);
 }
 
 // One network layer on the tensor cores: H[M, N] = GELU(alpha * A[M, K] . W[N, K]^T + bias)
@@ -1742,6 +1895,40 @@ int launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s) {
         case 129: return launch_tc_impl<64, 4, true>(a, s);
         default: return OPB_E_UNSUPPORTED;
     }
+}
+
+// Whether a squaring of d states runs under a tile plan (its stages are 64 deep, it is one
+// launch), and the tiles it then has.
+bool tile_plan_for(int d, int &tm, int &tn) {
+    if (!g_band_skip || g_bk256 != TC_BK) return false;
+    tn = tile_for(d, d);
+    tm = g_pair && tn == 256 && d % (2 * TC_BM) == 0 ? 2 * TC_BM : TC_BM;
+    return true;
+}
+
+int launch_tile_plan_single(const TilePlan &pl, int d, int tm, int tn, const int *band, int level, const uint8_t *occ,
+                            uint8_t *clear, const double *partial, int nparts, double2 *fix, cudaStream_t s) {
+    TilePlanArgs a{};
+    a.list[0] = TilePlanList{nullptr, (d / tm) * (d / tn), tm, tn, pl.order, pl.kmask, pl.count};
+    a.nw = pl.nw; a.level = level; a.band_skip = 1;
+    a.d = d; a.group_m = g_group_m; a.band = band; a.occ = occ;
+    a.clear = clear; a.clear_bytes = (long long)tile_plan_marks(d); a.done = pl.done;
+    a.partial = partial; a.nparts = nparts; a.fix = fix;
+    return launch_tile_plan(a, s);
+}
+
+int launch_tile_plan_batched(const TilePlan *pl, const uint32_t *const *work, const int *n, const int *tm, const int *tn,
+                             const TcProblem *probs, const TcProblem *other, int level, uint8_t *clear,
+                             long long clear_bytes, const BatchLattice *lats, int nlat, int parts_div,
+                             long long total_rows, cudaStream_t s) {
+    TilePlanArgs a{};
+    for (int i = 0; i < 2; i++)
+        a.list[i] = TilePlanList{work[i], n[i], tm[i], tn[i], pl[i].order, pl[i].kmask, pl[i].count};
+    a.nw = pl[0].nw; a.level = level; a.band_skip = 1;
+    a.probs = probs; a.other = other;
+    a.clear = clear; a.clear_bytes = clear_bytes; a.done = pl[0].done;
+    a.lats = lats; a.nlat = nlat; a.parts_div = parts_div; a.total_rows = total_rows;
+    return launch_tile_plan(a, s);
 }
 
 #include "row_chain.cuh"

@@ -73,6 +73,8 @@ struct Bufs {
     double *Vd;    // FP64 option values of the backward induction, d x nKp
     int *band;     // the ELL generator's half-bandwidth, found on the device per solve
     double *xpad;  // spot values of the padded lattice (split modes, d % 128 != 0)
+    uint8_t *occ[2];     // marks of the two part sets, opb::tile_plan_marks(d) each
+    opb::TilePlan plan;  // (occ[1] and plan.done lie next to each other)
 };
 
 inline int padded_nk(int nK, int mode) { return tc_mode(mode) ? (nK + 63) / 64 * 64 : nK; }
@@ -106,6 +108,14 @@ Bufs carve(Ws &w, int d, int nK, int mode, bool pad = false) {
         b.Vd = w.take<double>((size_t)d * nK);
         b.band = w.take<int>(1);
         if (pad) b.xpad = w.take<double>((size_t)d);
+        const size_t tiles = (size_t)(d / 128) * (d / 64);  // of the narrowest tile
+        b.plan.nw = opb::tile_plan_words(d);
+        b.occ[0] = w.take<uint8_t>(opb::tile_plan_marks(d));
+        b.occ[1] = w.take<uint8_t>(opb::tile_plan_marks(d) + 64);
+        b.plan.done = reinterpret_cast<unsigned *>(b.occ[1] + opb::tile_plan_marks(d));
+        b.plan.order = w.take<uint32_t>(tiles);
+        b.plan.kmask = w.take<uint32_t>(tiles * b.plan.nw);
+        b.plan.count = w.take<uint16_t>(tiles);
     } else {
         b.G = w.take<float>((size_t)d * nK);
         b.part = w.take<double>((size_t)d);
@@ -236,7 +246,14 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
     // (lattices not fused, opb::fused_single: a renormalisation kernel after every level,
     // which writes the next level's parts)
     const bool fused = opb::fused_single(d);
-    if (fused && L.niter > 1) {
+    // Under a tile plan (from OPB_PLAN_MIN_D states) the second and later levels issue only the
+    // K-blocks that the previous output's marks show to be non-zero; then no block is read
+    // that its level did not write, and B needs no zeros.
+    int tm = 0, tn = 0;
+    const bool planned = d >= opb::OPB_PLAN_MIN_D && L.niter > 1 && g_ksplit <= 1 && opb::tile_plan_for(d, tm, tn);
+    if (planned)
+        LT((int)cudaMemsetAsync(b.occ[1], 0, opb::tile_plan_marks(d) + 64, s));
+    else if (fused && L.niter > 1) {
         LT((int)cudaMemsetAsync(b.Bhi, 0, sizeof(__nv_bfloat16) * (size_t)d * d, s));
         LT((int)cudaMemsetAsync(b.Blo, 0, sizeof(__nv_bfloat16) * (size_t)d * d, s));
     }
@@ -259,18 +276,33 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
         g.level = r;
         // BF16 parts: the lo.lo product on the first levels (see OPB_LOLO_LEVELS)
         g.lolo = (!f16 && r < opb::g_lolo_levels) ? 1 : 0;
+        if (planned) {
+            g.occ = (last || !fused) ? nullptr : b.occ[(r & 1) ^ 1];
+            if (r > 0) {
+                // (fused: the plan forms the row fixes of the previous level too)
+                LT(opb::launch_tile_plan_single(b.plan, d, tm, tn, g.band, r, b.occ[r & 1], b.occ[(r & 1) ^ 1], b.part, np,
+                                                fused ? b.fix : nullptr, s));
+                g.order = b.plan.order; g.kmask = b.plan.kmask; g.nw = b.plan.nw;
+                g.occ_in = b.occ[r & 1];
+            }
+        }
         LT(tc_gemm_ksplit(g, s));
         // the last level emits P1 = I + E and its splits (row-major into A: the first
         // chain's A and pricing's; row-major into B: every chain's B); the others only the
         // row fixes of their output
         if (last) LT(opb::launch_renorm_to_p(d, b.X, b.part, np, b.Ahi, b.Alo, b.Bhi, b.Blo, s, ss));
-        else if (fused) LT(opb::launch_rowfix(d, b.part, np, 1, b.fix, s));
-        else LT(opb::launch_renorm(d, b.X, b.part, np, 1, b.Ahi, b.Alo, nullptr, nullptr, s, ss, 0, b.fix));
+        else if (!fused)
+            LT(opb::launch_renorm(d, b.X, b.part, np, 1, b.Ahi, b.Alo, nullptr, nullptr, s, ss, 0, b.fix,
+                                  planned ? b.occ[(r & 1) ^ 1] : nullptr));
+        else if (!planned) LT(opb::launch_rowfix(d, b.part, np, 1, b.fix, s));
     }
     g.Ahi = b.Ahi; g.Alo = b.Alo;
     g.cin_fix = nullptr;
     g.fixmode = opb::OPB_FIX_NONE;
     g.Shi = g.Slo = nullptr;
+    g.occ = nullptr;
+    g.occ_in = nullptr;
+    g.order = g.kmask = nullptr;
     g.band = nullptr;
     g.band_skip = 0;
     g.level = 0;

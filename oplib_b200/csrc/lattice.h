@@ -61,6 +61,25 @@ __device__ __forceinline__ void split2x2(float a, float b, uint32_t &hi, uint32_
     }
 }
 
+// Row fixes from FP64 row-sum partials, with the arithmetic of the renormalisation
+// kernels' row sums (renorm64_sums): s = sum of the nparts partials in order; E-form inv =
+// 1 / (1 + s), P-form inv = 1 / s.
+__device__ __forceinline__ double2 row_fix(const double *__restrict__ partial, int d, int nparts, int row, int eform) {
+    double s = 0.0;
+    const double *q = partial + row;
+    int p = 0;
+    for (; p + 8 <= nparts; p += 8) {
+        double v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = q[(long long)(p + j) * d];
+#pragma unroll
+        for (int j = 0; j < 8; j++) s += v[j];
+    }
+    for (; p < nparts; p++) s += q[(long long)p * d];
+    const double den = nparts == 0 ? 1.0 : (eform ? 1.0 + s : s);
+    return make_double2(s, den != 0.0 ? 1.0 / den : 0.0);
+}
+
 // gemm_simt.cu
 int sgemm_rm(int M, int N, int K, float alpha, const float *A, int lda, const float *B, int ldb, float beta,
              float *C, int ldc, cudaStream_t s);
@@ -88,10 +107,11 @@ int launch_split(int rows, int cols, const float *X, long long ld, __nv_bfloat16
                  __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, long long ldt, cudaStream_t s, float sscale = 0.f);
 int launch_rowsum(int d, const float *X, double *partial, cudaStream_t s);
 // write_x = 0 leaves X as it is (only the splits are written; d % 64 == 0); fix (optional,
-// E-form) receives the per-row (s, inv) that a following product applies to X as its Cin.
+// E-form) receives the per-row (s, inv) that a following product applies to X as its Cin; occ
+// (optional, d % 64 == 0) the marks of the written A parts (TcGemmArgs::occ).
 int launch_renorm(int d, float *X, const double *partial, int nparts, int eform, __nv_bfloat16 *Ahi,
                   __nv_bfloat16 *Alo, __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale = 0.f,
-                  int write_x = 1, double2 *fix = nullptr);
+                  int write_x = 1, double2 *fix = nullptr, uint8_t *occ = nullptr);
 int launch_add_identity(int d, float *X, cudaStream_t s);
 // dscale (device, optional): FP16 payoff split scale from launch_payoff_scale
 int launch_payoff_scale(int d, const double *x, int nK, const double *K, float *out, cudaStream_t s);
@@ -221,6 +241,14 @@ struct TcGemmArgs {
     // value it stores, row-major with leading dimension ldc; C may then be null (parts only)
     __nv_bfloat16 *Shi, *Slo;
     float sscale;
+    // optional (squarings, 64-deep stages): the tile plan of this product (k_tile_plan): its
+    // items in issue order and nw mask words per item, one bit per K-block
+    const uint32_t *order, *kmask;
+    int nw;
+    // marks of 32 x 64 blocks (row-major, one byte each), bit 0: the hi parts are not all zero,
+    // bit 1: the FP32 values are not all zero (or have not been so at an earlier level).
+    uint8_t *occ;           // optional, with Shi: written for the output's blocks
+    const uint8_t *occ_in;  // with a plan: Cin's, blocks without bit 1 hold zeros
 };
 // Deferred normalisation in the epilogue, with cin_fix[i] = (s_i, inv_i) of the operand
 // rows (E-form: the row sums s of P = I + E' are 1 + s, inv = 1 / (1 + s); P-form: s the row
@@ -259,6 +287,8 @@ extern int g_band_skip;    // 1: squarings leave out the K-blocks outside the op
 constexpr int OPB_FUSED_AUTO_MIN_D = 4096;
 extern int g_fused_max_d;  // opb_set_fused_normalisation; < 0: automatic
 inline bool fused_single(int d) { return g_fused_max_d < 0 ? d >= OPB_FUSED_AUTO_MIN_D : d <= g_fused_max_d; }
+// Single lattices of at least this many states square under a tile plan (tile_plan.cuh).
+constexpr int OPB_PLAN_MIN_D = 1536;
 // K-slices that fill the GPU with the tiles of a small-N product (1 = none), at most 4
 int tc_gemm_split_for(int M, int N, int K);
 int tc_gemm_tile_n(int N);                    // tile width chosen for N (0 if unsupported)
@@ -287,6 +317,8 @@ struct TcProblem {
     float alpha, beta;
     const double2 *cin_fix;  // as TcGemmArgs::cin_fix
     __nv_bfloat16 *Shi, *Slo;  // as TcGemmArgs::Shi / Slo (optional)
+    uint8_t *occ;              // as TcGemmArgs::occ (optional)
+    const uint8_t *occ_in;     // as TcGemmArgs::occ_in
 };
 // Four maps (Ahi, Alo, Bhi, Blo) of one problem: A with 128-row boxes; B K-major (N x K,
 // bn-row boxes) or, with b_kn, K x N row-major read as an MN-major operand (64 x 64
@@ -294,20 +326,47 @@ struct TcProblem {
 int tc_make_maps(CUtensorMap *out4, const __nv_bfloat16 *Ahi, const __nv_bfloat16 *Alo, long long M, long long lda,
                  const __nv_bfloat16 *Bhi, const __nv_bfloat16 *Blo, long long N, long long ldb, long long K, int bn,
                  int f16 = 0, int b_kn = 0);
-// work: packed (problem << 16 | m-tile << 8 | n-tile); bn in {64, 128, 256}; K-major B
-// (b_kn = 0) only for bn = 64
-// level, lolo: as TcGemmArgs (band per problem in TcProblem::band)
-// fixmode, sscale: as TcGemmArgs (the problems' cin_fix and Shi / Slo); fuse: the epilogue
-// form (0: FP32 output, OPB_FIX_CIN; 1: squaring with its output's parts, OPB_FIX_SQUARE;
-// 2: parts only, OPB_FIX_ROWSCALE), MN-major B only
+// A batched launch: level, lolo, band_skip, fixmode, sscale, order, kmask, nw as TcGemmArgs
+// (band, cin_fix, Shi / Slo, occ per problem); fuse: 1 = squaring with its output's parts
+// (OPB_FIX_SQUARE, MN-major B), 0 = FP32 output
+struct TcBatchArgs {
+    int f16, b_kn;
+    int level, lolo, band_skip, fixmode;
+    float sscale;
+    int fuse;
+    const uint32_t *order, *kmask;
+    int nw;
+};
+// work: packed (problem << 16 | m-tile << 8 | n-tile); bn in {64, 128, 256}, without fuse 64
 int launch_tc_gemm_batched(int bn, const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
-                           int grid, cudaStream_t s, int f16, int b_kn, int level = 0, int lolo = 0,
-                           int band_skip = 0, int fixmode = 0, float sscale = 0.f, int fuse = 0);
+                           int grid, cudaStream_t s, const TcBatchArgs &b);
 // 256 x 256 items (256-row / 256-column units) on 2-CTA clusters, each CTA loading its
-// 128 rows of A and 128 columns of B; MN-major B maps; problems with M, N multiples of 256
+// 128 rows of A and 128 columns of B; squarings of problems with M, N multiples of 256
 int launch_tc_gemm_batched_pair(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
-                                cudaStream_t s, int f16, int b_kn, int level = 0,
-                                int lolo = 0, int band_skip = 0, int fixmode = 0, float sscale = 0.f, int fuse = 0);
+                                cudaStream_t s, const TcBatchArgs &b);
+
+// tile_plan.cuh (in gemm_tc.cu) -- which K-blocks each output tile of a squaring issues.
+// Bytes of a matrix's marks (one per 32 x 64 block, d % 128 == 0; a multiple of 16)
+inline size_t tile_plan_marks(int d) { return ((size_t)(d / 32) * (d / 64) + 15) & ~size_t(15); }
+inline int tile_plan_words(int d) { return (d / 64 + 31) / 32; }
+struct TilePlan {
+    uint32_t *order, *kmask;
+    uint16_t *count;
+    int nw;
+    unsigned *done;  // zero before the first plan; each plan leaves it zero
+};
+bool tile_plan_for(int d, int &tm, int &tn);
+// The plan of level `level`'s squaring from its operands' marks, clearing the marks that the
+// squaring writes; with fix, the row fixes from the previous product's partials (as
+// launch_rowfix, E-form).
+int launch_tile_plan_single(const TilePlan &pl, int d, int tm, int tn, const int *band, int level, const uint8_t *occ,
+                            uint8_t *clear, const double *partial, int nparts, double2 *fix, cudaStream_t s);
+// Two work lists of one level (problems `probs`; their operands' marks are written by the
+// other part set's problems), and the row fixes of the lattices that square at this level.
+int launch_tile_plan_batched(const TilePlan *pl, const uint32_t *const *work, const int *n, const int *tm, const int *tn,
+                             const TcProblem *probs, const TcProblem *other, int level, uint8_t *clear,
+                             long long clear_bytes, const BatchLattice *lats, int nlat, int parts_div,
+                             long long total_rows, cudaStream_t s);
 
 // row_chain.cuh (in gemm_tc.cu) -- the quoted row of the chained kernels.
 // The quoted row of one lattice.

@@ -265,7 +265,8 @@ __device__ __forceinline__ void renorm64_sums(RenormSmem &sm, int d, const doubl
 __device__ __forceinline__ void renorm64_apply(RenormSmem &sm, int d, float *__restrict__ X, int mode,
                                                __nv_bfloat16 *__restrict__ Ahi, __nv_bfloat16 *__restrict__ Alo,
                                                __nv_bfloat16 *__restrict__ Bhi, __nv_bfloat16 *__restrict__ Blo,
-                                               int r0, int c0, float sscale, const float4 (&vin)[4], bool b_rm) {
+                                               int r0, int c0, float sscale, const float4 (&vin)[4], bool b_rm,
+                                               uint8_t *__restrict__ occ = nullptr) {
     const int tid = threadIdx.x;
     const bool eform = mode != 2;
     const bool transposed = Bhi && !b_rm;
@@ -296,6 +297,19 @@ __device__ __forceinline__ void renorm64_apply(RenormSmem &sm, int d, float *__r
             *reinterpret_cast<uint2 *>(Ahi + o) = make_uint2(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]));
             *reinterpret_cast<uint2 *>(Alo + o) = make_uint2(pack_bf16(l[0], l[1]), pack_bf16(l[2], l[3]));
         }
+        // marks for the next product's tile plan (a warp's two rows lie in one 32 x 64 block;
+        // several warps may set the same mark)
+        if (occ) {
+            const uint32_t nz = pack_bf16(h[0], h[1]) | pack_bf16(h[2], h[3]);
+            const uint32_t nx = __float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w);
+            const bool np = __any_sync(0xffffffffu, nz != 0), ne = __any_sync(0xffffffffu, nx != 0);
+            if (ne && (tid & 31) == 0) {
+                const size_t at = (size_t)(r >> 5) * (d >> 6) + (c0 >> 6);
+                const uint32_t bits = np ? 3u : 2u;
+                if ((reinterpret_cast<volatile uint8_t *>(occ)[at] & bits) != bits)
+                    atomicOr(reinterpret_cast<uint32_t *>(occ) + (at >> 2), bits << (8 * (at & 3)));
+            }
+        }
         if (Bhi && b_rm) {
             *reinterpret_cast<uint2 *>(Bhi + o) = make_uint2(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]));
             *reinterpret_cast<uint2 *>(Blo + o) = make_uint2(pack_bf16(l[0], l[1]), pack_bf16(l[2], l[3]));
@@ -324,7 +338,8 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
                                                int nparts, int mode, __nv_bfloat16 *__restrict__ Ahi,
                                                __nv_bfloat16 *__restrict__ Alo, __nv_bfloat16 *__restrict__ Bhi,
                                                __nv_bfloat16 *__restrict__ Blo, int r0, int first, int step,
-                                               float sscale, double2 *__restrict__ fix, bool b_rm) {
+                                               float sscale, double2 *__restrict__ fix, bool b_rm,
+                                               uint8_t *__restrict__ occ = nullptr) {
     const int nt = d / 64, tid = threadIdx.x;
     const int cnt = first < nt ? (nt - 1 - first) / step + 1 : 0;
 #pragma unroll
@@ -342,7 +357,7 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
         cp_async_wait<RN_RING - 1>();  // this thread's copies of tile k have landed
         const int sl = k % RN_RING;
         const float4 v[4] = {rg.v[sl][0][tid], rg.v[sl][1][tid], rg.v[sl][2][tid], rg.v[sl][3][tid]};
-        renorm64_apply(sm, d, Xout, mode, Ahi, Alo, Bhi, Blo, r0, (first + k * step) * 64, sscale, v, b_rm);
+        renorm64_apply(sm, d, Xout, mode, Ahi, Alo, Bhi, Blo, r0, (first + k * step) * 64, sscale, v, b_rm, occ);
     }
 }
 
@@ -355,13 +370,14 @@ __global__ void __launch_bounds__(256) k_renorm64(int d, float *__restrict__ X, 
                                                   int nparts, int mode, __nv_bfloat16 *__restrict__ Ahi,
                                                   __nv_bfloat16 *__restrict__ Alo, __nv_bfloat16 *__restrict__ Bhi,
                                                   __nv_bfloat16 *__restrict__ Blo, float sscale, int write_x = 1,
-                                                  double2 *__restrict__ fix = nullptr, int b_rm = 0) {
+                                                  double2 *__restrict__ fix = nullptr, int b_rm = 0,
+                                                  uint8_t *__restrict__ occ = nullptr) {
     extern __shared__ __align__(16) uint8_t rn_smem[];
     RenormSmem &sm = *reinterpret_cast<RenormSmem *>(rn_smem);
     RenormRing &rg = *reinterpret_cast<RenormRing *>(rn_smem + sizeof(RenormSmem));
     renorm64_strip(sm, rg, d, X, write_x ? X : nullptr, partial, nparts, mode, Ahi, Alo, Bhi, Blo,
                    (int)blockIdx.y * 64, (int)blockIdx.x, (int)gridDim.x, sscale, blockIdx.x == 0 ? fix : nullptr,
-                   b_rm != 0);
+                   b_rm != 0, occ);
 }
 
 // Column chunks of a k_renorm64 launch: about 8 blocks per SM in total.
@@ -470,25 +486,6 @@ __global__ void k_row_quotes_batched(const BatchLattice *__restrict__ lats, cons
     if (f16) disc /= (double)L.gscale[0];
     disc *= rows[l].qinv[i];
     quotes[((long long)l * nmat + m0 + i) * nK + k] = disc * (double)L.V[(long long)i * ldk + k];
-}
-
-// Row fixes from FP64 row-sum partials, with the arithmetic of the renormalisation
-// kernels' row sums (renorm64_sums): s = sum of the nparts partials in order; E-form inv =
-// 1 / (1 + s), P-form inv = 1 / s.
-__device__ __forceinline__ double2 row_fix(const double *__restrict__ partial, int d, int nparts, int row, int eform) {
-    double s = 0.0;
-    const double *q = partial + row;
-    int p = 0;
-    for (; p + 8 <= nparts; p += 8) {
-        double v[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = q[(long long)(p + j) * d];
-#pragma unroll
-        for (int j = 0; j < 8; j++) s += v[j];
-    }
-    for (; p < nparts; p++) s += q[(long long)p * d];
-    const double den = nparts == 0 ? 1.0 : (eform ? 1.0 + s : s);
-    return make_double2(s, den != 0.0 ? 1.0 / den : 0.0);
 }
 
 __global__ void k_rowfix(int d, const double *__restrict__ partial, int nparts, int eform, double2 *__restrict__ fix) {
@@ -735,14 +732,14 @@ int launch_rowsum(int d, const float *X, double *partial, cudaStream_t s) {
 
 int launch_renorm(int d, float *X, const double *partial, int nparts, int eform, __nv_bfloat16 *Ahi,
                   __nv_bfloat16 *Alo, __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale,
-                  int write_x, double2 *fix) {
+                  int write_x, double2 *fix, uint8_t *occ) {
     if (d % 64 == 0 && (Ahi != nullptr) == (Alo != nullptr)) {
         if (int r = renorm64_prepare()) return r;
         k_renorm64<<<renorm64_grid(d), 256, RN_SMEM, s>>>(d, X, partial, nparts, eform ? 0 : 2, Ahi, Alo, Bhi, Blo,
-                                                          sscale, write_x, eform ? fix : nullptr);
+                                                          sscale, write_x, eform ? fix : nullptr, 0, occ);
         return (int)cudaGetLastError();
     }
-    if (!write_x || fix) return OPB_E_UNSUPPORTED;
+    if (!write_x || fix || occ) return OPB_E_UNSUPPORTED;
     dim3 g((d + 31) / 32, (d + 31) / 32);
     k_renorm<<<g, 256, 0, s>>>(d, X, partial, nparts, eform, Ahi, Alo, Bhi, Blo, sscale);
     return (int)cudaGetLastError();
