@@ -323,8 +323,8 @@ unsigned long long opb_batch_workspace_size(const opb_batch_desc *b, int mode);
 int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *workspace, unsigned long long ws_bytes,
                           opb_batch_plan **out);
 int opb_batch_plan_destroy(opb_batch_plan *plan);
-/* cfg < opb_batch_num_configs(): tile width x work order (128, 64, 256-mixed or 256 on
- * CTA pairs mixed; longest first or lattice order); grid 0 = one CTA per SM */
+/* cfg < opb_batch_num_configs(): tile width x work order (128, 64, 256 or 256 on CTA pairs;
+ * longest first or lattice order); grid 0 = one CTA per SM */
 int opb_batch_set_config(opb_batch_plan *plan, int cfg, int grid);
 int opb_batch_num_configs(void);
 int opb_batch_execute(opb_batch_plan *plan, double *quotes);
@@ -333,7 +333,7 @@ int opb_batch_execute(opb_batch_plan *plan, double *quotes);
  * one batched tensor-core product per date over all lattices; quotes: device [nlat][nK]
  * FP64 values at each lattice's y0 */
 int opb_batch_execute_bermudan(opb_batch_plan *plan, int put, int exercise, double barrier, double *quotes);
-/* times the chain product (all lattices, dense operands) for every configuration
+/* times the plan's squarings (with the generators as they are) for every configuration
  * (ms_out: opb_batch_num_configs() floats) and keeps the fastest */
 int opb_batch_autotune(opb_batch_plan *plan, int reps, float *ms_out, int *best_cfg);
 int opb_batch_launches(const opb_batch_plan *plan);

@@ -55,14 +55,13 @@ struct opb_batch_desc {
 
 namespace {
 
-// (bn, order): (128, LPT), (64, LPT), (128, lattice), (64, lattice), (256 mixed, LPT),
-// (256 mixed, lattice), (256 pair mixed, LPT), (256 pair mixed, lattice).  "256 mixed":
-// 128 x 256 tiles for the lattices whose size is a multiple of 256, 128 x 128 tiles for
-// the rest (two launches per level); "256 pair mixed": 256 x 256 tiles on 2-CTA clusters
-// for those lattices instead.
+// (bn, order): (128, LPT), (64, LPT), (128, lattice), (64, lattice), (256, LPT), (256,
+// lattice), (256 pair, LPT), (256 pair, lattice): 128 x bn tiles on one CTA, or 256 x 256 tiles
+// on 2-CTA clusters ("pair").
 constexpr int NCFG = 8;
 constexpr int CFG_BN[NCFG] = {128, 64, 128, 64, 256, 256, 256, 256};
 constexpr bool CFG_PAIR[NCFG] = {false, false, false, false, false, false, true, true};
+constexpr int kTwin[NCFG] = {0, 1, 0, 1, 4, 4, 6, 6};  // the same tiles, longest first
 
 // mirror of opb_lattice_desc (lattice.cu), used for the FP32 per-lattice path
 struct LatticeDescMirror {
@@ -114,16 +113,17 @@ struct opb_batch_plan {
     // backward induction: A = P1's parts, B = the option values' parts read d x ldk row-major
     CUtensorMap *maps_berm = nullptr;
     uint32_t *work = nullptr;
-    // tile plans of a level's two launches, and the marks of the two part sets (all lattices,
-    // each set occ_bytes; the plans' counter lies behind set 1)
-    opb::TilePlan plan[2];
+    // the tile plan of a level, and the marks of the two part sets (all lattices, each set
+    // occ_bytes; the plan's counters lie behind set 0)
+    opb::TilePlan plan;
     uint8_t *occ[2] = {nullptr, nullptr};
     size_t occ_bytes = 0;
     float *E_base = nullptr;
-    size_t E_bytes = 0;
+    size_t E_bytes = 0;  // E and both part sets of all lattices
+    double *part = nullptr;  // the row-sum partials of all lattices
+    size_t part_bytes = 0;
     // work lists (offsets into `work`)
     std::vector<ListRef> gemm_level[NCFG];
-    std::vector<ListRef> gemm_level_rest[NCFG];  // pair configurations: the 128 x 256 items
     ListRef gemm_price;                // every 128-row tile (the induction's products)
     ListRef gemm_rows;                 // one tile per lattice (the priced rows)
     ListRef row_items;                 // the chained rows' 64-column items
@@ -237,10 +237,10 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     auto mp = c.take<CUtensorMap>(4 * (size_t)n);
     size_t Etot = 0;
     for (int i = 0; i < n; i++) Etot += (size_t)b->d[i] * b->d[i];
-    float *E = c.take<float>(Etot);
-    float *Pa = c.take<float>(Etot);
-    __nv_bfloat16 *Ah = c.take<__nv_bfloat16>(Etot), *Al = c.take<__nv_bfloat16>(Etot);
-    __nv_bfloat16 *Bh = c.take<__nv_bfloat16>(Etot), *Bl = c.take<__nv_bfloat16>(Etot);
+    // a lattice's E and parts lie together (E, A hi, A lo, B hi, B lo: 12 d^2 bytes), so that a
+    // tile's rows of all five share pages where the lattice is small
+    float *E = c.take<float>(3 * Etot);
+    (void)c.take<__nv_bfloat16>(2 * (size_t)opb::kRowSlots * off[n]);  // the priced rows' parts
     float *V = c.take<float>((size_t)off[n] * ldk);
     __nv_bfloat16 *Gh = c.take<__nv_bfloat16>((size_t)off[n] * ldk), *Gl = c.take<__nv_bfloat16>((size_t)off[n] * ldk);
     size_t parts = 0;
@@ -256,15 +256,15 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
         tiles += (size_t)(b->d[i] / 128) * (b->d[i] / 64);
         nw = std::max(nw, opb::tile_plan_words(b->d[i]));
     }
-    uint8_t *occ0 = c.take<uint8_t>(marks), *occ1 = c.take<uint8_t>(marks + 64);
-    opb::TilePlan plan[2];
-    for (auto &pl : plan) {
-        pl.order = c.take<uint32_t>(tiles);
-        pl.kmask = c.take<uint32_t>(tiles * nw);
-        pl.count = c.take<uint16_t>(tiles);
-        pl.nw = nw;
-        pl.done = reinterpret_cast<unsigned *>(occ1 + marks);
-    }
+    uint8_t *occ0 = c.take<uint8_t>(marks + 64), *occ1 = c.take<uint8_t>(marks);
+    opb::TilePlan plan;
+    plan.order = c.take<uint2>(tiles);
+    plan.kmask = c.take<uint32_t>(tiles * nw);
+    plan.tile = c.take<uint32_t>(tiles);
+    plan.count = c.take<uint16_t>(tiles);
+    plan.nw = nw;
+    plan.done = reinterpret_cast<unsigned *>(occ0 + marks);
+    plan.nlist = plan.done + 1;
     (void)c.take<double>((size_t)off[n] * ldk);     // FP64 option values of the backward induction
 
     // ---- work lists (host), appended into one blob
@@ -275,16 +275,13 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     std::stable_sort(lpt.begin(), lpt.end(), [&](int a, int bb) { return b->d[a] > b->d[bb]; });
     int maxn = 0;
     for (int i = 0; i < n; i++) maxn = std::max(maxn, b->niter[i]);
-    // sel: 0 every lattice, 1 only sizes that are multiples of 256, 2 only the others.  A
-    // size that is not a multiple of bn gets a last column tile that overhangs the matrix:
-    // its B columns beyond d load as zeros and its output groups beyond d are not stored.
-    auto gemm_list = [&](const std::vector<int> &order, int bn, int level, int sel = 0, int tile_m = 128,
-                         bool by_work = false) {
+    // A size that is not a multiple of the tile gets last tiles that overhang the matrix: their
+    // A rows and B columns beyond d load as zeros and their outputs beyond d are not stored.
+    auto gemm_list = [&](const std::vector<int> &order, int bn, int level, int tile_m, bool by_work) {
         ListRef r{W.size(), 0};
         for (int i : order) {
             if (b->niter[i] <= level) continue;
-            if ((sel == 1 && b->d[i] % 256) || (sel == 2 && b->d[i] % 256 == 0)) continue;
-            const int mt = b->d[i] / tile_m, nt = (b->d[i] + bn - 1) / bn;
+            const int mt = (b->d[i] + tile_m - 1) / tile_m, nt = (b->d[i] + bn - 1) / bn;
             for (int a = 0; a < mt; a++)
                 for (int bb = 0; bb < nt; bb++) W.push_back(((uint32_t)i << 16) | ((uint32_t)a << 8) | (uint32_t)bb);
         }
@@ -299,23 +296,11 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
         }
         return r;
     };
-    std::vector<ListRef> gl[NCFG], glr[NCFG];
+    std::vector<ListRef> gl[NCFG];
     for (int cfg = 0; cfg < NCFG; cfg++) {
         const bool longest = cfg < 2 || cfg == 4 || cfg == 6;
-        const auto &order = longest ? lpt : nat;
-        if (CFG_PAIR[cfg]) {
-            // 256 x 256 pair items for the multiples of 256, then 128 x 256 items (column
-            // overhang) for the other sizes
-            for (int lv = 0; lv < maxn; lv++) {
-                gl[cfg].push_back(gemm_list(order, 256, lv, 1, 256, longest));
-                glr[cfg].push_back(gemm_list(order, 256, lv, 2, 128, longest));
-            }
-        } else {
-            for (int lv = 0; lv < maxn; lv++) {
-                gl[cfg].push_back(gemm_list(order, CFG_BN[cfg], lv, 0, 128, longest));
-                glr[cfg].push_back(ListRef{W.size(), 0});
-            }
-        }
+        for (int lv = 0; lv < maxn; lv++)
+            gl[cfg].push_back(gemm_list(longest ? lpt : nat, CFG_BN[cfg], lv, CFG_PAIR[cfg] ? 256 : 128, longest));
     }
     ListRef gpr{W.size(), 0};
     for (int i : lpt)
@@ -370,12 +355,12 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     for (int k = 0; k < 2; k++) P->maps_sq[k] = msq + 4 * (size_t)n * k;
     P->maps_price = mp;
     P->maps_berm = mbm; P->work = work;
-    P->plan[0] = plan[0]; P->plan[1] = plan[1];
+    P->plan = plan;
     P->occ[0] = occ0; P->occ[1] = occ1; P->occ_bytes = marks;
-    P->E_base = E; P->E_bytes = Etot * sizeof(float);
+    P->E_base = E; P->E_bytes = 3 * Etot * sizeof(float);
+    P->part = part; P->part_bytes = parts * sizeof(double);
     for (int cfg = 0; cfg < NCFG; cfg++) {
         P->gemm_level[cfg] = gl[cfg];
-        P->gemm_level_rest[cfg] = glr[cfg];
     }
     P->gemm_price = gpr; P->gemm_rows = grw; P->row_items = gri; P->rn_level = rl; P->rn_init = rinit;
     if (work_out) *work_out = W;
@@ -471,9 +456,8 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
     cv.take<CUtensorMap>(8 * (size_t)n); cv.take<CUtensorMap>(4 * (size_t)n);
     size_t Etot = 0;
     for (int i = 0; i < n; i++) Etot += (size_t)b->d[i] * b->d[i];
-    float *E = cv.take<float>(Etot), *Pa = cv.take<float>(Etot);
-    __nv_bfloat16 *Ah = cv.take<__nv_bfloat16>(Etot), *Al = cv.take<__nv_bfloat16>(Etot);
-    __nv_bfloat16 *Bh = cv.take<__nv_bfloat16>(Etot), *Bl = cv.take<__nv_bfloat16>(Etot);
+    float *E = cv.take<float>(3 * Etot);
+    __nv_bfloat16 *Q = cv.take<__nv_bfloat16>(2 * (size_t)opb::kRowSlots * P->total_rows);
     float *V = cv.take<float>((size_t)P->total_rows * P->ldk);
     __nv_bfloat16 *Gh = cv.take<__nv_bfloat16>((size_t)P->total_rows * P->ldk);
     __nv_bfloat16 *Gl = cv.take<__nv_bfloat16>((size_t)P->total_rows * P->ldk);
@@ -497,14 +481,16 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
         L.d = d; L.y0 = b->y0[i]; L.row_off = ro; L.dt = b->dt[i]; L.rate = b->rate[i]; L.period = b->period;
         L.d_src = cb->d[i]; L.src_off = so;
         so += cb->d[i];
-        L.E = E + eo; L.Pa = Pa + eo; L.V = V + (size_t)ro * P->ldk;
+        L.E = E + 3 * eo; L.V = V + (size_t)ro * P->ldk;
         L.GThi = Gh + (size_t)ro * P->ldk; L.GTlo = Gl + (size_t)ro * P->ldk;
         L.gscale = gsc + i;
         L.Vd = vd + (size_t)ro * P->ldk;
         double *pi = part + po;
         L.niter = b->niter[i]; L.partial = pi; L.fix = fix + ro;
+        __nv_bfloat16 *Ah = reinterpret_cast<__nv_bfloat16 *>(L.E + dd), *Al = Ah + dd, *Bh = Al + dd, *Bl = Bh + dd;
+        L.Ahi = Ah; L.Alo = Al; L.occ0 = P->occ[0] + mo;
         // part sets: squarings between A and B
-        __nv_bfloat16 *sh[2] = {Ah + eo, Bh + eo}, *sl[2] = {Al + eo, Bl + eo};
+        __nv_bfloat16 *sh[2] = {Ah, Bh}, *sl[2] = {Al, Bl};
         for (int k = 0; k < 2 && rc_status == OPB_OK; k++) {
             // squaring: E' = 2E + E.E in place of E (as the previous level's GEMM left it, its
             // normalisation deferred into this epilogue through the row fixes), the output's
@@ -515,20 +501,21 @@ OPB_API int opb_batch_plan_create(const opb_batch_desc *b, int mode, void *works
                                           64, f16, 1);
         }
         // the quoted row of the chained kernels: FP32 rows in E (done with after the
-        // squarings), the parts to be priced in Pa, their row scales in the row-sum partials
+        // squarings), the parts to be priced in Q, their row scales in the row-sum partials
         opb::RowChainLat &R = rw[i];
         R.d = d;
-        R.hi = Ah + eo + (size_t)L.y0 * d; R.lo = Al + eo + (size_t)L.y0 * d;
+        R.hi = Ah + (size_t)L.y0 * d; R.lo = Al + (size_t)L.y0 * d;
         R.C[0] = L.E; R.C[1] = L.E + d;
-        R.Qhi = reinterpret_cast<__nv_bfloat16 *>(Pa + eo); R.Qlo = R.Qhi + (size_t)opb::kRowSlots * d;
+        R.Qhi = Q + 2 * (size_t)opb::kRowSlots * ro; R.Qlo = R.Qhi + (size_t)opb::kRowSlots * d;
         R.qinv = pi;
         if (rc_status == OPB_OK)
             rc_status = opb::tc_make_maps(&mp[4 * (size_t)i], R.Qhi, R.Qlo, opb::kRowSlots, d, L.GThi, L.GTlo, P->ldk,
                                           d, d, 64, f16);
         pr[i] = opb::TcProblem{d, P->ldk, d, 0, L.V, nullptr, nullptr, P->ldk, un1, 0.f, nullptr};
-        rs[i] = opb::RenormProblem{d, 0, L.E, pi, Ah + eo, Al + eo, Bh + eo, Bl + eo, fix + ro};
+        rs[i] = opb::RenormProblem{d, 0, L.E, pi, Ah, Al, Bh, Bl, fix + ro,
+                                   P->occ[b->niter[i] & 1] + mo};
         if (rc_status == OPB_OK)  // the same buffers, the value parts read d x ldk row-major
-            rc_status = opb::tc_make_maps(&mbm[4 * (size_t)i], Ah + eo, Al + eo, d, d, L.GThi, L.GTlo, P->ldk,
+            rc_status = opb::tc_make_maps(&mbm[4 * (size_t)i], Ah, Al, d, d, L.GThi, L.GTlo, P->ldk,
                                           P->ldk, d, 64, f16, 1);
         eo += dd;
         mo += opb::tile_plan_marks(d);
@@ -575,9 +562,8 @@ OPB_API int opb_batch_plan_destroy(opb_batch_plan *P) {
 }
 
 // Selects the launch configuration: cfg 0..7 = (BN 128, longest-K first), (64, longest
-// first), (128, lattice order), (64, lattice order), (128 x 256 tiles for every size,
-// longest first), (the same, lattice order), (256 x 256 pair items for the multiples of
-// 256 and 128 x 256 tiles for the rest, longest first), (the same, lattice order); grid 0
+// first), (128, lattice order), (64, lattice order), (128 x 256 tiles, longest first), (the
+// same, lattice order), (256 x 256 pair items, longest first), (the same, lattice order); grid 0
 // = one CTA per SM (the pair launches size their own grid).
 OPB_API int opb_batch_set_config(opb_batch_plan *P, int cfg, int grid) {
     OPB_REQUIRE(P, OPB_E_NULL);
@@ -589,25 +575,15 @@ OPB_API int opb_batch_set_config(opb_batch_plan *P, int cfg, int grid) {
 
 namespace {
 
-// One squaring level under configuration cfg: one launch, or two for the pair configurations
-// (256 x 256 pair items, then 128 x 256 ones).  The level reads the part set level % 2;
+// One squaring level under configuration cfg.  The level reads the part set level % 2;
 // fixmode: how the problems' row fixes apply.
 int cfg_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s, int lolo, int skip, int fixmode, bool planned) {
-    const int bn = CFG_BN[cfg], k = level & 1;
-    const CUtensorMap *maps = P->maps_sq[k];
-    const opb::TcProblem *probs = P->sq[k];
-    const ListRef &l = P->gemm_level[cfg][level], &rest = P->gemm_level_rest[cfg][level];
-    opb::TcBatchArgs a{P->f16, 1, level, lolo, skip, fixmode, P->f16 ? F16S : 0.f, 1, nullptr, nullptr, 0};
-    auto use = [&](const opb::TilePlan &pl) {
-        if (planned) { a.order = pl.order; a.kmask = pl.kmask; a.nw = pl.nw; }
-    };
-    use(P->plan[0]);
-    int r = CFG_PAIR[cfg] ? opb::launch_tc_gemm_batched_pair(maps, probs, P->work + l.off, l.n, s, a)
-                          : opb::launch_tc_gemm_batched(bn, maps, probs, P->work + l.off, l.n, P->grid, s, a);
-    use(P->plan[1]);
-    if (r == 0 && rest.n > 0)
-        r = opb::launch_tc_gemm_batched(256, maps, probs, P->work + rest.off, rest.n, P->grid, s, a);
-    return r;
+    const CUtensorMap *maps = P->maps_sq[level & 1];
+    const opb::TcProblem *probs = P->sq[level & 1];
+    const ListRef &l = P->gemm_level[cfg][level];
+    const opb::TcBatchArgs a{P->f16, 1, level, lolo, skip, fixmode, P->f16 ? F16S : 0.f, 1, planned ? &P->plan : nullptr};
+    return CFG_PAIR[cfg] ? opb::launch_tc_gemm_batched_pair(maps, probs, P->work + l.off, l.n, s, a)
+                         : opb::launch_tc_gemm_batched(CFG_BN[cfg], maps, probs, P->work + l.off, l.n, P->grid, s, a);
 }
 
 // Squaring level `level` of every lattice still squaring; each lattice's operands are
@@ -618,30 +594,24 @@ int cfg_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s, int lolo, in
 int level_gemm(opb_batch_plan *P, int cfg, int level, cudaStream_t s) {
     const int lolo = (!P->f16 && level < opb::g_lolo_levels) ? 1 : 0;
     return cfg_gemm(P, cfg, level, s, lolo, opb::g_band_skip, level > 0 ? opb::OPB_FIX_SQUARE : opb::OPB_FIX_NONE,
-                    level > 0 && opb::g_band_skip);
+                    opb::g_band_skip != 0);
 }
 
-// The tile plans of level `level` >= 1 under configuration cfg (which K-blocks each item
-// issues, from the marks that the previous level left), and its row fixes.
+// The tile plan of level `level` under configuration cfg (which K-blocks each item issues, from
+// the marks of E0 or those that the previous level left), and its row fixes.
 int level_plan(opb_batch_plan *P, int cfg, int level, cudaStream_t s) {
     const int bn = CFG_BN[cfg], k = level & 1;
-    const ListRef &l = P->gemm_level[cfg][level], &rest = P->gemm_level_rest[cfg][level];
-    const uint32_t *work[2] = {P->work + l.off, P->work + rest.off};
-    const int n[2] = {l.n, rest.n}, tm[2] = {CFG_PAIR[cfg] ? 256 : 128, 128}, tn[2] = {CFG_PAIR[cfg] ? 256 : bn, 256};
-    return opb::launch_tile_plan_batched(P->plan, work, n, tm, tn, P->sq[k], P->sq[k ^ 1], level, P->occ[k ^ 1],
-                                         (long long)P->occ_bytes, P->lats, P->nlat, bn < 128 ? bn : 128, P->total_rows, s);
-}
-
-// What the autotuner times: the first level's squaring of every lattice, without its band.
-int dense_gemm(opb_batch_plan *P, int cfg, cudaStream_t s) {
-    return cfg_gemm(P, cfg, 0, s, 0, 0, opb::OPB_FIX_NONE, false);
+    const ListRef &l = P->gemm_level[cfg][level];
+    return opb::launch_tile_plan_batched(P->plan, P->work + l.off, l.n, CFG_PAIR[cfg] ? 256 : 128, bn, P->sq[k], level,
+                                         P->occ[k ^ 1], (long long)P->occ_bytes, P->lats, P->nlat, bn < 128 ? bn : 128,
+                                         P->total_rows, s);
 }
 
 // E0 build and every squaring level: P1 of every lattice as row-major parts in its A and B
 // buffers.  Per level the tile plan with the row fixes of the level before, one GEMM, and the
 // renormalisation (to P1) of the lattices whose last level it was.
-int batch_square(opb_batch_plan *P, cudaStream_t s) {
-    const int cfg = P->cfg, bn = CFG_BN[cfg], pdiv = bn < 128 ? bn : 128;
+int batch_square(opb_batch_plan *P, int cfg, cudaStream_t s) {
+    const int bn = CFG_BN[cfg], pdiv = bn < 128 ? bn : 128;
     const float ss = P->f16 ? F16S : 0.f;
     int r = 0;
     // lattices off the 128 grid: the caller's generators and spot values into the padded rows
@@ -649,20 +619,22 @@ int batch_square(opb_batch_plan *P, cudaStream_t s) {
     if (P->padded)
         r = opb::launch_pad_batched(P->lats, P->nlat, P->total_rows, P->ell_width, P->cols_src, P->vals_src,
                                     P->x_src, P->cols_pad, P->vals_pad, P->x_pad, s);
-    if (r == 0) r = (int)cudaMemsetAsync(P->E_base, 0, P->E_bytes, s);
-    // Under the tile plans no block is read that its level did not write.  Without them (band
-    // skipping off) every level writes every tile.
+    // Under the tile plans every level writes the blocks that are or become non-zero: both part
+    // sets start as zeros, with the row-sum partials and the marks.  Without them (band skipping
+    // off) every level writes every tile.
     const bool planned = opb::g_band_skip != 0;
-    if (r == 0 && planned) r = (int)cudaMemsetAsync(P->occ[1], 0, P->occ_bytes + 64, s);
-    if (r == 0) r = opb::launch_ek_batched(P->lats, P->nlat, P->total_rows, P->ell_width, P->cols, P->vals, s);
-    if (r == 0) r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_init.off, P->rn_init.n, 0, s, ss);
+    if (r == 0) r = (int)cudaMemsetAsync(P->E_base, 0, P->E_bytes, s);
+    if (r == 0 && planned) r = (int)cudaMemsetAsync(P->part, 0, P->part_bytes, s);
+    if (r == 0 && planned) r = (int)cudaMemsetAsync(P->occ[0], 0, P->occ_bytes + 64, s);
+    if (r == 0)
+        r = opb::launch_ek_batched(P->lats, P->nlat, P->total_rows, P->ell_width, P->cols, P->vals, s, planned, ss);
+    if (r == 0 && !planned) r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_init.off, P->rn_init.n, 0, s, ss);
     for (int lv = 0; lv < P->maxn && r == 0; lv++) {
-        if (lv > 0)
-            r = planned ? level_plan(P, cfg, lv, s)
-                        : opb::launch_rowfix_batched(P->lats, P->nlat, P->total_rows, pdiv, lv - 1, s);
+        if (planned) r = level_plan(P, cfg, lv, s);
+        else if (lv > 0) r = opb::launch_rowfix_batched(P->lats, P->nlat, P->total_rows, pdiv, lv - 1, s);
         if (r == 0) r = level_gemm(P, cfg, lv, s);
         if (r == 0 && P->rn_level[lv].n > 0)
-            r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_level[lv].off, P->rn_level[lv].n, pdiv, s, ss);
+            r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_level[lv].off, P->rn_level[lv].n, pdiv, s, ss, planned);
     }
     return r;
 }
@@ -688,7 +660,7 @@ OPB_API int opb_batch_execute(opb_batch_plan *P, double *quotes) {
                                  P->fp32_ws_bytes, quotes + (size_t)i * P->nmat * P->nK, nullptr));
         return set_status(OPB_OK);
     }
-    BT(batch_square(P, s));
+    BT(batch_square(P, P->cfg, s));
     BT(opb::launch_payoff_batched(P->lats, P->nlat, P->total_rows, P->nK, P->ldk, P->x, P->strikes, s, P->f16));
     // chains: the quoted row of P_m = P_{m-1} . P1 for every lattice (row_chain.cuh), its
     // normalisation deferred into the next step and into the quotes; one product prices up
@@ -735,7 +707,7 @@ OPB_API int opb_batch_execute_bermudan(opb_batch_plan *P, int put, int exercise,
                                     exercise, barrier, P->fp32_ws[0], P->fp32_ws_bytes, quotes + (size_t)i * P->nK));
         return set_status(OPB_OK);
     }
-    BT(batch_square(P, s));
+    BT(batch_square(P, P->cfg, s));
     BT(opb::launch_berm_batched_init(P->lats, P->nlat, P->total_rows, P->nK, P->ldk, P->x, P->strikes, put, barrier,
                                      P->f16, s));
     for (int m = P->nmat - 1; m >= 0; m--) {
@@ -748,9 +720,13 @@ OPB_API int opb_batch_execute_bermudan(opb_batch_plan *P, int put, int exercise,
     return set_status(OPB_OK);
 }
 
-// Times a dense squaring (all lattices active: the shape of every squaring level once the
-// operands have filled in) for every configuration with CUDA events and keeps the
-// fastest; ms[cfg] (optional, opb_batch_num_configs() entries) receives the times.
+// Times the squarings of the plan's generators under every configuration with CUDA events and
+// keeps the fastest (which K-blocks a tile issues depends on the generators' spread, so a dense
+// product says little: it prefers 256 x 256 tiles where 128 x 256 ones take 15.0 ms to their
+// 15.7 for 256 lattices of the sweep).  A tile plan orders the items by what they issue, whatever
+// order they are listed in, so one run of each tile form is timed and its two orders share it; without
+// plans (band skipping off) every configuration is, reps times.  ms[cfg] (optional,
+// opb_batch_num_configs() entries) receives the times.
 // Blocking; leaves the plan's buffers in an arbitrary state (run execute afterwards).
 OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *best_cfg) {
     OPB_REQUIRE(P, OPB_E_NULL);
@@ -766,18 +742,29 @@ OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *
     float best = 1e30f;
     int bc = 0;
     for (int cfg = 0; cfg < NCFG; cfg++) {
-        int r = dense_gemm(P, cfg, s);  // warm-up (also sets the smem attribute)
+        const bool planned = opb::g_band_skip != 0;
+        if (planned && kTwin[cfg] != cfg) {
+            if (ms_out) ms_out[cfg] = ms_out[kTwin[cfg]];
+            continue;
+        }
+        // warm-up (sets the shared-memory attributes): one whole run, which also initialises the
+        // marks and the plan's counters, then the first level alone
+        int r = 0;
+        if (cfg == 0) r = batch_square(P, cfg, s);
+        if (r == 0 && cfg > 0 && planned) r = level_plan(P, cfg, 0, s);
+        if (r == 0 && cfg > 0) r = level_gemm(P, cfg, 0, s);
         if (r) return set_status(r);
+        const int n = planned ? 1 : reps;
         OPB_TRY(cudaEventRecord(e0, s));
-        for (int i = 0; i < reps; i++) {
-            r = dense_gemm(P, cfg, s);
+        for (int i = 0; i < n; i++) {
+            r = batch_square(P, cfg, s);
             if (r) return set_status(r);
         }
         OPB_TRY(cudaEventRecord(e1, s));
         OPB_TRY(cudaEventSynchronize(e1));
         float ms = 0.f;
         OPB_TRY(cudaEventElapsedTime(&ms, e0, e1));
-        ms /= reps;
+        ms /= n;
         if (ms_out) ms_out[cfg] = ms;
         if (ms < best) { best = ms; bc = cfg; }
     }
@@ -792,11 +779,9 @@ OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *
 OPB_API int opb_batch_launches(const opb_batch_plan *P) {
     if (!P) return 0;
     if (!tc_mode_b(P->mode)) return -1;
-    int extra = 0;  // the pair configurations' second GEMM launch per level
-    for (int lv = 0; lv < P->maxn; lv++) extra += P->gemm_level_rest[P->cfg][lv].n > 0 ? 1 : 0;
-    int per_level = 0;  // plan with row fixes (from the second level on), GEMM, renormalisation (some end)
-    for (int lv = 0; lv < P->maxn; lv++) per_level += 1 + (lv > 0 ? 1 : 0) + (P->rn_level[lv].n > 0 ? 1 : 0);
+    int per_level = 0;  // plan with row fixes, GEMM, renormalisation (some end)
+    for (int lv = 0; lv < P->maxn; lv++) per_level += 2 + (P->rn_level[lv].n > 0 ? 1 : 0);
     // a row launch per maturity; a product and a quote launch per group of priced maturities
     const int groups = (P->nmat + opb::kRowSlots - 1) / opb::kRowSlots;
-    return 4 + (P->padded ? 1 : 0) + per_level + 1 + (P->f16 ? 1 : 0) + P->nmat + 2 * groups + extra;
+    return 4 + (P->padded ? 1 : 0) + per_level + 1 + (P->f16 ? 1 : 0) + P->nmat + 2 * groups;
 }

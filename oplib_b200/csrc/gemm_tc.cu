@@ -330,7 +330,9 @@ struct TcParams {
     int fixmode;             // as TcGemmArgs::fixmode
     __nv_bfloat16 *Shi, *Slo;  // as TcGemmArgs::Shi / Slo (single products; batched: TcProblem)
     float sscale;            // as TcGemmArgs::sscale
-    const uint32_t *order, *kmask;  // as TcGemmArgs::plan (order and masks of this launch's items)
+    const uint2 *order;      // the plan of this launch (TilePlan), kmask null: none
+    const uint32_t *kmask;
+    const unsigned *nlist;
     int nw;
     uint8_t *occ;            // as TcGemmArgs::occ, occ_in (single products; batched: TcProblem)
     const uint8_t *occ_in;
@@ -429,7 +431,8 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int mtiles = p.M / Cfg::TILE_M, ntiles_n = p.N / BN;
     const int nsplit = (!BATCHED && p.ksplit > 1) ? p.ksplit : 1;  // K-slices of a single product
-    const int nitems = BATCHED ? bt.nwork : mtiles * ntiles_n * nsplit;
+    int nitems = BATCHED ? bt.nwork : mtiles * ntiles_n * nsplit;
+    if (PLANNED && p.kmask) nitems = (int)*p.nlist;  // the plan leaves out the tiles with nothing to do
     // pair mode: rank within the 2-CTA cluster, items walked per cluster
     const uint32_t rank = PAIR ? cluster_rank() : 0u;
     const int item0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
@@ -437,14 +440,23 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     // item t -> (problem, m0, n0, K-blocks, first K-block, K-slice); a single product split
     // into nsplit K-slices has nsplit consecutive items per output tile
     // mk: the item's K-block mask when the launch has a plan (kmask); its chunks keep their
-    // K-blocks, and those whose operand parts are zero are left out
-    auto get_item = [&](int t, int &prob, int &m0, int &n0, int &nkb, int &kb0, int &slice, const uint32_t *&mk) {
+    // K-blocks, and those whose operand parts are zero are left out.  The plan's entry of an
+    // item (mask index, packed tile) is fetched one item ahead.
+    auto entry = [&](int t) -> uint2 {
+        return PLANNED && p.kmask && t < nitems ? __ldg(p.order + t) : make_uint2(0u, 0u);
+    };
+    auto get_item = [&](int t, const uint2 &e, int &prob, int &m0, int &n0, int &nkb, int &kb0, int &slice,
+                        const uint32_t *&mk) {
         mk = nullptr;
+        slice = 0;
         if (PLANNED && p.kmask) {
-            t = (int)p.order[t];
-            mk = p.kmask + (long long)t * p.nw;
-        }
-        if constexpr (BATCHED) {
+            mk = p.kmask + (long long)e.x * p.nw;
+            prob = BATCHED ? (int)(e.y >> 16) : 0;
+            m0 = (int)(BATCHED ? (e.y >> 8) & 255u : e.y >> 16) * Cfg::TILE_M;
+            n0 = (int)(e.y & (BATCHED ? 255u : 0xffffu)) * BN;
+            nkb = (BATCHED ? bt.probs[prob].K : p.K) / BK;
+            kb0 = 0;
+        } else if constexpr (BATCHED) {
             const uint32_t w = bt.work[t];
             prob = (int)(w >> 16);
             m0 = (int)((w >> 8) & 255u) * Cfg::TILE_M;  // pair mode: 256-row items
@@ -452,33 +464,20 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
             const TcProblem &pr = bt.probs[prob];
             const long long h = (pr.band > 0 && p.band_skip) ? level_band(pr.band, p.level) : -1;
             band_kblocks(h, m0, Cfg::TILE_M, n0, BN, pr.K, BK, Cfg::CHUNK, kb0, nkb);
-            slice = 0;
         } else {
             slice = t % nsplit;
             t /= nsplit;
-            const int GM = p.group_m > 0 ? p.group_m : 8;
-            const int per_group = GM * ntiles_n;
-            const int group = t / per_group;
-            const int first_m = group * GM;
-            const int gm = min(mtiles - first_m, GM);
-            const int r = t - group * per_group;
+            int mt, nt;
+            raster_tile(t, mtiles, ntiles_n, p.group_m, mt, nt);
             prob = 0;
-            m0 = (first_m + r % gm) * Cfg::TILE_M;
-            n0 = (r / gm) * BN;
+            m0 = mt * Cfg::TILE_M;
+            n0 = nt * BN;
             nkb = p.K / BK / nsplit;
             kb0 = slice * nkb;
             if (p.band && p.band_skip && nsplit == 1) {
                 const int h0 = *p.band;
                 band_kblocks(h0 > 0 ? level_band(h0, p.level) : -1, m0, Cfg::TILE_M, n0, BN, p.K, BK, Cfg::CHUNK,
                              kb0, nkb);
-            }
-        }
-        if (PLANNED && mk) {
-            if (nkb == 0) mk = nullptr;  // outside twice the band: nothing to issue, nothing to write
-            else {
-                if constexpr (BATCHED) nkb = bt.probs[prob].K / BK;
-                else nkb = p.K / BK;
-                kb0 = 0;
             }
         }
     };
@@ -558,10 +557,12 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                         tma_load_2d(bres_base + kb * Cfg::B_BYTES, &mBhi, bres_bar, kb * BK, 0);
                 }
             }
+            uint2 next = entry(item0);
             for (int t = item0; t < nitems && ok; t += istep) {
                 int prob, m0, n0, nkb, kb0, slice;
                 const uint32_t *mk;
-                get_item(t, prob, m0, n0, nkb, kb0, slice, mk);
+                get_item(t, next, prob, m0, n0, nkb, kb0, slice, mk);
+                next = entry(t + istep);
                 uint32_t mw = 0;
                 const int ma = m0 + (int)rank * TC_BM;          // this CTA's A rows
                 const int nb = n0 + (int)rank * Cfg::B_ROWS;    // this CTA's B rows
@@ -649,10 +650,12 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     tc_fence_after();
                 }
             }
+            uint2 next = entry(item0);
             for (int t = item0; t < nitems && ok; t += istep) {
                 int prob, m0, n0, nkb, kb0, slice;
                 const uint32_t *mk;
-                get_item(t, prob, m0, n0, nkb, kb0, slice, mk);
+                get_item(t, next, prob, m0, n0, nkb, kb0, slice, mk);
+                next = entry(t + istep);
                 uint32_t mw = 0;
                 const bool lolo = item_lolo(prob);
                 const int nch = (nkb + Cfg::CHUNK - 1) / Cfg::CHUNK;
@@ -738,11 +741,13 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
         float sum[CPT];
         long g = 0;
         bool ok = true;
+        uint2 next = entry(item0);
         for (int t = item0; t < nitems && ok; t += istep) {
             int prob, m0, n0, nkb, kb0, slice;
             const uint32_t *mk;
-            get_item(t, prob, m0, n0, nkb, kb0, slice, mk);
-            const bool reached = nkb > 0;
+            get_item(t, next, prob, m0, n0, nkb, kb0, slice, mk);
+            next = entry(t + istep);
+            const bool reached = nkb > 0;  // (a plan has no item that is not)
             int nch = (nkb + Cfg::CHUNK - 1) / Cfg::CHUNK;
             if (PLANNED && mk) {  // the chunks with a K-block to issue
                 static_assert(!PLANNED || Cfg::CHUNK == 2, "two mask bits per chunk");
@@ -753,58 +758,43 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
 #pragma unroll
                 for (int j = 0; j < CPT; j++) sum[j] = 0.f;
             }
-            // a batched item's last column tile may overhang its matrix (zero B columns
-            // beyond N): this thread's column group then has nothing to store
-            const bool group_in = !BATCHED || n0 + h * CPT < bt.probs[prob].N;
             const int rbase = m0 + (int)rank * TC_BM + q * 32, col0 = n0 + h * CPT;
+            // a batched item's last tiles may overhang their matrix (zero A rows and B columns
+            // beyond it): this warp's rows or columns then have nothing to store
+            const bool group_in = !BATCHED || (col0 < bt.probs[prob].N && rbase < bt.probs[prob].M);
             // this thread's Cin row segment is prefetched into L2 about three chunks before
             // the output needs it (the live 64-column blocks); the row and column fixes are
             // loaded here, while the MMAs run
             const float *pf = nullptr;
             long long pf_ld = 0;
             const double2 *fix = nullptr;
-            const uint8_t *mi = nullptr;  // marks of the operand's blocks (E before this level)
-            // 64-column blocks that are not zero, or on the diagonal; the second level still
-            // writes every block of its tiles, so that both part sets hold what the marks say
+            // 64-column blocks that are marked; those and the ones on the diagonal
             uint32_t had = 0, live = ~0u;
-            bool fill = false;            // a zero block's parts are still to be written as zeros
             double2 rfix = make_double2(0.0, 0.0);
             float scol[CPT / 32];
             if constexpr (EPIMODE == 0) {
-                int h0 = 0;
+                const uint8_t *mi = nullptr;  // marks of the operand's blocks (E before this level)
                 if constexpr (BATCHED) {
                     const TcProblem &pr = bt.probs[prob];
                     pf = group_in ? pr.Cin : nullptr;
                     pf_ld = pr.ldc;
                     fix = pr.cin_fix;
-                    if (OCC && p.kmask && group_in) {
-                        mi = pr.occ_in;
-                        h0 = pr.band;
-                    }
+                    mi = OCC && p.kmask && group_in ? pr.occ_in : nullptr;
                 } else {
                     pf = p.Cin;
                     pf_ld = p.ldc;
                     fix = p.cin_fix;
-                    if (OCC && p.kmask) {
-                        mi = p.occ_in;
-                        h0 = p.band ? *p.band : 0;
-                    }
+                    mi = OCC && p.kmask ? p.occ_in : nullptr;
                 }
-                if (!reached) mi = nullptr;
                 if (OCC && mi) {
+                    live = 0;
 #pragma unroll
                     for (int b = 0; b < CPT / 64; b++) {
                         const int c = col0 + 64 * b;
-                        if ((mi[(long long)(rbase >> 5) * (pf_ld >> 6) + (c >> 6)] & 2) || (rbase < c + 64 && c < rbase + 32))
-                            had |= 1u << b;
+                        if (mi[(long long)(rbase >> 5) * (pf_ld >> 6) + (c >> 6)] & 2) had |= 1u << b;
+                        if (rbase < c + 64 && c < rbase + 32) live |= 1u << b;
                     }
-                    if (p.level >= 2) live = had;
-                    if (FUSE == 1 && h0 > 0 && p.level >= 2) {
-                        const int K = BATCHED ? bt.probs[prob].K : p.K;
-                        int lo, cnt;
-                        band_kblocks(level_band(h0, p.level - 2), m0, Cfg::TILE_M, n0, BN, K, BK, Cfg::CHUNK, lo, cnt);
-                        fill = cnt == 0;
-                    }
+                    live |= had;
                 }
                 if (fix && group_in && (FUSE == 0 || p.fixmode != OPB_FIX_NONE)) {
                     rfix = fix[rbase + lane];
@@ -977,19 +967,8 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     uint32_t any = 0;
 #pragma unroll
                     for (int i = 0; i < 64; i++) any |= __float_as_uint(sum[64 * b + i]);
-                    if (!__any_sync(0xffffffffu, any != 0)) {
-                        // zero before, nothing added: E, updated in place, is zero already, and so
-                        // are its parts in this set unless the tile is new to it
-                        if (FUSE == 1 && Shi && fill) {
-#pragma unroll
-                            for (int i = 0; i < 8; i++) {
-                                const long long so = (long long)(rbase + 4 * i + tr) * ldc + col0 + 64 * b + 8 * tc;
-                                *reinterpret_cast<uint4 *>(Shi + so) = make_uint4(0, 0, 0, 0);
-                                *reinterpret_cast<uint4 *>(Slo + so) = make_uint4(0, 0, 0, 0);
-                            }
-                        }
-                        continue;
-                    }
+                    // zero before, nothing added: E, updated in place, and its parts are zero already
+                    if (!__any_sync(0xffffffffu, any != 0)) continue;
                     if (FUSE != 2 && Cin) load_cin(cv[0], 2 * b, 0);
                 }
                 uint32_t nzp = 0, nze = 0;  // any bit of this block's hi parts, of its values
@@ -1013,12 +992,22 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                             for (int u = 0; u < 4; u++) sj[u] = __shfl_sync(0xffffffffu, scol[j], 4 * tc + u);
                         }
                     }
+                    // the half block in four passes over its four rows a lane -- sums in, values,
+                    // C out, parts out -- so that four independent chains are in flight (row by
+                    // row, a load could not pass the stores before it, which may alias for all
+                    // the compiler knows)
+                    const int gcol = col0 + 32 * j + 4 * tc;
+                    float o[4][4];
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const int rr = 4 * (4 * hb + i) + tr;
-                        const int grow = rbase + rr, gcol = col0 + 32 * j + 4 * tc;
                         const float4 sv = st[rr * 8 + (tc ^ (rr & 7))];
-                        float o[4] = {alpha * sv.x, alpha * sv.y, alpha * sv.z, alpha * sv.w};
+                        o[i][0] = alpha * sv.x; o[i][1] = alpha * sv.y; o[i][2] = alpha * sv.z; o[i][3] = alpha * sv.w;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int rr = 4 * (4 * hb + i) + tr;
+                        const int grow = rbase + rr;
                         const float4 &cf = cv[hf & 1][i];
                         if constexpr (FUSE == 1) {
                             // squaring with the parts of its output: alpha acc + beta E', and with
@@ -1033,13 +1022,13 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                                 const float inv = __shfl_sync(0xffffffffu, rinv, rr), bi = beta - si;
 #pragma unroll
                                 for (int u = 0; u < 4; u++) {
-                                    float x = fmaf(bi - sj[u], c4[u], o[u]);
+                                    float x = fmaf(bi - sj[u], c4[u], o[i][u]);
                                     if (grow == gcol + u) x += si * (si - beta);
-                                    o[u] = x * inv;
+                                    o[i][u] = x * inv;
                                 }
                             } else {
 #pragma unroll
-                                for (int u = 0; u < 4; u++) o[u] = fmaf(beta, c4[u], o[u]);
+                                for (int u = 0; u < 4; u++) o[i][u] = fmaf(beta, c4[u], o[i][u]);
                             }
                         } else if constexpr (FUSE == 2) {
                             // parts only, A's rows normalised here (OPB_FIX_ROWSCALE; FP32 inv:
@@ -1047,7 +1036,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                             if (fm == OPB_FIX_ROWSCALE) {
                                 const float inv = __shfl_sync(0xffffffffu, rinv, rr);
 #pragma unroll
-                                for (int u = 0; u < 4; u++) o[u] *= inv;
+                                for (int u = 0; u < 4; u++) o[i][u] *= inv;
                             }
                         } else if (Cin) {
                             float c4[4] = {cf.x, cf.y, cf.z, cf.w};
@@ -1065,32 +1054,49 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                                 }
                             }
 #pragma unroll
-                            for (int u = 0; u < 4; u++) o[u] = fmaf(beta, c4[u], o[u]);
+                            for (int u = 0; u < 4; u++) o[i][u] = fmaf(beta, c4[u], o[i][u]);
                         }
-                        if (C) *reinterpret_cast<float4 *>(C + (long long)grow * ldc + gcol) = make_float4(o[0], o[1], o[2], o[3]);
-                        if constexpr (FUSE != 0) {
-                            if (Shi) {
-                                uint32_t hh[2], ll[2];
-                                split2x2(o[0], o[1], hh[0], ll[0], p.sscale);
-                                split2x2(o[2], o[3], hh[1], ll[1], p.sscale);
-                                const long long so = (long long)grow * ldc + gcol;
-                                *reinterpret_cast<uint2 *>(Shi + so) = make_uint2(hh[0], hh[1]);
-                                *reinterpret_cast<uint2 *>(Slo + so) = make_uint2(ll[0], ll[1]);
-                                if constexpr (OCC) {
-                                    nzp |= hh[0] | hh[1];
-                                    nze |= __float_as_uint(o[0]) | __float_as_uint(o[1]) | __float_as_uint(o[2]) |
-                                           __float_as_uint(o[3]);
-                                }
+                    }
+                    const long long so = (long long)(rbase + 16 * hb + tr) * ldc + gcol;
+                    if (C) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            *reinterpret_cast<float4 *>(C + so + 4 * i * ldc) = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
+                    }
+                    if (rowsum) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            acc[4 * hb + i] += (double)o[i][0] + (double)o[i][1] + (double)o[i][2] + (double)o[i][3];
+                    }
+                    if constexpr (OCC) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            nze |= __float_as_uint(o[i][0]) | __float_as_uint(o[i][1]) | __float_as_uint(o[i][2]) |
+                                   __float_as_uint(o[i][3]);
+                    }
+                    if constexpr (FUSE != 0) {
+                        if (Shi) {
+                            uint32_t hh[4][2], ll[4][2];
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                split2x2(o[i][0], o[i][1], hh[i][0], ll[i][0], p.sscale);
+                                split2x2(o[i][2], o[i][3], hh[i][1], ll[i][1], p.sscale);
+                                nzp |= hh[i][0] | hh[i][1];
+                            }
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                *reinterpret_cast<uint2 *>(Shi + so + 4 * i * ldc) = make_uint2(hh[i][0], hh[i][1]);
+                                *reinterpret_cast<uint2 *>(Slo + so + 4 * i * ldc) = make_uint2(ll[i][0], ll[i][1]);
                             }
                         }
-                        if (rowsum) acc[4 * hb + i] += (double)o[0] + (double)o[1] + (double)o[2] + (double)o[3];
                     }
                 }
                 __syncwarp();  // before the next block overwrites the buffer
-                if constexpr (OCC && FUSE == 1) {
+                if constexpr (OCC) {
                     if (occ) {
                         const bool np = __any_sync(0xffffffffu, nzp != 0), ne = __any_sync(0xffffffffu, nze != 0);
-                        // (a block once non-zero keeps its mark: its parts stay in the other set)
+                        // (a block once marked stays marked: each level then rewrites its parts in
+                        // the set it writes, and an unmarked block's are zero in both)
                         if (lane == 0)
                             occ[(long long)(rbase >> 5) * (ldc >> 6) + ((col0 + 64 * b) >> 6)] =
                                 (uint8_t)((np ? 1u : 0u) | (ne || ((had >> b) & 1u) ? 2u : 0u));
@@ -1301,6 +1307,14 @@ static int set_smem_attr() {
     return 0;
 }
 
+static void set_plan(TcParams &p, const TilePlan *pl) {
+    if (!pl) return;
+    p.order = pl->order;
+    p.kmask = pl->kmask;
+    p.nlist = pl->nlist;
+    p.nw = pl->nw;
+}
+
 template <int BN, int STAGES, bool F16, int BK = TC_BK, bool BMN = false, int FUSE = 0>
 static int launch_tc_impl(const TcGemmArgs &a, cudaStream_t s) {
     using Cfg = TcCfg<BN, STAGES, 3, BK>;
@@ -1324,9 +1338,7 @@ static int launch_tc_impl(const TcGemmArgs &a, cudaStream_t s) {
     p.Shi = a.Shi;
     p.Slo = a.Slo;
     p.sscale = a.sscale;
-    p.order = a.order;
-    p.kmask = a.kmask;
-    p.nw = a.nw;
+    set_plan(p, a.plan);
     p.occ = a.occ;
     p.occ_in = a.occ_in;
     const int ntiles = (a.M / TC_BM) * (a.N / BN) * p.ksplit;
@@ -1363,9 +1375,7 @@ static int launch_tc_pair(const TcGemmArgs &a, cudaStream_t s) {
     p.Shi = a.Shi;
     p.Slo = a.Slo;
     p.sscale = a.sscale;
-    p.order = a.order;
-    p.kmask = a.kmask;
-    p.nw = a.nw;
+    set_plan(p, a.plan);
     p.occ = a.occ;
     p.occ_in = a.occ_in;
     TcBatch none{nullptr, nullptr, nullptr, 0};
@@ -1428,9 +1438,7 @@ static int launch_batched_impl(const CUtensorMap *maps, const TcProblem *probs, 
     p.band_skip = b.band_skip;
     p.fixmode = b.fixmode;
     p.sscale = b.sscale;
-    p.order = b.order;
-    p.kmask = b.kmask;
-    p.nw = b.nw;
+    set_plan(p, b.plan);
     TcBatch bt{maps, probs, work, nwork};
     k_tc_gemm<BN, STAGES, true, F16, 3, 0, TC_BK, false, BMN, FUSE><<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(
         dummy, dummy, dummy, dummy, p, bt);
@@ -1439,7 +1447,9 @@ static int launch_batched_impl(const CUtensorMap *maps, const TcProblem *probs, 
 
 // Batched 256 x 256 items on 2-CTA clusters: work items (problem << 16 | m-tile << 8 |
 // n-tile) in 256-row / 256-column units, maps with 128-row boxes for A and B (each CTA
-// loads its own half), problems with M % 256 == 0 and N % 256 == 0.
+// loads its own half).  A size that is an odd multiple of 128 overhangs by half a tile, whose
+// operands load as zeros: (ceil(d / 256) * 256 / d)^2 of the products (1.11 at d = 1152), against a
+// second launch of one-CTA tiles, with its own tail, per level.
 template <bool F16, bool BMN, int FUSE>
 static int launch_batched_pair_impl(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
                                     cudaStream_t s, const TcBatchArgs &b) {
@@ -1481,9 +1491,7 @@ static int launch_batched_pair_impl(const CUtensorMap *maps, const TcProblem *pr
     p.band_skip = b.band_skip;
     p.fixmode = b.fixmode;
     p.sscale = b.sscale;
-    p.order = b.order;
-    p.kmask = b.kmask;
-    p.nw = b.nw;
+    set_plan(p, b.plan);
     TcBatch bt{maps, probs, work, nwork};
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, dummy, dummy, dummy, dummy, p, bt);
     return e == cudaSuccess ? (int)cudaGetLastError() : (int)e;
@@ -1909,24 +1917,22 @@ bool tile_plan_for(int d, int &tm, int &tn) {
 int launch_tile_plan_single(const TilePlan &pl, int d, int tm, int tn, const int *band, int level, const uint8_t *occ,
                             uint8_t *clear, const double *partial, int nparts, double2 *fix, cudaStream_t s) {
     TilePlanArgs a{};
-    a.list[0] = TilePlanList{nullptr, (d / tm) * (d / tn), tm, tn, pl.order, pl.kmask, pl.count};
-    a.nw = pl.nw; a.level = level; a.band_skip = 1;
+    a.n = (d / tm) * (d / tn); a.tm = tm; a.tn = tn; a.pl = pl;
+    a.level = level;
     a.d = d; a.group_m = g_group_m; a.band = band; a.occ = occ;
-    a.clear = clear; a.clear_bytes = (long long)tile_plan_marks(d); a.done = pl.done;
+    a.clear = clear; a.clear_bytes = (long long)tile_plan_marks(d);
     a.partial = partial; a.nparts = nparts; a.fix = fix;
     return launch_tile_plan(a, s);
 }
 
-int launch_tile_plan_batched(const TilePlan *pl, const uint32_t *const *work, const int *n, const int *tm, const int *tn,
-                             const TcProblem *probs, const TcProblem *other, int level, uint8_t *clear,
-                             long long clear_bytes, const BatchLattice *lats, int nlat, int parts_div,
-                             long long total_rows, cudaStream_t s) {
+int launch_tile_plan_batched(const TilePlan &pl, const uint32_t *work, int n, int tm, int tn, const TcProblem *probs,
+                             int level, uint8_t *clear, long long clear_bytes, const BatchLattice *lats, int nlat,
+                             int parts_div, long long total_rows, cudaStream_t s) {
     TilePlanArgs a{};
-    for (int i = 0; i < 2; i++)
-        a.list[i] = TilePlanList{work[i], n[i], tm[i], tn[i], pl[i].order, pl[i].kmask, pl[i].count};
-    a.nw = pl[0].nw; a.level = level; a.band_skip = 1;
-    a.probs = probs; a.other = other;
-    a.clear = clear; a.clear_bytes = clear_bytes; a.done = pl[0].done;
+    a.work = work; a.n = n; a.tm = tm; a.tn = tn; a.pl = pl;
+    a.level = level;
+    a.probs = probs;
+    a.clear = clear; a.clear_bytes = clear_bytes;
     a.lats = lats; a.nlat = nlat; a.parts_div = parts_div; a.total_rows = total_rows;
     return launch_tile_plan(a, s);
 }

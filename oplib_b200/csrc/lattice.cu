@@ -74,7 +74,7 @@ struct Bufs {
     int *band;     // the ELL generator's half-bandwidth, found on the device per solve
     double *xpad;  // spot values of the padded lattice (split modes, d % 128 != 0)
     uint8_t *occ[2];     // marks of the two part sets, opb::tile_plan_marks(d) each
-    opb::TilePlan plan;  // (occ[1] and plan.done lie next to each other)
+    opb::TilePlan plan;  // (occ[0] and plan.done lie next to each other)
 };
 
 inline int padded_nk(int nK, int mode) { return tc_mode(mode) ? (nK + 63) / 64 * 64 : nK; }
@@ -110,10 +110,12 @@ Bufs carve(Ws &w, int d, int nK, int mode, bool pad = false) {
         if (pad) b.xpad = w.take<double>((size_t)d);
         const size_t tiles = (size_t)(d / 128) * (d / 64);  // of the narrowest tile
         b.plan.nw = opb::tile_plan_words(d);
-        b.occ[0] = w.take<uint8_t>(opb::tile_plan_marks(d));
-        b.occ[1] = w.take<uint8_t>(opb::tile_plan_marks(d) + 64);
-        b.plan.done = reinterpret_cast<unsigned *>(b.occ[1] + opb::tile_plan_marks(d));
-        b.plan.order = w.take<uint32_t>(tiles);
+        b.occ[0] = w.take<uint8_t>(opb::tile_plan_marks(d) + 64);
+        b.occ[1] = w.take<uint8_t>(opb::tile_plan_marks(d));
+        b.plan.done = reinterpret_cast<unsigned *>(b.occ[0] + opb::tile_plan_marks(d));
+        b.plan.nlist = b.plan.done + 1;
+        b.plan.order = w.take<uint2>(tiles);
+        b.plan.tile = w.take<uint32_t>(tiles);
         b.plan.kmask = w.take<uint32_t>(tiles * b.plan.nw);
         b.plan.count = w.take<uint16_t>(tiles);
     } else {
@@ -223,15 +225,33 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
     // E0 = dt*L in FP32 (FP64 arithmetic), then its splits.  An ELL generator's band h0
     // bounds E_r's to h0 * 2^r: the squarings skip the K-blocks (and whole output tiles) that
     // only multiply zeros, with bit-identical results.
+    // Under a tile plan (from OPB_PLAN_MIN_D states) a level issues only the K-blocks that its
+    // operand's marks show to be non-zero, and writes only the blocks that are or become so:
+    // the parts (of both sets, fused), the marks and the row-sum partials start as zeros, and an
+    // ELL generator's E0 goes in with its parts and marks.
+    int tm = 0, tn = 0;
+    const bool fused = opb::fused_single(d);
+    const bool planned = d >= opb::OPB_PLAN_MIN_D && L.niter > 0 && g_ksplit <= 1 && opb::tile_plan_for(d, tm, tn);
+    opb::E0Parts e0{};
+    if (planned) {
+        const bool ell = L.ell_width > 0;
+        LT((int)cudaMemsetAsync(b.Ahi, 0, sizeof(__nv_bfloat16) * (fused ? 4 : 2) * (size_t)d * d, s));
+        LT((int)cudaMemsetAsync(b.part, 0, sizeof(double) * (size_t)np * d, s));
+        // (a dense generator: every block marked, its parts from the split below)
+        LT((int)cudaMemsetAsync(b.occ[0], ell ? 0 : 3, opb::tile_plan_marks(d), s));
+        LT((int)cudaMemsetAsync(b.plan.done, 0, 64, s));
+        if (ell) e0 = opb::E0Parts{b.Ahi, b.Alo, b.occ[0], ss};
+    }
     // (d_gen < d: the generator's d_gen states, then absorbing padding states)
-    if (d_gen != d) LT(opb::launch_ek_padded(d_gen, d, L.ell_width, L.gen_cols, L.gen_vals, L.gen_dense, L.dt, b.X, s));
+    if (d_gen != d)
+        LT(opb::launch_ek_padded(d_gen, d, L.ell_width, L.gen_cols, L.gen_vals, L.gen_dense, L.dt, b.X, s, e0));
     if (L.ell_width > 0) {
-        if (d_gen == d) LT(opb::launch_ek_ell(d, L.ell_width, L.gen_cols, L.gen_vals, L.dt, 1, b.X, s));
+        if (d_gen == d) LT(opb::launch_ek_ell(d, L.ell_width, L.gen_cols, L.gen_vals, L.dt, 1, b.X, s, e0));
         LT(opb::launch_ell_band(d_gen, L.ell_width, L.gen_cols, b.band, s));
     } else if (d_gen == d) {
         LT(opb::launch_ek_dense(d, L.gen_dense, L.dt, 1, b.X, s));
     }
-    LT(opb::launch_split(d, d, b.X, d, b.Ahi, b.Alo, nullptr, nullptr, d, s, ss));
+    if (!e0.hi) LT(opb::launch_split(d, d, b.X, d, b.Ahi, b.Alo, nullptr, nullptr, d, s, ss));
     // every squaring and chain product reads its B operand K x N row-major (MN-major):
     // a squaring's B is E's own row-major parts, a chain product's B the row-major parts of
     // P1 kept in the B buffers
@@ -245,15 +265,7 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
     // B starts zeroed; the band only grows, so the tiles a level skips are zero in both.
     // (lattices not fused, opb::fused_single: a renormalisation kernel after every level,
     // which writes the next level's parts)
-    const bool fused = opb::fused_single(d);
-    // Under a tile plan (from OPB_PLAN_MIN_D states) the second and later levels issue only the
-    // K-blocks that the previous output's marks show to be non-zero; then no block is read
-    // that its level did not write, and B needs no zeros.
-    int tm = 0, tn = 0;
-    const bool planned = d >= opb::OPB_PLAN_MIN_D && L.niter > 1 && g_ksplit <= 1 && opb::tile_plan_for(d, tm, tn);
-    if (planned)
-        LT((int)cudaMemsetAsync(b.occ[1], 0, opb::tile_plan_marks(d) + 64, s));
-    else if (fused && L.niter > 1) {
+    if (fused && !planned && L.niter > 1) {
         LT((int)cudaMemsetAsync(b.Bhi, 0, sizeof(__nv_bfloat16) * (size_t)d * d, s));
         LT((int)cudaMemsetAsync(b.Blo, 0, sizeof(__nv_bfloat16) * (size_t)d * d, s));
     }
@@ -276,24 +288,23 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
         g.level = r;
         // BF16 parts: the lo.lo product on the first levels (see OPB_LOLO_LEVELS)
         g.lolo = (!f16 && r < opb::g_lolo_levels) ? 1 : 0;
+        uint8_t *mo = planned ? b.occ[(r & 1) ^ 1] : nullptr;  // the output's marks
         if (planned) {
-            g.occ = (last || !fused) ? nullptr : b.occ[(r & 1) ^ 1];
-            if (r > 0) {
-                // (fused: the plan forms the row fixes of the previous level too)
-                LT(opb::launch_tile_plan_single(b.plan, d, tm, tn, g.band, r, b.occ[r & 1], b.occ[(r & 1) ^ 1], b.part, np,
-                                                fused ? b.fix : nullptr, s));
-                g.order = b.plan.order; g.kmask = b.plan.kmask; g.nw = b.plan.nw;
-                g.occ_in = b.occ[r & 1];
-            }
+            // (fused: the plan forms the row fixes of the previous level too)
+            LT(opb::launch_tile_plan_single(b.plan, d, tm, tn, g.band, r, b.occ[r & 1], mo, b.part, np,
+                                            fused && r > 0 ? b.fix : nullptr, s));
+            g.plan = &b.plan;
+            g.occ_in = b.occ[r & 1];
+            g.occ = mo;
         }
         LT(tc_gemm_ksplit(g, s));
         // the last level emits P1 = I + E and its splits (row-major into A: the first
         // chain's A and pricing's; row-major into B: every chain's B); the others only the
         // row fixes of their output
-        if (last) LT(opb::launch_renorm_to_p(d, b.X, b.part, np, b.Ahi, b.Alo, b.Bhi, b.Blo, s, ss));
+        if (last)
+            LT(opb::launch_renorm_to_p(d, b.X, b.part, np, b.Ahi, b.Alo, b.Bhi, b.Blo, s, ss, fused ? mo : nullptr));
         else if (!fused)
-            LT(opb::launch_renorm(d, b.X, b.part, np, 1, b.Ahi, b.Alo, nullptr, nullptr, s, ss, 0, b.fix,
-                                  planned ? b.occ[(r & 1) ^ 1] : nullptr));
+            LT(opb::launch_renorm(d, b.X, b.part, np, 1, b.Ahi, b.Alo, nullptr, nullptr, s, ss, 0, b.fix, mo));
         else if (!planned) LT(opb::launch_rowfix(d, b.part, np, 1, b.fix, s));
     }
     g.Ahi = b.Ahi; g.Alo = b.Alo;
@@ -302,7 +313,7 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
     g.Shi = g.Slo = nullptr;
     g.occ = nullptr;
     g.occ_in = nullptr;
-    g.order = g.kmask = nullptr;
+    g.plan = nullptr;
     g.band = nullptr;
     g.band_skip = 0;
     g.level = 0;

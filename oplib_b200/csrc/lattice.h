@@ -94,12 +94,19 @@ int sgemm_rm_strided(bool ta, bool tb, int M, int N, int K, float alpha, const f
 // lattice_kernels.cu
 // *out = max |col - row| over the ELL entries (the generator's half-bandwidth)
 int launch_ell_band(int d, int w, const int *cols, int *out, cudaStream_t s);
+// Parts and marks that the ELL builds of E0 write beside it (hi null: none), for planned
+// squarings; the matrices and the marks must be zero.
+struct E0Parts {
+    __nv_bfloat16 *hi, *lo;
+    uint8_t *occ;
+    float sscale;
+};
 int launch_ek_ell(int d, int w, const int *cols, const double *vals, double dt, int eform, float *out,
-                  cudaStream_t s);
+                  cudaStream_t s, const E0Parts &parts = E0Parts{});
 // E0 = dt L (E-form) of a d-state generator (ELL when w > 0, else dense) into a dpad x dpad
 // matrix whose states d..dpad-1 are absorbing (zero rows and columns)
 int launch_ek_padded(int d, int dpad, int w, const int *cols, const double *vals, const double *dense, double dt,
-                     float *out, cudaStream_t s);
+                     float *out, cudaStream_t s, const E0Parts &parts = E0Parts{});
 // xpad[i] = x[min(i, d - 1)], i < dpad
 int launch_pad_x(int d, int dpad, const double *x, double *xpad, cudaStream_t s);
 int launch_ek_dense(int d, const double *L, double dt, int eform, float *out, cudaStream_t s);
@@ -108,7 +115,8 @@ int launch_split(int rows, int cols, const float *X, long long ld, __nv_bfloat16
 int launch_rowsum(int d, const float *X, double *partial, cudaStream_t s);
 // write_x = 0 leaves X as it is (only the splits are written; d % 64 == 0); fix (optional,
 // E-form) receives the per-row (s, inv) that a following product applies to X as its Cin; occ
-// (optional, d % 64 == 0) the marks of the written A parts (TcGemmArgs::occ).
+// (optional, d % 64 == 0): X's marks (TcGemmArgs::occ), whose unmarked blocks are left out and
+// which receive those of the written A parts.
 int launch_renorm(int d, float *X, const double *partial, int nparts, int eform, __nv_bfloat16 *Ahi,
                   __nv_bfloat16 *Alo, __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale = 0.f,
                   int write_x = 1, double2 *fix = nullptr, uint8_t *occ = nullptr);
@@ -135,7 +143,6 @@ struct BatchLattice {
     long long row_off;    // first global row (rows of all lattices concatenated)
     double dt, rate, period;
     float *E;             // d x d FP32 (E-form, then P1)
-    float *Pa;            // d x d FP32 chain product
     float *V;             // d x ldk FP32 pricing result
     __nv_bfloat16 *GThi, *GTlo;  // ldk x d payoff splits (or, in the induction, d x ldk value splits)
     float *gscale;        // device scalar: FP16 payoff split scale
@@ -148,6 +155,8 @@ struct BatchLattice {
     // caller's generator and spot arrays
     int d_src;
     long long src_off;
+    __nv_bfloat16 *Ahi, *Alo;  // E0's parts and marks
+    uint8_t *occ0;
 };
 // Padded copies of the caller's ELL generator (w slots per row; padding rows get column -1)
 // and spot values (padding rows repeat the last state's) in the plan's padded row space.
@@ -166,6 +175,7 @@ struct RenormProblem {
     const double *partial;
     __nv_bfloat16 *Ahi, *Alo, *Bhi, *Blo;
     double2 *fix;  // mode-0 items: per-row (s, inv) for the next product's Cin (cin_fix)
+    uint8_t *occ;  // marks of the last level's output
 };
 // Batched backward induction over all lattices of a sweep (lattice_kernels.cu): per-lattice
 // split scales, terminal values and one induction date (quotes [nlat][nK] at the last)
@@ -184,12 +194,15 @@ int launch_berm_step(int d, int nK, int ldk, const float *C, double disc, const 
                      const float *dscale, int y0, double *quotes, cudaStream_t s, int nslice = 1,
                      long long slice_stride = 0);
 int launch_renorm_to_p(int d, float *X, const double *partial, int nparts, __nv_bfloat16 *Ahi, __nv_bfloat16 *Alo,
-                       __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale = 0.f);
+                       __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale = 0.f,
+                       const uint8_t *occ = nullptr);
+// marks: leave out the tiles that RenormProblem::occ shows to be zero.
 // work items: problem << 16 | mode << 14 | strip << 7 | chunk (see renorm_chunks)
 int launch_renorm_batched(const RenormProblem *probs, const uint32_t *work, int nwork, int parts_div, cudaStream_t s,
-                          float sscale = 0.f);
+                          float sscale = 0.f, int marks = 0);
+// parts: E0's 16-bit parts and marks too (planned squarings)
 int launch_ek_batched(const BatchLattice *lats, int nlat, long long total_rows, int w, const int *cols,
-                      const double *vals, cudaStream_t s);
+                      const double *vals, cudaStream_t s, int parts = 0, float sscale = 0.f);
 int launch_payoff_batched(const BatchLattice *lats, int nlat, long long total_rows, int nK, int ldk, const double *x,
                           const double *strikes, cudaStream_t s, int f16 = 0);
 // Quotes of nm priced rows of every lattice (row slot i: maturity m0 + i + 1)
@@ -241,13 +254,10 @@ struct TcGemmArgs {
     // value it stores, row-major with leading dimension ldc; C may then be null (parts only)
     __nv_bfloat16 *Shi, *Slo;
     float sscale;
-    // optional (squarings, 64-deep stages): the tile plan of this product (k_tile_plan): its
-    // items in issue order and nw mask words per item, one bit per K-block
-    const uint32_t *order, *kmask;
-    int nw;
+    const struct TilePlan *plan;  // optional (squarings, 64-deep stages): the plan of this product
     // marks of 32 x 64 blocks (row-major, one byte each), bit 0: the hi parts are not all zero,
-    // bit 1: the FP32 values are not all zero (or have not been so at an earlier level).
-    uint8_t *occ;           // optional, with Shi: written for the output's blocks
+    // bit 1: the FP32 values are not all zero, or have not been so at an earlier level.
+    uint8_t *occ;           // optional: written for the output's blocks (bit 0 with Shi)
     const uint8_t *occ_in;  // with a plan: Cin's, blocks without bit 1 hold zeros
 };
 // Deferred normalisation in the epilogue, with cin_fix[i] = (s_i, inv_i) of the operand
@@ -326,7 +336,7 @@ struct TcProblem {
 int tc_make_maps(CUtensorMap *out4, const __nv_bfloat16 *Ahi, const __nv_bfloat16 *Alo, long long M, long long lda,
                  const __nv_bfloat16 *Bhi, const __nv_bfloat16 *Blo, long long N, long long ldb, long long K, int bn,
                  int f16 = 0, int b_kn = 0);
-// A batched launch: level, lolo, band_skip, fixmode, sscale, order, kmask, nw as TcGemmArgs
+// A batched launch: level, lolo, band_skip, fixmode, sscale, plan as TcGemmArgs
 // (band, cin_fix, Shi / Slo, occ per problem); fuse: 1 = squaring with its output's parts
 // (OPB_FIX_SQUARE, MN-major B), 0 = FP32 output
 struct TcBatchArgs {
@@ -334,14 +344,13 @@ struct TcBatchArgs {
     int level, lolo, band_skip, fixmode;
     float sscale;
     int fuse;
-    const uint32_t *order, *kmask;
-    int nw;
+    const struct TilePlan *plan;
 };
 // work: packed (problem << 16 | m-tile << 8 | n-tile); bn in {64, 128, 256}, without fuse 64
 int launch_tc_gemm_batched(int bn, const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
                            int grid, cudaStream_t s, const TcBatchArgs &b);
-// 256 x 256 items (256-row / 256-column units) on 2-CTA clusters, each CTA loading its
-// 128 rows of A and 128 columns of B; squarings of problems with M, N multiples of 256
+// 256 x 256 items (256-row / 256-column units, the last ones may overhang) on 2-CTA clusters,
+// each CTA loading its 128 rows of A and 128 columns of B; squarings
 int launch_tc_gemm_batched_pair(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
                                 cudaStream_t s, const TcBatchArgs &b);
 
@@ -350,10 +359,13 @@ int launch_tc_gemm_batched_pair(const CUtensorMap *maps, const TcProblem *probs,
 inline size_t tile_plan_marks(int d) { return ((size_t)(d / 32) * (d / 64) + 15) & ~size_t(15); }
 inline int tile_plan_words(int d) { return (d / 64 + 31) / 32; }
 struct TilePlan {
-    uint32_t *order, *kmask;
-    uint16_t *count;
+    uint2 *order;      // nlist items in issue order: index of the item's mask, packed tile
+    uint32_t *kmask;   // nw words per item, one bit per K-block
+    unsigned *nlist;
+    uint32_t *tile;    // scratch
+    uint16_t *count;   // scratch
     int nw;
-    unsigned *done;  // zero before the first plan; each plan leaves it zero
+    unsigned *done;    // zero before the first plan; each plan leaves it zero
 };
 bool tile_plan_for(int d, int &tm, int &tn);
 // The plan of level `level`'s squaring from its operands' marks, clearing the marks that the
@@ -361,12 +373,11 @@ bool tile_plan_for(int d, int &tm, int &tn);
 // launch_rowfix, E-form).
 int launch_tile_plan_single(const TilePlan &pl, int d, int tm, int tn, const int *band, int level, const uint8_t *occ,
                             uint8_t *clear, const double *partial, int nparts, double2 *fix, cudaStream_t s);
-// Two work lists of one level (problems `probs`; their operands' marks are written by the
-// other part set's problems), and the row fixes of the lattices that square at this level.
-int launch_tile_plan_batched(const TilePlan *pl, const uint32_t *const *work, const int *n, const int *tm, const int *tn,
-                             const TcProblem *probs, const TcProblem *other, int level, uint8_t *clear,
-                             long long clear_bytes, const BatchLattice *lats, int nlat, int parts_div,
-                             long long total_rows, cudaStream_t s);
+// The work list of one level (problems `probs`), and the row fixes of the lattices that square
+// at this level.
+int launch_tile_plan_batched(const TilePlan &pl, const uint32_t *work, int n, int tm, int tn, const TcProblem *probs,
+                             int level, uint8_t *clear, long long clear_bytes, const BatchLattice *lats, int nlat,
+                             int parts_div, long long total_rows, cudaStream_t s);
 
 // row_chain.cuh (in gemm_tc.cu) -- the quoted row of the chained kernels.
 // The quoted row of one lattice.

@@ -31,9 +31,16 @@ __global__ void k_zero_set_diag(int d, float *__restrict__ U, float v) {
     if (y < d) U[(long long)y * d + y] = v;
 }
 
+// The parts and marks of one entry of E0 (planned squarings: the matrices and the marks start zeroed).
+__device__ __forceinline__ void e0_parts(const E0Parts &p, long long y, int z, long long ld, float f) {
+    const long long o = y * ld + z;
+    split2(f, p.hi[o], p.lo[o], p.sscale);
+    p.occ[(y >> 5) * (ld >> 6) + (z >> 6)] = 3;
+}
+
 // ELL generator: row y holds w (col, val) pairs; col < 0 marks padding.
 __global__ void k_ek_scatter_ell(int d, int w, const int *__restrict__ cols, const double *__restrict__ vals,
-                                 double dt, int eform, float *__restrict__ out, long long ld) {
+                                 double dt, int eform, float *__restrict__ out, long long ld, E0Parts parts) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)d * w) return;
     int y = (int)(t / w);
@@ -42,6 +49,7 @@ __global__ void k_ek_scatter_ell(int d, int w, const int *__restrict__ cols, con
     double v = dt * vals[t];
     if (!eform && z == y) v += 1.0;
     out[(long long)y * ld + z] = (float)v;
+    if (parts.hi) e0_parts(parts, y, z, ld, (float)v);
 }
 
 // Half-bandwidth of an ELL generator: max |col - row| over its entries (padding excluded),
@@ -197,9 +205,12 @@ __global__ void k_renorm(int d, float *__restrict__ X, const double *__restrict_
 // squaring level); 2 = P-form in and out.  nparts = 0 skips the scaling (pure split).
 // Each (hi, lo) pair is one 32-bit shared word; the 65-word row stride keeps both the
 // row-wise stores and the column-wise reads of the transpose at most 2-way bank-conflicted.
-struct RenormSmem {
+constexpr int RN_LIVE = 512;  // column tiles of a strip that a block can pick out by their marks
+struct alignas(16) RenormSmem {
     double s_sum[64], s_inv[64];
     uint32_t t[64][65];
+    uint16_t live[RN_LIVE];
+    int nlive;
 };
 
 // Input staging: a ring of RN_RING tiles in shared memory filled by cp.async (16 bytes per
@@ -209,6 +220,7 @@ struct RenormSmem {
 struct RenormRing {
     float4 v[RN_RING][4][256];
 };
+static_assert(sizeof(RenormSmem) % 16 == 0, "the ring behind it holds 16-byte copies");
 constexpr int RN_SMEM = (int)(sizeof(RenormSmem) + sizeof(RenormRing));
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
@@ -297,17 +309,14 @@ __device__ __forceinline__ void renorm64_apply(RenormSmem &sm, int d, float *__r
             *reinterpret_cast<uint2 *>(Ahi + o) = make_uint2(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]));
             *reinterpret_cast<uint2 *>(Alo + o) = make_uint2(pack_bf16(l[0], l[1]), pack_bf16(l[2], l[3]));
         }
-        // marks for the next product's tile plan (a warp's two rows lie in one 32 x 64 block;
-        // several warps may set the same mark)
-        if (occ) {
+        // marks for the next product's tile plan: the values' came with the product, the parts' are
+        // set here (a warp's two rows lie in one 32 x 64 block, which several warps may mark)
+        if (occ && mode == 0) {
             const uint32_t nz = pack_bf16(h[0], h[1]) | pack_bf16(h[2], h[3]);
-            const uint32_t nx = __float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w);
-            const bool np = __any_sync(0xffffffffu, nz != 0), ne = __any_sync(0xffffffffu, nx != 0);
-            if (ne && (tid & 31) == 0) {
+            if (__any_sync(0xffffffffu, nz != 0) && (tid & 31) == 0) {
                 const size_t at = (size_t)(r >> 5) * (d >> 6) + (c0 >> 6);
-                const uint32_t bits = np ? 3u : 2u;
-                if ((reinterpret_cast<volatile uint8_t *>(occ)[at] & bits) != bits)
-                    atomicOr(reinterpret_cast<uint32_t *>(occ) + (at >> 2), bits << (8 * (at & 3)));
+                if (!(reinterpret_cast<volatile uint8_t *>(occ)[at] & 1u))
+                    atomicOr(reinterpret_cast<uint32_t *>(occ) + (at >> 2), 1u << (8 * (at & 3)));
             }
         }
         if (Bhi && b_rm) {
@@ -341,10 +350,30 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
                                                float sscale, double2 *__restrict__ fix, bool b_rm,
                                                uint8_t *__restrict__ occ = nullptr) {
     const int nt = d / 64, tid = threadIdx.x;
-    const int cnt = first < nt ? (nt - 1 - first) / step + 1 : 0;
+    int cnt = first < nt ? (nt - 1 - first) / step + 1 : 0;
+    // under a tile plan the tiles without a mark (off the diagonal) are zero and stay zero, and so
+    // are their parts: left alone
+    const bool pick = occ != nullptr && cnt <= RN_LIVE;
+    if (pick) {
+        if (tid < 32) {
+            int n = 0;
+            for (int k0 = 0; k0 < cnt; k0 += 32) {
+                const int t = first + (k0 + tid) * step;
+                const bool on = k0 + tid < cnt && (t * 64 == r0 || (occ[(long long)(r0 >> 5) * nt + t] & 2) ||
+                                                   (occ[(long long)((r0 >> 5) + 1) * nt + t] & 2));
+                const uint32_t m = __ballot_sync(0xffffffffu, on);
+                if (on) sm.live[n + __popc(m & ((1u << tid) - 1u))] = (uint16_t)t;
+                n += __popc(m);
+            }
+            if (tid == 0) sm.nlive = n;
+        }
+        __syncthreads();
+        cnt = sm.nlive;
+    }
+    auto col0 = [&](int k) { return (pick ? (int)sm.live[k] : first + k * step) * 64; };
 #pragma unroll
     for (int k = 0; k < RN_RING - 1; k++) {
-        if (k < cnt) renorm64_issue(rg, k, d, X, r0, (first + k * step) * 64);
+        if (k < cnt) renorm64_issue(rg, k, d, X, r0, col0(k));
         cp_async_commit();  // possibly empty: every iteration commits exactly one group
     }
     renorm64_sums(sm, d, partial, nparts, mode, r0, fix);
@@ -352,12 +381,12 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
     for (int k = 0; k < cnt; k++) {
         // the slot refilled here was read (and its values used) in iteration k - 1
         const int kn = k + RN_RING - 1;
-        if (kn < cnt) renorm64_issue(rg, kn % RN_RING, d, X, r0, (first + kn * step) * 64);
+        if (kn < cnt) renorm64_issue(rg, kn % RN_RING, d, X, r0, col0(kn));
         cp_async_commit();
         cp_async_wait<RN_RING - 1>();  // this thread's copies of tile k have landed
         const int sl = k % RN_RING;
         const float4 v[4] = {rg.v[sl][0][tid], rg.v[sl][1][tid], rg.v[sl][2][tid], rg.v[sl][3][tid]};
-        renorm64_apply(sm, d, Xout, mode, Ahi, Alo, Bhi, Blo, r0, (first + k * step) * 64, sscale, v, b_rm, occ);
+        renorm64_apply(sm, d, Xout, mode, Ahi, Alo, Bhi, Blo, r0, col0(k), sscale, v, b_rm, occ);
     }
 }
 
@@ -398,7 +427,7 @@ static dim3 renorm64_grid(int d) {
 // row-major A parts as their B operand.
 __global__ void __launch_bounds__(256) k_renorm64_batched(const RenormProblem *__restrict__ probs,
                                                           const uint32_t *__restrict__ work, int parts_div,
-                                                          float sscale) {
+                                                          float sscale, int marks) {
     extern __shared__ __align__(16) uint8_t rn_smem[];
     RenormSmem &sm = *reinterpret_cast<RenormSmem *>(rn_smem);
     RenormRing &rg = *reinterpret_cast<RenormRing *>(rn_smem + sizeof(RenormSmem));
@@ -409,7 +438,7 @@ __global__ void __launch_bounds__(256) k_renorm64_batched(const RenormProblem *_
     const int r0 = (int)((w >> 7) & 127u) * 64, chunk = (int)(w & 127u);
     renorm64_strip(sm, rg, pr.d, pr.X, nullptr, pr.partial, nparts, mode, pr.Ahi, pr.Alo,
                    mode == 1 ? pr.Bhi : nullptr, mode == 1 ? pr.Blo : nullptr, r0, chunk, renorm_chunks(pr.d),
-                   sscale, mode == 0 && chunk == 0 ? pr.fix : nullptr, true);
+                   sscale, mode == 0 && chunk == 0 ? pr.fix : nullptr, true, marks ? pr.occ : nullptr);
 }
 
 // Opts both renormalisation kernels into RN_SMEM bytes of dynamic shared memory (once per
@@ -432,7 +461,8 @@ static int renorm64_prepare() {
 // Batched ELL scatter into zeroed dense E-form matrices: thread per global ELL slot
 // (rows of all lattices concatenated; row_off[i] = first global row of lattice i).
 __global__ void k_ek_scatter_batched(const BatchLattice *__restrict__ lats, int nlat, long long total_rows, int w,
-                                     const int *__restrict__ cols, const double *__restrict__ vals) {
+                                     const int *__restrict__ cols, const double *__restrict__ vals, int parts,
+                                     float sscale) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= total_rows * w) return;
     const long long grow = t / w;
@@ -445,7 +475,9 @@ __global__ void k_ek_scatter_batched(const BatchLattice *__restrict__ lats, int 
     const int y = (int)(grow - L.row_off);
     const int z = cols[t];
     if (z < 0 || z >= L.d) return;
-    L.E[(long long)y * L.d + z] = (float)(L.dt * vals[t]);
+    const float f = (float)(L.dt * vals[t]);
+    L.E[(long long)y * L.d + z] = f;
+    if (parts) e0_parts(E0Parts{L.Ahi, L.Alo, L.occ0, sscale}, y, z, L.d, f);
 }
 
 // Batched payoff splits: G^T[k][z] = (x_z - K_k)^+ for strikes k < nK of lattice i and 0
@@ -676,12 +708,12 @@ __global__ void k_berm_step(int d, int nK, int ldk, const float *__restrict__ C,
 static inline int blocks_for(long long n, int threads) { return (int)((n + threads - 1) / threads); }
 
 int launch_ek_ell(int d, int w, const int *cols, const double *vals, double dt, int eform, float *out,
-                  cudaStream_t s) {
+                  cudaStream_t s, const E0Parts &parts) {
     cudaError_t e = cudaMemsetAsync(out, 0, sizeof(float) * (size_t)d * d, s);
     if (e != cudaSuccess) return (int)e;
     if (!eform) k_zero_set_diag<<<blocks_for(d, 256), 256, 0, s>>>(d, out, 1.0f);
     long long n = (long long)d * w;
-    if (n > 0) k_ek_scatter_ell<<<blocks_for(n, 256), 256, 0, s>>>(d, w, cols, vals, dt, eform, out, d);
+    if (n > 0) k_ek_scatter_ell<<<blocks_for(n, 256), 256, 0, s>>>(d, w, cols, vals, dt, eform, out, d, parts);
     return (int)cudaGetLastError();
 }
 
@@ -699,12 +731,12 @@ int launch_ek_dense(int d, const double *L, double dt, int eform, float *out, cu
 }
 
 int launch_ek_padded(int d, int dpad, int w, const int *cols, const double *vals, const double *dense, double dt,
-                     float *out, cudaStream_t s) {
+                     float *out, cudaStream_t s, const E0Parts &parts) {
     cudaError_t e = cudaMemsetAsync(out, 0, sizeof(float) * (size_t)dpad * dpad, s);
     if (e != cudaSuccess) return (int)e;
     if (w > 0) {
         long long n = (long long)d * w;
-        if (n > 0) k_ek_scatter_ell<<<blocks_for(n, 256), 256, 0, s>>>(d, w, cols, vals, dt, 1, out, dpad);
+        if (n > 0) k_ek_scatter_ell<<<blocks_for(n, 256), 256, 0, s>>>(d, w, cols, vals, dt, 1, out, dpad, parts);
     } else {
         long long n = (long long)d * d;
         int b = blocks_for(n, 256), cap = 16 * num_sms();
@@ -749,19 +781,19 @@ int launch_renorm(int d, float *X, const double *partial, int nparts, int eform,
 // (the last squaring level: P1 is the A of the first chain product and of pricing, and
 // the B of every chain product).
 int launch_renorm_to_p(int d, float *X, const double *partial, int nparts, __nv_bfloat16 *Ahi, __nv_bfloat16 *Alo,
-                       __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale) {
+                       __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale, const uint8_t *occ) {
     if (d % 64) return OPB_E_UNSUPPORTED;
     if (int r = renorm64_prepare()) return r;
     k_renorm64<<<renorm64_grid(d), 256, RN_SMEM, s>>>(d, X, partial, nparts, 1, Ahi, Alo, Bhi, Blo, sscale, 1,
-                                                      nullptr, 1);
+                                                      nullptr, 1, const_cast<uint8_t *>(occ));
     return (int)cudaGetLastError();
 }
 
 int launch_renorm_batched(const RenormProblem *probs, const uint32_t *work, int nwork, int parts_div, cudaStream_t s,
-                          float sscale) {
+                          float sscale, int marks) {
     if (nwork <= 0) return OPB_OK;
     if (int r = renorm64_prepare()) return r;
-    k_renorm64_batched<<<nwork, 256, RN_SMEM, s>>>(probs, work, parts_div, sscale);
+    k_renorm64_batched<<<nwork, 256, RN_SMEM, s>>>(probs, work, parts_div, sscale, marks);
     return (int)cudaGetLastError();
 }
 
@@ -803,10 +835,10 @@ int launch_pad_batched(const BatchLattice *lats, int nlat, long long total_rows,
 }
 
 int launch_ek_batched(const BatchLattice *lats, int nlat, long long total_rows, int w, const int *cols,
-                      const double *vals, cudaStream_t s) {
+                      const double *vals, cudaStream_t s, int parts, float sscale) {
     long long n = total_rows * w;
     if (n <= 0) return OPB_OK;
-    k_ek_scatter_batched<<<(int)((n + 255) / 256), 256, 0, s>>>(lats, nlat, total_rows, w, cols, vals);
+    k_ek_scatter_batched<<<(int)((n + 255) / 256), 256, 0, s>>>(lats, nlat, total_rows, w, cols, vals, parts, sscale);
     return (int)cudaGetLastError();
 }
 
