@@ -4,11 +4,13 @@
 //   opcuda_sgemm  (oplib/opcuda/sgemm.cu:41-44, column-major, alpha/beta),
 //   opcuda_ssqmm  (oplib/opcuda/ssqmm.cu:119-179, batched d x d via device pointer tables),
 //   opcuda_sgemm4 (oplib/opcuda/sgemm4.cu:84-154, ragged batch through a per-block task table).
-// The reference kernels are 64x16-tile Volkov-style SIMT loops for sm_1x; here one core
-// kernel computes a row-major 128x128 CTA tile with 8x8 outputs per thread, a
-// double-buffered shared-memory K pipeline and float4 shared-memory fragments.
+// The reference kernels are 64x16-tile Volkov-style SIMT loops for sm_1x; here large products
+// take row-major 128x128 CTA tiles with 8x8 outputs per thread, small ones and the task tables
+// tiles of a warp each (below).
 // Column-major calls are mapped onto it through C^T = B^T . A^T (a column-major matrix
 // is the row-major storage of its transpose), so the kernel never transposes data.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace opb {
@@ -268,6 +270,178 @@ __global__ void __launch_bounds__(SG_THREADS, 2) k_sgemm_pipe(SgemmArgs p) {
     }
 }
 
+// ---- small tiles: a warp computes 8 RPT x 16 outputs (a thread RPT x 4), for products whose
+// 128 x 128 tiles leave SMs idle, and for the task tables, whose tiles are 64 x 16.
+//
+// The tile is written column-major (X contiguous in the left operand and in C, K contiguous in
+// the right one), which is what the tables hold; a row-major product is C^T = B^T . A^T.  K runs
+// in steps of 16 through a ring of shared stages filled by 16-byte cp.async (4-byte ones where an
+// operand's rows are not 16-byte aligned), each operand as it lies in memory: transposing the
+// right one with 4-byte copies cost about a cycle an element, 1000 cycles a stage (512^3: 27 us
+// whatever the tile).  Four steps of K at a time, a thread issues four to eight 128-bit loads of
+// the left tile (its X pairs come packed), four of the right one (along K, each value duplicated
+// by a move) and 4 RPT / 2 x 4 packed FMAs, so the FMA pipe is what bounds it.  Every output
+// sums its products in k order with fma, as the other kernels here do: the same bits.
+constexpr int ST_BK = 16, ST_STAGES = 4;
+
+// 16 bytes of global memory into shared memory, bytes beyond `valid` as zeros (valid 0: all).
+__device__ __forceinline__ void st_cp16(float *dst, const float *src, int valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(valid)
+                 : "memory");
+}
+__device__ __forceinline__ void st_cp4(float *dst, const float *src, int valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(valid)
+                 : "memory");
+}
+
+// A stage's left tile: X columns [x0, x0 + TX) of K rows [k0, k0 + 16), element (x, k) at
+// A[k * lda + x], into dst[k][x] (pitch floats a row), by `nthr` threads of which this is `tid`.
+template <int TX>
+__device__ __forceinline__ void st_load_a(float *dst, int pitch, const float *A, long long lda, int X, int K, int x0,
+                                          int k0, bool vec, int tid, int nthr) {
+    if (vec) {
+        for (int e = tid; e < ST_BK * TX / 4; e += nthr) {
+            const int k = e / (TX / 4), x = (e % (TX / 4)) * 4;
+            const int left = k0 + k < K ? X - (x0 + x) : 0;
+            const int valid = left >= 4 ? 16 : left > 0 ? 4 * left : 0;
+            st_cp16(dst + k * pitch + x, valid ? A + (long long)(k0 + k) * lda + x0 + x : A, valid);
+        }
+    } else {
+        for (int e = tid; e < ST_BK * TX; e += nthr) {
+            const int k = e / TX, x = e % TX;
+            const bool in = k0 + k < K && x0 + x < X;
+            st_cp4(dst + k * pitch + x, in ? A + (long long)(k0 + k) * lda + x0 + x : A, in ? 4 : 0);
+        }
+    }
+}
+// A stage's right tile: Y columns [y0, y0 + TY), element (k, y) at B[y * ldb + k], into
+// dst[y * ST_BP + k].
+constexpr int ST_BP = ST_BK + 4;  // four neighbouring y fall on different banks
+template <int TY>
+__device__ __forceinline__ void st_load_b(float *dst, const float *B, long long ldb, int Y, int K, int y0, int k0,
+                                          bool vec, int tid, int nthr) {
+    if (vec) {
+        for (int e = tid; e < ST_BK * TY / 4; e += nthr) {
+            const int k = (e % (ST_BK / 4)) * 4, y = e / (ST_BK / 4);
+            const int left = y0 + y < Y ? K - (k0 + k) : 0;
+            const int valid = left >= 4 ? 16 : left > 0 ? 4 * left : 0;
+            st_cp16(dst + y * ST_BP + k, valid ? B + (long long)(y0 + y) * ldb + k0 + k : B, valid);
+        }
+    } else {
+        for (int e = tid; e < ST_BK * TY; e += nthr) {
+            const int k = e % ST_BK, y = e / ST_BK;
+            const bool in = k0 + k < K && y0 + y < Y;
+            st_cp4(dst + y * ST_BP + k, in ? B + (long long)(y0 + y) * ldb + k0 + k : B, in ? 4 : 0);
+        }
+    }
+}
+
+// One step of K: this thread's X values at `as` (and, RPT = 8, 32 further on) times its four Y values.
+template <int RPT>
+__device__ __forceinline__ void st_step(uint64_t (&acc)[RPT / 2][4], const float *as, float b0, float b1, float b2,
+                                        float b3) {
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(as);
+    ulonglong2 a1 = a0;
+    if constexpr (RPT == 8) a1 = *reinterpret_cast<const ulonglong2 *>(as + 32);
+    const uint64_t bb[4] = {f2_pack(b0, b0), f2_pack(b1, b1), f2_pack(b2, b2), f2_pack(b3, b3)};
+    const uint64_t aa[4] = {a0.x, a0.y, a1.x, a1.y};
+#pragma unroll
+    for (int i = 0; i < RPT / 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = f2_fma(aa[i], bb[j], acc[i][j]);
+}
+// A stage of kn (<= 16) steps; the thread's Y columns are 4 apart, from bs on.
+template <int RPT>
+__device__ __forceinline__ void st_steps(uint64_t (&acc)[RPT / 2][4], const float *as, int ap, const float *bs, int kn) {
+    if (kn == ST_BK) {
+#pragma unroll
+        for (int k = 0; k < ST_BK; k += 4) {
+            float4 b[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) b[j] = *reinterpret_cast<const float4 *>(bs + 4 * j * ST_BP + k);
+            st_step<RPT>(acc, as + k * ap, b[0].x, b[1].x, b[2].x, b[3].x);
+            st_step<RPT>(acc, as + (k + 1) * ap, b[0].y, b[1].y, b[2].y, b[3].y);
+            st_step<RPT>(acc, as + (k + 2) * ap, b[0].z, b[1].z, b[2].z, b[3].z);
+            st_step<RPT>(acc, as + (k + 3) * ap, b[0].w, b[1].w, b[2].w, b[3].w);
+        }
+    } else {
+        for (int k = 0; k < kn; k++)
+            st_step<RPT>(acc, as + k * ap, bs[k], bs[4 * ST_BP + k], bs[8 * ST_BP + k], bs[12 * ST_BP + k]);
+    }
+}
+// Stores this thread's outputs: rows x.. (and x + 32..), columns y, y + 4, y + 8, y + 12 of
+// column-major C.
+template <int RPT>
+__device__ __forceinline__ void st_store(const uint64_t (&acc)[RPT / 2][4], float *C, long long ldc, int X, int Y, int x,
+                                         int y, float alpha, float beta, bool vec) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (y + 4 * j >= Y) continue;
+#pragma unroll
+        for (int h = 0; h < RPT / 4; h++) {
+            float v[4];
+            f2_unpack(acc[2 * h][j], v[0], v[1]);
+            f2_unpack(acc[2 * h + 1][j], v[2], v[3]);
+            float *c = C + (long long)(y + 4 * j) * ldc + x + 32 * h;
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] *= alpha;
+            if (vec && x + 32 * h + 4 <= X) {
+                if (beta != 0.f) {
+                    const float4 o = *reinterpret_cast<const float4 *>(c);
+                    v[0] = fmaf(beta, o.x, v[0]); v[1] = fmaf(beta, o.y, v[1]);
+                    v[2] = fmaf(beta, o.z, v[2]); v[3] = fmaf(beta, o.w, v[3]);
+                }
+                *reinterpret_cast<float4 *>(c) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (x + 32 * h + i < X) c[i] = beta != 0.f ? fmaf(beta, c[i], v[i]) : v[i];
+            }
+        }
+    }
+}
+
+// Row-major C[M,N] = alpha * A . B + beta * C on tiles of 8 RPT WX columns of N x 16 WY rows of M;
+// grid (N tiles, M tiles, batch).
+template <int RPT, int WX, int WY>
+__global__ void __launch_bounds__(32 * WX * WY) k_sgemm_small(SgemmArgs p) {
+    constexpr int TX = 8 * RPT * WX, TY = 16 * WY, AP = TX + 4, NT = 32 * WX * WY;
+    __shared__ __align__(16) float As[ST_STAGES][ST_BK * AP], Bs[ST_STAGES][TY * ST_BP];
+    const int z = blockIdx.z;
+    const float *L = p.B_tab ? p.B_tab[z] : p.B + z * p.sB;  // K x N: X contiguous
+    const float *R = p.A_tab ? p.A_tab[z] : p.A + z * p.sA;  // M x K: K contiguous
+    float *C = p.C_tab ? p.C_tab[z] : p.C + z * p.sC;
+    auto al = [](const void *q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && ld % 4 == 0; };
+    const bool vl = al(L, p.ldb), vr = al(R, p.lda), vc = al(C, p.ldc);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+    const int xl = (warp % WX) * 8 * RPT + (lane & 7) * 4, yl = (warp / WX) * 16 + (lane >> 3);
+    uint64_t acc[RPT / 2][4];
+#pragma unroll
+    for (int i = 0; i < RPT / 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
+    const int nk = (p.K + ST_BK - 1) / ST_BK;
+    auto load = [&](int t) {
+        if (t < nk) {
+            st_load_a<TX>(As[t % ST_STAGES], AP, L, p.ldb, p.N, p.K, x0, t * ST_BK, vl, tid, NT);
+            st_load_b<TY>(Bs[t % ST_STAGES], R, p.lda, p.M, p.K, y0, t * ST_BK, vr, tid, NT);
+        }
+        sf_commit();
+    };
+#pragma unroll
+    for (int t = 0; t < ST_STAGES - 1; t++) load(t);
+    for (int t = 0; t < nk; t++) {
+        sf_wait<ST_STAGES - 2>();
+        __syncthreads();  // stage t has landed for every thread; stage t - 1 is free to refill
+        load(t + ST_STAGES - 1);
+        st_steps<RPT>(acc, As[t % ST_STAGES] + xl, AP, Bs[t % ST_STAGES] + yl * ST_BP, min(ST_BK, p.K - t * ST_BK));
+    }
+    st_store<RPT>(acc, C, p.ldc, p.N, p.M, x0 + xl, y0 + yl, p.alpha, p.beta, vc);
+}
+
 static bool sgemm_pipe_ok(const SgemmArgs &a, int batch) {
     auto al = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     return !a.A_tab && !a.B_tab && !a.C_tab && a.M % SG_BM == 0 && a.N % SG_BN == 0 && a.K % SF_BK == 0 &&
@@ -275,9 +449,27 @@ static bool sgemm_pipe_ok(const SgemmArgs &a, int batch) {
            (batch == 1 || (a.sA % 4 == 0 && a.sB % 4 == 0 && a.sC % 4 == 0));
 }
 
+// Which kernel a plain product runs on, by the measured times (B200, us; small = k_sgemm_small):
+//   aligned, whole 128-tiles   512^3: small 22, pipe 58; 1024^3: 79, 112; 1280^3 (100 tiles): 130,
+//                              140; 1408^3 (121): 177, 152; 4096^3: 3272, 2712 -> the pipe from 112 tiles on
+//   aligned, ragged            577 .. 4100: small at every size (4100^3: 3394 against 3576 of k_sgemm_rm)
+//   unaligned rows             1001^3 (64 tiles): small 97, rm 138; 2047^3 (256): 568, 456 -> rm from
+//                              a tile per SM on (the 4-byte copies)
+// and of the small tiles 64 x 64 from 240 of them on (1000^3: 79 against 79), 64 x 32 below.
+constexpr int SG_PIPE_TILES = 112, ST_WIDE_TILES = 240;
+
 int sgemm_rowmajor(const SgemmArgs &a, int batch, cudaStream_t s, bool ta = false, bool tb = false) {
     if (a.M <= 0 || a.N <= 0 || batch <= 0) return OPB_OK;
-    if (!ta && !tb && sgemm_pipe_ok(a, batch)) {
+    const long long tiles = (long long)((a.M + SG_BM - 1) / SG_BM) * ((a.N + SG_BN - 1) / SG_BN) * batch;
+    const bool pipe = !ta && !tb && sgemm_pipe_ok(a, batch) && tiles >= SG_PIPE_TILES;
+    const bool rows16 = a.lda % 4 == 0 && a.ldb % 4 == 0;
+    if (!ta && !tb && !pipe && (rows16 || tiles < num_sms()) && a.M <= 65535 * 64) {  // (grid rows)
+        const dim3 g64((a.N + 63) / 64, (a.M + 63) / 64, batch);
+        if ((long long)g64.x * g64.y * g64.z >= ST_WIDE_TILES) k_sgemm_small<8, 1, 4><<<g64, 128, 0, s>>>(a);
+        else k_sgemm_small<4, 2, 2><<<dim3(g64.x, (a.M + 31) / 32, batch), 128, 0, s>>>(a);
+        return static_cast<int>(cudaGetLastError());
+    }
+    if (pipe) {
         static bool attr[64] = {false};
         int dev = 0;
         cudaGetDevice(&dev);
@@ -336,45 +528,109 @@ struct Sgemm4Task {
     uint64_t A, B, C;
 };
 
-__global__ void __launch_bounds__(256) k_sgemm4(const uint64_t *argptr_bid) {
-    const Sgemm4Task *tp = reinterpret_cast<const Sgemm4Task *>(argptr_bid[blockIdx.x]);
-    __shared__ Sgemm4Task t;
-    if (threadIdx.x == 0) t = *tp;
+// A block takes four consecutive tasks, a warp each.  Neighbouring tasks of a table mostly share
+// a tile (the same rows of A along by, the same columns of B along bx), so each distinct tile is
+// staged once for the warps that read it; tasks that share nothing stage their own.  What a
+// block computes does not depend on which they share.  (One 64 x 16 tile per 256-thread block,
+// every operand of A from L1: 9.2 TFLOP/s over 40 products of 576^3, 1657 us; now 475.)
+constexpr int S4_TASKS = 4, S4_AP = 64 + 4;
+constexpr int S4_A = ST_BK * S4_AP, S4_B = 16 * ST_BP;   // floats of a left, a right tile
+constexpr int S4_POOL = 2 * S4_TASKS * (S4_A + S4_B);        // two stages without sharing
+static_assert(4 * S4_POOL <= 48 * 1024, "static limit");
+
+__global__ void __launch_bounds__(32 * S4_TASKS) k_sgemm4(const uint64_t *argptr_bid, int ntasks) {
+    __shared__ Sgemm4Task task[S4_TASKS];
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cnt = min(S4_TASKS, ntasks - (int)blockIdx.x * S4_TASKS);
+    if (tid < cnt) task[tid] = *reinterpret_cast<const Sgemm4Task *>(argptr_bid[blockIdx.x * S4_TASKS + tid]);
     __syncthreads();
-    const float *A = reinterpret_cast<const float *>(t.A);
-    const float *B = reinterpret_cast<const float *>(t.B);
-    float *C = reinterpret_cast<float *>(t.C);
-    const int row0 = t.bx * 64, col0 = t.by * 16;
-    // thread -> (row, 4 columns): 64 rows x 4 column groups of 4
-    const int r = threadIdx.x & 63;
-    const int cg = threadIdx.x >> 6;
-    __shared__ float Bs[32][16];
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const int row = row0 + r;
-    for (int k0 = 0; k0 < t.k; k0 += 32) {
-        for (int e = threadIdx.x; e < 32 * 16; e += 256) {
-            int kk = e & 31, cc = e >> 5;
-            int gk = k0 + kk, gc = col0 + cc;
-            Bs[kk][cc] = (gk < t.k && gc < t.n) ? B[(long long)gc * t.k + gk] : 0.f;
-        }
-        __syncthreads();
-        int kmax = min(32, t.k - k0);
-        if (row < t.m) {
-            for (int kk = 0; kk < kmax; kk++) {
-                float a = A[(long long)(k0 + kk) * t.m + row];
+    // the tiles of each task, as offsets (floats) into a stage: those of the first task that has
+    // the same one
+    int oa[S4_TASKS], ob[S4_TASKS], stage = 0, kmax = 0;
+    uint32_t owner = 0;  // bits i, 4 + i: task i stages its own left, right tile
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[j] = fmaf(a, Bs[kk][cg * 4 + j], acc[j]);
+    for (int i = 0; i < S4_TASKS; i++) {
+        oa[i] = ob[i] = 0;
+        if (i >= cnt) continue;
+        const Sgemm4Task &t = task[i];
+        kmax = max(kmax, t.k);
+        int ja = i, jb = i;
+#pragma unroll
+        for (int j = i - 1; j >= 0; j--) {
+            const Sgemm4Task &u = task[j];
+            if (u.A == t.A && u.m == t.m && u.k == t.k && u.bx == t.bx) ja = j;
+            if (u.B == t.B && u.n == t.n && u.k == t.k && u.by == t.by) jb = j;
+        }
+        if (ja == i) {
+            owner |= 1u << i;
+            oa[i] = stage;
+            stage += S4_A;
+        }
+        if (jb == i) {
+            owner |= 16u << i;
+            ob[i] = stage;
+            stage += S4_B;
+        }
+#pragma unroll
+        for (int j = 0; j < S4_TASKS; j++) {  // (registers: no indexing by ja, jb)
+            if (j == ja && j < i) oa[i] = oa[j];
+            if (j == jb && j < i) ob[i] = ob[j];
+        }
+    }
+    auto load = [&](int t, int ns) {
+        const int k0 = t * ST_BK;
+        if (k0 < kmax) {
+            float *st = sm + (t % ns) * stage;
+#pragma unroll
+            for (int i = 0; i < S4_TASKS; i++) {
+                if (i >= cnt || k0 >= task[i].k) continue;
+                const Sgemm4Task &u = task[i];
+                if ((owner >> i) & 1u)
+                    st_load_a<64>(st + oa[i], S4_AP, reinterpret_cast<const float *>(u.A), u.m, u.m, u.k, u.bx * 64, k0,
+                                  u.m % 4 == 0 && u.A % 16 == 0, tid, 32 * S4_TASKS);
+                if ((owner >> (4 + i)) & 1u)
+                    st_load_b<16>(st + ob[i], reinterpret_cast<const float *>(u.B), u.k, u.n, u.k, u.by * 16, k0,
+                                  u.k % 4 == 0 && u.B % 16 == 0, tid, 32 * S4_TASKS);
             }
         }
-        __syncthreads();
-    }
-    if (row < t.m) {
+        sf_commit();
+    };
+    uint64_t acc[4][4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int c = col0 + cg * 4 + j;
-            if (c < t.n) C[(long long)c * t.m + row] = acc[j];
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
+    const bool mine = warp < cnt;
+    const int k = mine ? task[warp].k : 0, xl = (lane & 7) * 4, yl = lane >> 3;
+    int wa = 0, wb = 0;
+#pragma unroll
+    for (int i = 0; i < S4_TASKS; i++)
+        if (i == warp) {
+            wa = oa[i];
+            wb = ob[i];
         }
-    }
+    // as many stages as the block's memory holds of these tiles: four for tasks that share,
+    // two for four strangers
+    auto run = [&](auto depth) {
+        constexpr int NS = decltype(depth)::value;
+#pragma unroll
+        for (int t = 0; t < NS - 1; t++) load(t, NS);
+        for (int t = 0, k0 = 0; k0 < kmax; t++, k0 += ST_BK) {
+            sf_wait<NS - 2>();
+            __syncthreads();
+            load(t + NS - 1, NS);
+            const float *st = sm + (t % NS) * stage;
+            if (k0 < k) st_steps<8>(acc, st + wa + xl, S4_AP, st + wb + yl * ST_BP, min(ST_BK, k - k0));
+        }
+    };
+    if (4 * stage <= S4_POOL) run(std::integral_constant<int, 4>{});
+    else if (3 * stage <= S4_POOL) run(std::integral_constant<int, 3>{});
+    else run(std::integral_constant<int, 2>{});
+    if (!mine) return;
+    const Sgemm4Task &t = task[warp];
+    st_store<8>(acc, reinterpret_cast<float *>(t.C), t.m, t.m, t.n, t.bx * 64 + xl, t.by * 16 + yl, 1.f, 0.f,
+                t.m % 4 == 0 && t.C % 16 == 0);
 }
 
 }  // namespace opb
@@ -428,7 +684,8 @@ OPB_API int opcuda_sgemm4(int nblocks, uint64_t argptr_bid) {
     OPB_REQUIRE(nblocks >= 0, OPB_E_ARG);
     if (nblocks == 0) return set_status(OPB_OK);
     OPB_REQUIRE(argptr_bid != 0, OPB_E_NULL);
-    k_sgemm4<<<nblocks, 256, 0, stream()>>>(reinterpret_cast<const uint64_t *>(argptr_bid));
+    k_sgemm4<<<(nblocks + S4_TASKS - 1) / S4_TASKS, 32 * S4_TASKS, 4 * S4_POOL, stream()>>>(
+        reinterpret_cast<const uint64_t *>(argptr_bid), nblocks);
     return launch_check();
 }
 
