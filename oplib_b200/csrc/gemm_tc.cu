@@ -407,7 +407,9 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     using Cfg = TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>;
     constexpr int EPI = Cfg::EPI_WARPS;
     constexpr int CPT = Cfg::CPT;
-    constexpr bool PLANNED = NPROD == 3 && BK == 64;  // launches that may carry a tile plan
+    // launches that may carry a tile plan: squarings on 64-deep stages, single ones from 128-wide
+    // tiles on (the small kernels stay without the code)
+    constexpr bool PLANNED = NPROD == 3 && BK == 64 && (BATCHED ? FUSE == 1 : BN >= 128);
     constexpr bool OCC = PLANNED && EPIMODE == 0 && FUSE != 2;  // and marks of their blocks
     static_assert(!BMN || (NPROD == 3 && Cfg::B_ROWS % 64 == 0), "MN-major B: split products");
     extern __shared__ uint8_t smem_raw[];
@@ -1847,6 +1849,8 @@ int launch_mlp_fused(long long M, const __nv_bfloat16 *Xp, const __nv_bfloat16 *
     return (int)cudaGetLastError();
 }
 
+static int tile_of(const TcGemmArgs &a) { return a.tile_n && a.N % a.tile_n == 0 ? a.tile_n : tile_for(a.M, a.N, a.ksplit); }
+
 // The epilogue form of a product (the FUSE template parameter of k_tc_gemm).
 static int fuse_of(const TcGemmArgs &a) {
     if (a.fixmode == OPB_FIX_SQUARE || (a.Shi && a.Cin)) return 1;
@@ -1858,7 +1862,7 @@ static int fuse_of(const TcGemmArgs &a) {
 // chain products, in any of the three epilogue forms.
 template <int FUSE>
 static int launch_tc_kn(const TcGemmArgs &a, cudaStream_t s, bool pair) {
-    switch (tile_for(a.M, a.N, a.ksplit) * 2 + (a.f16 ? 1 : 0)) {
+    switch (tile_of(a) * 2 + (a.f16 ? 1 : 0)) {
         case 512:
             if (pair)
                 return g_bk256 == 32 ? launch_tc_pair<false, true, 6, 32, FUSE>(a, s)
@@ -1890,7 +1894,7 @@ int launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s) {
         return launch_tc_kn<0>(a, s, pair);
     }
     if (fuse) return OPB_E_UNSUPPORTED;  // fused epilogues: MN-major B only
-    switch (tile_for(a.M, a.N, a.ksplit) * 2 + (a.f16 ? 1 : 0)) {
+    switch (tile_of(a) * 2 + (a.f16 ? 1 : 0)) {
         case 512:
             if (pair) return launch_tc_pair<false, false>(a, s);
             return g_bk256 == 32 ? launch_tc_impl<256, 4, false, 32>(a, s) : launch_tc_impl<256, 2, false>(a, s);
@@ -1910,6 +1914,7 @@ int launch_tc_gemm(const TcGemmArgs &a, cudaStream_t s) {
 bool tile_plan_for(int d, int &tm, int &tn) {
     if (!g_band_skip || g_bk256 != TC_BK) return false;
     tn = tile_for(d, d);
+    if (tn < 128) return false;  // (products of a wave of 64-wide tiles; see k_tc_gemm's PLANNED)
     tm = g_pair && tn == 256 && d % (2 * TC_BM) == 0 ? 2 * TC_BM : TC_BM;
     return true;
 }

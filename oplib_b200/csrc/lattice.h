@@ -259,6 +259,7 @@ struct TcGemmArgs {
     // bit 1: the FP32 values are not all zero, or have not been so at an earlier level.
     uint8_t *occ;           // optional: written for the output's blocks (bit 0 with Shi)
     const uint8_t *occ_in;  // with a plan: Cin's, blocks without bit 1 hold zeros
+    int tile_n;             // output tile width (64, 128 or 256, dividing N); 0: the launcher's choice
 };
 // Deferred normalisation in the epilogue, with cin_fix[i] = (s_i, inv_i) of the operand
 // rows (E-form: the row sums s of P = I + E' are 1 + s, inv = 1 / (1 + s); P-form: s the row

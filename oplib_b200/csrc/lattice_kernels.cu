@@ -342,6 +342,7 @@ __device__ __forceinline__ void renorm64_apply(RenormSmem &sm, int d, float *__r
 // Column tiles first, first + step, ... of the 64-row strip at r0, through the cp.async
 // ring; the row sums are formed once, while the first tiles are in flight.  Xout (may be
 // null) receives the renormalised values; fix (optional) the per-row (s, inv).
+template <bool MARKS>
 __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, int d, const float *__restrict__ X,
                                                float *__restrict__ Xout, const double *__restrict__ partial,
                                                int nparts, int mode, __nv_bfloat16 *__restrict__ Ahi,
@@ -353,8 +354,8 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
     int cnt = first < nt ? (nt - 1 - first) / step + 1 : 0;
     // under a tile plan the tiles without a mark (off the diagonal) are zero and stay zero, and so
     // are their parts: left alone
-    const bool pick = occ != nullptr && cnt <= RN_LIVE;
-    if (pick) {
+    const bool pick = MARKS && cnt <= RN_LIVE;
+    if (MARKS && pick) {
         if (tid < 32) {
             int n = 0;
             for (int k0 = 0; k0 < cnt; k0 += 32) {
@@ -370,7 +371,7 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
         __syncthreads();
         cnt = sm.nlive;
     }
-    auto col0 = [&](int k) { return (pick ? (int)sm.live[k] : first + k * step) * 64; };
+    auto col0 = [&](int k) { return (MARKS && pick ? (int)sm.live[k] : first + k * step) * 64; };
 #pragma unroll
     for (int k = 0; k < RN_RING - 1; k++) {
         if (k < cnt) renorm64_issue(rg, k, d, X, r0, col0(k));
@@ -386,7 +387,7 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
         cp_async_wait<RN_RING - 1>();  // this thread's copies of tile k have landed
         const int sl = k % RN_RING;
         const float4 v[4] = {rg.v[sl][0][tid], rg.v[sl][1][tid], rg.v[sl][2][tid], rg.v[sl][3][tid]};
-        renorm64_apply(sm, d, Xout, mode, Ahi, Alo, Bhi, Blo, r0, col0(k), sscale, v, b_rm, occ);
+        renorm64_apply(sm, d, Xout, mode, Ahi, Alo, Bhi, Blo, r0, col0(k), sscale, v, b_rm, MARKS ? occ : nullptr);
     }
 }
 
@@ -395,6 +396,7 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
 // to the splits alone); fix (optional) receives the per-row (s, inv), written by the
 // blocks of column chunk 0; b_rm: B parts row-major (else transposed).  Dynamic shared
 // memory RN_SMEM.
+template <bool MARKS>
 __global__ void __launch_bounds__(256) k_renorm64(int d, float *__restrict__ X, const double *__restrict__ partial,
                                                   int nparts, int mode, __nv_bfloat16 *__restrict__ Ahi,
                                                   __nv_bfloat16 *__restrict__ Alo, __nv_bfloat16 *__restrict__ Bhi,
@@ -404,9 +406,9 @@ __global__ void __launch_bounds__(256) k_renorm64(int d, float *__restrict__ X, 
     extern __shared__ __align__(16) uint8_t rn_smem[];
     RenormSmem &sm = *reinterpret_cast<RenormSmem *>(rn_smem);
     RenormRing &rg = *reinterpret_cast<RenormRing *>(rn_smem + sizeof(RenormSmem));
-    renorm64_strip(sm, rg, d, X, write_x ? X : nullptr, partial, nparts, mode, Ahi, Alo, Bhi, Blo,
-                   (int)blockIdx.y * 64, (int)blockIdx.x, (int)gridDim.x, sscale, blockIdx.x == 0 ? fix : nullptr,
-                   b_rm != 0, occ);
+    renorm64_strip<MARKS>(sm, rg, d, X, write_x ? X : nullptr, partial, nparts, mode, Ahi, Alo, Bhi, Blo,
+                          (int)blockIdx.y * 64, (int)blockIdx.x, (int)gridDim.x, sscale, blockIdx.x == 0 ? fix : nullptr,
+                          b_rm != 0, occ);
 }
 
 // Column chunks of a k_renorm64 launch: about 8 blocks per SM in total.
@@ -436,9 +438,14 @@ __global__ void __launch_bounds__(256) k_renorm64_batched(const RenormProblem *_
     const int mode = (int)((w >> 14) & 3u);
     const int nparts = parts_div > 0 ? pr.d / parts_div : 0;
     const int r0 = (int)((w >> 7) & 127u) * 64, chunk = (int)(w & 127u);
-    renorm64_strip(sm, rg, pr.d, pr.X, nullptr, pr.partial, nparts, mode, pr.Ahi, pr.Alo,
+    if (marks)
+        renorm64_strip<true>(sm, rg, pr.d, pr.X, nullptr, pr.partial, nparts, mode, pr.Ahi, pr.Alo,
                    mode == 1 ? pr.Bhi : nullptr, mode == 1 ? pr.Blo : nullptr, r0, chunk, renorm_chunks(pr.d),
-                   sscale, mode == 0 && chunk == 0 ? pr.fix : nullptr, true, marks ? pr.occ : nullptr);
+                   sscale, mode == 0 && chunk == 0 ? pr.fix : nullptr, true, pr.occ);
+    else
+        renorm64_strip<false>(sm, rg, pr.d, pr.X, nullptr, pr.partial, nparts, mode, pr.Ahi, pr.Alo,
+                   mode == 1 ? pr.Bhi : nullptr, mode == 1 ? pr.Blo : nullptr, r0, chunk, renorm_chunks(pr.d),
+                   sscale, mode == 0 && chunk == 0 ? pr.fix : nullptr, true, nullptr);
 }
 
 // Opts both renormalisation kernels into RN_SMEM bytes of dynamic shared memory (once per
@@ -449,7 +456,9 @@ static int renorm64_prepare() {
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return OPB_E_UNSUPPORTED;
     if (!done[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_renorm64, cudaFuncAttributeMaxDynamicSharedMemorySize, RN_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(k_renorm64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RN_SMEM);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_renorm64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RN_SMEM);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_renorm64_batched, cudaFuncAttributeMaxDynamicSharedMemorySize, RN_SMEM);
         if (e != cudaSuccess) return (int)e;
@@ -767,8 +776,9 @@ int launch_renorm(int d, float *X, const double *partial, int nparts, int eform,
                   int write_x, double2 *fix, uint8_t *occ) {
     if (d % 64 == 0 && (Ahi != nullptr) == (Alo != nullptr)) {
         if (int r = renorm64_prepare()) return r;
-        k_renorm64<<<renorm64_grid(d), 256, RN_SMEM, s>>>(d, X, partial, nparts, eform ? 0 : 2, Ahi, Alo, Bhi, Blo,
-                                                          sscale, write_x, eform ? fix : nullptr, 0, occ);
+        auto kern = occ ? k_renorm64<true> : k_renorm64<false>;
+        kern<<<renorm64_grid(d), 256, RN_SMEM, s>>>(d, X, partial, nparts, eform ? 0 : 2, Ahi, Alo, Bhi, Blo, sscale,
+                                                    write_x, eform ? fix : nullptr, 0, occ);
         return (int)cudaGetLastError();
     }
     if (!write_x || fix || occ) return OPB_E_UNSUPPORTED;
@@ -784,7 +794,8 @@ int launch_renorm_to_p(int d, float *X, const double *partial, int nparts, __nv_
                        __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale, const uint8_t *occ) {
     if (d % 64) return OPB_E_UNSUPPORTED;
     if (int r = renorm64_prepare()) return r;
-    k_renorm64<<<renorm64_grid(d), 256, RN_SMEM, s>>>(d, X, partial, nparts, 1, Ahi, Alo, Bhi, Blo, sscale, 1,
+    auto kern = occ ? k_renorm64<true> : k_renorm64<false>;
+    kern<<<renorm64_grid(d), 256, RN_SMEM, s>>>(d, X, partial, nparts, 1, Ahi, Alo, Bhi, Blo, sscale, 1,
                                                       nullptr, 1, const_cast<uint8_t *>(occ));
     return (int)cudaGetLastError();
 }
@@ -1166,7 +1177,7 @@ OPB_API int opb_renorm_rows(int d, float *X, const double *partial, int nparts, 
                     (!Bhi || (opb::aligned(Bhi, 8) && opb::aligned(Blo, 8))),
                 OPB_E_ALIGN);
     if (int r = opb::renorm64_prepare()) return opb::set_status(r);
-    opb::k_renorm64<<<opb::renorm64_grid(d), 256, opb::RN_SMEM, opb::stream()>>>(
+    opb::k_renorm64<false><<<opb::renorm64_grid(d), 256, opb::RN_SMEM, opb::stream()>>>(
         d, X, partial, nparts, mode, reinterpret_cast<__nv_bfloat16 *>(Ahi), reinterpret_cast<__nv_bfloat16 *>(Alo),
         mode == 2 ? nullptr : reinterpret_cast<__nv_bfloat16 *>(Bhi),
         mode == 2 ? nullptr : reinterpret_cast<__nv_bfloat16 *>(Blo), f16 ? 32768.f : 0.f);

@@ -86,13 +86,47 @@ __device__ __forceinline__ float gelu_grad(float z) {
     return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-// Z += b (per column), H = GELU(Z).  Z, H: [B x n] row-major.  H (optional) in FP32 and/or
-// its BF16 parts Hhi / Hlo (optional, for the tensor-core products).
-__global__ void k_bias_gelu(long long total, int n, float *__restrict__ Z, const float *__restrict__ b,
-                            float *__restrict__ H, __nv_bfloat16 *__restrict__ Hhi, __nv_bfloat16 *__restrict__ Hlo) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const float z = Z[i] + b[i % n];
+// A training step is some twenty dependent launches over 4 MB matrices, so what bounds it is the
+// number of launches and the passes between the products: 47 launches took 318 us at B = 4096
+// (228 us of kernels).  Each element-wise pass below therefore writes everything the following
+// products read (the parts, row-major and transposed) and the column sums it passes over (bias,
+// first-layer and output-layer gradients, as partial sums per row block), and one launch at the
+// end adds up all partial sums in a fixed order: 20 launches, 317 -> 164 us.
+
+constexpr int MLP_RB = 16;  // rows per block of the backward element-wise pass (two blocks an SM at B = 4096)
+
+// First layer: Z = X W^T + b (8 inputs, summed in order), H = GELU(Z) in FP32 and/or as parts; thread
+// per column, MLP_RB rows per block.  Blocks from nrow on write the parts of the working weights of
+// the hidden layers (three 256 x 256 matrices from wh, the biases between them) instead.
+__global__ void __launch_bounds__(MLP_H) k_mlp_first(int B, const float *__restrict__ X, const float *__restrict__ W,
+                                                     const float *__restrict__ b, float *__restrict__ Z,
+                                                     float *__restrict__ H, __nv_bfloat16 *__restrict__ Hhi,
+                                                     __nv_bfloat16 *__restrict__ Hlo, int nrow,
+                                                     const float *__restrict__ wh, __nv_bfloat16 *const Wp0h,
+                                                     __nv_bfloat16 *const Wp0l, __nv_bfloat16 *const Wp1h,
+                                                     __nv_bfloat16 *const Wp1l, __nv_bfloat16 *const Wp2h,
+                                                     __nv_bfloat16 *const Wp2l) {
+    const int c = threadIdx.x;
+    if ((int)blockIdx.x >= nrow) {  // a row of a weight matrix
+        const int i = (int)blockIdx.x - nrow, l = i / MLP_H, o = (i % MLP_H) * MLP_H + c;
+        __nv_bfloat16 *hi = l == 0 ? Wp0h : l == 1 ? Wp1h : Wp2h, *lo = l == 0 ? Wp0l : l == 1 ? Wp1l : Wp2l;
+        split2(wh[(long long)l * (MLP_H * MLP_H + MLP_H) + o], hi[o], lo[o]);
+        return;
+    }
+    __shared__ float xs[MLP_RB][MLP_IN];
+    const int r0 = blockIdx.x * MLP_RB, n = min(MLP_RB, B - r0);
+    if (c < n * MLP_IN) xs[c / MLP_IN][c % MLP_IN] = X[(long long)r0 * MLP_IN + c];
+    float w[MLP_IN];
+#pragma unroll
+    for (int k = 0; k < MLP_IN; k++) w[k] = W[c * MLP_IN + k];
+    const float bc = b[c];
+    __syncthreads();
+    for (int r = 0; r < n; r++) {
+        float z = 0.f;
+#pragma unroll
+        for (int k = 0; k < MLP_IN; k++) z = fmaf(xs[r][k], w[k], z);
+        z += bc;
+        const long long i = (long long)(r0 + r) * MLP_H + c;
         Z[i] = z;
         const float h = gelu(z);
         if (H) H[i] = h;
@@ -100,115 +134,248 @@ __global__ void k_bias_gelu(long long total, int n, float *__restrict__ Z, const
     }
 }
 
-// y[r] = H[r, :] . w + b0 (warp per row), and (optional) dy = 2 (y - t) / B, loss partials.
-__global__ void k_out_layer(int B, const float *__restrict__ H, const float *__restrict__ w, const float *__restrict__ b,
-                            float *__restrict__ y, const float *__restrict__ t, float *__restrict__ dy,
-                            double *__restrict__ loss_part) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+// Z += b (per column), H = GELU(Z), four columns a thread.  Z, H: [B x 256] row-major.  H
+// (optional) in FP32 and/or its BF16 parts Hhi / Hlo (optional, for the tensor-core products).
+__global__ void k_bias_gelu(long long total4, float *__restrict__ Z, const float *__restrict__ b,
+                            float *__restrict__ H, __nv_bfloat16 *__restrict__ Hhi, __nv_bfloat16 *__restrict__ Hlo) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= total4) return;
+    const float4 zv = reinterpret_cast<const float4 *>(Z)[i], bv = reinterpret_cast<const float4 *>(b)[i % (MLP_H / 4)];
+    const float z[4] = {zv.x + bv.x, zv.y + bv.y, zv.z + bv.z, zv.w + bv.w};
+    float h[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) h[j] = gelu(z[j]);
+    reinterpret_cast<float4 *>(Z)[i] = make_float4(z[0], z[1], z[2], z[3]);
+    if (H) reinterpret_cast<float4 *>(H)[i] = make_float4(h[0], h[1], h[2], h[3]);
+    if (Hhi) {
+        uint2 hi, lo;
+        split2x2(h[0], h[1], hi.x, lo.x, 0.f);
+        split2x2(h[2], h[3], hi.y, lo.y, 0.f);
+        reinterpret_cast<uint2 *>(Hhi)[i] = hi;
+        reinterpret_cast<uint2 *>(Hlo)[i] = lo;
+    }
+}
+
+// Last hidden layer's bias and GELU with the output layer (warp per row, eight rows per block):
+// Z += b, y = GELU(Z) . w5 + b5, and with targets dy = 2 (y - t) / B and the block's sums of the
+// squared errors and of dy.
+__global__ void __launch_bounds__(256) k_mlp_out(int B, float *__restrict__ Z, const float *__restrict__ b,
+                                                 const float *__restrict__ w5, const float *__restrict__ b5,
+                                                 float *__restrict__ y, const float *__restrict__ t,
+                                                 float *__restrict__ dy, double *__restrict__ loss_part,
+                                                 float *__restrict__ dy_part) {
+    __shared__ double se_s[8];
+    __shared__ float dy_s[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long r = blockIdx.x * 8LL + warp;
     double se = 0.0;
-    if (warp < B) {
-        const float *h = H + (long long)warp * MLP_H;
+    float d = 0.f;
+    if (r < B) {
         float s = 0.f;
-        for (int j = lane; j < MLP_H; j += 32) s = fmaf(h[j], w[j], s);
+#pragma unroll
+        for (int i = 0; i < MLP_H / 32; i++) {
+            const int c = lane + 32 * i;
+            const float z = Z[r * MLP_H + c] + b[c];
+            Z[r * MLP_H + c] = z;
+            s = fmaf(gelu(z), w5[c], s);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        const float v = s + b[0];
-        if (lane == 0) {
-            y[warp] = v;
-            if (t) {
-                const float e = v - t[warp];
-                dy[warp] = 2.f * e / (float)B;
-                se = (double)e * (double)e;
+        const float v = s + b5[0];
+        if (lane == 0) y[r] = v;
+        if (t) {
+            const float e = v - t[r];
+            d = 2.f * e / (float)B;
+            se = (double)e * (double)e;
+            if (lane == 0) dy[r] = d;
+        }
+    }
+    if (!t) return;
+    if (lane == 0) {
+        se_s[warp] = se;
+        dy_s[warp] = d;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = 0.0;
+        float g = 0.f;
+        for (int i = 0; i < 8; i++) {
+            a += se_s[i];
+            g += dy_s[i];
+        }
+        loss_part[blockIdx.x] = a;
+        dy_part[blockIdx.x] = g;
+    }
+}
+
+// Backward element-wise pass of one hidden layer, two columns a thread, MLP_RB rows per block:
+// dZ = dH * GELU'(Z), with dH = dy (outer) w5 for the last layer (dH null).  Writes dZ in FP32
+// (optional), its BF16 parts row-major and transposed ([256 x B]; both or neither, B a multiple of
+// MLP_RB then), and the block's column sums: of dZ into bsum[block][256]; of dy H (last layer, H =
+// GELU(Z) again) into wsum[block][256]; of dZ X (first layer, X non-null) into wsum[block][8][256].
+// Rows past the end read the last one and count as zeros, so that all loads are in flight at once.
+template <bool LAST, bool FIRST>
+__global__ void __launch_bounds__(MLP_H / 2) k_mlp_dz(int B, const float *__restrict__ Z, const float *__restrict__ dH,
+                                                      const float *__restrict__ dy, const float *__restrict__ w5,
+                                                      const float *__restrict__ X, float *__restrict__ dZ,
+                                                      __nv_bfloat16 *__restrict__ Ghi, __nv_bfloat16 *__restrict__ Glo,
+                                                      __nv_bfloat16 *__restrict__ Thi, __nv_bfloat16 *__restrict__ Tlo,
+                                                      float *__restrict__ bsum, float *__restrict__ wsum) {
+    const int c = 2 * threadIdx.x, r0 = blockIdx.x * MLP_RB, n = min(MLP_RB, B - r0);
+    __shared__ float xs[MLP_RB][MLP_IN];
+    if (FIRST) {
+        if ((int)threadIdx.x < n * MLP_IN) xs[threadIdx.x / MLP_IN][threadIdx.x % MLP_IN] = X[(long long)r0 * MLP_IN + threadIdx.x];
+        __syncthreads();
+    }
+    auto at = [&](int r) { return ((long long)r0 + min(r, n - 1)) * MLP_H + c; };
+    float2 g[MLP_RB];
+    float2 sb = make_float2(0.f, 0.f), sw[FIRST ? MLP_IN : 1];
+#pragma unroll
+    for (int k = 0; k < (FIRST ? MLP_IN : 1); k++) sw[k] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < MLP_RB; r++) {
+        if (LAST) {
+            const float d = dy[r0 + min(r, n - 1)];
+            const float2 wc = *reinterpret_cast<const float2 *>(w5 + c);
+            g[r] = make_float2(d * wc.x, d * wc.y);
+        } else {
+            g[r] = *reinterpret_cast<const float2 *>(dH + at(r));
+        }
+    }
+    float2 z[MLP_RB];
+#pragma unroll
+    for (int r = 0; r < MLP_RB; r++) z[r] = *reinterpret_cast<const float2 *>(Z + at(r));
+#pragma unroll
+    for (int r = 0; r < MLP_RB; r++) {
+        const bool in = r < n;
+        if (LAST) {
+            const float d = in ? dy[r0 + r] : 0.f;
+            sw[0].x = fmaf(d, gelu(z[r].x), sw[0].x);
+            sw[0].y = fmaf(d, gelu(z[r].y), sw[0].y);
+        }
+        g[r].x = in ? g[r].x * gelu_grad(z[r].x) : 0.f;
+        g[r].y = in ? g[r].y * gelu_grad(z[r].y) : 0.f;
+        sb.x += g[r].x;
+        sb.y += g[r].y;
+        if (FIRST && in) {
+#pragma unroll
+            for (int k = 0; k < MLP_IN; k++) {
+                sw[k].x = fmaf(g[r].x, xs[r][k], sw[k].x);
+                sw[k].y = fmaf(g[r].y, xs[r][k], sw[k].y);
+            }
+        }
+        if (dZ && in) *reinterpret_cast<float2 *>(dZ + at(r)) = g[r];
+    }
+    if (!FIRST && Ghi) {
+        uint32_t h[2][MLP_RB / 2], l[2][MLP_RB / 2];  // per column, rows in pairs
+#pragma unroll
+        for (int r = 0; r < MLP_RB; r += 2) {
+            const int q = r / 2;
+            split2x2(g[r].x, g[r + 1].x, h[0][q], l[0][q], 0.f);
+            split2x2(g[r].y, g[r + 1].y, h[1][q], l[1][q], 0.f);
+            *reinterpret_cast<uint32_t *>(Ghi + at(r)) = __byte_perm(h[0][q], h[1][q], 0x5410);
+            *reinterpret_cast<uint32_t *>(Glo + at(r)) = __byte_perm(l[0][q], l[1][q], 0x5410);
+            *reinterpret_cast<uint32_t *>(Ghi + at(r + 1)) = __byte_perm(h[0][q], h[1][q], 0x7632);
+            *reinterpret_cast<uint32_t *>(Glo + at(r + 1)) = __byte_perm(l[0][q], l[1][q], 0x7632);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            uint4 *th = reinterpret_cast<uint4 *>(Thi + (long long)(c + u) * B + r0);
+            uint4 *tl = reinterpret_cast<uint4 *>(Tlo + (long long)(c + u) * B + r0);
+#pragma unroll
+            for (int q = 0; q < MLP_RB / 8; q++) {
+                th[q] = make_uint4(h[u][4 * q], h[u][4 * q + 1], h[u][4 * q + 2], h[u][4 * q + 3]);
+                tl[q] = make_uint4(l[u][4 * q], l[u][4 * q + 1], l[u][4 * q + 2], l[u][4 * q + 3]);
             }
         }
     }
-    if (loss_part && lane == 0) atomicAdd(loss_part, se);
-}
-
-// dZ = dH * GELU'(Z); its BF16 parts (optional) row-major too.
-__global__ void k_gelu_back(long long total, const float *__restrict__ Z, const float *__restrict__ dH,
-                            float *__restrict__ dZ, __nv_bfloat16 *__restrict__ dZhi, __nv_bfloat16 *__restrict__ dZlo) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const float g = dH[i] * gelu_grad(Z[i]);
-        dZ[i] = g;
-        if (dZhi) split2(g, dZhi[i], dZlo[i]);
+    *reinterpret_cast<float2 *>(bsum + (long long)blockIdx.x * MLP_H + c) = sb;
+    if (LAST) *reinterpret_cast<float2 *>(wsum + (long long)blockIdx.x * MLP_H + c) = sw[0];
+    if (FIRST) {
+#pragma unroll
+        for (int k = 0; k < MLP_IN; k++)
+            *reinterpret_cast<float2 *>(wsum + ((long long)blockIdx.x * MLP_IN + k) * MLP_H + c) = sw[k];
     }
 }
 
-// First-layer weight gradient dW[c][k] = sum_r dZ[r, c] X[r, k] (n columns, 8 inputs) in the
-// two fixed-order passes of the column sums: block (x, y) forms the 8 sums of its rows for 32
-// columns into part[(y * 8 + k) * n + c]; k_wgrad_in_fin adds the row blocks in order.
-__global__ void k_wgrad_in_part(int B, int n, int rows_per, const float *__restrict__ dZ, const float *__restrict__ X,
-                                float *__restrict__ part) {
-    __shared__ float red[8][MLP_IN][33];
-    const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane, rg = threadIdx.x >> 5;
-    const int r0 = blockIdx.y * rows_per, r1 = min(B, r0 + rows_per);
-    float s[MLP_IN];
-#pragma unroll
-    for (int k = 0; k < MLP_IN; k++) s[k] = 0.f;
-    if (c < n)
-        for (int r = r0 + rg; r < r1; r += 8) {
-            const float g = dZ[(long long)r * n + c];
-#pragma unroll
-            for (int k = 0; k < MLP_IN; k++) s[k] = fmaf(g, X[(long long)r * MLP_IN + k], s[k]);
+// All partial sums of a step into the gradient, in a fixed order.  Blocks [0, 3 * 256): the
+// hidden layers' weight gradients, a row each, over their np[l] slices (np 0: already there); the
+// next ones a row of column sums each, over nb row blocks (four biases, then w5, then the eight
+// first-layer inputs) by four groups of 64 columns; the last one b5 and the loss over no blocks.
+struct MlpFinish {
+    const float *wpart[3];  // [np][256 x 256]
+    int np[3];
+    float *dW[3];
+    const float *bsum[4], *w5sum, *w1sum;  // [nb][256], [nb][256], [nb][8][256]
+    float *db[4], *dw5, *dw1, *db5;
+    int nb;
+    const double *loss_part;
+    const float *dy_part;
+    double *loss;  // optional
+    int no;
+};
+__global__ void __launch_bounds__(256) k_mlp_finish(MlpFinish f) {
+    const int tid = threadIdx.x;
+    int blk = blockIdx.x;
+    if (blk < 3 * MLP_H) {
+        const int l = blk / MLP_H;
+        const long long i = (long long)(blk % MLP_H) * MLP_H + tid;
+        if (f.np[l] == 0) return;
+        float acc = 0.f;
+#pragma unroll 8
+        for (int p = 0; p < f.np[l]; p++) acc += f.wpart[l][(long long)p * MLP_H * MLP_H + i];
+        f.dW[l][i] = acc;
+        return;
+    }
+    blk -= 3 * MLP_H;
+    __shared__ float red[4][64];
+    if (blk < 13 * 4) {
+        const int row = blk / 4, c = (blk % 4) * 64 + (tid & 63), grp = tid >> 6;
+        const float *src;
+        long long step = MLP_H;
+        if (row < 4) src = f.bsum[row];
+        else if (row == 4) src = f.w5sum;
+        else {
+            src = f.w1sum + (long long)(row - 5) * MLP_H;
+            step = (long long)MLP_IN * MLP_H;
         }
-#pragma unroll
-    for (int k = 0; k < MLP_IN; k++) red[rg][k][lane] = s[k];
-    __syncthreads();
-    if (rg == 0 && c < n) {
-        for (int k = 0; k < MLP_IN; k++) {
-            float t = 0.f;
-            for (int i = 0; i < 8; i++) t += red[i][k][lane];
-            part[((long long)blockIdx.y * MLP_IN + k) * n + c] = t;
+        // four contiguous quarters of the row blocks, added in order
+        const int q = (f.nb + 3) / 4, p0 = grp * q, p1 = min(f.nb, p0 + q);
+        float acc = 0.f;
+#pragma unroll 8
+        for (int p = p0; p < p1; p++) acc += src[p * step + c];
+        red[grp][tid & 63] = acc;
+        __syncthreads();
+        if (grp == 0) {
+            const float v = red[0][tid] + red[1][tid] + red[2][tid] + red[3][tid];
+            if (row < 4) f.db[row][c] = v;
+            else if (row == 4) f.dw5[c] = v;
+            else f.dw1[c * MLP_IN + (row - 5)] = v;
         }
+        return;
     }
-}
-
-__global__ void k_wgrad_in_fin(int nb, int n, const float *__restrict__ part, float *__restrict__ dW) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;  // i = c * 8 + k
-    if (i >= n * MLP_IN) return;
-    const int c = i / MLP_IN, k = i - c * MLP_IN;
-    float t = 0.f;
-    for (int b = 0; b < nb; b++) t += part[((long long)b * MLP_IN + k) * n + c];
-    dW[i] = t;
-}
-
-// Weighted column sums over the batch in two fixed-order passes, so that the reduction
-// spreads over many SMs: block (x, y) sums rows [y * rows_per, (y + 1) * rows_per) of 32
-// columns (8 row groups, then in order) into part[y * n + c]; k_colsum_fin adds the row
-// blocks in order.  w (optional): row weights.
-__global__ void k_colsum_part(int B, int n, int rows_per, const float *__restrict__ M, const float *__restrict__ w,
-                              float *__restrict__ part) {
-    __shared__ float red[8][33];
-    const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane, rg = threadIdx.x >> 5;
-    const int r0 = blockIdx.y * rows_per, r1 = min(B, r0 + rows_per);
-    float s = 0.f;
-    if (c < n)
-        for (int r = r0 + rg; r < r1; r += 8) s = w ? fmaf(w[r], M[(long long)r * n + c], s) : s + M[(long long)r * n + c];
-    red[rg][lane] = s;
+    __shared__ double rl[256];
+    __shared__ float rd[256];
+    double a = 0.0;
+    float g = 0.f;
+    for (int p = tid; p < f.no; p += 256) {
+        a += f.loss_part[p];
+        g += f.dy_part[p];
+    }
+    rl[tid] = a;
+    rd[tid] = g;
     __syncthreads();
-    if (rg == 0 && c < n) {
-        float t = 0.f;
-        for (int i = 0; i < 8; i++) t += red[i][lane];
-        part[(long long)blockIdx.y * n + c] = t;
+    for (int o = 128; o > 0; o >>= 1) {
+        if (tid < o) {
+            rl[tid] += rl[tid + o];
+            rd[tid] += rd[tid + o];
+        }
+        __syncthreads();
     }
-}
-
-__global__ void k_colsum_fin(int nb, int n, const float *__restrict__ part, float *__restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    float t = 0.f;
-    for (int b = 0; b < nb; b++) t += part[(long long)b * n + c];
-    out[c] = t;
-}
-
-// dH4 = dy (outer) w5
-__global__ void k_out_back(int B, const float *__restrict__ dy, const float *__restrict__ w, float *__restrict__ dH) {
-    const long long total = (long long)B * MLP_H;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x)
-        dH[i] = dy[i / MLP_H] * w[i % MLP_H];
+    if (tid == 0) {
+        *f.db5 = rd[0];
+        if (f.loss) *f.loss = rl[0];
+    }
 }
 
 // Adam on the FP32 master weights; refreshes the BF16 working copy.
@@ -287,16 +454,20 @@ namespace {
 
 struct MlpWs {  // training workspace carve (floats)
     float *Z[4], *H[4], *dZ, *dH, *y, *dy, *part;
-    double *loss;
+    // partial sums: [nb][256] per layer's bias and for w5, [nb][8][256] for the first layer, [no] per
+    // row block of the output layer
+    float *bsum[4], *w5sum, *w1sum, *dysum;
+    double *lossp;
     // 16-bit parts for the tensor-core products of the hidden layers 1..3 (split2, BF16):
     // Hp[l][0/1] of H[l] (l = 0..2, B x 256 row-major), dZp of dZ (B x 256), dZt of dZ^T
     // (256 x B), Wp[l][0/1] of the working weights W_{l+1} (256 x 256, exact BF16: lo = 0)
     __nv_bfloat16 *Hp[3][2], *dZp[2], *dZt[2], *Wp[3][2];
+    size_t floats;
 };
 
-// Weight gradients reduce over the batch (K = B): split into at most MLP_KSPLIT chunks,
-// one batched SIMT launch over the chunks, then a fixed-order sum of the partials, so
-// that the reduction keeps every SM busy and stays deterministic.
+// Weight gradients reduce over the batch (K = B): split into at most MLP_KSPLIT chunks whose
+// partial products the step's last launch adds in a fixed order, so that the reduction keeps
+// every SM busy and stays deterministic.
 constexpr int MLP_KSPLIT = 32;
 
 int grid_ew(long long n);
@@ -304,34 +475,41 @@ int grid_ew(long long n);
 MlpWs carve_mlp(float *ws, int B) {
     MlpWs w{};
     size_t o = 0;
-    for (int l = 0; l < 4; l++) {
-        w.Z[l] = ws + o; o += (size_t)B * MLP_H;
-        w.H[l] = ws + o; o += (size_t)B * MLP_H;
-    }
-    w.dZ = ws + o; o += (size_t)B * MLP_H;
-    w.dH = ws + o; o += (size_t)B * MLP_H;
-    w.y = ws + o; o += (size_t)B;
-    w.dy = ws + o; o += (size_t)B;
-    o = (o + 3) & ~size_t(3);
-    w.part = ws + o; o += (size_t)MLP_KSPLIT * MLP_H * MLP_H;
-    o = (o + 1) & ~size_t(1);
-    w.loss = reinterpret_cast<double *>(ws + o);
-    o += 2;
-    // parts: 64-float (256-byte) aligned pieces, each n bf16 values in n / 2 floats
-    auto parts = [&](size_t n) {
+    auto take = [&](size_t n) {  // 256-byte aligned pieces
         o = (o + 63) & ~size_t(63);
-        __nv_bfloat16 *q = reinterpret_cast<__nv_bfloat16 *>(ws + o);
-        o += n / 2;
+        float *q = ws + o;
+        o += n;
         return q;
     };
-    const size_t bh = (size_t)B * MLP_H;
+    auto parts = [&](size_t n) { return reinterpret_cast<__nv_bfloat16 *>(take((n + 1) / 2)); };  // n BF16 values
+    const size_t bh = (size_t)B * MLP_H, nb = ((size_t)B + MLP_RB - 1) / MLP_RB, no = ((size_t)B + 7) / 8;
+    for (int l = 0; l < 4; l++) {
+        w.Z[l] = take(bh);
+        w.H[l] = take(bh);
+    }
+    w.dZ = take(bh);
+    w.dH = take(bh);
+    w.y = take(B);
+    w.dy = take(B);
+    w.part = take(3 * (size_t)MLP_KSPLIT * MLP_H * MLP_H);
+    for (int l = 0; l < 4; l++) w.bsum[l] = take(nb * MLP_H);
+    w.w5sum = take(nb * MLP_H);
+    w.w1sum = take(nb * MLP_IN * MLP_H);
+    w.dysum = take(no);
+    w.lossp = reinterpret_cast<double *>(take(2 * no));
     for (int l = 0; l < 3; l++)
         for (int k = 0; k < 2; k++) w.Hp[l][k] = parts(bh);
     for (int k = 0; k < 2; k++) w.dZp[k] = parts(bh);
     for (int k = 0; k < 2; k++) w.dZt[k] = parts(bh);
     for (int l = 0; l < 3; l++)
         for (int k = 0; k < 2; k++) w.Wp[l][k] = parts((size_t)MLP_H * MLP_H);
+    w.floats = o;
     return w;
+}
+
+// The workspace's carve starts at the next 256-byte boundary.
+float *mlp_ws_base(float *ws) {
+    return reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(ws) + 255) & ~uintptr_t(255));
 }
 
 // The hidden layers' products run on the tensor cores (split-BF16, three products, FP32
@@ -343,10 +521,10 @@ bool mlp_tc(int B) { return g_mlp_tc && B % 128 == 0; }
 // C[M x N] = A[M x K] . B^T with A's parts row-major (lda) and B's parts N x K row-major
 // (b_kn = 0) or K x N row-major (b_kn = 1); ksplit > 1: K-slices into C + s * M * N.
 int mlp_tc_gemm(int M, int N, int K, __nv_bfloat16 *const *A, long long lda, __nv_bfloat16 *const *Bp,
-                long long ldb, int b_kn, float *C, int ksplit, cudaStream_t s) {
+                long long ldb, int b_kn, float *C, int ksplit, cudaStream_t s, int tile_n = 0) {
     TcGemmArgs a{};
     a.M = M; a.N = N; a.K = K; a.Ahi = A[0]; a.Alo = A[1]; a.lda = lda; a.Bhi = Bp[0]; a.Blo = Bp[1]; a.ldb = ldb;
-    a.b_kn = b_kn; a.C = C; a.ldc = N; a.alpha = 1.f; a.beta = 0.f;
+    a.b_kn = b_kn; a.C = C; a.ldc = N; a.alpha = 1.f; a.beta = 0.f; a.tile_n = tile_n;
     if (ksplit > 1) {
         a.ksplit = ksplit;
         a.c_slice = (long long)M * N;
@@ -354,43 +532,25 @@ int mlp_tc_gemm(int M, int N, int K, __nv_bfloat16 *const *A, long long lda, __n
     return launch_tc_gemm(a, s);
 }
 
-__global__ void k_sum_parts(int nparts, long long n, const float *__restrict__ part, float *__restrict__ out) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        float acc = 0.f;
-        for (int p = 0; p < nparts; p++) acc += part[p * n + i];
-        out[i] = acc;
-    }
-}
-
-// dW[out x in] = dZ[B x out]^T . in[B x in], split over the batch.
-int mlp_weight_grad(int out, int in, int B, const float *dZ, const float *X, float *dW, float *part,
-                    cudaStream_t s) {
+// Partial products of dW[256 x 256] = dZ[B x 256]^T . in[B x 256], split over the batch, on the
+// SIMT kernels; returns through *np how many.
+int mlp_weight_grad(int B, const float *dZ, const float *in, float *part, int *np, cudaStream_t s) {
     int nch = (B + 63) / 64;
     if (nch > MLP_KSPLIT) nch = MLP_KSPLIT;
     const int kc = (B + nch - 1) / nch;
     const int full = B / kc, rem = B - full * kc;
-    const long long n = (long long)out * in;
+    const long long n = (long long)MLP_H * MLP_H;
     if (full > 0) {
-        int r = sgemm_rm_strided(true, false, out, in, kc, 1.f, dZ, out, (long long)kc * out, X, in,
-                                 (long long)kc * in, 0.f, part, in, n, full, s);
+        int r = sgemm_rm_strided(true, false, MLP_H, MLP_H, kc, 1.f, dZ, MLP_H, (long long)kc * MLP_H, in, MLP_H,
+                                 (long long)kc * MLP_H, 0.f, part, MLP_H, n, full, s);
         if (r) return r;
     }
     if (rem > 0) {
-        int r = sgemm_rm_t(true, false, out, in, rem, 1.f, dZ + (long long)full * kc * out, out,
-                           X + (long long)full * kc * in, in, 0.f, part + (long long)full * n, in, s);
+        int r = sgemm_rm_t(true, false, MLP_H, MLP_H, rem, 1.f, dZ + (long long)full * kc * MLP_H, MLP_H,
+                           in + (long long)full * kc * MLP_H, MLP_H, 0.f, part + (long long)full * n, MLP_H, s);
         if (r) return r;
     }
-    const int np = full + (rem > 0 ? 1 : 0);
-    k_sum_parts<<<grid_ew(n), 256, 0, s>>>(np, n, part, dW);
-    return (int)cudaGetLastError();
-}
-
-// out[c] = sum_r (w[r] *) M[r, c] for c < n over B rows (part: scratch of 32 n floats).
-int mlp_colsum(int B, int n, const float *M, const float *w, float *part, float *out, cudaStream_t s) {
-    const int nb = B < 32 * 128 ? (B + 127) / 128 : 32;
-    const int rows_per = (B + nb - 1) / nb;
-    k_colsum_part<<<dim3((n + 31) / 32, nb), 256, 0, s>>>(B, n, rows_per, M, w, part);
-    k_colsum_fin<<<(n + 255) / 256, 256, 0, s>>>(nb, n, part, out);
+    *np = full + (rem > 0 ? 1 : 0);
     return (int)cudaGetLastError();
 }
 
@@ -406,28 +566,27 @@ int grid_ew(long long n) {
         if (_r) return set_status(_r);    \
     } while (0)
 
+// The forward pass up to the last hidden layer's product (its bias, GELU and the output layer
+// are k_mlp_out's).
 int mlp_forward(const float *thb, const float *X, int B, MlpWs &w, cudaStream_t s) {
     const MlpLayout L = mlp_layout();
     const bool tc = mlp_tc(B);
-    if (tc)
-        for (int l = 1; l < 4; l++)
-            MT(launch_split(MLP_H, MLP_H, thb + L.w[l], MLP_H, w.Wp[l - 1][0], w.Wp[l - 1][1], nullptr, nullptr, 0,
-                            s));
-    const float *in = X;
-    for (int l = 0; l < 4; l++) {
+    const int nrow = (B + MLP_RB - 1) / MLP_RB;
+    // with the tensor cores, layers 0..2 store only their activations' parts (the next
+    // product's A and the weight gradient's B)
+    k_mlp_first<<<nrow + (tc ? 3 * MLP_H : 0), MLP_H, 0, s>>>(
+        B, X, thb + L.w[0], thb + L.b[0], w.Z[0], tc ? nullptr : w.H[0], tc ? w.Hp[0][0] : nullptr,
+        tc ? w.Hp[0][1] : nullptr, nrow, thb + L.w[1], w.Wp[0][0], w.Wp[0][1], w.Wp[1][0], w.Wp[1][1], w.Wp[2][0], w.Wp[2][1]);
+    for (int l = 1; l < 4; l++) {
         // Z = in . W^T  (W stored out x in: the TB form)
-        if (tc && l > 0)
-            MT(mlp_tc_gemm(B, MLP_H, MLP_H, w.Hp[l - 1], MLP_H, w.Wp[l - 1], MLP_H, 0, w.Z[l], 1, s));
+        if (tc) MT(mlp_tc_gemm(B, MLP_H, MLP_H, w.Hp[l - 1], MLP_H, w.Wp[l - 1], MLP_H, 0, w.Z[l], 1, s));
         else
-            MT(sgemm_rm_t(false, true, B, L.out[l], L.in[l], 1.f, in, L.in[l], thb + L.w[l], L.in[l], 0.f, w.Z[l],
-                          L.out[l], s));
-        const long long tot = (long long)B * L.out[l];
-        // with the tensor cores, layers 0..2 store only their activations' parts (the next
-        // product's A and the weight gradient's B); the last one FP32 for the output layer
-        const bool parts = tc && l < 3;
-        k_bias_gelu<<<grid_ew(tot), 256, 0, s>>>(tot, L.out[l], w.Z[l], thb + L.b[l], parts ? nullptr : w.H[l],
-                                                 parts ? w.Hp[l][0] : nullptr, parts ? w.Hp[l][1] : nullptr);
-        in = w.H[l];
+            MT(sgemm_rm_t(false, true, B, MLP_H, MLP_H, 1.f, w.H[l - 1], MLP_H, thb + L.w[l], MLP_H, 0.f, w.Z[l], MLP_H,
+                          s));
+        if (l == 3) break;
+        const long long t4 = (long long)B * MLP_H / 4;
+        k_bias_gelu<<<(unsigned)((t4 + 255) / 256), 256, 0, s>>>(t4, w.Z[l], thb + L.b[l], tc ? nullptr : w.H[l],
+                                                                 tc ? w.Hp[l][0] : nullptr, tc ? w.Hp[l][1] : nullptr);
     }
     return (int)cudaGetLastError();
 }
@@ -438,10 +597,8 @@ OPB_API int opb_mlp_param_count(void) { return MLP_NPARAM; }
 
 // floats of training workspace for batch B
 OPB_API long long opb_mlp_workspace_floats(int B) {
-    // FP32 buffers, then the tensor-core parts (5 B x 256 + 3 x 256 x 256 floats of BF16 pairs)
-    // with their alignment
-    return 10LL * B * MLP_H + 2LL * B + 4 + (long long)MLP_KSPLIT * MLP_H * MLP_H + 8 + 5LL * B * MLP_H +
-           3LL * MLP_H * MLP_H + 14 * 64;
+    if (B <= 0) return 0;
+    return (long long)carve_mlp(nullptr, B).floats + 64;  // (+ the alignment of its base)
 }
 
 // 1 (default): the hidden layers' training products on the tensor cores (batches of a
@@ -467,76 +624,72 @@ OPB_API int opb_mlp_round(const float *theta, float *theta_bf, void *theta_b16) 
 }
 
 // Forward pass of B rows of X [B x 8] with the working weights thb; y [B].  The workspace
-// keeps the pre-activations for a following opb_mlp_backward.
+// keeps the pre-activations.
 OPB_API int opb_mlp_forward(const float *thb, const float *X, int B, float *ws, float *y) {
     OPB_REQUIRE(thb && X && ws && y, OPB_E_NULL);
     OPB_REQUIRE(B > 0, OPB_E_ARG);
-    MlpWs w = carve_mlp(ws, B);
+    MlpWs w = carve_mlp(mlp_ws_base(ws), B);
     cudaStream_t s = stream();
     MT(mlp_forward(thb, X, B, w, s));
     const MlpLayout L = mlp_layout();
-    k_out_layer<<<(B * 32 + 255) / 256, 256, 0, s>>>(B, w.H[3], thb + L.w[4], thb + L.b[4], y, nullptr, nullptr,
-                                                      nullptr);
+    k_mlp_out<<<(B + 7) / 8, 256, 0, s>>>(B, w.Z[3], thb + L.b[3], thb + L.w[4], thb + L.b[4], y, nullptr, nullptr,
+                                          nullptr, nullptr);
     return launch_check();
 }
 
-// Loss (mean squared error against t) and its gradient with respect to the working weights,
-// written into grad [param count].  loss (device, 1 double, optional) receives the mean.
+// Loss (sum of squared errors against t) and the gradient of the mean squared error with respect
+// to the working weights, written into grad [param count].  loss: device, 1 double, optional.
 OPB_API int opb_mlp_loss_grad(const float *thb, const float *X, const float *t, int B, float *ws, float *grad,
                               double *loss) {
     OPB_REQUIRE(thb && X && t && ws && grad, OPB_E_NULL);
     OPB_REQUIRE(B > 0, OPB_E_ARG);
-    MlpWs w = carve_mlp(ws, B);
+    MlpWs w = carve_mlp(mlp_ws_base(ws), B);
     cudaStream_t s = stream();
     const MlpLayout L = mlp_layout();
     MT(mlp_forward(thb, X, B, w, s));
-    MT((int)cudaMemsetAsync(w.loss, 0, sizeof(double), s));
-    k_out_layer<<<(B * 32 + 255) / 256, 256, 0, s>>>(B, w.H[3], thb + L.w[4], thb + L.b[4], w.y, t, w.dy, w.loss);
-    // output layer
-    // (column sums over the batch in two fixed-order passes over many blocks)
-    MT(mlp_colsum(B, MLP_H, w.H[3], w.dy, w.part, grad + L.w[4], s));
-    MT(mlp_colsum(B, 1, w.dy, nullptr, w.part, grad + L.b[4], s));
-    k_out_back<<<grid_ew((long long)B * MLP_H), 256, 0, s>>>(B, w.dy, thb + L.w[4], w.dH);
+    const int no = (B + 7) / 8, nb = (B + MLP_RB - 1) / MLP_RB;
+    k_mlp_out<<<no, 256, 0, s>>>(B, w.Z[3], thb + L.b[3], thb + L.w[4], thb + L.b[4], w.y, t, w.dy, w.lossp, w.dysum);
     const bool tc = mlp_tc(B);
-    // weight-gradient K-slices on the tensor cores: at most MLP_KSPLIT, dividing B / 64
-    int ks = B / 64 < MLP_KSPLIT ? B / 64 : MLP_KSPLIT;
+    // weight-gradient K-slices on the tensor cores: at most 16, dividing B / 64.  Sixteen slices of
+    // 128 x 64 tiles are 128 CTAs; with 32 slices of 128 x 256 ones (64 CTAs) the output phase of
+    // the wide tile was most of the launch
+    int ks = B / 64 < MLP_KSPLIT / 2 ? B / 64 : MLP_KSPLIT / 2;
     while (ks > 1 && (B / 64) % ks) ks--;
-    for (int l = 3; l >= 0; l--) {
-        const long long tot = (long long)B * L.out[l];
-        const bool parts = tc && l > 0;
-        k_gelu_back<<<grid_ew(tot), 256, 0, s>>>(tot, w.Z[l], w.dH, w.dZ, parts ? w.dZp[0] : nullptr,
-                                                 parts ? w.dZp[1] : nullptr);
-        const float *in = l > 0 ? w.H[l - 1] : X;
-        if (parts) {
-            // dZ's parts transposed (for dW; the row-major ones, for dH, came with dZ)
-            MT(launch_split(B, MLP_H, w.dZ, MLP_H, nullptr, nullptr, w.dZt[0], w.dZt[1], B, s));
-            // dW = dZ^T . in: A = dZ^T's parts (256 x B), B = in's parts read K x N (B x 256)
-            MT(mlp_tc_gemm(MLP_H, MLP_H, B, w.dZt, B, w.Hp[l - 1], MLP_H, 1, w.part, ks, s));
-            k_sum_parts<<<grid_ew((long long)MLP_H * MLP_H), 256, 0, s>>>(ks, (long long)MLP_H * MLP_H, w.part,
-                                                                          grad + L.w[l]);
-        } else if (l == 0) {
-            // dW = dZ^T . X (8 inputs): eight weighted column sums
-            const int nb = B < 32 * 128 ? (B + 127) / 128 : 32;
-            const int rows_per = (B + nb - 1) / nb;
-            k_wgrad_in_part<<<dim3(MLP_H / 32, nb), 256, 0, s>>>(B, MLP_H, rows_per, w.dZ, X, w.part);
-            k_wgrad_in_fin<<<(MLP_H * MLP_IN + 255) / 256, 256, 0, s>>>(nb, MLP_H, w.part, grad + L.w[0]);
+    MlpFinish f{};
+    for (int l = 3; l >= 1; l--) {
+        float *dZ = tc ? nullptr : w.dZ;
+        __nv_bfloat16 *gh = tc ? w.dZp[0] : nullptr, *gl = tc ? w.dZp[1] : nullptr;
+        if (l == 3) {
+            // (with SIMT products the last activations are wanted in FP32 by nobody but this pass)
+            k_mlp_dz<true, false><<<nb, MLP_H / 2, 0, s>>>(B, w.Z[3], nullptr, w.dy, thb + L.w[4], nullptr, dZ, gh, gl, w.dZt[0],
+                                                       w.dZt[1], w.bsum[3], w.w5sum);
         } else {
-            // dW = dZ^T . in  (A = dZ stored B x out: the TA form)
-            MT(mlp_weight_grad(L.out[l], L.in[l], B, w.dZ, in, grad + L.w[l], w.part, s));
+            k_mlp_dz<false, false><<<nb, MLP_H / 2, 0, s>>>(B, w.Z[l], w.dH, nullptr, nullptr, nullptr, dZ, gh, gl, w.dZt[0],
+                                                        w.dZt[1], w.bsum[l], nullptr);
         }
-        MT(mlp_colsum(B, L.out[l], w.dZ, nullptr, w.part, grad + L.b[l], s));
-        if (l > 0) {
+        float *part = w.part + (size_t)(l - 1) * MLP_KSPLIT * MLP_H * MLP_H;
+        f.wpart[l - 1] = part;
+        f.dW[l - 1] = grad + L.w[l];
+        if (tc) {
+            // dW = dZ^T . in: A = dZ^T's parts (256 x B), B = in's parts read K x N (B x 256);
             // dH = dZ . W: B = W's parts read K x N (out x in)
-            if (tc) MT(mlp_tc_gemm(B, MLP_H, MLP_H, w.dZp, MLP_H, w.Wp[l - 1], MLP_H, 1, w.dH, 1, s));
-            else
-                MT(sgemm_rm_t(false, false, B, L.in[l], L.out[l], 1.f, w.dZ, L.out[l], thb + L.w[l], L.in[l], 0.f,
-                              w.dH, L.in[l], s));
+            f.np[l - 1] = ks;
+            MT(mlp_tc_gemm(MLP_H, MLP_H, B, w.dZt, B, w.Hp[l - 1], MLP_H, 1, part, ks, s, 64));
+            MT(mlp_tc_gemm(B, MLP_H, MLP_H, w.dZp, MLP_H, w.Wp[l - 1], MLP_H, 1, w.dH, 1, s));
+        } else {
+            MT(mlp_weight_grad(B, w.dZ, w.H[l - 1], part, &f.np[l - 1], s));
+            MT(sgemm_rm_t(false, false, B, MLP_H, MLP_H, 1.f, w.dZ, MLP_H, thb + L.w[l], MLP_H, 0.f, w.dH, MLP_H, s));
         }
     }
-    if (loss) {
-        // mean of the squared errors
-        MT((int)cudaMemcpyAsync(loss, w.loss, sizeof(double), cudaMemcpyDeviceToDevice, s));
+    k_mlp_dz<false, true><<<nb, MLP_H / 2, 0, s>>>(B, w.Z[0], w.dH, nullptr, nullptr, X, nullptr, nullptr, nullptr, nullptr,
+                                               nullptr, w.bsum[0], w.w1sum);
+    for (int l = 0; l < 4; l++) {
+        f.bsum[l] = w.bsum[l];
+        f.db[l] = grad + L.b[l];
     }
+    f.w5sum = w.w5sum; f.w1sum = w.w1sum; f.dw5 = grad + L.w[4]; f.dw1 = grad + L.w[0]; f.db5 = grad + L.b[4];
+    f.nb = nb; f.loss_part = w.lossp; f.dy_part = w.dysum; f.loss = loss; f.no = no;
+    k_mlp_finish<<<3 * MLP_H + 13 * 4 + 1, 256, 0, s>>>(f);
     return launch_check();
 }
 
