@@ -43,6 +43,38 @@ struct NvtxRange {
     NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
+// Programmatic dependent launch.  A kernel launched by launch_pdl may be set up (its launch, and
+// what it does before pdl_wait) while the kernel before it in the stream still runs; pdl_wait
+// returns once that kernel has completed and its writes are visible, so every thread of a kernel
+// launched this way calls it before it touches global memory.  pdl_next lets the kernel's own
+// successor be set up in turn, once all its blocks have called it or ended.  It stands after the
+// wait, so that one successor at most is resident and order stays transitive, and after the
+// block's tensor memory is allocated: a successor may sit on tensor memory while it waits for
+// this kernel, which therefore must not still be asking for its own.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() {
+    pdl_wait();
+    pdl_next();
+}
+
+template <class... P, class... A>
+inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
+
 }  // namespace opb
 
 #define OPB_NVTX(name) opb::NvtxRange opb_nvtx_range_(name)

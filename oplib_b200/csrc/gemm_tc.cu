@@ -434,7 +434,6 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     const int mtiles = p.M / Cfg::TILE_M, ntiles_n = p.N / BN;
     const int nsplit = (!BATCHED && p.ksplit > 1) ? p.ksplit : 1;  // K-slices of a single product
     int nitems = BATCHED ? bt.nwork : mtiles * ntiles_n * nsplit;
-    if (PLANNED && p.kmask) nitems = (int)*p.nlist;  // the plan leaves out the tiles with nothing to do
     // pair mode: rank within the 2-CTA cluster, items walked per cluster
     const uint32_t rank = PAIR ? cluster_rank() : 0u;
     const int item0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
@@ -533,6 +532,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     float *svec = reinterpret_cast<float *>(gbase + Cfg::RING_BYTES + 256 + Cfg::OUT_BYTES);
     const bool vec_smem = EPIMODE != 0 && p.N == BN;
     if (vec_smem) {
+        pdl_wait();
         for (int i = threadIdx.x; i < BN; i += blockDim.x) {
             svec[i] = p.bias[i];
             if (EPIMODE == 2) svec[BN + i] = p.w5[i];
@@ -543,6 +543,8 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers initialised before any cross-CTA signal
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (!vec_smem) pdl_wait();  // (barriers and tensor memory are set up while the kernel before runs)
+    if (PLANNED && p.kmask) nitems = (int)*p.nlist;  // the plan leaves out the tiles with nothing to do
 
     if (warp >= EPI) {
         if constexpr (Cfg::REGSPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_REST));
@@ -628,6 +630,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     kbg++;
                 }
             }
+            pdl_next();  // nothing left to load: the next kernel may be set up
             if (!ok) {
                 atomicExch(&g_tc_error, 1);
                 *abort_flag = 1;
@@ -1346,8 +1349,8 @@ static int launch_tc_impl(const TcGemmArgs &a, cudaStream_t s) {
     const int ntiles = (a.M / TC_BM) * (a.N / BN) * p.ksplit;
     const int grid = ntiles < num_sms() ? ntiles : num_sms();
     TcBatch none{nullptr, nullptr, nullptr, 0};
-    k_tc_gemm<BN, STAGES, false, F16, 3, 0, BK, false, BMN, FUSE><<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(
-        mAh, mAl, mBh, mBl, p, none);
+    launch_pdl(k_tc_gemm<BN, STAGES, false, F16, 3, 0, BK, false, BMN, FUSE>, grid, Cfg::THREADS, Cfg::SMEM, s, mAh,
+               mAl, mBh, mBl, p, none);
     return (int)cudaGetLastError();
 }
 
@@ -1381,7 +1384,9 @@ static int launch_tc_pair(const TcGemmArgs &a, cudaStream_t s) {
     p.occ = a.occ;
     p.occ_in = a.occ_in;
     TcBatch none{nullptr, nullptr, nullptr, 0};
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2;
     at[0].val.clusterDim.y = 1;
@@ -1404,6 +1409,7 @@ static int launch_tc_pair(const TcGemmArgs &a, cudaStream_t s) {
         if (n <= 0) return OPB_E_UNSUPPORTED;
         max_clusters[dev] = n;
     }
+    cfg.numAttrs = 2;
     const int ntiles = (a.M / (2 * TC_BM)) * (a.N / BN);
     const int nclusters = ntiles < max_clusters[dev] ? ntiles : max_clusters[dev];
     cfg.gridDim = dim3(2 * nclusters);
@@ -1426,6 +1432,12 @@ int tc_make_maps(CUtensorMap *out4, const __nv_bfloat16 *Ahi, const __nv_bfloat1
     return OPB_OK;
 }
 
+// A batched launch overlaps its set-up with the kernel before it up to this many items per CTA
+// (or pair); longer lists gain nothing from it (56 lattices of 256 to 640 states, under 10 items
+// a CTA: 1406 us a calibration pass with, 1446 without; 256 lattices up to 2048 states, 94 items
+// a pair: 15.13 ms with it, 15.09 without).
+constexpr int TC_PDL_ITEMS = 64;
+
 template <int BN, int STAGES, bool F16, bool BMN, int FUSE>
 static int launch_batched_impl(const CUtensorMap *maps, const TcProblem *probs, const uint32_t *work, int nwork,
                                int grid, cudaStream_t s, const TcBatchArgs &b) {
@@ -1442,8 +1454,9 @@ static int launch_batched_impl(const CUtensorMap *maps, const TcProblem *probs, 
     p.sscale = b.sscale;
     set_plan(p, b.plan);
     TcBatch bt{maps, probs, work, nwork};
-    k_tc_gemm<BN, STAGES, true, F16, 3, 0, TC_BK, false, BMN, FUSE><<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(
-        dummy, dummy, dummy, dummy, p, bt);
+    auto kern = k_tc_gemm<BN, STAGES, true, F16, 3, 0, TC_BK, false, BMN, FUSE>;
+    if (nwork <= TC_PDL_ITEMS * grid) launch_pdl(kern, grid, Cfg::THREADS, Cfg::SMEM, s, dummy, dummy, dummy, dummy, p, bt);
+    else kern<<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(dummy, dummy, dummy, dummy, p, bt);
     return (int)cudaGetLastError();
 }
 
@@ -1460,7 +1473,9 @@ static int launch_batched_pair_impl(const CUtensorMap *maps, const TcProblem *pr
     auto kern = k_tc_gemm<BN, STAGES, true, F16, 3, 0, TC_BK, true, BMN, FUSE>;
     int e0 = set_smem_attr<BN, STAGES, true, F16, 3, 0, TC_BK, true, BMN, FUSE>();
     if (e0) return e0;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2;
     at[0].val.clusterDim.y = 1;
@@ -1484,6 +1499,7 @@ static int launch_batched_pair_impl(const CUtensorMap *maps, const TcProblem *pr
         max_clusters[dev] = n;
     }
     const int ncl = nwork < max_clusters[dev] ? nwork : max_clusters[dev];
+    cfg.numAttrs = nwork <= TC_PDL_ITEMS * ncl ? 2 : 1;
     cfg.gridDim = dim3(2 * ncl);
     CUtensorMap dummy;
     std::memset(&dummy, 0, sizeof(dummy));
@@ -1562,9 +1578,11 @@ int launch_tc_layer(int M, int N, int K, const __nv_bfloat16 *A, long long lda, 
     const int grid = ntiles < num_sms() ? ntiles : num_sms();
     TcBatch none{nullptr, nullptr, nullptr, 0};
     if (fused)
-        k_tc_gemm<BN, STAGES, false, false, 1, 2><<<grid, Cfg2::THREADS, Cfg2::SMEM, s>>>(mA, mA, mW, mW, p, none);
+        launch_pdl(k_tc_gemm<BN, STAGES, false, false, 1, 2>, grid, Cfg2::THREADS, Cfg2::SMEM, s, mA, mA, mW, mW, p,
+                   none);
     else
-        k_tc_gemm<BN, STAGES, false, false, 1, 1><<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(mA, mA, mW, mW, p, none);
+        launch_pdl(k_tc_gemm<BN, STAGES, false, false, 1, 1>, grid, Cfg::THREADS, Cfg::SMEM, s, mA, mA, mW, mW, p,
+                   none);
     return (int)cudaGetLastError();
 }
 
@@ -1648,11 +1666,13 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    pdl_wait();
     for (int i = threadIdx.x; i < 5 * 256; i += blockDim.x) svec[i] = p.vec[i];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_next();
 
     // The steps (tile j of this CTA, layer l) in MMA order: pairs of tiles, layer by layer,
     // the pair's two tiles alternating; tile j lives in slot j & 1 as that slot's use j >> 1.
@@ -1845,7 +1865,7 @@ int launch_mlp_fused(long long M, const __nv_bfloat16 *Xp, const __nv_bfloat16 *
     FmParams p{M, vec, ypart};
     const long long ntiles = M / TC_BM;
     const int grid = ntiles < num_sms() ? (int)ntiles : num_sms();
-    k_mlp_fused<<<grid, FM_THREADS, FM_SMEM, s>>>(mX, mW1, mWH, p);
+    launch_pdl(k_mlp_fused, grid, FM_THREADS, FM_SMEM, s, mX, mW1, mWH, p);
     return (int)cudaGetLastError();
 }
 

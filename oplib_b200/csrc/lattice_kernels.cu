@@ -27,6 +27,7 @@
 namespace opb {
 
 __global__ void k_zero_set_diag(int d, float *__restrict__ U, float v) {
+    pdl_begin();
     int y = blockIdx.x * blockDim.x + threadIdx.x;
     if (y < d) U[(long long)y * d + y] = v;
 }
@@ -41,6 +42,7 @@ __device__ __forceinline__ void e0_parts(const E0Parts &p, long long y, int z, l
 // ELL generator: row y holds w (col, val) pairs; col < 0 marks padding.
 __global__ void k_ek_scatter_ell(int d, int w, const int *__restrict__ cols, const double *__restrict__ vals,
                                  double dt, int eform, float *__restrict__ out, long long ld, E0Parts parts) {
+    pdl_begin();
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)d * w) return;
     int y = (int)(t / w);
@@ -55,6 +57,7 @@ __global__ void k_ek_scatter_ell(int d, int w, const int *__restrict__ cols, con
 // Half-bandwidth of an ELL generator: max |col - row| over its entries (padding excluded),
 // by one block.  The squarings read it to leave out the K-blocks that multiply zeros.
 __global__ void __launch_bounds__(1024) k_ell_band(int d, int w, const int *__restrict__ cols, int *__restrict__ out) {
+    pdl_begin();
     __shared__ int wmax[32];
     int m = 0;
     const long long n = (long long)d * w;
@@ -77,6 +80,7 @@ __global__ void __launch_bounds__(1024) k_ell_band(int d, int w, const int *__re
 // Dense FP64 generator, row-major (source-major), into rows of leading dimension ld.
 __global__ void k_ek_dense(int d, const double *__restrict__ L, double dt, int eform, float *__restrict__ out,
                            long long ld) {
+    pdl_begin();
     long long n = (long long)d * d;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
          t += (long long)gridDim.x * blockDim.x) {
@@ -89,6 +93,7 @@ __global__ void k_ek_dense(int d, const double *__restrict__ L, double dt, int e
 
 // Spot values of a lattice padded with absorbing states: xpad[i] = x[min(i, d - 1)].
 __global__ void k_pad_x(int d, int dpad, const double *__restrict__ x, double *__restrict__ xpad) {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < dpad) xpad[i] = x[i < d ? i : d - 1];
 }
@@ -99,6 +104,7 @@ __global__ void k_split_tr(int rows, int cols, const float *__restrict__ X, long
                            __nv_bfloat16 *__restrict__ Ahi, __nv_bfloat16 *__restrict__ Alo,
                            __nv_bfloat16 *__restrict__ Bhi, __nv_bfloat16 *__restrict__ Blo, long long ldt,
                            float sscale) {
+    pdl_begin();
     __shared__ __nv_bfloat16 th[32][34], tl[32][34];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
@@ -130,6 +136,7 @@ __global__ void k_split_tr(int rows, int cols, const float *__restrict__ X, long
 
 // FP64 row sums of an FP32 matrix, one block per row -> partial[row].
 __global__ void k_rowsum(int d, const float *__restrict__ X, double *__restrict__ partial) {
+    pdl_begin();
     const int y = blockIdx.x;
     const float *row = X + (long long)y * d;
     double s = 0.0;
@@ -153,6 +160,7 @@ __global__ void k_rowsum(int d, const float *__restrict__ X, double *__restrict_
 __global__ void k_renorm(int d, float *__restrict__ X, const double *__restrict__ partial, int nparts, int eform,
                          __nv_bfloat16 *__restrict__ Ahi, __nv_bfloat16 *__restrict__ Alo,
                          __nv_bfloat16 *__restrict__ Bhi, __nv_bfloat16 *__restrict__ Blo, float sscale) {
+    pdl_begin();
     __shared__ double s_sum[32], s_inv[32];
     __shared__ __nv_bfloat16 th[32][34], tl[32][34];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -400,9 +408,10 @@ template <bool MARKS>
 __global__ void __launch_bounds__(256) k_renorm64(int d, float *__restrict__ X, const double *__restrict__ partial,
                                                   int nparts, int mode, __nv_bfloat16 *__restrict__ Ahi,
                                                   __nv_bfloat16 *__restrict__ Alo, __nv_bfloat16 *__restrict__ Bhi,
-                                                  __nv_bfloat16 *__restrict__ Blo, float sscale, int write_x = 1,
-                                                  double2 *__restrict__ fix = nullptr, int b_rm = 0,
-                                                  uint8_t *__restrict__ occ = nullptr) {
+                                                  __nv_bfloat16 *__restrict__ Blo, float sscale, int write_x,
+                                                  double2 *__restrict__ fix, int b_rm,
+                                                  uint8_t *__restrict__ occ) {
+    pdl_begin();
     extern __shared__ __align__(16) uint8_t rn_smem[];
     RenormSmem &sm = *reinterpret_cast<RenormSmem *>(rn_smem);
     RenormRing &rg = *reinterpret_cast<RenormRing *>(rn_smem + sizeof(RenormSmem));
@@ -530,6 +539,7 @@ __global__ void k_row_quotes_batched(const BatchLattice *__restrict__ lats, cons
 }
 
 __global__ void k_rowfix(int d, const double *__restrict__ partial, int nparts, int eform, double2 *__restrict__ fix) {
+    pdl_begin();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < d) fix[r] = row_fix(partial, d, nparts, r, eform);
 }
@@ -553,6 +563,7 @@ __global__ void k_rowfix_batched(const BatchLattice *__restrict__ lats, int nlat
 
 // E-form -> P-form: P = I + E (in place), FP32.
 __global__ void k_add_identity(int d, float *__restrict__ X) {
+    pdl_begin();
     int y = blockIdx.x * blockDim.x + threadIdx.x;
     if (y < d) {
         long long o = (long long)y * d + y;
@@ -566,6 +577,7 @@ __global__ void k_add_identity(int d, float *__restrict__ X) {
 __global__ void k_payoff(int d, int nK, int ldk, const double *__restrict__ x, const double *__restrict__ K,
                          float *__restrict__ G, __nv_bfloat16 *__restrict__ GThi, __nv_bfloat16 *__restrict__ GTlo,
                          const float *__restrict__ dscale) {
+    pdl_begin();
     const float sscale = dscale ? *dscale : 0.f;
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)d * ldk) return;
@@ -593,6 +605,7 @@ __device__ __forceinline__ double sum_slices(const float *__restrict__ P, long l
 __global__ void k_discount(int d, int nK, int ldk, const float *__restrict__ V32, double disc,
                            double *__restrict__ V64, int y0, double *__restrict__ quotes, const float *__restrict__ dscale,
                            int nslice, long long slice_stride, const double2 *__restrict__ rowfix) {
+    pdl_begin();
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)d * nK) return;
     int y = (int)(t / nK), k = (int)(t - (long long)y * nK);
@@ -607,6 +620,7 @@ __global__ void k_discount(int d, int nK, int ldk, const float *__restrict__ V32
 __global__ void k_row_quotes(int nm, int m0, int nK, int ldk, const float *__restrict__ V, double rate, double period,
                              const double *__restrict__ qinv, const float *__restrict__ dscale, int nslice,
                              long long slice_stride, double *__restrict__ quotes) {
+    pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nm * nK) return;
     const int i = t / nK, k = t - i * nK;
@@ -632,6 +646,7 @@ __device__ __forceinline__ double berm_exercise(double x, double K, int put) {
 // largest exercise value (max x - min K for calls, max K - min x for puts).
 __global__ void k_berm_scale(int d, const double *__restrict__ x, int nK, const double *__restrict__ K, int put,
                              float *__restrict__ out) {
+    pdl_begin();
     __shared__ double s0[256], s1[256];
     double a = -1e300, b = 1e300;  // calls: max x, min K; puts: max K, min x
     for (int i = threadIdx.x; i < d; i += blockDim.x) {
@@ -665,6 +680,7 @@ __global__ void k_berm_scale(int d, const double *__restrict__ x, int nK, const 
 __global__ void k_berm_init(int d, int nK, int ldk, const double *__restrict__ x, const double *__restrict__ K,
                             int put, double barrier, double *__restrict__ V, __nv_bfloat16 *__restrict__ Vhi,
                             __nv_bfloat16 *__restrict__ Vlo, float *__restrict__ Vf, const float *__restrict__ dscale) {
+    pdl_begin();
     const float sscale = dscale ? *dscale : 0.f;
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)d * ldk) return;
@@ -690,6 +706,7 @@ __global__ void k_berm_step(int d, int nK, int ldk, const float *__restrict__ C,
                             int exercise, double *__restrict__ V, __nv_bfloat16 *__restrict__ Vhi,
                             __nv_bfloat16 *__restrict__ Vlo, float *__restrict__ Vf, const float *__restrict__ dscale,
                             int y0, double *__restrict__ quotes, int nslice, long long slice_stride) {
+    pdl_begin();
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)d * ldk) return;
     const int z = (int)(t / ldk), k = (int)(t - (long long)z * ldk);
@@ -720,14 +737,15 @@ int launch_ek_ell(int d, int w, const int *cols, const double *vals, double dt, 
                   cudaStream_t s, const E0Parts &parts) {
     cudaError_t e = cudaMemsetAsync(out, 0, sizeof(float) * (size_t)d * d, s);
     if (e != cudaSuccess) return (int)e;
-    if (!eform) k_zero_set_diag<<<blocks_for(d, 256), 256, 0, s>>>(d, out, 1.0f);
+    if (!eform) launch_pdl(k_zero_set_diag, blocks_for(d, 256), 256, 0, s, d, out, 1.0f);
     long long n = (long long)d * w;
-    if (n > 0) k_ek_scatter_ell<<<blocks_for(n, 256), 256, 0, s>>>(d, w, cols, vals, dt, eform, out, d, parts);
+    if (n > 0) launch_pdl(k_ek_scatter_ell, blocks_for(n, 256), 256, 0, s, d, w, cols, vals, dt, eform, out, d,
+                          parts);
     return (int)cudaGetLastError();
 }
 
 int launch_ell_band(int d, int w, const int *cols, int *out, cudaStream_t s) {
-    k_ell_band<<<1, 1024, 0, s>>>(d, w, cols, out);
+    launch_pdl(k_ell_band, 1, 1024, 0, s, d, w, cols, out);
     return (int)cudaGetLastError();
 }
 
@@ -735,7 +753,7 @@ int launch_ek_dense(int d, const double *L, double dt, int eform, float *out, cu
     long long n = (long long)d * d;
     int b = blocks_for(n, 256);
     int cap = 16 * num_sms();
-    k_ek_dense<<<b < cap ? b : cap, 256, 0, s>>>(d, L, dt, eform, out, d);
+    launch_pdl(k_ek_dense, b < cap ? b : cap, 256, 0, s, d, L, dt, eform, out, d);
     return (int)cudaGetLastError();
 }
 
@@ -745,29 +763,30 @@ int launch_ek_padded(int d, int dpad, int w, const int *cols, const double *vals
     if (e != cudaSuccess) return (int)e;
     if (w > 0) {
         long long n = (long long)d * w;
-        if (n > 0) k_ek_scatter_ell<<<blocks_for(n, 256), 256, 0, s>>>(d, w, cols, vals, dt, 1, out, dpad, parts);
+        if (n > 0) launch_pdl(k_ek_scatter_ell, blocks_for(n, 256), 256, 0, s, d, w, cols, vals, dt, 1, out, dpad,
+                              parts);
     } else {
         long long n = (long long)d * d;
         int b = blocks_for(n, 256), cap = 16 * num_sms();
-        k_ek_dense<<<b < cap ? b : cap, 256, 0, s>>>(d, dense, dt, 1, out, dpad);
+        launch_pdl(k_ek_dense, b < cap ? b : cap, 256, 0, s, d, dense, dt, 1, out, dpad);
     }
     return (int)cudaGetLastError();
 }
 
 int launch_pad_x(int d, int dpad, const double *x, double *xpad, cudaStream_t s) {
-    k_pad_x<<<blocks_for(dpad, 256), 256, 0, s>>>(d, dpad, x, xpad);
+    launch_pdl(k_pad_x, blocks_for(dpad, 256), 256, 0, s, d, dpad, x, xpad);
     return (int)cudaGetLastError();
 }
 
 int launch_split(int rows, int cols, const float *X, long long ld, __nv_bfloat16 *Ahi, __nv_bfloat16 *Alo,
                  __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, long long ldt, cudaStream_t s, float sscale) {
     dim3 g((cols + 31) / 32, (rows + 31) / 32);
-    k_split_tr<<<g, 256, 0, s>>>(rows, cols, X, ld, Ahi, Alo, Bhi, Blo, ldt, sscale);
+    launch_pdl(k_split_tr, g, 256, 0, s, rows, cols, X, ld, Ahi, Alo, Bhi, Blo, ldt, sscale);
     return (int)cudaGetLastError();
 }
 
 int launch_rowsum(int d, const float *X, double *partial, cudaStream_t s) {
-    k_rowsum<<<d, 256, 0, s>>>(d, X, partial);
+    launch_pdl(k_rowsum, d, 256, 0, s, d, X, partial);
     return (int)cudaGetLastError();
 }
 
@@ -777,13 +796,13 @@ int launch_renorm(int d, float *X, const double *partial, int nparts, int eform,
     if (d % 64 == 0 && (Ahi != nullptr) == (Alo != nullptr)) {
         if (int r = renorm64_prepare()) return r;
         auto kern = occ ? k_renorm64<true> : k_renorm64<false>;
-        kern<<<renorm64_grid(d), 256, RN_SMEM, s>>>(d, X, partial, nparts, eform ? 0 : 2, Ahi, Alo, Bhi, Blo, sscale,
-                                                    write_x, eform ? fix : nullptr, 0, occ);
+        launch_pdl(kern, renorm64_grid(d), 256, RN_SMEM, s, d, X, partial, nparts, eform ? 0 : 2, Ahi, Alo, Bhi,
+                   Blo, sscale, write_x, eform ? fix : nullptr, 0, occ);
         return (int)cudaGetLastError();
     }
     if (!write_x || fix || occ) return OPB_E_UNSUPPORTED;
     dim3 g((d + 31) / 32, (d + 31) / 32);
-    k_renorm<<<g, 256, 0, s>>>(d, X, partial, nparts, eform, Ahi, Alo, Bhi, Blo, sscale);
+    launch_pdl(k_renorm, g, 256, 0, s, d, X, partial, nparts, eform, Ahi, Alo, Bhi, Blo, sscale);
     return (int)cudaGetLastError();
 }
 
@@ -795,8 +814,8 @@ int launch_renorm_to_p(int d, float *X, const double *partial, int nparts, __nv_
     if (d % 64) return OPB_E_UNSUPPORTED;
     if (int r = renorm64_prepare()) return r;
     auto kern = occ ? k_renorm64<true> : k_renorm64<false>;
-    kern<<<renorm64_grid(d), 256, RN_SMEM, s>>>(d, X, partial, nparts, 1, Ahi, Alo, Bhi, Blo, sscale, 1,
-                                                      nullptr, 1, const_cast<uint8_t *>(occ));
+    launch_pdl(kern, renorm64_grid(d), 256, RN_SMEM, s, d, X, partial, nparts, 1, Ahi, Alo, Bhi, Blo, sscale, 1,
+               nullptr, 1, const_cast<uint8_t *>(occ));
     return (int)cudaGetLastError();
 }
 
@@ -841,7 +860,7 @@ int launch_pad_batched(const BatchLattice *lats, int nlat, long long total_rows,
     const long long n = total_rows * w;
     if (n <= 0) return OPB_OK;
     k_pad_batched<<<(int)((n + 255) / 256), 256, 0, s>>>(lats, nlat, total_rows, w, cols_src, vals_src, x_src, cols,
-                                                          vals, x);
+                                                         vals, x);
     return (int)cudaGetLastError();
 }
 
@@ -988,7 +1007,7 @@ int launch_berm_batched_init(const BatchLattice *lats, int nlat, long long total
     if (n <= 0) return OPB_OK;
     if (f16) k_berm_scale_batched<<<nlat, 256, 0, s>>>(lats, x, nK, strikes, put);
     k_berm_init_batched<<<blocks_for(n, 256), 256, 0, s>>>(lats, nlat, total_rows, nK, ldk, x, strikes, put, barrier,
-                                                          f16);
+                                                           f16);
     return (int)cudaGetLastError();
 }
 
@@ -998,7 +1017,7 @@ int launch_berm_batched_step(const BatchLattice *lats, int nlat, long long total
     const long long n = total_rows * ldk;
     if (n <= 0) return OPB_OK;
     k_berm_step_batched<<<blocks_for(n, 256), 256, 0, s>>>(lats, nlat, total_rows, nK, ldk, x, strikes, put, barrier,
-                                                          exercise, last, f16, quotes);
+                                                           exercise, last, f16, quotes);
     return (int)cudaGetLastError();
 }
 
@@ -1020,13 +1039,13 @@ int launch_row_quotes_batched(const BatchLattice *lats, const RowChainLat *rows,
 
 int launch_row_quotes(int nm, int m0, int nK, int ldk, const float *V, double rate, double period, const double *qinv,
                       const float *dscale, int nslice, long long slice_stride, double *quotes, cudaStream_t s) {
-    k_row_quotes<<<blocks_for((long long)nm * nK, 256), 256, 0, s>>>(nm, m0, nK, ldk, V, rate, period, qinv, dscale,
-                                                                    nslice > 1 ? nslice : 1, slice_stride, quotes);
+    launch_pdl(k_row_quotes, blocks_for((long long)nm * nK, 256), 256, 0, s, nm, m0, nK, ldk, V, rate, period, qinv,
+               dscale, nslice > 1 ? nslice : 1, slice_stride, quotes);
     return (int)cudaGetLastError();
 }
 
 int launch_rowfix(int d, const double *partial, int nparts, int eform, double2 *fix, cudaStream_t s) {
-    k_rowfix<<<blocks_for(d, 256), 256, 0, s>>>(d, partial, nparts, eform, fix);
+    launch_pdl(k_rowfix, blocks_for(d, 256), 256, 0, s, d, partial, nparts, eform, fix);
     return (int)cudaGetLastError();
 }
 
@@ -1038,7 +1057,7 @@ int launch_rowfix_batched(const BatchLattice *lats, int nlat, long long total_ro
 }
 
 int launch_add_identity(int d, float *X, cudaStream_t s) {
-    k_add_identity<<<blocks_for(d, 256), 256, 0, s>>>(d, X);
+    launch_pdl(k_add_identity, blocks_for(d, 256), 256, 0, s, d, X);
     return (int)cudaGetLastError();
 }
 
@@ -1046,6 +1065,7 @@ int launch_add_identity(int d, float *X, cudaStream_t s) {
 // with max payoff = max(x) - min(K) (one block).
 __global__ void k_payoff_scale(int d, const double *__restrict__ x, int nK, const double *__restrict__ K,
                                float *__restrict__ out) {
+    pdl_begin();
     __shared__ double sx[256], sk[256];
     double mx = -1e300, mk = 1e300;
     for (int i = threadIdx.x; i < d; i += blockDim.x) mx = fmax(mx, x[i]);
@@ -1069,26 +1089,26 @@ __global__ void k_payoff_scale(int d, const double *__restrict__ x, int nK, cons
 }
 
 int launch_payoff_scale(int d, const double *x, int nK, const double *K, float *out, cudaStream_t s) {
-    k_payoff_scale<<<1, 256, 0, s>>>(d, x, nK, K, out);
+    launch_pdl(k_payoff_scale, 1, 256, 0, s, d, x, nK, K, out);
     return (int)cudaGetLastError();
 }
 
 int launch_payoff(int d, int nK, int ldk, const double *x, const double *K, float *G, __nv_bfloat16 *GThi,
                   __nv_bfloat16 *GTlo, cudaStream_t s, const float *dscale) {
     long long n = (long long)d * ldk;
-    k_payoff<<<blocks_for(n, 256), 256, 0, s>>>(d, nK, ldk, x, K, G, GThi, GTlo, dscale);
+    launch_pdl(k_payoff, blocks_for(n, 256), 256, 0, s, d, nK, ldk, x, K, G, GThi, GTlo, dscale);
     return (int)cudaGetLastError();
 }
 
 int launch_berm_scale(int d, const double *x, int nK, const double *K, int put, float *out, cudaStream_t s) {
-    k_berm_scale<<<1, 256, 0, s>>>(d, x, nK, K, put, out);
+    launch_pdl(k_berm_scale, 1, 256, 0, s, d, x, nK, K, put, out);
     return (int)cudaGetLastError();
 }
 
 int launch_berm_init(int d, int nK, int ldk, const double *x, const double *K, int put, double barrier, double *V,
                      __nv_bfloat16 *Vhi, __nv_bfloat16 *Vlo, float *Vf, const float *dscale, cudaStream_t s) {
     const long long n = (long long)d * ldk;
-    k_berm_init<<<blocks_for(n, 256), 256, 0, s>>>(d, nK, ldk, x, K, put, barrier, V, Vhi, Vlo, Vf, dscale);
+    launch_pdl(k_berm_init, blocks_for(n, 256), 256, 0, s, d, nK, ldk, x, K, put, barrier, V, Vhi, Vlo, Vf, dscale);
     return (int)cudaGetLastError();
 }
 
@@ -1097,16 +1117,16 @@ int launch_berm_step(int d, int nK, int ldk, const float *C, double disc, const 
                      const float *dscale, int y0, double *quotes, cudaStream_t s, int nslice,
                      long long slice_stride) {
     const long long n = (long long)d * ldk;
-    k_berm_step<<<blocks_for(n, 256), 256, 0, s>>>(d, nK, ldk, C, disc, x, K, put, barrier, exercise, V, Vhi, Vlo,
-                                                   Vf, dscale, y0, quotes, nslice > 1 ? nslice : 1, slice_stride);
+    launch_pdl(k_berm_step, blocks_for(n, 256), 256, 0, s, d, nK, ldk, C, disc, x, K, put, barrier, exercise, V,
+               Vhi, Vlo, Vf, dscale, y0, quotes, nslice > 1 ? nslice : 1, slice_stride);
     return (int)cudaGetLastError();
 }
 
 int launch_discount(int d, int nK, int ldk, const float *V32, double disc, double *V64, int y0, double *quotes,
                     cudaStream_t s, const float *dscale, int nslice, long long slice_stride, const double2 *rowfix) {
     long long n = (long long)d * nK;
-    k_discount<<<blocks_for(n, 256), 256, 0, s>>>(d, nK, ldk, V32, disc, V64, y0, quotes, dscale,
-                                                  nslice > 1 ? nslice : 1, slice_stride, rowfix);
+    launch_pdl(k_discount, blocks_for(n, 256), 256, 0, s, d, nK, ldk, V32, disc, V64, y0, quotes, dscale, nslice > 1
+               ? nslice : 1, slice_stride, rowfix);
     return (int)cudaGetLastError();
 }
 
@@ -1122,6 +1142,7 @@ int launch_discount(int d, int nK, int ldk, const float *V32, double disc, doubl
 // IEEE FP32 division.  The lattice path builds its U0 in FP64 elsewhere; this is the drop-in.
 __global__ void k_sek(int d, const float *__restrict__ gen, float dt, float *__restrict__ out,
                       const float *__restrict__ r, const float *__restrict__ lambda) {
+    opb::pdl_begin();
     long long n = (long long)d * d;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
          t += (long long)gridDim.x * blockDim.x) {
@@ -1142,10 +1163,9 @@ static int sek_common(int d, uint64_t gen, float dt, uint64_t tpk, uint64_t r, u
     long long n = (long long)d * d;
     int b = (int)((n + 255) / 256);
     int cap = 16 * opb::num_sms();
-    k_sek<<<b < cap ? b : cap, 256, 0, opb::stream()>>>(d, reinterpret_cast<const float *>(gen), dt,
-                                                         reinterpret_cast<float *>(tpk),
-                                                         reinterpret_cast<const float *>(r),
-                                                         reinterpret_cast<const float *>(lambda));
+    opb::launch_pdl(k_sek, b < cap ? b : cap, 256, 0, opb::stream(), d, reinterpret_cast<const float *>(gen), dt,
+                    reinterpret_cast<float *>(tpk), reinterpret_cast<const float *>(r), reinterpret_cast<const float
+                    *>(lambda));
     return opb::launch_check();
 }
 
@@ -1177,9 +1197,10 @@ OPB_API int opb_renorm_rows(int d, float *X, const double *partial, int nparts, 
                     (!Bhi || (opb::aligned(Bhi, 8) && opb::aligned(Blo, 8))),
                 OPB_E_ALIGN);
     if (int r = opb::renorm64_prepare()) return opb::set_status(r);
-    opb::k_renorm64<false><<<opb::renorm64_grid(d), 256, opb::RN_SMEM, opb::stream()>>>(
-        d, X, partial, nparts, mode, reinterpret_cast<__nv_bfloat16 *>(Ahi), reinterpret_cast<__nv_bfloat16 *>(Alo),
-        mode == 2 ? nullptr : reinterpret_cast<__nv_bfloat16 *>(Bhi),
-        mode == 2 ? nullptr : reinterpret_cast<__nv_bfloat16 *>(Blo), f16 ? 32768.f : 0.f);
+    opb::launch_pdl(opb::k_renorm64<false>, opb::renorm64_grid(d), 256, opb::RN_SMEM, opb::stream(), d, X, partial,
+                    nparts, mode, reinterpret_cast<__nv_bfloat16 *>(Ahi), reinterpret_cast<__nv_bfloat16 *>(Alo),
+                    mode == 2 ? nullptr : reinterpret_cast<__nv_bfloat16 *>(Bhi),
+                    mode == 2 ? nullptr : reinterpret_cast<__nv_bfloat16 *>(Blo), f16 ? 32768.f : 0.f, 1, nullptr, 0,
+                    nullptr);
     return opb::launch_check();
 }

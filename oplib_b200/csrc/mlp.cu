@@ -55,6 +55,7 @@ __device__ __forceinline__ uint32_t hash32(uint64_t x) {
 
 // Uniform(-a, a) weights with a = sqrt(6 / fan_in) (He-uniform), zero biases.
 __global__ void k_mlp_init(float *__restrict__ theta, uint64_t seed) {
+    pdl_begin();
     const MlpLayout L = mlp_layout();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < MLP_NPARAM;
          i += (long long)gridDim.x * blockDim.x) {
@@ -74,6 +75,7 @@ __global__ void k_mlp_init(float *__restrict__ theta, uint64_t seed) {
 // inference (same layout).
 __global__ void k_mlp_round(const float *__restrict__ theta, float *__restrict__ theta_bf,
                             __nv_bfloat16 *__restrict__ theta_b16, int n) {
+    pdl_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const __nv_bfloat16 b = __float2bfloat16_rn(theta[i]);
         if (theta_bf) theta_bf[i] = __bfloat162float(b);
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(MLP_H) k_mlp_first(int B, const float *__restr
                                                      __nv_bfloat16 *const Wp0l, __nv_bfloat16 *const Wp1h,
                                                      __nv_bfloat16 *const Wp1l, __nv_bfloat16 *const Wp2h,
                                                      __nv_bfloat16 *const Wp2l) {
+    pdl_begin();
     const int c = threadIdx.x;
     if ((int)blockIdx.x >= nrow) {  // a row of a weight matrix
         const int i = (int)blockIdx.x - nrow, l = i / MLP_H, o = (i % MLP_H) * MLP_H + c;
@@ -138,6 +141,7 @@ __global__ void __launch_bounds__(MLP_H) k_mlp_first(int B, const float *__restr
 // (optional) in FP32 and/or its BF16 parts Hhi / Hlo (optional, for the tensor-core products).
 __global__ void k_bias_gelu(long long total4, float *__restrict__ Z, const float *__restrict__ b,
                             float *__restrict__ H, __nv_bfloat16 *__restrict__ Hhi, __nv_bfloat16 *__restrict__ Hlo) {
+    pdl_begin();
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= total4) return;
     const float4 zv = reinterpret_cast<const float4 *>(Z)[i], bv = reinterpret_cast<const float4 *>(b)[i % (MLP_H / 4)];
@@ -164,6 +168,7 @@ __global__ void __launch_bounds__(256) k_mlp_out(int B, float *__restrict__ Z, c
                                                  float *__restrict__ y, const float *__restrict__ t,
                                                  float *__restrict__ dy, double *__restrict__ loss_part,
                                                  float *__restrict__ dy_part) {
+    pdl_begin();
     __shared__ double se_s[8];
     __shared__ float dy_s[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -221,6 +226,7 @@ __global__ void __launch_bounds__(MLP_H / 2) k_mlp_dz(int B, const float *__rest
                                                       __nv_bfloat16 *__restrict__ Ghi, __nv_bfloat16 *__restrict__ Glo,
                                                       __nv_bfloat16 *__restrict__ Thi, __nv_bfloat16 *__restrict__ Tlo,
                                                       float *__restrict__ bsum, float *__restrict__ wsum) {
+    pdl_begin();
     const int c = 2 * threadIdx.x, r0 = blockIdx.x * MLP_RB, n = min(MLP_RB, B - r0);
     __shared__ float xs[MLP_RB][MLP_IN];
     if (FIRST) {
@@ -315,6 +321,7 @@ struct MlpFinish {
     int no;
 };
 __global__ void __launch_bounds__(256) k_mlp_finish(MlpFinish f) {
+    pdl_begin();
     const int tid = threadIdx.x;
     int blk = blockIdx.x;
     if (blk < 3 * MLP_H) {
@@ -382,6 +389,7 @@ __global__ void __launch_bounds__(256) k_mlp_finish(MlpFinish f) {
 __global__ void k_adam(int n, float *__restrict__ theta, float *__restrict__ m, float *__restrict__ v,
                        const float *__restrict__ g, float lr, float b1, float b2, float eps, float c1, float c2,
                        float *__restrict__ theta_bf) {
+    pdl_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -402,6 +410,7 @@ __global__ void k_adam_sched(int n, float *__restrict__ theta, float *__restrict
                              const float *__restrict__ g, const float *__restrict__ lr_table,
                              const int *__restrict__ step, float b1, float b2, float eps,
                              float *__restrict__ theta_bf) {
+    pdl_begin();
     const int s = *step + 1;
     const float c1 = 1.f - powf(b1, (float)s), c2 = 1.f - powf(b2, (float)s);
     const float lr = lr_table[s - 1];
@@ -417,7 +426,10 @@ __global__ void k_adam_sched(int n, float *__restrict__ theta, float *__restrict
     }
 }
 
-__global__ void k_step_inc(int *step) { *step += 1; }
+__global__ void k_step_inc(int *step) {
+    pdl_begin();
+    *step += 1;
+}
 
 // ---- implied volatility of call prices (FP64 bisection on the Black-Scholes price)
 __device__ double bs_call(double s, double k, double r, double sig, double t) {
@@ -429,6 +441,7 @@ __device__ double bs_call(double s, double k, double r, double sig, double t) {
 __global__ void k_implied_vol(long long n, const double *__restrict__ price, const double *__restrict__ K,
                               const double *__restrict__ T, const double *__restrict__ r,
                               const double *__restrict__ S0, double *__restrict__ iv) {
+    pdl_begin();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         const double p = price[i], k = K[i], t = T[i], rr = r[i], s0 = S0[i];
@@ -574,9 +587,9 @@ int mlp_forward(const float *thb, const float *X, int B, MlpWs &w, cudaStream_t 
     const int nrow = (B + MLP_RB - 1) / MLP_RB;
     // with the tensor cores, layers 0..2 store only their activations' parts (the next
     // product's A and the weight gradient's B)
-    k_mlp_first<<<nrow + (tc ? 3 * MLP_H : 0), MLP_H, 0, s>>>(
-        B, X, thb + L.w[0], thb + L.b[0], w.Z[0], tc ? nullptr : w.H[0], tc ? w.Hp[0][0] : nullptr,
-        tc ? w.Hp[0][1] : nullptr, nrow, thb + L.w[1], w.Wp[0][0], w.Wp[0][1], w.Wp[1][0], w.Wp[1][1], w.Wp[2][0], w.Wp[2][1]);
+    launch_pdl(k_mlp_first, nrow + (tc ? 3 * MLP_H : 0), MLP_H, 0, s, B, X, thb + L.w[0], thb + L.b[0], w.Z[0],
+               tc ? nullptr : w.H[0], tc ? w.Hp[0][0] : nullptr, tc ? w.Hp[0][1] : nullptr, nrow, thb + L.w[1],
+               w.Wp[0][0], w.Wp[0][1], w.Wp[1][0], w.Wp[1][1], w.Wp[2][0], w.Wp[2][1]);
     for (int l = 1; l < 4; l++) {
         // Z = in . W^T  (W stored out x in: the TB form)
         if (tc) MT(mlp_tc_gemm(B, MLP_H, MLP_H, w.Hp[l - 1], MLP_H, w.Wp[l - 1], MLP_H, 0, w.Z[l], 1, s));
@@ -585,8 +598,8 @@ int mlp_forward(const float *thb, const float *X, int B, MlpWs &w, cudaStream_t 
                           s));
         if (l == 3) break;
         const long long t4 = (long long)B * MLP_H / 4;
-        k_bias_gelu<<<(unsigned)((t4 + 255) / 256), 256, 0, s>>>(t4, w.Z[l], thb + L.b[l], tc ? nullptr : w.H[l],
-                                                                 tc ? w.Hp[l][0] : nullptr, tc ? w.Hp[l][1] : nullptr);
+        launch_pdl(k_bias_gelu, (unsigned)((t4 + 255) / 256), 256, 0, s, t4, w.Z[l], thb + L.b[l],
+                   tc ? nullptr : w.H[l], tc ? w.Hp[l][0] : nullptr, tc ? w.Hp[l][1] : nullptr);
     }
     return (int)cudaGetLastError();
 }
@@ -611,15 +624,15 @@ OPB_API int opb_mlp_set_tensor_cores(int on) {
 
 OPB_API int opb_mlp_init(float *theta, unsigned long long seed) {
     OPB_REQUIRE(theta, OPB_E_NULL);
-    k_mlp_init<<<grid_ew(MLP_NPARAM), 256, 0, stream()>>>(theta, seed);
+    launch_pdl(k_mlp_init, grid_ew(MLP_NPARAM), 256, 0, stream(), theta, seed);
     return launch_check();
 }
 
 // theta_bf: BF16-rounded FP32 working copy (optional); theta_b16: BF16 storage (optional)
 OPB_API int opb_mlp_round(const float *theta, float *theta_bf, void *theta_b16) {
     OPB_REQUIRE(theta, OPB_E_NULL);
-    k_mlp_round<<<grid_ew(MLP_NPARAM), 256, 0, stream()>>>(theta, theta_bf, reinterpret_cast<__nv_bfloat16 *>(theta_b16),
-                                                            MLP_NPARAM);
+    launch_pdl(k_mlp_round, grid_ew(MLP_NPARAM), 256, 0, stream(), theta, theta_bf,
+               reinterpret_cast<__nv_bfloat16 *>(theta_b16), MLP_NPARAM);
     return launch_check();
 }
 
@@ -632,8 +645,8 @@ OPB_API int opb_mlp_forward(const float *thb, const float *X, int B, float *ws, 
     cudaStream_t s = stream();
     MT(mlp_forward(thb, X, B, w, s));
     const MlpLayout L = mlp_layout();
-    k_mlp_out<<<(B + 7) / 8, 256, 0, s>>>(B, w.Z[3], thb + L.b[3], thb + L.w[4], thb + L.b[4], y, nullptr, nullptr,
-                                          nullptr, nullptr);
+    launch_pdl(k_mlp_out, (B + 7) / 8, 256, 0, s, B, w.Z[3], thb + L.b[3], thb + L.w[4], thb + L.b[4], y, nullptr,
+               nullptr, nullptr, nullptr);
     return launch_check();
 }
 
@@ -648,7 +661,8 @@ OPB_API int opb_mlp_loss_grad(const float *thb, const float *X, const float *t, 
     const MlpLayout L = mlp_layout();
     MT(mlp_forward(thb, X, B, w, s));
     const int no = (B + 7) / 8, nb = (B + MLP_RB - 1) / MLP_RB;
-    k_mlp_out<<<no, 256, 0, s>>>(B, w.Z[3], thb + L.b[3], thb + L.w[4], thb + L.b[4], w.y, t, w.dy, w.lossp, w.dysum);
+    launch_pdl(k_mlp_out, no, 256, 0, s, B, w.Z[3], thb + L.b[3], thb + L.w[4], thb + L.b[4], w.y, t, w.dy, w.lossp,
+               w.dysum);
     const bool tc = mlp_tc(B);
     // weight-gradient K-slices on the tensor cores: at most 16, dividing B / 64.  Sixteen slices of
     // 128 x 64 tiles are 128 CTAs; with 32 slices of 128 x 256 ones (64 CTAs) the output phase of
@@ -661,11 +675,11 @@ OPB_API int opb_mlp_loss_grad(const float *thb, const float *X, const float *t, 
         __nv_bfloat16 *gh = tc ? w.dZp[0] : nullptr, *gl = tc ? w.dZp[1] : nullptr;
         if (l == 3) {
             // (with SIMT products the last activations are wanted in FP32 by nobody but this pass)
-            k_mlp_dz<true, false><<<nb, MLP_H / 2, 0, s>>>(B, w.Z[3], nullptr, w.dy, thb + L.w[4], nullptr, dZ, gh, gl, w.dZt[0],
-                                                       w.dZt[1], w.bsum[3], w.w5sum);
+            launch_pdl(k_mlp_dz<true, false>, nb, MLP_H / 2, 0, s, B, w.Z[3], nullptr, w.dy, thb + L.w[4], nullptr,
+                       dZ, gh, gl, w.dZt[0], w.dZt[1], w.bsum[3], w.w5sum);
         } else {
-            k_mlp_dz<false, false><<<nb, MLP_H / 2, 0, s>>>(B, w.Z[l], w.dH, nullptr, nullptr, nullptr, dZ, gh, gl, w.dZt[0],
-                                                        w.dZt[1], w.bsum[l], nullptr);
+            launch_pdl(k_mlp_dz<false, false>, nb, MLP_H / 2, 0, s, B, w.Z[l], w.dH, nullptr, nullptr, nullptr, dZ,
+                       gh, gl, w.dZt[0], w.dZt[1], w.bsum[l], nullptr);
         }
         float *part = w.part + (size_t)(l - 1) * MLP_KSPLIT * MLP_H * MLP_H;
         f.wpart[l - 1] = part;
@@ -681,15 +695,15 @@ OPB_API int opb_mlp_loss_grad(const float *thb, const float *X, const float *t, 
             MT(sgemm_rm_t(false, false, B, MLP_H, MLP_H, 1.f, w.dZ, MLP_H, thb + L.w[l], MLP_H, 0.f, w.dH, MLP_H, s));
         }
     }
-    k_mlp_dz<false, true><<<nb, MLP_H / 2, 0, s>>>(B, w.Z[0], w.dH, nullptr, nullptr, X, nullptr, nullptr, nullptr, nullptr,
-                                               nullptr, w.bsum[0], w.w1sum);
+    launch_pdl(k_mlp_dz<false, true>, nb, MLP_H / 2, 0, s, B, w.Z[0], w.dH, nullptr, nullptr, X, nullptr, nullptr,
+               nullptr, nullptr, nullptr, w.bsum[0], w.w1sum);
     for (int l = 0; l < 4; l++) {
         f.bsum[l] = w.bsum[l];
         f.db[l] = grad + L.b[l];
     }
     f.w5sum = w.w5sum; f.w1sum = w.w1sum; f.dw5 = grad + L.w[4]; f.dw1 = grad + L.w[0]; f.db5 = grad + L.b[4];
     f.nb = nb; f.loss_part = w.lossp; f.dy_part = w.dysum; f.loss = loss; f.no = no;
-    k_mlp_finish<<<3 * MLP_H + 13 * 4 + 1, 256, 0, s>>>(f);
+    launch_pdl(k_mlp_finish, 3 * MLP_H + 13 * 4 + 1, 256, 0, s, f);
     return launch_check();
 }
 
@@ -698,7 +712,8 @@ OPB_API int opb_mlp_adam(float *theta, float *m, float *v, const float *grad, in
     OPB_REQUIRE(theta && m && v && grad && theta_bf, OPB_E_NULL);
     OPB_REQUIRE(step >= 1 && lr > 0.f, OPB_E_ARG);
     const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-    k_adam<<<grid_ew(MLP_NPARAM), 256, 0, stream()>>>(MLP_NPARAM, theta, m, v, grad, lr, b1, b2, eps, c1, c2, theta_bf);
+    launch_pdl(k_adam, grid_ew(MLP_NPARAM), 256, 0, stream(), MLP_NPARAM, theta, m, v, grad, lr, b1, b2, eps, c1,
+               c2, theta_bf);
     return launch_check();
 }
 
@@ -709,9 +724,9 @@ OPB_API int opb_mlp_adam(float *theta, float *m, float *v, const float *grad, in
 OPB_API int opb_mlp_adam_sched(float *theta, float *m, float *v, const float *grad, int *step, const float *lr_table,
                                float b1, float b2, float eps, float *theta_bf) {
     OPB_REQUIRE(theta && m && v && grad && step && lr_table && theta_bf, OPB_E_NULL);
-    k_adam_sched<<<grid_ew(MLP_NPARAM), 256, 0, stream()>>>(MLP_NPARAM, theta, m, v, grad, lr_table, step, b1, b2,
-                                                             eps, theta_bf);
-    k_step_inc<<<1, 1, 0, stream()>>>(step);
+    launch_pdl(k_adam_sched, grid_ew(MLP_NPARAM), 256, 0, stream(), MLP_NPARAM, theta, m, v, grad, lr_table, step,
+               b1, b2, eps, theta_bf);
+    launch_pdl(k_step_inc, 1, 1, 0, stream(), step);
     return launch_check();
 }
 
@@ -722,7 +737,7 @@ OPB_API int opb_implied_vol(long long n, const double *price, const double *K, c
     OPB_REQUIRE(n >= 0, OPB_E_ARG);
     if (n == 0) return set_status(OPB_OK);
     OPB_REQUIRE(price && K && T && r && S0 && iv, OPB_E_NULL);
-    k_implied_vol<<<grid_ew(n), 256, 0, stream()>>>(n, price, K, T, r, S0, iv);
+    launch_pdl(k_implied_vol, grid_ew(n), 256, 0, stream(), n, price, K, T, r, S0, iv);
     return launch_check();
 }
 
@@ -736,6 +751,7 @@ constexpr long long MLP_PACK_W1 = 256LL * 64 * 2, MLP_PACK_WH = 256LL * 256 * 2;
 constexpr long long MLP_PACK_BYTES = MLP_PACK_W1 + 3 * MLP_PACK_WH + (4 * 256 + 256 + 1) * 4;
 
 __global__ void k_mlp_pack(const float *__restrict__ theta, uint8_t *__restrict__ packed) {
+    pdl_begin();
     const MlpLayout L = mlp_layout();
     __nv_bfloat16 *w1 = reinterpret_cast<__nv_bfloat16 *>(packed);
     __nv_bfloat16 *wh = reinterpret_cast<__nv_bfloat16 *>(packed + MLP_PACK_W1);
@@ -760,6 +776,7 @@ __global__ void k_mlp_pack(const float *__restrict__ theta, uint8_t *__restrict_
 
 // X [n x 8] FP32 -> Xp [n x 64] BF16 (zero padded)
 __global__ void k_mlp_pad_input(long long n, const float *__restrict__ X, __nv_bfloat16 *__restrict__ Xp) {
+    pdl_begin();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * 64;
          i += (long long)gridDim.x * blockDim.x) {
         const long long r = i / 64;
@@ -775,6 +792,7 @@ constexpr int MLP_YPARTS = 256 / TC_LAYER_CPT;
 __global__ void k_mlp_ensemble(long long n, long long np, int nmem, const float *__restrict__ yp,
                                const uint8_t *__restrict__ packed, long long stride, long long b5_off,
                                float *__restrict__ mean, float *__restrict__ spread) {
+    pdl_begin();
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {
         float s = 0.f, lo = 3.4e38f, hi = -3.4e38f;
         for (int m = 0; m < nmem; m++) {
@@ -798,7 +816,7 @@ OPB_API long long opb_mlp_packed_bytes(void) { return MLP_PACK_BYTES; }
 OPB_API int opb_mlp_pack(const float *theta, void *packed) {
     OPB_REQUIRE(theta && packed, OPB_E_NULL);
     OPB_REQUIRE(aligned(packed, 16), OPB_E_ALIGN);
-    k_mlp_pack<<<grid_ew(3LL * 256 * 256), 256, 0, stream()>>>(theta, reinterpret_cast<uint8_t *>(packed));
+    launch_pdl(k_mlp_pack, grid_ew(3LL * 256 * 256), 256, 0, stream(), theta, reinterpret_cast<uint8_t *>(packed));
     return launch_check();
 }
 
@@ -830,7 +848,7 @@ OPB_API int opb_mlp_infer(const void *packed, int nmem, long long member_stride,
     __nv_bfloat16 *Hb = Ha + np * 256;
     float *ym = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(Hb + np * 256));
     MT((int)cudaMemsetAsync(Xp, 0, np * 64 * 2, s));
-    k_mlp_pad_input<<<grid_ew(n * 64), 256, 0, s>>>(n, X, Xp);
+    launch_pdl(k_mlp_pad_input, grid_ew(n * 64), 256, 0, s, n, X, Xp);
     for (int m = 0; m < nmem; m++) {
         const uint8_t *pk = reinterpret_cast<const uint8_t *>(packed) + (long long)m * member_stride;
         const __nv_bfloat16 *W1 = reinterpret_cast<const __nv_bfloat16 *>(pk);
@@ -847,8 +865,8 @@ OPB_API int opb_mlp_infer(const void *packed, int nmem, long long member_stride,
         MT(launch_tc_layer((int)np, 256, 256, Ha, 256, WH + 2 * 65536, 256, 1.f, f + 768, nullptr, 256, s, f + 1024,
                            ym + (long long)MLP_YPARTS * m * np));
     }
-    k_mlp_ensemble<<<grid_ew(n), 256, 0, s>>>(n, np, nmem, ym, reinterpret_cast<const uint8_t *>(packed),
-                                              member_stride, MLP_PACK_W1 + 3 * MLP_PACK_WH + 1280LL * 4, mean, spread);
+    launch_pdl(k_mlp_ensemble, grid_ew(n), 256, 0, s, n, np, nmem, ym, reinterpret_cast<const uint8_t *>(packed),
+               member_stride, MLP_PACK_W1 + 3 * MLP_PACK_WH + 1280LL * 4, mean, spread);
     return launch_check();
 }
 

@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(RS_THREADS)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot_s);
+    pdl_begin();  // (the shared and tensor memory set up while the previous step ran)
 
     if (warp == 4) {
         if (lane == 0) {
@@ -332,6 +333,7 @@ __global__ void __launch_bounds__(RS_THREADS)
 // The last maturity's row into its pricing slot (block per lattice); p.m is one past it.
 template <bool BATCHED>
 __global__ void __launch_bounds__(RS_PREP) k_row_finish(RowChainLat one, RowStepParams p, const RowChainLat *__restrict__ lats) {
+    pdl_begin();
     __shared__ double red[4];
     const RowChainLat &L = BATCHED ? lats[blockIdx.x] : one;
     const double inv = row_parts(L, p, red, [&](int e, const uint4 &h, const uint4 &l) { row_slot(L, p.m, e, h, l); });
@@ -376,8 +378,10 @@ int launch_row_step(const RowChainLat &L, const __nv_bfloat16 *Bhi, const __nv_b
     if ((r = make_map_mn(&ml, Blo, L.d, L.d, L.d, f16)) != OPB_OK) return r;
     const int items = L.d / RS_BN, smem = row_step_smem(L.d, p.stages);
     const int cap = num_sms() * (smem <= 110 * 1024 ? 2 : 1), grid = items < cap ? items : cap;
-    if (f16) k_row_step<false, true><<<grid, RS_THREADS, smem, s>>>(mh, ml, L, p, nullptr, nullptr, nullptr, items);
-    else k_row_step<false, false><<<grid, RS_THREADS, smem, s>>>(mh, ml, L, p, nullptr, nullptr, nullptr, items);
+    if (f16) launch_pdl(k_row_step<false, true>, grid, RS_THREADS, smem, s, mh, ml, L, p, nullptr, nullptr, nullptr,
+                        items);
+    else launch_pdl(k_row_step<false, false>, grid, RS_THREADS, smem, s, mh, ml, L, p, nullptr, nullptr, nullptr,
+                    items);
     return (int)cudaGetLastError();
 }
 
@@ -400,7 +404,7 @@ int launch_row_step_batched(const RowChainLat *lats, const CUtensorMap *maps, co
 
 int launch_row_finish(const RowChainLat &L, int m, int fused, float sscale, cudaStream_t s) {
     RowStepParams p{m + 1, fused, 0, L.d, 1.f, sscale};
-    k_row_finish<false><<<1, RS_PREP, 0, s>>>(L, p, nullptr);
+    launch_pdl(k_row_finish<false>, 1, RS_PREP, 0, s, L, p, nullptr);
     return (int)cudaGetLastError();
 }
 

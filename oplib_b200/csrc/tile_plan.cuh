@@ -55,6 +55,7 @@ __device__ __forceinline__ void raster_tile(int t, int mtiles, int ntiles, int g
 }
 
 __global__ void __launch_bounds__(TP_THREADS) k_tile_plan(TilePlanArgs a) {
+    pdl_begin();
     const long long tid = blockIdx.x * (long long)TP_THREADS + threadIdx.x, nth = (long long)gridDim.x * TP_THREADS;
     for (long long i = tid; i < a.clear_bytes / 16; i += nth) reinterpret_cast<uint4 *>(a.clear)[i] = make_uint4(0, 0, 0, 0);
     // ---- row fixes
@@ -183,6 +184,6 @@ static int launch_tile_plan(TilePlanArgs &a, cudaStream_t s) {
     const long long want = std::max({(items + 7) / 8, (rows + TP_THREADS - 1) / TP_THREADS,
                                      (a.clear_bytes / 16 + TP_THREADS - 1) / TP_THREADS, 1LL});
     const int grid = (int)std::min<long long>(want, 4LL * num_sms());
-    k_tile_plan<<<grid, TP_THREADS, 0, s>>>(a);
+    launch_pdl(k_tile_plan, grid, TP_THREADS, 0, s, a);
     return (int)cudaGetLastError();
 }
