@@ -1,0 +1,49 @@
+"""Cumulative rows and guide tables at the widths where their tiles end, against numpy."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def rows_for(d, nrows, cuda, seed=3):
+    from oplib_b200.model import cumulative_rows
+    rng = np.random.default_rng(seed)
+    P = (rng.random((nrows, d)) ** 8).astype(np.float32)
+    P[rng.random((nrows, d)) < 0.3] = 0
+    P[0, : d // 2] -= 0.01  # residues below zero count as zero
+    dP = torch.from_numpy(P).to(cuda)
+    return P, cumulative_rows(dP)
+
+
+@pytest.mark.parametrize("d,nrows", [(1, 1), (3, 5), (128, 4), (513, 7), (1023, 2), (1024, 9), (1025, 6), (2051, 3)])
+def test_cumulative_rows_and_guide_at_the_edges(cuda, d, nrows):
+    from oplib_b200.model import guide_table
+    P, C = rows_for(d, nrows, cuda)
+    p = np.where(P > 0, P, np.float32(0))
+    acc = np.cumsum(p, axis=1, dtype=np.float32)  # sequential FP32 sums
+    with np.errstate(invalid="ignore"):
+        want = acc / acc[:, -1:]
+    want = np.where(want < 1, want, np.float32(1))
+    got = C.cpu().numpy()
+    assert np.array_equal(got, want)
+    for nb in (1, 64, 1024):
+        g = guide_table(C, nb).cpu().numpy().view(np.uint32)
+        for r in range(nrows):
+            lo = np.searchsorted(got[r], np.arange(nb) / nb, side="right").clip(max=d - 1)
+            hi = np.searchsorted(got[r], np.arange(1, nb + 1) / nb, side="left").clip(max=d - 1)
+            hi[-1] = d - 1
+            assert np.array_equal(g[r] & 0xffff, lo) and np.array_equal(g[r] >> 16, np.maximum(lo, hi))
+
+
+def test_guide_of_a_row_longer_than_the_staged_one(cuda):
+    from oplib_b200.model import guide_table
+    d = 12 * 1024 + 5
+    _, C = rows_for(d, 2, cuda)
+    got = C.cpu().numpy()
+    g = guide_table(C, 256).cpu().numpy().view(np.uint32)
+    for r in range(2):
+        lo = np.searchsorted(got[r], np.arange(256) / 256, side="right").clip(max=d - 1)
+        hi = np.searchsorted(got[r], np.arange(1, 257) / 256, side="left").clip(max=d - 1)
+        hi[-1] = d - 1
+        assert np.array_equal(g[r] & 0xffff, lo) and np.array_equal(g[r] >> 16, np.maximum(lo, hi))
