@@ -51,6 +51,7 @@ struct McArgs {
     long long ms;
     const uint32_t *guide;   // optional [d][nb] brackets (row-major rows only)
     int nb;
+    uint32_t rs4;            // rs in bytes (guided form)
     int d, y0, nsteps;
     uint32_t seed;
     const uint32_t *seeds;   // optional [kMcStreams] stream seeds (replaces seed)
@@ -68,9 +69,19 @@ struct McArgs {
 };
 
 // EVAL: block sums are (sum v, sum v^2) of the evaluator's path values instead of the
-// fused barrier / Asian payoffs.
-template <bool ANY_LENGTH, bool EVAL = false>
-__global__ void __launch_bounds__(256) k_mc(McArgs a) {
+// fused barrier / Asian payoffs.  GUIDED: a guide table is given and a row's pitch in bytes
+// fits 32 bits (McArgs::rs4), which makes a row's address one multiply-add.  STATES: ypaths is
+// given.
+//
+// What bounds it: issue slots, half of them of the integer pipe (one instruction in two cycles
+// a scheduler), so it is the instructions per step that count -- one tw() per output however
+// many cursors (mt19937.cuh), the barrier as a flag instead of a running FP64 minimum, no
+// branches for what the launch does not ask for.  Six blocks of 256 an SM (40 registers) hide
+// the step's chain of dependent loads (guide word, row entry, next guide word); the form for
+// longer runs gains more from registers than from warps.  2^20 paths x 504 steps over 512
+// states: 2.51 -> 1.81 ms.
+template <bool ANY_LENGTH, bool GUIDED, bool EVAL, bool STATES>
+__global__ void __launch_bounds__(256, ANY_LENGTH ? 4 : 6) k_mc(McArgs a) {
     double s_bar = 0.0, s_asi = 0.0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     const float nbf = (float)a.nb;
@@ -82,26 +93,38 @@ __global__ void __launch_bounds__(256) k_mc(McArgs a) {
             key1 = (uint32_t)(g >> kMcStreamsLog2);
         }
         int y = a.y0;
-        double xmin = 1e300, xsum = 0.0, xlast = 0.0;
+        double xsum = 0.0;
+        bool above = true;  // no node value at or below the barrier so far
         double v = 0.0;
         bool alive = true;
+        short *yp = a.ypaths + p;
         mt19937_stream<ANY_LENGTH>(seed, key1, a.nsteps, [&](int k, uint32_t bits) {
             const float u = mt_uniform_open0(bits);
-            const float *row = a.C + (long long)y * a.rs + (a.m_k ? (long long)__ldg(a.m_k + k) * a.ms : 0LL);
+            const float *row;
             int lo = 0, hi = a.d - 1;
-            if (a.guide) {
+            if constexpr (GUIDED) {
+                row = reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.C) +
+                                                      (unsigned long long)(uint32_t)y * a.rs4);
+            } else {
+                row = a.C + (long long)y * a.rs + (a.m_k ? (long long)__ldg(a.m_k + k) * a.ms : 0LL);
+            }
+            if (GUIDED || a.guide) {
                 int bkt = (int)__fmul_rn(u, nbf);
                 bkt = bkt < a.nb ? bkt : a.nb - 1;
-                uint32_t g = __ldg(a.guide + (long long)y * a.nb + bkt);
-                lo = (int)(g & 0xffffu);
-                hi = (int)(g >> 16);
+                const uint32_t gw = __ldg(a.guide + (uint32_t)(y * a.nb + bkt));
+                lo = (int)(gw & 0xffffu);
+                hi = (int)(gw >> 16);
             }
             while (lo < hi) {
-                int mid = (lo + hi) >> 1;
-                if (u < __ldg(row + (long long)mid * a.cs)) hi = mid; else lo = mid + 1;
+                const int mid = (lo + hi) >> 1;
+                const float c = GUIDED ? __ldg(row + mid) : __ldg(row + (long long)mid * a.cs);
+                if (u < c) hi = mid; else lo = mid + 1;
             }
             y = lo;
-            if (a.ypaths) a.ypaths[p + a.npaths * (long long)k] = (short)y;
+            if constexpr (STATES) {
+                *yp = (short)y;
+                yp += a.npaths;
+            }
             if constexpr (EVAL) {
                 const long long o = (long long)k * a.d + y;
                 if (alive) {
@@ -109,10 +132,9 @@ __global__ void __launch_bounds__(256) k_mc(McArgs a) {
                     else v += __ldg(a.cf + o);
                 }
             } else if (a.x) {
-                double xv = __ldg(a.x + y);
-                xmin = xv < xmin ? xv : xmin;
+                const double xv = __ldg(a.x + y);
+                above = above && !(xv <= a.barrier);
                 xsum += xv;
-                xlast = xv;
             }
         });
         if constexpr (EVAL) {
@@ -120,8 +142,8 @@ __global__ void __launch_bounds__(256) k_mc(McArgs a) {
             s_bar += v;
             s_asi += v * v;
         } else if (a.x) {
-            double pay = xlast - a.strike;
-            if (xmin > a.barrier && pay > 0.0) s_bar += a.disc * pay;
+            double pay = __ldg(a.x + y) - a.strike;
+            if (above && a.barrier < 1e300 && pay > 0.0) s_bar += a.disc * pay;
             double avg = xsum / (double)a.nsteps - a.strike;
             if (avg > 0.0) s_asi += a.disc * avg;
         }
@@ -181,28 +203,48 @@ __global__ void k_mt_raw(uint32_t seed, long long nstreams, int n, uint32_t *__r
     mt19937_stream<ANY_LENGTH>(seed + (uint32_t)s, 0u, n, [&](int j, uint32_t bits) { out[s * n + j] = bits; });
 }
 
+// Paths to blocks.  A path is one thread's work from end to end, so blocks are what the SMs can
+// be evened out with: up to 24 blocks an SM, four times what is resident, each of as few
+// threads as that allows (64 at least) -- a grid of the resident blocks alone walks 3.46 paths
+// a thread at 2^20 paths and waits for the fourth.  100,003 paths of 700 steps: 391 blocks of
+// 256 (three on an SM, or two) 554 us, 1563 of 64 443.
+constexpr int MC_BLOCKS_PER_SM = 24;
+
+static int mc_threads(long long npaths) {
+    const long long cap = (long long)MC_BLOCKS_PER_SM * num_sms();
+    return npaths <= 64 * cap ? 64 : npaths <= 128 * cap ? 128 : 256;
+}
+int mc_grid(long long npaths) {
+    const int threads = mc_threads(npaths);
+    const long long b = (npaths + threads - 1) / threads, cap = (long long)MC_BLOCKS_PER_SM * num_sms();
+    return (int)(b < 1 ? 1 : b < cap ? b : cap);
+}
+
 // The register-only generator up to 623 steps, the cursor/state-array one beyond; the
 // evaluator form when a cashflow table is given.
-void launch_mc(int grid, const McArgs &a) {
-    if (a.cf) {
-        if (a.nsteps <= kMtCursorMax) k_mc<false, true><<<grid, 256, 0, stream()>>>(a);
-        else k_mc<true, true><<<grid, 256, 0, stream()>>>(a);
-    } else if (a.nsteps <= kMtCursorMax) {
-        k_mc<false><<<grid, 256, 0, stream()>>>(a);
+template <bool ANY_LENGTH, bool GUIDED>
+static void launch_mc_form(int grid, int threads, const McArgs &a) {
+    if (a.cf && a.ypaths) k_mc<ANY_LENGTH, GUIDED, true, true><<<grid, threads, 0, stream()>>>(a);
+    else if (a.cf) k_mc<ANY_LENGTH, GUIDED, true, false><<<grid, threads, 0, stream()>>>(a);
+    else if (a.ypaths) k_mc<ANY_LENGTH, GUIDED, false, true><<<grid, threads, 0, stream()>>>(a);
+    else k_mc<ANY_LENGTH, GUIDED, false, false><<<grid, threads, 0, stream()>>>(a);
+}
+static int launch_mc(McArgs &a) {
+    const int grid = mc_grid(a.npaths), threads = mc_threads(a.npaths);
+    const bool guided = a.guide && a.rs >= 0 && a.rs < (1LL << 30);
+    a.rs4 = guided ? (uint32_t)(a.rs * 4) : 0u;
+    if (a.nsteps <= kMtCursorMax) {
+        if (guided) launch_mc_form<false, true>(grid, threads, a);
+        else launch_mc_form<false, false>(grid, threads, a);
     } else {
-        k_mc<true><<<grid, 256, 0, stream()>>>(a);
+        if (guided) launch_mc_form<true, true>(grid, threads, a);
+        else launch_mc_form<true, false>(grid, threads, a);
     }
+    return grid;
 }
 void launch_mt_bench(int grid, uint32_t seed, const uint32_t *seeds, long long nstreams, int nper, float *unif) {
     if (nper <= kMtCursorMax) k_mt_bench<false><<<grid, 256, 0, stream()>>>(seed, seeds, nstreams, nper, unif);
     else k_mt_bench<true><<<grid, 256, 0, stream()>>>(seed, seeds, nstreams, nper, unif);
-}
-
-int mc_grid(long long npaths) {
-    long long b = (npaths + 255) / 256;
-    long long cap = 8LL * num_sms();  // 8 x 256 threads per SM resident
-    if (b > cap) b = cap;
-    return (int)(b < 1 ? 1 : b);
 }
 
 }  // namespace opb
@@ -237,8 +279,7 @@ OPB_API int opb_mc_mt19937(const float *C, long long row_stride, long long col_s
     a.d = d; a.y0 = y0; a.nsteps = nsteps; a.seed = seed; a.path0 = path0; a.npaths = npaths;
     a.ypaths = ypaths; a.x = x; a.strike = strike; a.barrier = barrier; a.disc = disc;
     a.block_sums = x ? scratch : nullptr;
-    int grid = mc_grid(npaths);
-    launch_mc(grid, a);
+    const int grid = launch_mc(a);
     if (x) k_reduce_pairs<<<1, 256, 0, stream()>>>(grid, scratch, sums);
     return launch_check();
 }
@@ -268,8 +309,7 @@ OPB_API int opb_mc_mt19937_eval(const float *C, long long row_stride, long long 
     a.C = C; a.rs = row_stride; a.cs = col_stride; a.guide = guide; a.nb = nb;
     a.d = d; a.y0 = y0; a.nsteps = nsteps; a.seed = seed; a.path0 = path0; a.npaths = npaths;
     a.ypaths = ypaths; a.cf = cashflow; a.ko = knockout; a.pv = path_values; a.block_sums = scratch;
-    const int grid = mc_grid(npaths);
-    launch_mc(grid, a);
+    const int grid = launch_mc(a);
     k_reduce_pairs<<<1, 256, 0, stream()>>>(grid, scratch, sums);
     return launch_check();
 }
@@ -343,7 +383,7 @@ OPB_API int opcuda_mc1f(uint64_t mtptr, int y0, uint64_t y_sk, int nscen, int nk
         a.d = d; a.y0 = y0; a.nsteps = nk; a.path0 = path0; a.npaths = nscen;
         a.seeds = reinterpret_cast<const uint32_t *>(mtptr) + kMcStatusHeader;
         a.ypaths = reinterpret_cast<short *>(y_sk);
-        launch_mc(mc_grid(nscen), a);
+        launch_mc(a);
         OPB_TRY(cudaGetLastError());
     }
     path0 += (unsigned long long)nscen;
@@ -383,7 +423,7 @@ OPB_API int opcuda_mc1f_eval(uint64_t mtptr, int y0, uint64_t y_sk, int nscen, i
         a.cf = reinterpret_cast<const double *>(cashflow);
         a.ko = reinterpret_cast<const unsigned char *>(knockout);
         a.pv = reinterpret_cast<double *>(results);
-        launch_mc(mc_grid(nscen), a);
+        launch_mc(a);
         OPB_TRY(cudaGetLastError());
     }
     path0 += (unsigned long long)nscen;
@@ -426,8 +466,8 @@ OPB_API int opb_mt_uniforms(uint32_t seed, long long nstreams, int nper, float *
 // The per-block payoff partial sums live in a fixed file-scope device array of
 // OPB_MC_NOALLOC_MAX_BLOCKS x 2 doubles (64 KiB), which every GPU that loads the library
 // keeps until the process exits.  The grid is the one opb_mc_mt19937 uses for the same
-// npaths (at most 8 blocks per SM), so results are bit-identical to it; a grid larger than
-// the array -- only possible on a device with more than 512 SMs -- is rejected with
+// npaths (at most 24 blocks per SM), so results are bit-identical to it; a grid larger than
+// the array -- only possible on a device with more than 170 SMs -- is rejected with
 // OPB_E_UNSUPPORTED.  Runs longer than 623 steps are rejected with OPB_E_UNSUPPORTED too:
 // opb_mc_mt19937 serves them with a per-thread local-memory state array, and the CUDA
 // driver may grow its local-memory reservation for that kernel on first use, an allocation

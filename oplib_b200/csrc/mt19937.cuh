@@ -19,12 +19,15 @@
 //   i <  454 : mt'[i] = mt[i+170] ^ tw(mt[i-227], mt[i-226]) ^ tw(mt[i], mt[i+1])
 //   i <  623 : mt'[i] = mt[i-57] ^ tw(mt[i-454], mt[i-453]) ^ tw(mt[i-227], mt[i-226])
 //                       ^ tw(mt[i], mt[i+1])
+// and tw is linear over XOR, so that the cursors' words are XORed first and one tw() is left:
+// tw(a, b) ^ tw(c, d) = tw(a ^ c, b ^ d); the first operand's XOR is the previous word's second.
 // Output 623 would need mt'[0] as the second operand of its tw(), i.e. a word of the
 // regenerated state, which is where the cursor form stops.
 //
 // mt19937_any (any n): the first 623 outputs come from the same cursors, and each
-// regenerated word is also stored in a per-thread 624-word array (local memory on the
-// device, 2496 bytes a thread), so no separate initialisation pass is needed.  Output 623
+// regenerated word that a later output reads is also stored in a per-thread 624-word array
+// (local memory on the device, 2496 bytes a thread), so no separate initialisation pass is
+// needed.  Output 623
 // closes the first regeneration (mt'[623] = mt'[396] ^ tw(mt[623], mt'[0]), with the
 // initial word mt[623] taken from the cursor), and every later output regenerates one word
 // of the array:
@@ -50,12 +53,22 @@ namespace opb {
 // Longest stream mt19937_first serves.
 constexpr int kMtCursorMax = 623;
 
+// Outputs per trip of the output loops: four keep enough independent work in flight that a
+// caller's dependent loads per output do not idle a warp, and no words are moved between
+// registers at the end of one (Monte Carlo at 2^20 paths x 504 steps: 2.30 ms at one output a
+// trip, 2.19 at four).
+constexpr int kMtUnroll = 4;
 OPB_MT_FN uint32_t mt_init_next(uint32_t v, uint32_t i) {
     return 1812433253u * (v ^ (v >> 30)) + i;
 }
 OPB_MT_FN uint32_t mt_tw(uint32_t a, uint32_t b) {
     uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
     return (y >> 1) ^ ((b & 1u) ? 0x9908b0dfu : 0u);
+}
+// x ^ tw(a, b)
+OPB_MT_FN uint32_t mt_tw_xor(uint32_t a, uint32_t b, uint32_t x) {
+    const uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
+    return x ^ (y >> 1) ^ (b & 1u) * 0x9908b0dfu;
 }
 OPB_MT_FN uint32_t mt_temper(uint32_t y) {
     y ^= (y >> 11);
@@ -70,44 +83,51 @@ OPB_MT_FN uint32_t mt_temper(uint32_t y) {
 template <class F>
 OPB_MT_FN uint32_t mt19937_cursor_words(uint32_t seed, uint32_t key1, int n, F &&f) {
     const uint32_t m1 = mt_init_next(seed, 1u) + key1;
-    // cursor A at i: (a0, a1) = (mt[i], mt[i+1])
-    uint32_t a0 = seed, a1 = m1;
+    // cursor A: a1 = mt[i+1]; x0 = mt[i], from phase 2 on with the other cursors' words in it
+    uint32_t x0 = seed, a1 = m1, a0 = seed;
     // cursor B at i + 397
     uint32_t b = m1;
-#pragma unroll 1
+#pragma unroll 4
     for (uint32_t j = 2; j <= 397; j++) b = mt_init_next(b, j);
     const uint32_t m397 = b;
     uint32_t bi = 397;
     int i = 0;
     const int n1 = n < 227 ? n : 227;
-#pragma unroll 1
+#pragma unroll kMtUnroll
     for (; i < n1; i++) {
-        f(i, b ^ mt_tw(a0, a1));
-        a0 = a1; a1 = mt_init_next(a1, (uint32_t)i + 2u);
+        f(i, mt_tw_xor(x0, a1, b));
+        x0 = a0 = a1;
+        a1 = mt_init_next(a1, (uint32_t)i + 2u);
         bi++; b = mt_init_next(b, bi);
     }
     if (i >= n) return a0;
-    // phase 2: cursor C at i-227 from the seed, cursor B restarted at 397
-    uint32_t c0 = seed, c1 = m1;
+    // phase 2: cursor C (c1 = mt[i-226]) from the seed, cursor B restarted at 397
+    uint32_t c1 = m1;
+    x0 ^= seed;
     b = m397; bi = 397;
     const int n2 = n < 454 ? n : 454;
-#pragma unroll 1
+#pragma unroll kMtUnroll
     for (; i < n2; i++) {
-        f(i, b ^ mt_tw(c0, c1) ^ mt_tw(a0, a1));
-        a0 = a1; a1 = mt_init_next(a1, (uint32_t)i + 2u);
-        c0 = c1; c1 = mt_init_next(c1, (uint32_t)(i - 227) + 2u);
+        const uint32_t x1 = a1 ^ c1;
+        f(i, mt_tw_xor(x0, x1, b));
+        x0 = x1; a0 = a1;
+        a1 = mt_init_next(a1, (uint32_t)i + 2u);
+        c1 = mt_init_next(c1, (uint32_t)(i - 227) + 2u);
         bi++; b = mt_init_next(b, bi);
     }
     if (i >= n) return a0;
-    // phase 3: cursor D at i-454 from the seed, B restarted at 397 (= i-57 at i = 454)
-    uint32_t d0 = seed, d1 = m1;
+    // phase 3: cursor D (d1 = mt[i-453]) from the seed, B restarted at 397 (= i-57 at i = 454)
+    uint32_t d1 = m1;
+    x0 ^= seed;
     b = m397; bi = 397;
-#pragma unroll 1
+#pragma unroll kMtUnroll
     for (; i < n; i++) {
-        f(i, b ^ mt_tw(d0, d1) ^ mt_tw(c0, c1) ^ mt_tw(a0, a1));
-        a0 = a1; a1 = mt_init_next(a1, (uint32_t)i + 2u);
-        c0 = c1; c1 = mt_init_next(c1, (uint32_t)(i - 227) + 2u);
-        d0 = d1; d1 = mt_init_next(d1, (uint32_t)(i - 454) + 2u);
+        const uint32_t x1 = a1 ^ c1 ^ d1;
+        f(i, mt_tw_xor(x0, x1, b));
+        x0 = x1; a0 = a1;
+        a1 = mt_init_next(a1, (uint32_t)i + 2u);
+        c1 = mt_init_next(c1, (uint32_t)(i - 227) + 2u);
+        d1 = mt_init_next(d1, (uint32_t)(i - 454) + 2u);
         bi++; b = mt_init_next(b, bi);
     }
     return a0;
@@ -124,8 +144,10 @@ template <class F>
 OPB_MT_FN void mt19937_any(uint32_t seed, uint32_t key1, int n, F &&f) {
     uint32_t mt[624];
     const int n1 = n < kMtCursorMax ? n : kMtCursorMax;
+    // output 623 + j reads words j - 1, j and (j + 396) mod 624
+    const uint32_t more = n > kMtCursorMax ? (uint32_t)(n - kMtCursorMax) : 0u;
     const uint32_t init623 = mt19937_cursor_words(seed, key1, n1, [&](int k, uint32_t w) {
-        mt[k] = w;
+        if ((uint32_t)k < more || (uint32_t)(k - 396) < more) mt[k] = w;
         f(k, mt_temper(w));
     });
     if (n <= kMtCursorMax) return;
