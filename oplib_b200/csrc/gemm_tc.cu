@@ -91,6 +91,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if (gtimer() - t0 > limit_ns) return false;
     }
 }
+// The warp's wait: every lane waits, and the answer is the warp's.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag,
+                                               unsigned long long limit_ns) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit_ns));
+}
+// True in one lane of a converged warp, the same one each time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(e)::"memory");
+    return e != 0;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
@@ -430,7 +442,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
     const uint32_t bres_bar = bar0 + 8u * (2 * STAGES + 7);        // resident B loaded
     const uint32_t bres_base = base + STAGES * Cfg::STAGE_BYTES;   // resident B, K-block kb at + kb * B_BYTES
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int mtiles = p.M / Cfg::TILE_M, ntiles_n = p.N / BN;
     const int nsplit = (!BATCHED && p.ksplit > 1) ? p.ksplit : 1;  // K-slices of a single product
     int nitems = BATCHED ? bt.nwork : mtiles * ntiles_n * nsplit;
@@ -644,14 +656,18 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                                         100000000ull);
             }
         }
-        if (warp == EPI + 1 && lane == 0 && rank == 0) {
+        if (warp == EPI + 1 && rank == 0) {
             // ---------------- MMA issuer (pair mode: the even CTA issues for both)
+            // The whole warp walks the loop and one elected lane issues: in code that one lane
+            // runs alone the descriptors' way into the uniform registers, which is where the
+            // MMA takes them from, costs more than a narrow MMA (1024 states of 64-wide tiles
+            // 17.5 -> 15.7 us, the quoted row's step at d = 6144 71 -> 60).
             const uint32_t idesc = umma_idesc_16(BN, F16, Cfg::TILE_M, BMN);
             long kbg = 0, g = 0;  // K-blocks consumed, chunks issued
             bool ok = true;
             if constexpr (Cfg::BRES) {
                 if (item0 < nitems) {
-                    ok = mbar_wait(bres_bar, 0u, abort_flag, TC_WAIT_NS);
+                    ok = mbar_wait_warp(bres_bar, 0u, abort_flag, TC_WAIT_NS);
                     tc_fence_after();
                 }
             }
@@ -672,7 +688,8 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                         if (!bits) continue;
                     }
                     const int a = (int)(g & 1);
-                    if (g >= 2 && !mbar_wait(acce_bar(a), (uint32_t)(((g >> 1) + 1) & 1), abort_flag, TC_WAIT_NS)) {
+                    if (g >= 2 &&
+                        !mbar_wait_warp(acce_bar(a), (uint32_t)(((g >> 1) + 1) & 1), abort_flag, TC_WAIT_NS)) {
                         ok = false;
                         break;
                     }
@@ -683,7 +700,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     for (int kb = c * Cfg::CHUNK; kb < kb_end; kb++) {
                         if (PLANNED && mk && !((bits >> (kb - c * Cfg::CHUNK)) & 1u)) continue;
                         const int s = (int)(kbg % STAGES);
-                        if (!mbar_wait(full_bar(s), (uint32_t)((kbg / STAGES) & 1), abort_flag, TC_WAIT_NS)) {
+                        if (!mbar_wait_warp(full_bar(s), (uint32_t)((kbg / STAGES) & 1), abort_flag, TC_WAIT_NS)) {
                             ok = false;
                             break;
                         }
@@ -696,32 +713,34 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                         const uint32_t sBl = st + 2 * Cfg::A_BYTES + Cfg::B_BYTES;
                         const uint64_t dBh = BMN ? umma_desc_mn<BK>(sBh) : umma_desc_sw<BK>(sBh);
                         const uint64_t dBl = BMN ? umma_desc_mn<BK>(sBl) : umma_desc_sw<BK>(sBl);
+                        if (elect_one()) {
 #pragma unroll
-                        for (int k16 = 0; k16 < BK / 16; k16++) {
-                            const uint64_t adv = (uint64_t)((k16 * 32) >> 4);  // +32 bytes along K
-                            // MN-major B: +16 rows of 128 bytes along K
-                            const uint64_t advb = BMN ? (uint64_t)((k16 * 16 * 128) >> 4) : adv;
-                            const uint32_t acc0 = k16 > 0 ? 1u : fresh;
-                            if constexpr (PAIR) {
-                                umma_bf16_pair(dacc, dAh + adv, dBh + advb, idesc, acc0);
-                                umma_bf16_pair(dacc, dAh + adv, dBl + advb, idesc, 1u);
-                                umma_bf16_pair(dacc, dAl + adv, dBh + advb, idesc, 1u);
-                                if (lolo) umma_bf16_pair(dacc, dAl + adv, dBl + advb, idesc, 1u);
-                            } else {
-                                umma_bf16(dacc, dAh + adv, dBh + advb, idesc, acc0);
-                                if constexpr (NPROD == 3) {
-                                    umma_bf16(dacc, dAh + adv, dBl + advb, idesc, 1u);
-                                    umma_bf16(dacc, dAl + adv, dBh + advb, idesc, 1u);
-                                    if (lolo) umma_bf16(dacc, dAl + adv, dBl + advb, idesc, 1u);
+                            for (int k16 = 0; k16 < BK / 16; k16++) {
+                                const uint64_t adv = (uint64_t)((k16 * 32) >> 4);  // +32 bytes along K
+                                // MN-major B: +16 rows of 128 bytes along K
+                                const uint64_t advb = BMN ? (uint64_t)((k16 * 16 * 128) >> 4) : adv;
+                                const uint32_t acc0 = k16 > 0 ? 1u : fresh;
+                                if constexpr (PAIR) {
+                                    umma_bf16_pair(dacc, dAh + adv, dBh + advb, idesc, acc0);
+                                    umma_bf16_pair(dacc, dAh + adv, dBl + advb, idesc, 1u);
+                                    umma_bf16_pair(dacc, dAl + adv, dBh + advb, idesc, 1u);
+                                    if (lolo) umma_bf16_pair(dacc, dAl + adv, dBl + advb, idesc, 1u);
+                                } else {
+                                    umma_bf16(dacc, dAh + adv, dBh + advb, idesc, acc0);
+                                    if constexpr (NPROD == 3) {
+                                        umma_bf16(dacc, dAh + adv, dBl + advb, idesc, 1u);
+                                        umma_bf16(dacc, dAl + adv, dBh + advb, idesc, 1u);
+                                        if (lolo) umma_bf16(dacc, dAl + adv, dBl + advb, idesc, 1u);
+                                    }
                                 }
                             }
+                            if constexpr (PAIR) umma_commit_pair(empty_bar(s));
+                            else umma_commit(empty_bar(s));
                         }
                         fresh = 1u;
-                        if constexpr (PAIR) umma_commit_pair(empty_bar(s));
-                        else umma_commit(empty_bar(s));
                         kbg++;
                     }
-                    if (ok) {
+                    if (ok && elect_one()) {
                         if constexpr (PAIR) umma_commit_pair(accf_bar(a));
                         else umma_commit(accf_bar(a));
                     }
@@ -733,8 +752,10 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                 *abort_flag = 1;
             }
             // arrives once every issued MMA has completed
-            if constexpr (PAIR) umma_commit_pair(drain_bar);
-            else umma_commit(drain_bar);
+            if (elect_one()) {
+                if constexpr (PAIR) umma_commit_pair(drain_bar);
+                else umma_commit(drain_bar);
+            }
             (void)mbar_wait(drain_bar, 0, abort_flag, TC_WAIT_NS);
         }
         __syncwarp();

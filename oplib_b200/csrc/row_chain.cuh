@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(RS_THREADS)
     auto acce_bar = [&](int a) { return bar0 + 8u * (2 * RS_MAX_STAGES + RS_ACC + a); };
     const uint32_t row_bar = bar0 + 8u * (2 * RS_MAX_STAGES + 2 * RS_ACC);
     const uint32_t drain_bar = row_bar + 8u;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     const int m = p.m;
     const uint32_t ring = base + (uint32_t)row_step_atoms(p.dmax) * 4096u;
@@ -200,42 +200,42 @@ __global__ void __launch_bounds__(RS_THREADS)
         }
         __syncwarp();
     } else if (warp == 5) {
-        if (lane == 0) {
-            // ---------------- MMA issuer
-            const uint32_t idesc = umma_idesc_16(RS_BN, F16, TC_BM, true);
-            long kbg = 0, g = 0;
-            int item = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < nitems && ok; t += gridDim.x, item++) {
-                int n0;
-                const int li = lattice(t, n0);
-                const int d = BATCHED ? lats[li].d : one.d;
-                const int natoms = row_step_atoms(d);
-                if (!mbar_wait(row_bar, (uint32_t)(item & 1), abort_flag, TC_WAIT_NS)) {
+        // ---------------- MMA issuer: the whole warp walks the loop, one elected lane issues
+        const uint32_t idesc = umma_idesc_16(RS_BN, F16, TC_BM, true);
+        long kbg = 0, g = 0;
+        int item = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < nitems && ok; t += gridDim.x, item++) {
+            int n0;
+            const int li = lattice(t, n0);
+            const int d = BATCHED ? lats[li].d : one.d;
+            const int natoms = row_step_atoms(d);
+            if (!mbar_wait_warp(row_bar, (uint32_t)(item & 1), abort_flag, TC_WAIT_NS)) {
+                ok = false;
+                break;
+            }
+            for (int c = 0; c < d / 128 && ok; c++, g++) {
+                const int a = (int)(g % RS_ACC);
+                if (g >= RS_ACC &&
+                    !mbar_wait_warp(acce_bar(a), (uint32_t)(((g / RS_ACC) + 1) & 1), abort_flag, TC_WAIT_NS)) {
                     ok = false;
                     break;
                 }
-                for (int c = 0; c < d / 128 && ok; c++, g++) {
-                    const int a = (int)(g % RS_ACC);
-                    if (g >= RS_ACC &&
-                        !mbar_wait(acce_bar(a), (uint32_t)(((g / RS_ACC) + 1) & 1), abort_flag, TC_WAIT_NS)) {
+                tc_fence_after();
+                const uint32_t dacc = tmem + (uint32_t)(a * RS_BN);
+                for (int half = 0; half < 2; half++, kbg++) {
+                    const int s = (int)(kbg % p.stages);
+                    if (!mbar_wait_warp(full_bar(s), (uint32_t)((kbg / p.stages) & 1), abort_flag, TC_WAIT_NS)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t dacc = tmem + (uint32_t)(a * RS_BN);
-                    for (int half = 0; half < 2; half++, kbg++) {
-                        const int s = (int)(kbg % p.stages);
-                        if (!mbar_wait(full_bar(s), (uint32_t)((kbg / p.stages) & 1), abort_flag, TC_WAIT_NS)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t arow = base + (uint32_t)(half * natoms + (c >> 3)) * 1024u;
-                        const uint64_t dAh = umma_desc_sw<TC_BK>(arow);
-                        const uint64_t dAl = umma_desc_sw<TC_BK>(arow + (uint32_t)(2 * natoms) * 1024u);
-                        const uint64_t dBh = umma_desc_mn<TC_BK>(ring + s * RS_STAGE);
-                        const uint64_t dBl = umma_desc_mn<TC_BK>(ring + s * RS_STAGE + RS_BOX);
+                    const uint32_t arow = base + (uint32_t)(half * natoms + (c >> 3)) * 1024u;
+                    const uint64_t dAh = umma_desc_sw<TC_BK>(arow);
+                    const uint64_t dAl = umma_desc_sw<TC_BK>(arow + (uint32_t)(2 * natoms) * 1024u);
+                    const uint64_t dBh = umma_desc_mn<TC_BK>(ring + s * RS_STAGE);
+                    const uint64_t dBl = umma_desc_mn<TC_BK>(ring + s * RS_STAGE + RS_BOX);
+                    if (elect_one()) {
 #pragma unroll
                         for (int k16 = 0; k16 < TC_BK / 16; k16++) {
                             const uint64_t adv = (uint64_t)((k16 * 32) >> 4), advb = (uint64_t)((k16 * 16 * 128) >> 4);
@@ -245,16 +245,16 @@ __global__ void __launch_bounds__(RS_THREADS)
                         }
                         umma_commit(empty_bar(s));
                     }
-                    if (ok) umma_commit(accf_bar(a));
                 }
+                if (ok && elect_one()) umma_commit(accf_bar(a));
             }
-            if (!ok) {
-                atomicExch(&g_tc_error, 22);
-                *abort_flag = 1;
-            }
-            umma_commit(drain_bar);
-            (void)mbar_wait(drain_bar, 0, abort_flag, TC_WAIT_NS);
         }
+        if (!ok) {
+            atomicExch(&g_tc_error, 22);
+            *abort_flag = 1;
+        }
+        if (elect_one()) umma_commit(drain_bar);
+        (void)mbar_wait_warp(drain_bar, 0, abort_flag, TC_WAIT_NS);
         __syncwarp();
     } else {
         // ---------------- the row's parts, the chunk sums, the item's columns

@@ -1,6 +1,6 @@
 """Monte Carlo at the path counts where the launch shape changes (64, 128, 256 threads a block, a
 second path a thread) and at the run lengths where the generator's loops end, against the
-oracle's paths; cumulative rows and guide tables at the widths where their tiles end."""
+oracle's paths."""
 import numpy as np
 import pytest
 import torch
