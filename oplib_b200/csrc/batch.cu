@@ -126,7 +126,7 @@ struct opb_batch_plan {
     std::vector<ListRef> gemm_level[NCFG];
     ListRef gemm_price;                // every 128-row tile (the induction's products)
     ListRef gemm_rows;                 // one tile per lattice (the priced rows)
-    ListRef row_items;                 // the chained rows' 64-column items
+    ListRef row_items;                 // the chained rows' 128-column items
     std::vector<ListRef> rn_level;     // per level: the lattices whose last level it is (P1)
     ListRef rn_init;
     // FP32 path
@@ -311,7 +311,7 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     grw.n = (int)(W.size() - grw.off);
     ListRef gri{W.size(), 0};
     for (int i : lpt)
-        for (int a = 0; a < b->d[i] / 64; a++) W.push_back(((uint32_t)i << 16) | (uint32_t)a);
+        for (int a = 0; a < b->d[i] / 128; a++) W.push_back(((uint32_t)i << 16) | (uint32_t)a);
     gri.n = (int)(W.size() - gri.off);
     auto rn_list = [&](int level, int kind) {  // kind: 0 init split, 1 the lattices ending at `level`
         ListRef r{W.size(), 0};

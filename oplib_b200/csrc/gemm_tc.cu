@@ -143,20 +143,19 @@ __device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr) {
 }
 
 // kind::f16 instruction descriptor: D = F32, A = B = BF16 (format 1) or F16 (format 0),
-// A K-major, B K-major or (bmn) MN-major, N, M (128 for one CTA, 256 for a CTA pair).
-__host__ __device__ constexpr uint32_t umma_idesc_16(int n, bool f16, int m = TC_BM, bool bmn = false) {
-    return (1u << 4) | ((f16 ? 0u : 1u) << 7) | ((f16 ? 0u : 1u) << 10) | ((bmn ? 1u : 0u) << 16) |
-           ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+// A and B K-major or (amn, bmn) MN-major, N, M (128 for one CTA, 256 for a CTA pair).
+__host__ __device__ constexpr uint32_t umma_idesc_16(int n, bool f16, int m = TC_BM, bool bmn = false, bool amn = false) {
+    return (1u << 4) | ((f16 ? 0u : 1u) << 7) | ((f16 ? 0u : 1u) << 10) | ((amn ? 1u : 0u) << 15) |
+           ((bmn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
-    uint32_t z = 0;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {

@@ -397,7 +397,7 @@ int launch_row_step(const RowChainLat &L, const __nv_bfloat16 *Bhi, const __nv_b
                     float alpha, float sscale, cudaStream_t s);
 // P_m's row into its slot, after the last step.
 int launch_row_finish(const RowChainLat &L, int m, int fused, float sscale, cudaStream_t s);
-// All lattices of a plan: work items lattice << 16 | 64-column tile, maps 4 per lattice (the
+// All lattices of a plan: work items lattice << 16 | 128-column tile, maps 4 per lattice (the
 // last two P1's parts, MN-major), dmax the largest size.
 int launch_row_step_batched(const RowChainLat *lats, const CUtensorMap *maps, const uint32_t *work, int nwork, int dmax,
                             int m, int f16, float alpha, float sscale, cudaStream_t s);

@@ -11,29 +11,38 @@
 //
 // What bounds it: one pass over P1's parts per maturity (4 d^2 bytes, 151 MB at d = 6144:
 // 23 us of HBM) instead of a d^3 product; at d <= 2048 P1 stays in L2 and the chain of
-// dependent launches is what is left.  One item is 64 columns of the row: 96 CTAs stream P1
-// at d = 6144, each through a ring of 16 KB stages (hi and lo boxes of 64 x 64).  128-wide
-// items halve the CTAs that stream, and a CTA's stream, not the MMAs, is the limit.
+// dependent launches is what is left.  One item is 64 columns of the row, or 128 in the
+// batched form, where the SMs are full anyway; its P1 boxes (64 of K, hi and lo) come through a
+// ring of shared-memory stages.
 //
-// The MMA's M is 128 and one row of it is wanted.  The row's 128 K-values of chunk c sit in
-// row c % 8 of an 8-row swizzle atom (one atom for the chunk's first 64 of K, one for the
-// second), so the whole row takes 4 d bytes of shared memory instead of the 512 d of a
-// 128-row operand, and chunk c's sums are in TMEM lane c % 8.  The other rows multiply
-// whatever lies in shared memory there (other chunks' values, the ring): rows do not mix,
-// and nobody reads those lanes.
+// P1's columns are the MMA's M (M-major, as they lie in memory) and the row is its N, so that
+// the results are one TMEM column: each epilogue thread owns one column of the row and adds
+// its chunks in order.  (With the row as one of M's 128 rows the chunk sums lay across one
+// lane and went through shared memory.)  An MMA costs about 40 cycles however few columns it
+// has, and the issuing warp's own instructions between them count as much: at d = 6144 a step
+// took 60 us with a 64-bit modulo for the ring position, 43 without, 40 without the MMA's
+// optional lane mask; the loads alone take 26.
+//
+// The row's 128 K-values of chunk c sit in row c % 8 of an 8-row swizzle atom (one atom for the
+// chunk's first 64 of K, one for the second), so the whole row takes 4 d bytes of shared
+// memory, and chunk c's sums are in column c % 8.  N is 16, two atoms; the other rows multiply
+// whatever lies in shared memory there (other chunks' values, the ring), as do the 64 M-rows
+// past a 64-column item's box: neither rows nor columns mix, and nobody reads those sums.
 //
 // Measured on B200, whole calls, full chain products -> quoted row: the SV solve (d = 6144, 16
-// maturities) 24.65 -> 10.91 ms, its 15 chain products of 873 us becoming 15 row steps of 71 us;
-// 512 nodes, 8 maturities 481 -> 345 us (11.9 + 3.8 us of product and renormalisation per
-// maturity -> 9.3 us, and one pricing product for all); 256 lattices of the sweep 60.8 -> 38.7 ms.
+// maturities) 24.65 -> 10.91 ms, its 15 chain products of 873 us becoming 15 row steps of 71 us
+// (40 now); 512 nodes, 8 maturities 481 -> 345 us (11.9 + 3.8 us of product and
+// renormalisation per maturity -> 9.3 us, and one pricing product for all); 256 lattices of the
+// sweep 60.8 -> 38.7 ms.
 
-constexpr int RS_BN = 64;           // columns per item
-constexpr int RS_BOX = 64 * 64 * 2; // one 64 x 64 box of B parts
-constexpr int RS_STAGE = 2 * RS_BOX;
-constexpr int RS_ACC = 4;           // TMEM accumulators (64 columns each)
-constexpr int RS_PREP = 128;        // threads that prepare the row and finish the columns
+constexpr int RS_N = 16;        // the MMA's N: two 8-row atoms of the row
+constexpr int RS_ACC = 8;       // TMEM accumulators (RS_N columns each)
+constexpr int RS_PREP = 256;    // threads that prepare the row; the first W finish the columns
 constexpr int RS_THREADS = RS_PREP + 64;
 constexpr int RS_MAX_STAGES = 8, RS_MIN_STAGES = 3;
+constexpr int RS_MAX_D = 30336;
+
+__host__ __device__ constexpr int row_step_part(int w) { return w * 64 * 2; }  // W columns x 64 of K, one part
 
 struct RowStepParams {
     int m;           // the maturity this launch forms (P_m from P_{m-1}); m >= 2
@@ -44,9 +53,10 @@ struct RowStepParams {
 };
 
 __host__ __device__ inline int row_step_atoms(int d) { return (d / 128 + 7) / 8; }
-// shared memory: the row's parts (2 parts x 2 halves of a chunk), the ring, the chunk sums
-__host__ inline int row_step_smem(int d, int stages) {
-    return row_step_atoms(d) * 4096 + stages * RS_STAGE + (d / 128) * RS_BN * 4 + 1024 + 256;
+// shared memory: the row's parts (2 parts x 2 halves of a chunk), the ring, and behind it what a
+// 64-column item's MMA reads past the last stage's low parts
+__host__ inline int row_step_smem(int d, int w, int stages) {
+    return row_step_atoms(d) * 4096 + stages * 2 * row_step_part(w) + (w < 128 ? 8192 : 0) + 1024;
 }
 
 // The row of P_{m-1} as operand parts: P1's own for m = 2, else from the FP32 row that the
@@ -71,7 +81,9 @@ __device__ __forceinline__ double row_parts(const RowChainLat &L, const RowStepP
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((tid & 31) == 0) red[tid >> 5] = s;
     asm volatile("bar.sync 1, %0;" ::"n"(RS_PREP) : "memory");
-    s = red[0] + red[1] + red[2] + red[3];
+    s = 0.0;
+#pragma unroll
+    for (int i = 0; i < RS_PREP / 32; i++) s += red[i];
     const double inv = s != 0.0 ? 1.0 / s : 0.0;
     for (int j = tid; j < n8; j += RS_PREP) {
         const float4 a = c4[2 * j], b = c4[2 * j + 1];
@@ -97,17 +109,26 @@ __device__ __forceinline__ void row_slot(const RowChainLat &L, int m, int e, con
     *reinterpret_cast<uint4 *>(L.Qlo + o) = l;
 }
 
+// One column of an accumulator, 32 rows a warp.
+__device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
+    uint32_t v;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v)::"memory");
+    return __uint_as_float(v);
+}
+
 template <bool BATCHED, bool F16>
 __global__ void __launch_bounds__(RS_THREADS)
     k_row_step(const __grid_constant__ CUtensorMap mBhi, const __grid_constant__ CUtensorMap mBlo, RowChainLat one,
                RowStepParams p, const RowChainLat *__restrict__ lats, const CUtensorMap *__restrict__ maps,
                const uint32_t *__restrict__ work, int nitems) {
+    constexpr int W = BATCHED ? 128 : 64, PART = row_step_part(W), STAGE = 2 * PART;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *gbase = smem_raw + (base - raw);
     __shared__ uint64_t bars[2 * RS_MAX_STAGES + 2 * RS_ACC + 2];
-    __shared__ double red[4];
+    __shared__ double red[RS_PREP / 32];
     __shared__ uint32_t tmem_slot_s;
     __shared__ int abort_s;
     volatile int *abort_flag = &abort_s;
@@ -122,15 +143,14 @@ __global__ void __launch_bounds__(RS_THREADS)
 
     const int m = p.m;
     const uint32_t ring = base + (uint32_t)row_step_atoms(p.dmax) * 4096u;
-    float *sums = reinterpret_cast<float *>(gbase + row_step_atoms(p.dmax) * 4096 + p.stages * RS_STAGE);
     // item t -> lattice, first column
     auto lattice = [&](int t, int &n0) -> int {
         if constexpr (BATCHED) {
             const uint32_t w = work[t];
-            n0 = (int)(w & 0xffffu) * RS_BN;
+            n0 = (int)(w & 0xffffu) * W;
             return (int)(w >> 16);
         } else {
-            n0 = t * RS_BN;
+            n0 = t * W;
             return 0;
         }
     };
@@ -142,7 +162,7 @@ __global__ void __launch_bounds__(RS_THREADS)
         }
         for (int a = 0; a < RS_ACC; a++) {
             mbar_init(accf_bar(a), 1);
-            mbar_init(acce_bar(a), 1);
+            mbar_init(acce_bar(a), W / 32);
         }
         mbar_init(row_bar, RS_PREP);
         mbar_init(drain_bar, 1);
@@ -152,7 +172,7 @@ __global__ void __launch_bounds__(RS_THREADS)
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot_s)),
-                     "r"(RS_ACC * RS_BN)
+                     "r"(RS_ACC * RS_N)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -160,12 +180,15 @@ __global__ void __launch_bounds__(RS_THREADS)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot_s);
-    pdl_begin();  // (the shared and tensor memory set up while the previous step ran)
 
-    if (warp == 4) {
+    if (warp == RS_PREP / 32) {
         if (lane == 0) {
-            // ---------------- TMA producer: P1's parts, 64 rows of K x 64 columns at a time
-            long kbg = 0;
+            // ---------------- TMA producer: P1's parts, 64 rows of K x W columns at a time.  From
+            // m = 3 on P1 was there before the step that this launch follows (that step waited
+            // for it), so the ring fills without waiting for that step.
+            if (BATCHED || m == 2) pdl_wait();
+            int s = 0, issued = 0;
+            uint32_t ph = 1;  // the parity that a free stage's barrier has passed
             bool ok = true;
             for (int t = blockIdx.x; t < nitems && ok; t += gridDim.x) {
                 int n0;
@@ -177,33 +200,45 @@ __global__ void __launch_bounds__(RS_THREADS)
                     bl = maps + 4 * li + 3;
                     d = lats[li].d;
                 }
-                for (int kb = 0; kb < d / 64; kb++, kbg++) {
-                    const int s = (int)(kbg % p.stages);
-                    if (kbg >= p.stages &&
-                        !mbar_wait(empty_bar(s), (uint32_t)(((kbg / p.stages) + 1) & 1), abort_flag, TC_WAIT_NS)) {
+                for (int kb = 0; kb < d / 64; kb++) {
+                    if (issued == p.stages && !mbar_wait(empty_bar(s), ph, abort_flag, TC_WAIT_NS)) {
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(full_bar(s), RS_STAGE);
-                    tma_load_2d(ring + s * RS_STAGE, bh, full_bar(s), n0, kb * 64);
-                    tma_load_2d(ring + s * RS_STAGE + RS_BOX, bl, full_bar(s), n0, kb * 64);
+                    mbar_expect_tx(full_bar(s), STAGE);
+#pragma unroll
+                    for (int i = 0; i < W / 64; i++) {
+                        const uint32_t at = ring + s * STAGE + i * 8192;
+                        tma_load_2d(at, bh, full_bar(s), n0 + 64 * i, kb * 64);
+                        tma_load_2d(at + PART, bl, full_bar(s), n0 + 64 * i, kb * 64);
+                    }
+                    if (issued < p.stages) issued++;
+                    if (++s == p.stages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
                 }
             }
             if (!ok) {
                 atomicExch(&g_tc_error, 21);
                 *abort_flag = 1;
-                const long first = kbg > p.stages ? kbg - p.stages : 0;
-                for (long k = first; k < kbg; k++)
-                    (void)mbar_wait(full_bar((int)(k % p.stages)), (uint32_t)((k / p.stages) & 1), abort_flag,
-                                    100000000ull);
+                // (bounded) for the copies in flight: the ring's last use of each stage; ph is 1 in
+                // the even rounds of the ring
+                for (int k = 0; k < issued; k++) {
+                    s = s == 0 ? p.stages - 1 : s - 1;
+                    if (s == p.stages - 1) ph ^= 1;
+                    (void)mbar_wait(full_bar(s), ph ^ 1, abort_flag, 100000000ull);
+                }
             }
         }
         __syncwarp();
-    } else if (warp == 5) {
+    } else if (warp == RS_PREP / 32 + 1) {
         // ---------------- MMA issuer: the whole warp walks the loop, one elected lane issues
-        const uint32_t idesc = umma_idesc_16(RS_BN, F16, TC_BM, true);
-        long kbg = 0, g = 0;
-        int item = 0;
+        if (BATCHED) pdl_wait();
+        const uint32_t idesc = umma_idesc_16(RS_N, F16, TC_BM, false, true);
+        int s = 0, item = 0;
+        uint32_t ph = 0;
+        unsigned g = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < nitems && ok; t += gridDim.x, item++) {
             int n0;
@@ -216,34 +251,36 @@ __global__ void __launch_bounds__(RS_THREADS)
             }
             for (int c = 0; c < d / 128 && ok; c++, g++) {
                 const int a = (int)(g % RS_ACC);
-                if (g >= RS_ACC &&
-                    !mbar_wait_warp(acce_bar(a), (uint32_t)(((g / RS_ACC) + 1) & 1), abort_flag, TC_WAIT_NS)) {
+                if (g >= RS_ACC && !mbar_wait_warp(acce_bar(a), ((g / RS_ACC) + 1) & 1, abort_flag, TC_WAIT_NS)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t dacc = tmem + (uint32_t)(a * RS_BN);
-                for (int half = 0; half < 2; half++, kbg++) {
-                    const int s = (int)(kbg % p.stages);
-                    if (!mbar_wait_warp(full_bar(s), (uint32_t)((kbg / p.stages) & 1), abort_flag, TC_WAIT_NS)) {
+                const uint32_t dacc = tmem + (uint32_t)(a * RS_N);
+                for (int half = 0; half < 2; half++) {
+                    if (!mbar_wait_warp(full_bar(s), ph, abort_flag, TC_WAIT_NS)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t arow = base + (uint32_t)(half * natoms + (c >> 3)) * 1024u;
-                    const uint64_t dAh = umma_desc_sw<TC_BK>(arow);
-                    const uint64_t dAl = umma_desc_sw<TC_BK>(arow + (uint32_t)(2 * natoms) * 1024u);
-                    const uint64_t dBh = umma_desc_mn<TC_BK>(ring + s * RS_STAGE);
-                    const uint64_t dBl = umma_desc_mn<TC_BK>(ring + s * RS_STAGE + RS_BOX);
+                    const uint32_t brow = base + (uint32_t)(half * natoms + (c >> 3)) * 1024u;
+                    const uint64_t dBh = umma_desc_sw<TC_BK>(brow);
+                    const uint64_t dBl = umma_desc_sw<TC_BK>(brow + (uint32_t)(2 * natoms) * 1024u);
+                    const uint64_t dAh = umma_desc_mn<TC_BK>(ring + s * STAGE);
+                    const uint64_t dAl = umma_desc_mn<TC_BK>(ring + s * STAGE + PART);
                     if (elect_one()) {
 #pragma unroll
                         for (int k16 = 0; k16 < TC_BK / 16; k16++) {
-                            const uint64_t adv = (uint64_t)((k16 * 32) >> 4), advb = (uint64_t)((k16 * 16 * 128) >> 4);
+                            const uint64_t adv = (uint64_t)((k16 * 16 * 128) >> 4), advb = (uint64_t)((k16 * 32) >> 4);
                             umma_bf16(dacc, dAh + adv, dBh + advb, idesc, (half || k16) ? 1u : 0u);
-                            umma_bf16(dacc, dAh + adv, dBl + advb, idesc, 1u);
                             umma_bf16(dacc, dAl + adv, dBh + advb, idesc, 1u);
+                            umma_bf16(dacc, dAh + adv, dBl + advb, idesc, 1u);
                         }
                         umma_commit(empty_bar(s));
+                    }
+                    if (++s == p.stages) {
+                        s = 0;
+                        ph ^= 1;
                     }
                 }
                 if (ok && elect_one()) umma_commit(accf_bar(a));
@@ -255,10 +292,10 @@ __global__ void __launch_bounds__(RS_THREADS)
         }
         if (elect_one()) umma_commit(drain_bar);
         (void)mbar_wait_warp(drain_bar, 0, abort_flag, TC_WAIT_NS);
-        __syncwarp();
     } else {
         // ---------------- the row's parts, the chunk sums, the item's columns
-        long g = 0;
+        pdl_begin();
+        unsigned g = 0;
         int held = -1;  // the lattice whose row is in shared memory
         double inv = 1.0;
         bool ok = true;
@@ -282,51 +319,37 @@ __global__ void __launch_bounds__(RS_THREADS)
                 held = li;
             }
             asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(row_bar) : "memory");
-            if (warp == 0) {
+            if (warp < W / 32) {
+                float acc = 0.f;
                 for (int c = 0; c < nch; c++, g++) {
                     const int a = (int)(g % RS_ACC);
-                    if (ok && !mbar_wait(accf_bar(a), (uint32_t)((g / RS_ACC) & 1), abort_flag, TC_WAIT_NS)) {
+                    if (ok && !mbar_wait_warp(accf_bar(a), (g / RS_ACC) & 1, abort_flag, TC_WAIT_NS)) {
                         atomicExch(&g_tc_error, 23);
                         *abort_flag = 1;
                         ok = false;
                     }
-                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
-#pragma unroll
-                    for (int hb = 0; hb < 2; hb++) {
-                        uint32_t v[32];
-                        tmem_ld32(tmem + (uint32_t)(a * RS_BN + 32 * hb), v);
-                        if (lane == (c & 7)) {
-                            uint4 *dst = reinterpret_cast<uint4 *>(sums + c * RS_BN + 32 * hb);
-#pragma unroll
-                            for (int i = 0; i < 8; i++) dst[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                        }
-                    }
+                    acc = __fadd_rn(acc, tmem_ld1(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(a * RS_N + (c & 7))));
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0)
                         asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(acce_bar(a)) : "memory");
                 }
-            }
-            // (after a failed wait the loop runs on without waiting, so that every thread meets
-            // the barriers; the error word tells the caller)
-            asm volatile("bar.sync 1, %0;" ::"n"(RS_PREP) : "memory");
-            if (threadIdx.x < RS_BN) {
-                float acc = 0.f;
-                for (int c = 0; c < nch; c++) acc = __fadd_rn(acc, sums[c * RS_BN + threadIdx.x]);
                 float o = p.alpha * acc;
                 if (p.fused && m > 2) o *= (float)inv;
                 L.C[m & 1][n0 + threadIdx.x] = o;
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(RS_PREP) : "memory");  // the sums are free again
+            // (after a failed wait the loop runs on without waiting, so that every thread meets
+            // the barriers; the error word tells the caller)
+            asm volatile("bar.sync 1, %0;" ::"n"(RS_PREP) : "memory");  // the row may go
         }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(RS_ACC * RS_BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(RS_ACC * RS_N) : "memory");
     }
 }
 
@@ -334,7 +357,7 @@ __global__ void __launch_bounds__(RS_THREADS)
 template <bool BATCHED>
 __global__ void __launch_bounds__(RS_PREP) k_row_finish(RowChainLat one, RowStepParams p, const RowChainLat *__restrict__ lats) {
     pdl_begin();
-    __shared__ double red[4];
+    __shared__ double red[RS_PREP / 32];
     const RowChainLat &L = BATCHED ? lats[blockIdx.x] : one;
     const double inv = row_parts(L, p, red, [&](int e, const uint4 &h, const uint4 &l) { row_slot(L, p.m, e, h, l); });
     if (threadIdx.x == 0) L.qinv[(p.m - 2) % kRowSlots] = inv;
@@ -355,28 +378,31 @@ static int row_step_attr() {
     return OPB_OK;
 }
 
-// Ring depth for rows of up to d states: two CTAs an SM where four stages allow it (d <= 4096:
-// one prepares its row while the other's MMAs run), else as deep as shared memory allows; 0: the
-// row does not fit.
-static int row_step_stages(int d) {
-    if (row_step_smem(d, 4) <= 110 * 1024) return 4;
+// Ring depth for `items` items of rows of up to d states.  Launches of one item an SM take what
+// shared memory holds, up to eight stages (a load takes about 1 us, a stage's MMAs 0.2).  With
+// more items two CTAs an SM hide as much and one prepares its row while the other's MMAs run,
+// as long as four stages (64 columns; three of 128) allow two.  0: the row does not fit.
+static int row_step_stages(int d, int w, int items) {
+    const int two = w < 128 ? 4 : RS_MIN_STAGES;
+    if (items > num_sms() && row_step_smem(d, w, two) <= 110 * 1024) return two;
     for (int st = RS_MAX_STAGES; st >= RS_MIN_STAGES; st--)
-        if (row_step_smem(d, st) <= 226 * 1024) return st;
+        if (row_step_smem(d, w, st) <= 226 * 1024) return st;
     return 0;
 }
 
-bool row_chain_fits(int d) { return d > 0 && d % 128 == 0 && row_step_stages(d) > 0; }
+bool row_chain_fits(int d) { return d > 0 && d % 128 == 0 && d <= RS_MAX_D && row_step_stages(d, 64, d / 64) > 0; }
 
 int launch_row_step(const RowChainLat &L, const __nv_bfloat16 *Bhi, const __nv_bfloat16 *Blo, int m, int fused, int f16,
                     float alpha, float sscale, cudaStream_t s) {
-    RowStepParams p{m, fused, row_step_stages(L.d), L.d, alpha, sscale};
     if (!row_chain_fits(L.d)) return OPB_E_UNSUPPORTED;
+    const int items = L.d / 64;
+    const RowStepParams p{m, fused, row_step_stages(L.d, 64, items), L.d, alpha, sscale};
     int r = f16 ? row_step_attr<false, true>() : row_step_attr<false, false>();
     if (r) return r;
     CUtensorMap mh, ml;
     if ((r = make_map_mn(&mh, Bhi, L.d, L.d, L.d, f16)) != OPB_OK) return r;
     if ((r = make_map_mn(&ml, Blo, L.d, L.d, L.d, f16)) != OPB_OK) return r;
-    const int items = L.d / RS_BN, smem = row_step_smem(L.d, p.stages);
+    const int smem = row_step_smem(L.d, 64, p.stages);
     const int cap = num_sms() * (smem <= 110 * 1024 ? 2 : 1), grid = items < cap ? items : cap;
     if (f16) launch_pdl(k_row_step<false, true>, grid, RS_THREADS, smem, s, mh, ml, L, p, nullptr, nullptr, nullptr,
                         items);
@@ -388,11 +414,11 @@ int launch_row_step(const RowChainLat &L, const __nv_bfloat16 *Bhi, const __nv_b
 int launch_row_step_batched(const RowChainLat *lats, const CUtensorMap *maps, const uint32_t *work, int nwork, int dmax,
                             int m, int f16, float alpha, float sscale, cudaStream_t s) {
     if (nwork <= 0) return OPB_OK;
-    if (!row_chain_fits(dmax)) return OPB_E_UNSUPPORTED;
-    RowStepParams p{m, 1, row_step_stages(dmax), dmax, alpha, sscale};
+    const RowStepParams p{m, 1, row_step_stages(dmax, 128, nwork), dmax, alpha, sscale};
+    if (!row_chain_fits(dmax) || p.stages == 0) return OPB_E_UNSUPPORTED;
     int r = f16 ? row_step_attr<true, true>() : row_step_attr<true, false>();
     if (r) return r;
-    const int smem = row_step_smem(dmax, p.stages);
+    const int smem = row_step_smem(dmax, 128, p.stages);
     const int cap = num_sms() * (smem <= 110 * 1024 ? 2 : 1), grid = nwork < cap ? nwork : cap;
     CUtensorMap none;
     std::memset(&none, 0, sizeof(none));

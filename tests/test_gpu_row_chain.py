@@ -48,3 +48,19 @@ def test_batched_rows_against_fp64(cuda):
         L = O.lv_generator_fast(x, 0.03 * x, O.lv_sigma(x, level=0.15 + 0.02 * i) * x)
         V, _, _ = O.solve_lattice_fp64(L, x, STRIKES, 0.03, period, nmat, dt0)
         assert np.abs(got[i] - V[:, lat.y0, :]).max() < 1e-5
+
+
+@pytest.mark.parametrize("n", [384, 640])
+def test_batched_rows_with_several_items_a_block(cuda, n):
+    """More items than blocks are resident: a block changes lattice (another row in its shared
+    memory) and goes on in the ring; equal lattices give equal bits, whichever block had them."""
+    from oplib_b200 import _lib
+    from oplib_b200.model import Batch, Lattice
+    lats = [Lattice.local_vol(n=n, level=0.2 + 0.1 * (i % 2), device=cuda) for i in range(130)]
+    got = Batch(lats, STRIKES, 4, 0.125, 2.0 ** -11, mode="bf16x3", autotune=False).execute()
+    torch.cuda.synchronize()
+    assert _lib.load().opb_tc_error() == 0
+    for k in range(2):
+        assert torch.equal(got[k::2], got[k:k + 1].expand_as(got[k::2]))
+        alone, _ = lats[k].solve(STRIKES, 4, 0.125, 2.0 ** -11, mode="bf16x3")
+        assert (got[k] - alone).abs().max() < 1e-5
