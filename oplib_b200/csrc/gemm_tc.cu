@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
         if constexpr (Cfg::REGSPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_REST));
         if (warp == EPI && lane == 0) {
             // ---------------- TMA producer
-            long kbg = 0;  // K-blocks issued over the CTA's lifetime (stage ring position)
+            unsigned kbg = 0;  // K-blocks issued over the CTA's lifetime (stage ring position)
             bool ok = true;
             if constexpr (Cfg::BRES) {
                 // every item's B is the whole weight matrix (N == BN, K <= 256): load it once
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     }
                     const int s = (int)(kbg % STAGES);
                     if (kbg >= STAGES &&
-                        !mbar_wait(empty_bar(s), (uint32_t)(((kbg / STAGES) + 1) & 1), abort_flag, TC_WAIT_NS)) {
+                        !mbar_wait(empty_bar(s), ((kbg / STAGES) + 1) & 1, abort_flag, TC_WAIT_NS)) {
                         ok = false;
                         break;
                     }
@@ -648,11 +648,10 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                 // wait (bounded) for the copies in flight; in pair mode they complete on the
                 // leader's barriers, and the closing cluster barrier keeps this CTA resident
                 // until the leader has drained them
-                const long first = kbg > STAGES ? kbg - STAGES : 0;
+                const unsigned first = kbg > STAGES ? kbg - STAGES : 0;
                 if (!PAIR || rank == 0)
-                    for (long k = first; k < kbg; k++)
-                        (void)mbar_wait(full_bar((int)(k % STAGES)), (uint32_t)((k / STAGES) & 1), abort_flag,
-                                        100000000ull);
+                    for (unsigned k = first; k < kbg; k++)
+                        (void)mbar_wait(full_bar((int)(k % STAGES)), (k / STAGES) & 1, abort_flag, 100000000ull);
             }
         }
         if (warp == EPI + 1 && rank == 0) {
@@ -662,7 +661,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
             // MMA takes them from, costs more than a narrow MMA (1024 states of 64-wide tiles
             // 17.5 -> 15.7 us, the quoted row's step at d = 6144 71 -> 60).
             const uint32_t idesc = umma_idesc_16(BN, F16, Cfg::TILE_M, BMN);
-            long kbg = 0, g = 0;  // K-blocks consumed, chunks issued
+            unsigned kbg = 0, g = 0;  // K-blocks consumed, chunks issued
             bool ok = true;
             if constexpr (Cfg::BRES) {
                 if (item0 < nitems) {
@@ -688,7 +687,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     }
                     const int a = (int)(g & 1);
                     if (g >= 2 &&
-                        !mbar_wait_warp(acce_bar(a), (uint32_t)(((g >> 1) + 1) & 1), abort_flag, TC_WAIT_NS)) {
+                        !mbar_wait_warp(acce_bar(a), ((g >> 1) + 1) & 1, abort_flag, TC_WAIT_NS)) {
                         ok = false;
                         break;
                     }
@@ -699,7 +698,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     for (int kb = c * Cfg::CHUNK; kb < kb_end; kb++) {
                         if (PLANNED && mk && !((bits >> (kb - c * Cfg::CHUNK)) & 1u)) continue;
                         const int s = (int)(kbg % STAGES);
-                        if (!mbar_wait_warp(full_bar(s), (uint32_t)((kbg / STAGES) & 1), abort_flag, TC_WAIT_NS)) {
+                        if (!mbar_wait_warp(full_bar(s), (kbg / STAGES) & 1, abort_flag, TC_WAIT_NS)) {
                             ok = false;
                             break;
                         }
@@ -764,7 +763,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
         const int q = warp & 3, h = warp >> 2;
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
         float sum[CPT];
-        long g = 0;
+        unsigned g = 0;
         bool ok = true;
         uint2 next = entry(item0);
         for (int t = item0; t < nitems && ok; t += istep) {
@@ -837,7 +836,7 @@ __global__ void __launch_bounds__(TcCfg<BN, STAGES, NPROD, BK, PAIR, EPIMODE>::T
                     for (int b = 0; b < CPT / 64; b++)
                         if ((live >> b) & 1u) prefetch_l2(pf + (long long)(rbase + lane) * pf_ld + col0 + 64 * b, 256);
                 }
-                if (!mbar_wait(accf_bar(a), (uint32_t)((g >> 1) & 1), abort_flag, TC_WAIT_NS)) {
+                if (!mbar_wait(accf_bar(a), (g >> 1) & 1, abort_flag, TC_WAIT_NS)) {
                     ok = false;
                     break;
                 }
