@@ -369,11 +369,12 @@ def run_b200(args, rank, world, local_rank):
 
     quotes_per_step = NMAT * NK * world
     value = quotes_per_step / (ms * 1e-3)
-    # gpu launches per step (library kernels): generator, E0 scatter, split, niter*(gemm+renorm),
-    # add_identity, split, payoff, nmat*(price gemm + discount), (nmat-1)*(chain gemm + renorm)
-    if mode == MODES["bf16x3"]:
-        # ... + the generator's band (one block)
-        launches = 1 + 1 + 1 + 1 + 2 * plan.niter + 1 + 1 + 1 + 2 * NMAT + 2 * (NMAT - 1)
+    # gpu launches per step (library kernels): generator, band, E0 scatter, niter * (tile plan +
+    # squaring), P1's renormalisation, payoff (FP16 parts: + its scale), nmat - 1 steps of the
+    # quoted row, its last slot, one pricing product, quotes.  FP32 modes: E0, split,
+    # niter * (gemm + renorm), payoff, nmat * (price gemm + discount), (nmat - 1) * (gemm + renorm)
+    if mode >= MODES["bf16x3"]:
+        launches = 1 + 1 + 1 + 2 * plan.niter + 1 + 1 + (mode != MODES["bf16x3"]) + (NMAT - 1) + 1 + 1 + 1
     else:
         launches = 1 + 2 + (3 if mode == 1 else 1) * plan.niter + 1 + 2 * NMAT + (3 if mode == 1 else 1) * (NMAT - 1)
     out = {

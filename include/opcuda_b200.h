@@ -280,8 +280,9 @@ int opb_set_ksplit(int s);
  * calibration sweep; with the default every sweep price is within 2e-6 of FP64 */
 int opb_set_lolo_levels(int n);
 /* new: 1 (default): squarings of an ELL generator's E_r = P(2^r dt) - I skip the K-blocks and
- * output tiles outside twice E_r's band (h0 * 2^r for the generator's half-bandwidth h0),
- * whose products are exact zeros; 0: every squaring runs the full product.  Results are
+ * output tiles outside twice E_r's band (h0 * 2^r for the generator's half-bandwidth h0) and,
+ * in batches and from 1536 states on, those whose blocks are zero inside it, whose products
+ * are exact zeros; 0: every squaring runs the full product.  Results are
  * bit-identical either way */
 int opb_set_band_skip(int on);
 /* new: the split-mode solves defer each product's FP64 row normalisation into the next
@@ -347,7 +348,7 @@ int opb_batch_launches(const opb_batch_plan *plan);
  * split-BF16 products (activations and gradients as hi + lo parts, FP32 accumulation) when
  * B is a multiple of 128; the first and output layers on SIMT kernels. */
 int opb_mlp_param_count(void);
-long long opb_mlp_workspace_floats(int B);
+long long opb_mlp_workspace_floats(int B); /* floats of ws for batches of B rows */
 /* new: 1 (default) tensor-core training products as above, 0 SIMT FP32 throughout */
 int opb_mlp_set_tensor_cores(int on);
 int opb_mlp_init(float *theta, unsigned long long seed);
@@ -411,7 +412,7 @@ int opcuda_mt_benchmark(uint64_t mtptr, uint64_t unif_ptr, int nscen);
  * Runs of up to 623 steps keep the generator in registers; longer runs hold the
  * 624-word state in per-thread local memory (2496 bytes a thread), which the CUDA
  * driver may provision on the first such launch. */
-int opb_mc_scratch_blocks(long long npaths);
+int opb_mc_scratch_blocks(long long npaths); /* blocks of a run: scratch holds two doubles for each */
 int opb_mc_mt19937(const float *C, long long row_stride, long long col_stride, const uint32_t *guide, int nb, int d,
                    int y0, int nsteps, uint32_t seed, unsigned long long path0, long long npaths, short *ypaths,
                    const double *x, double strike, double barrier, double disc, double *scratch, double *sums);

@@ -9,8 +9,8 @@ iteration:
 1. rewrites in place the device generators of every problem, at its trial point and at
    six parameter bumps for central differences (``opb_lv_params`` +
    ``opb_lv_generator_ell`` into the batch's ELL arrays);
-2. prices all 7 x M lattices with one ``opb_batch_execute``, i.e. one persistent
-   tensor-core launch and one renormalisation launch per squaring level;
+2. prices all 7 x M lattices with one ``opb_batch_execute``, i.e. one tile plan and
+   one persistent tensor-core launch per squaring level;
 3. per problem, on the host in FP64: accepts or rejects the trial, forms J^T J and J^T r
    from the bumped prices, and solves the damped 3 x 3 system for the next trial.
 

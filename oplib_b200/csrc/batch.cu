@@ -641,8 +641,8 @@ int batch_square(opb_batch_plan *P, int cfg, cudaStream_t s) {
 
 }  // namespace
 
-// Executes the plan on the library stream: E0 build, every squaring level (one GEMM +
-// one renormalisation launch each), chaining and pricing.  quotes: device
+// Executes the plan on the library stream: E0 build, every squaring level (tile plan and one
+// GEMM; the renormalisation of the lattices that end there), the quoted rows and pricing.  quotes: device
 // [nlat][nmat][nK] FP64.  No host synchronisation, no allocation (graph-capturable).
 OPB_API int opb_batch_execute(opb_batch_plan *P, double *quotes) {
     OPB_NVTX("opb_batch_execute");

@@ -14,21 +14,21 @@
 //   TMA warp, one lane : 4 tiled bulk-tensor loads per K-block (Ahi, Alo, Bhi, Blo; 128B
 //                        swizzle; no multicast) into a STAGES-deep ring, completion
 //                        tracked by mbarrier transaction counts.
-//   MMA warp, one lane : per 16-wide K step three tcgen05.mma.kind::f16 (BF16 x BF16 ->
-//                        FP32) into one of two TMEM accumulators (BN columns each), one
+//   MMA warp           : one elected lane, per 16-wide K step three tcgen05.mma.kind::f16
+//                        (BF16 x BF16 -> FP32) into one of two TMEM accumulators (BN columns each), one
 //                        accumulator per chunk of 2 K-blocks; tcgen05.commit releases
 //                        each stage and hands each finished chunk to the epilogue.
 //   epilogue warps     : (4 lane quadrants x BN/128 column groups) tcgen05.ld of each
 //                        finished chunk into FP32 round-to-nearest register sums; after a
 //                        tile's last chunk, the alpha/beta update (with the deferred
 //                        renormalisation of Cin, when given), FP32 stores staged through
-//                        shared memory in 32 x 32 blocks, and FP64 row sums of the
+//                        shared memory, and FP64 row sums of the
 //                        stored values (rowsum[group * M + row], one per 128 columns,
 //                        used by the row renormalisation).
 // CTA pairs (the default for M % 256 == 0 with 256-wide tiles): a 2-CTA cluster owns a
 // 256 x 256 output tile; each CTA loads its own 128 rows of A and 128 columns of B (3-stage
 // 64 KB ring per CTA, both CTAs' copies counted on the even CTA's full barrier), the even
-// CTA's MMA lane issues tcgen05.mma.cta_group::2 (M = 256) over both CTAs' shared memory
+// CTA's MMA warp issues tcgen05.mma.cta_group::2 (M = 256) over both CTAs' shared memory
 // into each CTA's own TMEM, and its commits arrive on both CTAs' barriers.  Operand bytes
 // through shared memory per MMA flop drop by a third against one CTA per 128 x 256 tile.
 // The tensor cores truncate their FP32 accumulator (about half an ulp per MMA); chunked

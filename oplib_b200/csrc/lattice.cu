@@ -231,7 +231,8 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
     // ELL generator's E0 goes in with its parts and marks.
     int tm = 0, tn = 0;
     const bool fused = opb::fused_single(d);
-    const bool planned = d >= opb::OPB_PLAN_MIN_D && L.niter > 0 && g_ksplit <= 1 && opb::tile_plan_for(d, tm, tn);
+    const bool planned = opb::g_band_skip && d >= opb::OPB_PLAN_MIN_D && L.niter > 0 && g_ksplit <= 1 &&
+                         opb::tile_plan_for(d, tm, tn);
     opb::E0Parts e0{};
     if (planned) {
         const bool ell = L.ell_width > 0;
