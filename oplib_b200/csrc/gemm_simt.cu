@@ -371,6 +371,33 @@ __device__ __forceinline__ void st_steps(uint64_t (&acc)[RPT / 2][4], const floa
             st_step<RPT>(acc, as + k * ap, bs[k], bs[4 * ST_BP + k], bs[8 * ST_BP + k], bs[12 * ST_BP + k]);
     }
 }
+// Two right tiles against one left tile: its values are read once for both.
+template <int RPT>
+__device__ __forceinline__ void st_steps2(uint64_t (&acc0)[RPT / 2][4], uint64_t (&acc1)[RPT / 2][4], const float *as,
+                                          int ap, const float *bs0, const float *bs1, int kn) {
+    if (kn == ST_BK) {
+#pragma unroll
+        for (int k = 0; k < ST_BK; k += 4) {
+            float4 b[4], c[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                b[j] = *reinterpret_cast<const float4 *>(bs0 + 4 * j * ST_BP + k);
+                c[j] = *reinterpret_cast<const float4 *>(bs1 + 4 * j * ST_BP + k);
+            }
+            st_step<RPT>(acc0, as + k * ap, b[0].x, b[1].x, b[2].x, b[3].x);
+            st_step<RPT>(acc1, as + k * ap, c[0].x, c[1].x, c[2].x, c[3].x);
+            st_step<RPT>(acc0, as + (k + 1) * ap, b[0].y, b[1].y, b[2].y, b[3].y);
+            st_step<RPT>(acc1, as + (k + 1) * ap, c[0].y, c[1].y, c[2].y, c[3].y);
+            st_step<RPT>(acc0, as + (k + 2) * ap, b[0].z, b[1].z, b[2].z, b[3].z);
+            st_step<RPT>(acc1, as + (k + 2) * ap, c[0].z, c[1].z, c[2].z, c[3].z);
+            st_step<RPT>(acc0, as + (k + 3) * ap, b[0].w, b[1].w, b[2].w, b[3].w);
+            st_step<RPT>(acc1, as + (k + 3) * ap, c[0].w, c[1].w, c[2].w, c[3].w);
+        }
+    } else {
+        st_steps<RPT>(acc0, as, ap, bs0, kn);
+        st_steps<RPT>(acc1, as, ap, bs1, kn);
+    }
+}
 // Stores this thread's outputs: rows x.. (and x + 32..), columns y, y + 4, y + 8, y + 12 of
 // column-major C.
 template <int RPT>
@@ -528,22 +555,32 @@ struct Sgemm4Task {
     uint64_t A, B, C;
 };
 
-// A block takes four consecutive tasks, a warp each.  Neighbouring tasks of a table mostly share
+// A block takes one, two or four consecutive tasks.  Neighbouring tasks of a table mostly share
 // a tile (the same rows of A along by, the same columns of B along bx), so each distinct tile is
-// staged once for the warps that read it; tasks that share nothing stage their own.  What a
-// block computes does not depend on which they share.  (One 64 x 16 tile per 256-thread block,
-// every operand of A from L1: 9.2 TFLOP/s over 40 products of 576^3, 1657 us; now 475.)
-constexpr int S4_TASKS = 4, S4_AP = 64 + 4;
+// staged once for the warps that read it, and a warp that has two tasks with one left tile reads
+// it from shared memory once for both: with one task a warp those reads, not the FMAs, were the
+// limit.  Tasks that share nothing stage their own.  What a block computes does not depend on
+// which they share.  (One 64 x 16 tile per 256-thread block, every operand of A from L1: 9.2
+// TFLOP/s over 40 products of 576^3, 1657 us; a task a warp 466; now 417.)
+//
+constexpr int S4_TASKS = 4, S4_THREADS = 16 * S4_TASKS, S4_AP = 64 + 4;
+// Tasks a block takes: one in tables of up to three tasks an SM, where a task's own chain over K is
+// the time, two (a warp each) up to fifteen, four (two a warp) beyond.  Measured, us, at 1 / 2 / 4
+// a block: 200 tasks 25 / 32 / 56, 400 31 / 33 / 56, 800 41 / 39 / 60, 1296 117 / 78 / 94, 3000
+// 131 / 97 / 97, 5184 383 / 218 / 201, 12960 920 / 515 / 417.
+constexpr int S4_ONE = 3, S4_PAIR = 15;
 constexpr int S4_A = ST_BK * S4_AP, S4_B = 16 * ST_BP;   // floats of a left, a right tile
-constexpr int S4_POOL = 2 * S4_TASKS * (S4_A + S4_B);        // two stages without sharing
-static_assert(4 * S4_POOL <= 48 * 1024, "static limit");
+// Shared memory of a block: three stages of tasks that share their left tile, or of strangers'
+// tiles one; six blocks an SM (two stages of strangers, 45 KB, left four: 447 us).
+constexpr int S4_POOL = 3 * (S4_A + S4_TASKS * S4_B);
+static_assert(4 * S4_POOL <= 48 * 1024 && S4_POOL >= S4_TASKS * (S4_A + S4_B), "default limit; a stage of strangers");
 
-__global__ void __launch_bounds__(32 * S4_TASKS) k_sgemm4(const uint64_t *argptr_bid, int ntasks) {
+__global__ void __launch_bounds__(S4_THREADS) k_sgemm4(const uint64_t *argptr_bid, int ntasks, int per) {
     __shared__ Sgemm4Task task[S4_TASKS];
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int cnt = min(S4_TASKS, ntasks - (int)blockIdx.x * S4_TASKS);
-    if (tid < cnt) task[tid] = *reinterpret_cast<const Sgemm4Task *>(argptr_bid[blockIdx.x * S4_TASKS + tid]);
+    const int cnt = min(per, ntasks - (int)blockIdx.x * per);
+    if (tid < cnt) task[tid] = *reinterpret_cast<const Sgemm4Task *>(argptr_bid[blockIdx.x * per + tid]);
     __syncthreads();
     // the tiles of each task, as offsets (floats) into a stage: those of the first task that has
     // the same one
@@ -588,49 +625,68 @@ __global__ void __launch_bounds__(32 * S4_TASKS) k_sgemm4(const uint64_t *argptr
                 const Sgemm4Task &u = task[i];
                 if ((owner >> i) & 1u)
                     st_load_a<64>(st + oa[i], S4_AP, reinterpret_cast<const float *>(u.A), u.m, u.m, u.k, u.bx * 64, k0,
-                                  u.m % 4 == 0 && u.A % 16 == 0, tid, 32 * S4_TASKS);
+                                  u.m % 4 == 0 && u.A % 16 == 0, tid, S4_THREADS);
                 if ((owner >> (4 + i)) & 1u)
                     st_load_b<16>(st + ob[i], reinterpret_cast<const float *>(u.B), u.k, u.n, u.k, u.by * 16, k0,
-                                  u.k % 4 == 0 && u.B % 16 == 0, tid, 32 * S4_TASKS);
+                                  u.k % 4 == 0 && u.B % 16 == 0, tid, S4_THREADS);
             }
         }
         sf_commit();
     };
-    uint64_t acc[4][4];
+    uint64_t acc0[4][4], acc1[4][4];
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
-    const bool mine = warp < cnt;
-    const int k = mine ? task[warp].k : 0, xl = (lane & 7) * 4, yl = lane >> 3;
-    int wa = 0, wb = 0;
+        for (int j = 0; j < 4; j++) acc0[i][j] = acc1[i][j] = 0ull;
+    const int t0 = per > 2 ? 2 * warp : warp, t1 = per > 2 ? 2 * warp + 1 : S4_TASKS;
+    const int ka = t0 < cnt ? task[t0].k : 0, kb = t1 < cnt ? task[t1].k : 0, xl = (lane & 7) * 4, yl = lane >> 3;
+    int wa0 = 0, wb0 = 0, wa1 = 0, wb1 = 0;
 #pragma unroll
-    for (int i = 0; i < S4_TASKS; i++)
-        if (i == warp) {
-            wa = oa[i];
-            wb = ob[i];
+    for (int i = 0; i < S4_TASKS; i++) {
+        if (i == t0) {
+            wa0 = oa[i];
+            wb0 = ob[i];
         }
-    // as many stages as the block's memory holds of these tiles: four for tasks that share,
-    // two for four strangers
+        if (i == t1) {
+            wa1 = oa[i];
+            wb1 = ob[i];
+        }
+    }
+    const bool both = ka > 0 && kb > 0 && wa0 == wa1;  // (the same left tile: the same k)
+    // as many stages as the block's memory holds of these tiles (one: load, then compute)
     auto run = [&](auto depth) {
         constexpr int NS = decltype(depth)::value;
 #pragma unroll
         for (int t = 0; t < NS - 1; t++) load(t, NS);
         for (int t = 0, k0 = 0; k0 < kmax; t++, k0 += ST_BK) {
-            sf_wait<NS - 2>();
+            if (NS == 1) {
+                if (t > 0) __syncthreads();
+                load(t, NS);
+            }
+            sf_wait<NS == 1 ? 0 : NS - 2>();
             __syncthreads();
-            load(t + NS - 1, NS);
+            if (NS > 1) load(t + NS - 1, NS);
             const float *st = sm + (t % NS) * stage;
-            if (k0 < k) st_steps<8>(acc, st + wa + xl, S4_AP, st + wb + yl * ST_BP, min(ST_BK, k - k0));
+            const float *bs0 = st + wb0 + yl * ST_BP, *bs1 = st + wb1 + yl * ST_BP;
+            if (both) {
+                if (k0 < ka) st_steps2<8>(acc0, acc1, st + wa0 + xl, S4_AP, bs0, bs1, min(ST_BK, ka - k0));
+            } else {
+                if (k0 < ka) st_steps<8>(acc0, st + wa0 + xl, S4_AP, bs0, min(ST_BK, ka - k0));
+                if (k0 < kb) st_steps<8>(acc1, st + wa1 + xl, S4_AP, bs1, min(ST_BK, kb - k0));
+            }
         }
     };
-    if (4 * stage <= S4_POOL) run(std::integral_constant<int, 4>{});
-    else if (3 * stage <= S4_POOL) run(std::integral_constant<int, 3>{});
-    else run(std::integral_constant<int, 2>{});
-    if (!mine) return;
-    const Sgemm4Task &t = task[warp];
-    st_store<8>(acc, reinterpret_cast<float *>(t.C), t.m, t.m, t.n, t.bx * 64 + xl, t.by * 16 + yl, 1.f, 0.f,
-                t.m % 4 == 0 && t.C % 16 == 0);
+    if (3 * stage <= S4_POOL) run(std::integral_constant<int, 3>{});
+    else if (2 * stage <= S4_POOL) run(std::integral_constant<int, 2>{});
+    else run(std::integral_constant<int, 1>{});
+    auto store = [&](int i, const uint64_t (&acc)[4][4]) {
+        if (i >= cnt) return;
+        const Sgemm4Task &t = task[i];
+        st_store<8>(acc, reinterpret_cast<float *>(t.C), t.m, t.m, t.n, t.bx * 64 + xl, t.by * 16 + yl, 1.f, 0.f,
+                    t.m % 4 == 0 && t.C % 16 == 0);
+    };
+    store(t0, acc0);
+    store(t1, acc1);
 }
 
 }  // namespace opb
@@ -684,8 +740,9 @@ OPB_API int opcuda_sgemm4(int nblocks, uint64_t argptr_bid) {
     OPB_REQUIRE(nblocks >= 0, OPB_E_ARG);
     if (nblocks == 0) return set_status(OPB_OK);
     OPB_REQUIRE(argptr_bid != 0, OPB_E_NULL);
-    k_sgemm4<<<(nblocks + S4_TASKS - 1) / S4_TASKS, 32 * S4_TASKS, 4 * S4_POOL, stream()>>>(
-        reinterpret_cast<const uint64_t *>(argptr_bid), nblocks);
+    const int per = nblocks <= S4_ONE * num_sms() ? 1 : nblocks <= S4_PAIR * num_sms() ? 2 : S4_TASKS;
+    k_sgemm4<<<(nblocks + per - 1) / per, S4_THREADS, 4 * S4_POOL, stream()>>>(
+        reinterpret_cast<const uint64_t *>(argptr_bid), nblocks, per);
     return launch_check();
 }
 

@@ -72,3 +72,32 @@ def test_grouped_products_in_any_order_of_the_table(cuda, shapes, order):
     assert lib.opcuda_sgemm4(len(tasks), ptrs.data_ptr()) == 0
     for A, B, _, _, C in mats:
         assert torch.equal(C.t(), _product(lib, A, B)[0])
+
+
+@pytest.mark.parametrize("count", [3, 15, 16, 75, 76, 149])  # tasks a block: 1 up to 444, 2 up to 2220, 4 beyond
+def test_grouped_products_across_the_table_sizes(cuda, count):
+    """Tables of 30 tasks a product (80 x 229 x 37), the last block of a table not full."""
+    from oplib_b200 import _lib
+    from oplib_b200.model import bind_stream
+    lib = _lib.load()
+    bind_stream(cuda)
+    g = torch.Generator(device=cuda).manual_seed(count)
+    m, n, k = 80, 229, 37
+    A = torch.randn(count, m, k, device=cuda, generator=g)
+    B = torch.randn(count, k, n, device=cuda, generator=g)
+    Ac, Bc = A.transpose(1, 2).contiguous(), B.transpose(1, 2).contiguous()
+    C = torch.full((count, n, m), float("nan"), device=cuda)
+    words = lib.opb_sgemm4_task_size() // 8
+    rec = np.zeros((count * 30 - 1, words), dtype=np.int64)  # without the last tile
+    for t in range(len(rec)):
+        i, bx, by = t // 30, t % 30 // 15, t % 15
+        rec[t, :3] = np.array([i, bx, by, m, n, k], dtype=np.int32).view(np.int64)
+        rec[t, 3:6] = Ac[i].data_ptr(), Bc[i].data_ptr(), C[i].data_ptr()
+    drec = torch.from_numpy(rec.ravel()).to(cuda)
+    ptrs = torch.arange(len(rec), dtype=torch.int64, device=cuda) * (8 * words) + drec.data_ptr()
+    assert lib.opcuda_sgemm4(len(rec), ptrs.data_ptr()) == 0
+    got = C.transpose(1, 2)
+    want = torch.stack([_product(lib, A[i], B[i])[0] for i in range(count)])
+    want[-1, 64:, 14 * 16:] = float("nan")
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(got.nan_to_num(), want.nan_to_num())
