@@ -564,10 +564,11 @@ struct Sgemm4Task {
 // TFLOP/s over 40 products of 576^3, 1657 us; a task a warp 466; now 417.)
 //
 constexpr int S4_TASKS = 4, S4_THREADS = 16 * S4_TASKS, S4_AP = 64 + 4;
-// Tasks a block takes: one in tables of up to three tasks an SM, where a task's own chain over K is
-// the time, two (a warp each) up to fifteen, four (two a warp) beyond.  Measured, us, at 1 / 2 / 4
-// a block: 200 tasks 25 / 32 / 56, 400 31 / 33 / 56, 800 41 / 39 / 60, 1296 117 / 78 / 94, 3000
-// 131 / 97 / 97, 5184 383 / 218 / 201, 12960 920 / 515 / 417.
+// Tasks a block takes: one (half of its rows a warp) in tables of up to three tasks an SM, where a
+// task's own chain over K is the time, two (a warp each) up to fifteen, four (two a warp) beyond.
+// Measured, us, one tile per 256-thread block / now: 20 tasks of K = 300 29 / 17, 400 33 / 21, one
+// product of 576^3 (324 tasks) 58 / 35; at 2 / 4 tasks a block: 800 39 / 60, 1296 78 / 94, 3000
+// 97 / 97, 5184 218 / 201, 12960 515 / 417.
 constexpr int S4_ONE = 3, S4_PAIR = 15;
 constexpr int S4_A = ST_BK * S4_AP, S4_B = 16 * ST_BP;   // floats of a left, a right tile
 // Shared memory of a block: three stages of tasks that share their left tile, or of strangers'
@@ -575,12 +576,13 @@ constexpr int S4_A = ST_BK * S4_AP, S4_B = 16 * ST_BP;   // floats of a left, a 
 constexpr int S4_POOL = 3 * (S4_A + S4_TASKS * S4_B);
 static_assert(4 * S4_POOL <= 48 * 1024 && S4_POOL >= S4_TASKS * (S4_A + S4_B), "default limit; a stage of strangers");
 
-__global__ void __launch_bounds__(S4_THREADS) k_sgemm4(const uint64_t *argptr_bid, int ntasks, int per) {
+template <int PER>
+__global__ void __launch_bounds__(S4_THREADS) k_sgemm4(const uint64_t *argptr_bid, int ntasks) {
     __shared__ Sgemm4Task task[S4_TASKS];
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int cnt = min(per, ntasks - (int)blockIdx.x * per);
-    if (tid < cnt) task[tid] = *reinterpret_cast<const Sgemm4Task *>(argptr_bid[blockIdx.x * per + tid]);
+    const int cnt = min(PER, ntasks - (int)blockIdx.x * PER);
+    if (tid < cnt) task[tid] = *reinterpret_cast<const Sgemm4Task *>(argptr_bid[blockIdx.x * PER + tid]);
     __syncthreads();
     // the tiles of each task, as offsets (floats) into a stage: those of the first task that has
     // the same one
@@ -633,13 +635,16 @@ __global__ void __launch_bounds__(S4_THREADS) k_sgemm4(const uint64_t *argptr_bi
         }
         sf_commit();
     };
-    uint64_t acc0[4][4], acc1[4][4];
+    // one task a block: a warp takes half of its rows, else a warp takes a task, or two
+    constexpr int RPT = PER == 1 ? 4 : 8;
+    uint64_t acc0[RPT / 2][4], acc1[RPT / 2][4];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < RPT / 2; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) acc0[i][j] = acc1[i][j] = 0ull;
-    const int t0 = per > 2 ? 2 * warp : warp, t1 = per > 2 ? 2 * warp + 1 : S4_TASKS;
-    const int ka = t0 < cnt ? task[t0].k : 0, kb = t1 < cnt ? task[t1].k : 0, xl = (lane & 7) * 4, yl = lane >> 3;
+    const int t0 = PER == 1 ? 0 : PER == 2 ? warp : 2 * warp, t1 = PER == 4 ? 2 * warp + 1 : S4_TASKS;
+    const int ka = t0 < cnt ? task[t0].k : 0, kb = t1 < cnt ? task[t1].k : 0;
+    const int xl = (lane & 7) * 4 + (PER == 1 ? 32 * warp : 0), yl = lane >> 3;
     int wa0 = 0, wb0 = 0, wa1 = 0, wb1 = 0;
 #pragma unroll
     for (int i = 0; i < S4_TASKS; i++) {
@@ -652,7 +657,7 @@ __global__ void __launch_bounds__(S4_THREADS) k_sgemm4(const uint64_t *argptr_bi
             wb1 = ob[i];
         }
     }
-    const bool both = ka > 0 && kb > 0 && wa0 == wa1;  // (the same left tile: the same k)
+    const bool both = PER == 4 && ka > 0 && kb > 0 && wa0 == wa1;  // (the same left tile: the same k)
     // as many stages as the block's memory holds of these tiles (one: load, then compute)
     auto run = [&](auto depth) {
         constexpr int NS = decltype(depth)::value;
@@ -669,24 +674,24 @@ __global__ void __launch_bounds__(S4_THREADS) k_sgemm4(const uint64_t *argptr_bi
             const float *st = sm + (t % NS) * stage;
             const float *bs0 = st + wb0 + yl * ST_BP, *bs1 = st + wb1 + yl * ST_BP;
             if (both) {
-                if (k0 < ka) st_steps2<8>(acc0, acc1, st + wa0 + xl, S4_AP, bs0, bs1, min(ST_BK, ka - k0));
+                if (k0 < ka) st_steps2<RPT>(acc0, acc1, st + wa0 + xl, S4_AP, bs0, bs1, min(ST_BK, ka - k0));
             } else {
-                if (k0 < ka) st_steps<8>(acc0, st + wa0 + xl, S4_AP, bs0, min(ST_BK, ka - k0));
-                if (k0 < kb) st_steps<8>(acc1, st + wa1 + xl, S4_AP, bs1, min(ST_BK, kb - k0));
+                if (k0 < ka) st_steps<RPT>(acc0, st + wa0 + xl, S4_AP, bs0, min(ST_BK, ka - k0));
+                if (PER == 4 && k0 < kb) st_steps<RPT>(acc1, st + wa1 + xl, S4_AP, bs1, min(ST_BK, kb - k0));
             }
         }
     };
     if (3 * stage <= S4_POOL) run(std::integral_constant<int, 3>{});
     else if (2 * stage <= S4_POOL) run(std::integral_constant<int, 2>{});
     else run(std::integral_constant<int, 1>{});
-    auto store = [&](int i, const uint64_t (&acc)[4][4]) {
+    auto store = [&](int i, const uint64_t (&acc)[RPT / 2][4]) {
         if (i >= cnt) return;
         const Sgemm4Task &t = task[i];
-        st_store<8>(acc, reinterpret_cast<float *>(t.C), t.m, t.m, t.n, t.bx * 64 + xl, t.by * 16 + yl, 1.f, 0.f,
+        st_store<RPT>(acc, reinterpret_cast<float *>(t.C), t.m, t.m, t.n, t.bx * 64 + xl, t.by * 16 + yl, 1.f, 0.f,
                     t.m % 4 == 0 && t.C % 16 == 0);
     };
     store(t0, acc0);
-    store(t1, acc1);
+    if (PER == 4) store(t1, acc1);
 }
 
 }  // namespace opb
@@ -740,9 +745,12 @@ OPB_API int opcuda_sgemm4(int nblocks, uint64_t argptr_bid) {
     OPB_REQUIRE(nblocks >= 0, OPB_E_ARG);
     if (nblocks == 0) return set_status(OPB_OK);
     OPB_REQUIRE(argptr_bid != 0, OPB_E_NULL);
-    const int per = nblocks <= S4_ONE * num_sms() ? 1 : nblocks <= S4_PAIR * num_sms() ? 2 : S4_TASKS;
-    k_sgemm4<<<(nblocks + per - 1) / per, S4_THREADS, 4 * S4_POOL, stream()>>>(
-        reinterpret_cast<const uint64_t *>(argptr_bid), nblocks, per);
+    const uint64_t *tab = reinterpret_cast<const uint64_t *>(argptr_bid);
+    cudaStream_t s = stream();
+    if (nblocks <= S4_ONE * num_sms()) k_sgemm4<1><<<nblocks, S4_THREADS, 4 * S4_POOL, s>>>(tab, nblocks);
+    else if (nblocks <= S4_PAIR * num_sms())
+        k_sgemm4<2><<<(nblocks + 1) / 2, S4_THREADS, 4 * S4_POOL, s>>>(tab, nblocks);
+    else k_sgemm4<S4_TASKS><<<(nblocks + S4_TASKS - 1) / S4_TASKS, S4_THREADS, 4 * S4_POOL, s>>>(tab, nblocks);
     return launch_check();
 }
 
