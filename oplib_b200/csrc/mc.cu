@@ -13,8 +13,8 @@
 // B200 design: one thread per path with the whole generator in registers for runs of up
 // to 623 steps (mt19937_first in mt19937.cuh walks the seeding recurrence with a few
 // cursors, no state array); longer runs (mt19937_any) take their first 623 outputs from
-// the same cursors while storing the regenerated words in a per-thread 624-word
-// local-memory array, which serves every later output.  They run in a separate
+// the same cursors while storing the regenerated words that are read again in a per-thread
+// 624-word local-memory array, which serves every later output.  They run in a separate
 // instantiation of the same kernels, so the register-only one carries no stack frame.
 // The inverse-CDF search starts from the guide-table bracket of the previous state's row
 // (about one probe per step) and falls back to the full row without a guide table.

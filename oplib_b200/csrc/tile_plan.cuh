@@ -13,10 +13,10 @@
 // Whoever writes the parts marks the blocks (32 rows x 64 columns) that hold a non-zero hi part
 // (lo parts are zero where hi is); before the next squaring one launch of k_tile_plan turns the
 // marks into one bit per K-block for every output tile, leaves out the tiles that are zero and
-// stay zero, orders the others by the K-blocks they issue, most first (the persistent CTAs walk the tiles round robin, and the counts now differ by
-// an order of magnitude between the diagonal and the corners), clears the marks that the
-// squaring is going to write, and forms the row fixes of the previous level on the way (it
-// replaces that kernel's launch).  It costs a launch of 4-6 us per level, so single lattices
+// stay zero, orders the others by the K-blocks they issue, most first (the persistent CTAs walk
+// the tiles round robin, and the counts now differ by an order of magnitude between the diagonal
+// and the corners), clears the marks that the squaring is going to write, and forms the row
+// fixes of the previous level on the way (it replaces that kernel's launch).  It costs a launch of 4-6 us per level, so single lattices
 // below OPB_PLAN_MIN_D states, whose whole product takes about 16 us, go without.
 
 struct TilePlanArgs {
