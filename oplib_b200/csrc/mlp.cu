@@ -140,13 +140,16 @@ __global__ void __launch_bounds__(MLP_H) k_mlp_first(int B, const float *__restr
 
 // Z += b (per column), H = GELU(Z), four columns a thread.  Z, H: [B x 256] row-major.  H
 // (optional) in FP32 and/or its BF16 parts Hhi / Hlo (optional, for the tensor-core products).
+// Z and H are the workspace's and 16-byte aligned; b is the caller's, any float address (a network
+// is 199,937 floats: in an array of several, every second row starts off the 8-byte grid).
 __global__ void k_bias_gelu(long long total4, float *__restrict__ Z, const float *__restrict__ b,
                             float *__restrict__ H, __nv_bfloat16 *__restrict__ Hhi, __nv_bfloat16 *__restrict__ Hlo) {
     pdl_begin();
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= total4) return;
-    const float4 zv = reinterpret_cast<const float4 *>(Z)[i], bv = reinterpret_cast<const float4 *>(b)[i % (MLP_H / 4)];
-    const float z[4] = {zv.x + bv.x, zv.y + bv.y, zv.z + bv.z, zv.w + bv.w};
+    const float4 zv = reinterpret_cast<const float4 *>(Z)[i];
+    const float *bc = b + 4 * (i % (MLP_H / 4));
+    const float z[4] = {zv.x + bc[0], zv.y + bc[1], zv.z + bc[2], zv.w + bc[3]};
     float h[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) h[j] = gelu(z[j]);
@@ -243,8 +246,7 @@ __global__ void __launch_bounds__(MLP_H / 2) k_mlp_dz(int B, const float *__rest
     for (int r = 0; r < MLP_RB; r++) {
         if (LAST) {
             const float d = dy[r0 + min(r, n - 1)];
-            const float2 wc = *reinterpret_cast<const float2 *>(w5 + c);
-            g[r] = make_float2(d * wc.x, d * wc.y);
+            g[r] = make_float2(d * w5[c], d * w5[c + 1]);  // (w5: the caller's, any float address)
         } else {
             g[r] = *reinterpret_cast<const float2 *>(dH + at(r));
         }
