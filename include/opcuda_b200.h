@@ -412,7 +412,9 @@ int opcuda_mt_benchmark(uint64_t mtptr, uint64_t unif_ptr, int nscen);
  * Runs of up to 623 steps keep the generator in registers; longer runs hold the
  * 624-word state in per-thread local memory (2496 bytes a thread), which the CUDA
  * driver may provision on the first such launch. */
-int opb_mc_scratch_blocks(long long npaths); /* blocks of a run: scratch holds two doubles for each */
+/* scratch holds two doubles for each of opb_mc_scratch_blocks(npaths) blocks; it never falls as
+ * npaths grows, so a buffer for the largest run serves the smaller ones */
+int opb_mc_scratch_blocks(long long npaths);
 int opb_mc_mt19937(const float *C, long long row_stride, long long col_stride, const uint32_t *guide, int nb, int d,
                    int y0, int nsteps, uint32_t seed, unsigned long long path0, long long npaths, short *ypaths,
                    const double *x, double strike, double barrier, double disc, double *scratch, double *sums);

@@ -220,6 +220,15 @@ int mc_grid(long long npaths) {
     return (int)(b < 1 ? 1 : b < cap ? b : cap);
 }
 
+// What a caller's scratch must hold two doubles for each of: the most blocks that any run of up to
+// npaths paths is launched with.  (mc_grid itself falls where the blocks get wider -- 3552, then
+// 1777 from 227,329 paths on -- and a buffer sized for a program's largest run serves its smaller
+// ones.)
+static int mc_scratch_blocks(long long npaths) {
+    const long long b = (npaths + 63) / 64, cap = (long long)MC_BLOCKS_PER_SM * num_sms();
+    return (int)(b < 1 ? 1 : b < cap ? b : cap);
+}
+
 // The register-only generator up to 623 steps, the cursor/state-array one beyond; the
 // evaluator form when a cashflow table is given.
 template <bool ANY_LENGTH, bool GUIDED>
@@ -257,8 +266,9 @@ using namespace opb;
 // (optional, source-major rows only) is the opb_guide_table of C with nb buckets.
 // ypaths (optional) receives int16 states y[p + npaths*k].  x (optional, d doubles)
 // enables the fused payoffs; sums[0] / sums[1] receive the discounted barrier / Asian
-// payoff sums.  scratch must hold 2*opb_mc_scratch_blocks(npaths) doubles.
-OPB_API int opb_mc_scratch_blocks(long long npaths) { return mc_grid(npaths); }
+// payoff sums.  scratch must hold 2*opb_mc_scratch_blocks(npaths) doubles (a buffer for npaths
+// holds every smaller run's).
+OPB_API int opb_mc_scratch_blocks(long long npaths) { return mc_scratch_blocks(npaths); }
 
 OPB_API int opb_mc_mt19937(const float *C, long long row_stride, long long col_stride, const uint32_t *guide,
                            int nb, int d, int y0, int nsteps, uint32_t seed, unsigned long long path0,

@@ -193,3 +193,17 @@ def test_fused_normalisation_knob_values(lib):
     """-1 restores the automatic rule, 0 and above set a size limit; neither needs a device."""
     for v in (0, 8192, -1):
         assert lib.opb_set_fused_normalisation(v) == 0
+
+
+def test_mc_scratch_never_falls_as_paths_grow(lib):
+    """A buffer sized for a program's largest run holds every smaller run's partial sums: the size
+    does not fall where the launch goes over to wider blocks (64, 128, 256 threads), and covers the
+    blocks of each."""
+    cap = lib.opb_mc_scratch_blocks(1 << 50)
+    sizes = sorted({n for w in (64, 128, 256) for k in (1, 2, cap // 2, cap, 2 * cap)
+                    for n in (w * k - 1, w * k, w * k + 1, w * k + w)} | {1, 63, 227_000, 300_000, 1 << 20, 1 << 40})
+    got = [lib.opb_mc_scratch_blocks(n) for n in sizes]
+    assert got == sorted(got)
+    for n, g in zip(sizes, got):
+        threads = 64 if n <= 64 * cap else 128 if n <= 128 * cap else 256
+        assert g >= min(-(-n // threads), cap)
