@@ -282,8 +282,9 @@ int opb_set_lolo_levels(int n);
 /* new: 1 (default): squarings of an ELL generator's E_r = P(2^r dt) - I skip the K-blocks and
  * output tiles outside twice E_r's band (h0 * 2^r for the generator's half-bandwidth h0) and,
  * in batches and from 1536 states on, those whose blocks are zero inside it, whose products
- * are exact zeros; 0: every squaring runs the full product.  Results are
- * bit-identical either way */
+ * are exact zeros; 0: every squaring runs the full product.  The results of finite generators are
+ * bit-identical either way; a value that is not finite spreads through all blocks inside the
+ * band, as in the full product, but not through those outside it */
 int opb_set_band_skip(int on);
 /* new: the split-mode solves defer each product's FP64 row normalisation into the next
  * product's epilogue, which also writes that product's 16-bit operand parts, so no

@@ -264,7 +264,8 @@ size_t layout(const opb_batch_desc *b, int mode, opb_batch_plan *P, char *base, 
     plan.count = c.take<uint16_t>(tiles);
     plan.nw = nw;
     plan.done = reinterpret_cast<unsigned *>(occ0 + marks);
-    plan.nlist = plan.done + 1;
+    plan.wild = plan.done + 1;
+    plan.nlist = plan.done + 2;
     (void)c.take<double>((size_t)off[n] * ldk);     // FP64 option values of the backward induction
 
     // ---- work lists (host), appended into one blob
@@ -623,18 +624,19 @@ int batch_square(opb_batch_plan *P, int cfg, cudaStream_t s) {
     // sets start as zeros, with the row-sum partials and the marks.  Without them (band skipping
     // off) every level writes every tile.
     const bool planned = opb::g_band_skip != 0;
+    unsigned *wild = planned ? P->plan.wild : nullptr;
     if (r == 0) r = (int)cudaMemsetAsync(P->E_base, 0, P->E_bytes, s);
     if (r == 0 && planned) r = (int)cudaMemsetAsync(P->part, 0, P->part_bytes, s);
     if (r == 0 && planned) r = (int)cudaMemsetAsync(P->occ[0], 0, P->occ_bytes + 64, s);
     if (r == 0)
-        r = opb::launch_ek_batched(P->lats, P->nlat, P->total_rows, P->ell_width, P->cols, P->vals, s, planned, ss);
+        r = opb::launch_ek_batched(P->lats, P->nlat, P->total_rows, P->ell_width, P->cols, P->vals, s, wild, ss);
     if (r == 0 && !planned) r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_init.off, P->rn_init.n, 0, s, ss);
     for (int lv = 0; lv < P->maxn && r == 0; lv++) {
         if (planned) r = level_plan(P, cfg, lv, s);
         else if (lv > 0) r = opb::launch_rowfix_batched(P->lats, P->nlat, P->total_rows, pdiv, lv - 1, s);
         if (r == 0) r = level_gemm(P, cfg, lv, s);
         if (r == 0 && P->rn_level[lv].n > 0)
-            r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_level[lv].off, P->rn_level[lv].n, pdiv, s, ss, planned);
+            r = opb::launch_renorm_batched(P->rn_sq, P->work + P->rn_level[lv].off, P->rn_level[lv].n, pdiv, s, ss, wild);
     }
     return r;
 }

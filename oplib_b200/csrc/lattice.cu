@@ -113,7 +113,8 @@ Bufs carve(Ws &w, int d, int nK, int mode, bool pad = false) {
         b.occ[0] = w.take<uint8_t>(opb::tile_plan_marks(d) + 64);
         b.occ[1] = w.take<uint8_t>(opb::tile_plan_marks(d));
         b.plan.done = reinterpret_cast<unsigned *>(b.occ[0] + opb::tile_plan_marks(d));
-        b.plan.nlist = b.plan.done + 1;
+        b.plan.wild = b.plan.done + 1;
+        b.plan.nlist = b.plan.done + 2;
         b.plan.order = w.take<uint2>(tiles);
         b.plan.tile = w.take<uint32_t>(tiles);
         b.plan.kmask = w.take<uint32_t>(tiles * b.plan.nw);
@@ -241,7 +242,7 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
         // (a dense generator: every block marked, its parts from the split below)
         LT((int)cudaMemsetAsync(b.occ[0], ell ? 0 : 3, opb::tile_plan_marks(d), s));
         LT((int)cudaMemsetAsync(b.plan.done, 0, 64, s));
-        if (ell) e0 = opb::E0Parts{b.Ahi, b.Alo, b.occ[0], ss};
+        if (ell) e0 = opb::E0Parts{b.Ahi, b.Alo, b.occ[0], ss, b.plan.wild};
     }
     // (d_gen < d: the generator's d_gen states, then absorbing padding states)
     if (d_gen != d)
@@ -303,9 +304,11 @@ int square_tc(const opb_lattice_desc &L, Bufs &b, cudaStream_t s, bool f16, opb:
         // chain's A and pricing's; row-major into B: every chain's B); the others only the
         // row fixes of their output
         if (last)
-            LT(opb::launch_renorm_to_p(d, b.X, b.part, np, b.Ahi, b.Alo, b.Bhi, b.Blo, s, ss, fused ? mo : nullptr));
+            LT(opb::launch_renorm_to_p(d, b.X, b.part, np, b.Ahi, b.Alo, b.Bhi, b.Blo, s, ss, fused ? mo : nullptr,
+                                       b.plan.wild));
         else if (!fused)
-            LT(opb::launch_renorm(d, b.X, b.part, np, 1, b.Ahi, b.Alo, nullptr, nullptr, s, ss, 0, b.fix, mo));
+            LT(opb::launch_renorm(d, b.X, b.part, np, 1, b.Ahi, b.Alo, nullptr, nullptr, s, ss, 0, b.fix, mo,
+                                 b.plan.wild));
         else if (!planned) LT(opb::launch_rowfix(d, b.part, np, 1, b.fix, s));
     }
     g.Ahi = b.Ahi; g.Alo = b.Alo;

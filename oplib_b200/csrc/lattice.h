@@ -61,6 +61,10 @@ __device__ __forceinline__ void split2x2(float a, float b, uint32_t &hi, uint32_
     }
 }
 
+// Whether a value of E = P - I, |E| <= 1 for a probability matrix P, may not be finite in 16-bit
+// parts (FP16 parts are scaled by 2^15) or is not itself, NaN included.
+__device__ __forceinline__ bool e_wild(float v) { return !(fabsf(v) < 1.99f); }
+
 // Row fixes from FP64 row-sum partials, with the arithmetic of the renormalisation
 // kernels' row sums (renorm64_sums): s = sum of the nparts partials in order; E-form inv =
 // 1 / (1 + s), P-form inv = 1 / s.
@@ -100,6 +104,7 @@ struct E0Parts {
     __nv_bfloat16 *hi, *lo;
     uint8_t *occ;
     float sscale;
+    unsigned *wild;  // TilePlan::wild
 };
 int launch_ek_ell(int d, int w, const int *cols, const double *vals, double dt, int eform, float *out,
                   cudaStream_t s, const E0Parts &parts = E0Parts{});
@@ -116,10 +121,10 @@ int launch_rowsum(int d, const float *X, double *partial, cudaStream_t s);
 // write_x = 0 leaves X as it is (only the splits are written; d % 64 == 0); fix (optional,
 // E-form) receives the per-row (s, inv) that a following product applies to X as its Cin; occ
 // (optional, d % 64 == 0): X's marks (TcGemmArgs::occ), whose unmarked blocks are left out and
-// which receive those of the written A parts.
+// which receive those of the written A parts; wild with it (TilePlan::wild).
 int launch_renorm(int d, float *X, const double *partial, int nparts, int eform, __nv_bfloat16 *Ahi,
                   __nv_bfloat16 *Alo, __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale = 0.f,
-                  int write_x = 1, double2 *fix = nullptr, uint8_t *occ = nullptr);
+                  int write_x = 1, double2 *fix = nullptr, uint8_t *occ = nullptr, unsigned *wild = nullptr);
 int launch_add_identity(int d, float *X, cudaStream_t s);
 // dscale (device, optional): FP16 payoff split scale from launch_payoff_scale
 int launch_payoff_scale(int d, const double *x, int nK, const double *K, float *out, cudaStream_t s);
@@ -195,14 +200,14 @@ int launch_berm_step(int d, int nK, int ldk, const float *C, double disc, const 
                      long long slice_stride = 0);
 int launch_renorm_to_p(int d, float *X, const double *partial, int nparts, __nv_bfloat16 *Ahi, __nv_bfloat16 *Alo,
                        __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale = 0.f,
-                       const uint8_t *occ = nullptr);
-// marks: leave out the tiles that RenormProblem::occ shows to be zero.
+                       const uint8_t *occ = nullptr, unsigned *wild = nullptr);
+// wild (TilePlan::wild, optional): leave out the tiles that RenormProblem::occ shows to be zero.
 // work items: problem << 16 | mode << 14 | strip << 7 | chunk (see renorm_chunks)
 int launch_renorm_batched(const RenormProblem *probs, const uint32_t *work, int nwork, int parts_div, cudaStream_t s,
-                          float sscale = 0.f, int marks = 0);
-// parts: E0's 16-bit parts and marks too (planned squarings)
+                          float sscale = 0.f, unsigned *wild = nullptr);
+// wild (TilePlan::wild, optional): E0's 16-bit parts and marks too (planned squarings)
 int launch_ek_batched(const BatchLattice *lats, int nlat, long long total_rows, int w, const int *cols,
-                      const double *vals, cudaStream_t s, int parts = 0, float sscale = 0.f);
+                      const double *vals, cudaStream_t s, unsigned *wild = nullptr, float sscale = 0.f);
 int launch_payoff_batched(const BatchLattice *lats, int nlat, long long total_rows, int nK, int ldk, const double *x,
                           const double *strikes, cudaStream_t s, int f16 = 0);
 // Quotes of nm priced rows of every lattice (row slot i: maturity m0 + i + 1)
@@ -362,7 +367,11 @@ inline int tile_plan_words(int d) { return (d / 64 + 31) / 32; }
 struct TilePlan {
     uint2 *order;      // nlist items in issue order: index of the item's mask, packed tile
     uint32_t *kmask;   // nw words per item, one bit per K-block
-    unsigned *nlist;
+    unsigned *nlist;   // [0] the items, [1] whether the product is to ignore them (wild); 8-byte aligned
+    // set, for the rest of a solve, by whoever stores a value far from any probability matrix's:
+    // where it or its parts are not finite, zero blocks have products that are not zero.  Zero
+    // before the first level.
+    unsigned *wild;
     uint32_t *tile;    // scratch
     uint16_t *count;   // scratch
     int nw;

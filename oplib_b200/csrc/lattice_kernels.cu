@@ -37,6 +37,7 @@ __device__ __forceinline__ void e0_parts(const E0Parts &p, long long y, int z, l
     const long long o = y * ld + z;
     split2(f, p.hi[o], p.lo[o], p.sscale);
     p.occ[(y >> 5) * (ld >> 6) + (z >> 6)] = 3;
+    if (e_wild(f)) *p.wild = 1u;
 }
 
 // ELL generator: row y holds w (col, val) pairs; col < 0 marks padding.
@@ -286,7 +287,7 @@ __device__ __forceinline__ void renorm64_apply(RenormSmem &sm, int d, float *__r
                                                __nv_bfloat16 *__restrict__ Ahi, __nv_bfloat16 *__restrict__ Alo,
                                                __nv_bfloat16 *__restrict__ Bhi, __nv_bfloat16 *__restrict__ Blo,
                                                int r0, int c0, float sscale, const float4 (&vin)[4], bool b_rm,
-                                               uint8_t *__restrict__ occ = nullptr) {
+                                               uint8_t *__restrict__ occ = nullptr, unsigned *wild = nullptr) {
     const int tid = threadIdx.x;
     const bool eform = mode != 2;
     const bool transposed = Bhi && !b_rm;
@@ -326,6 +327,7 @@ __device__ __forceinline__ void renorm64_apply(RenormSmem &sm, int d, float *__r
                 if (!(reinterpret_cast<volatile uint8_t *>(occ)[at] & 1u))
                     atomicOr(reinterpret_cast<uint32_t *>(occ) + (at >> 2), 1u << (8 * (at & 3)));
             }
+            if (e_wild(f[0]) || e_wild(f[1]) || e_wild(f[2]) || e_wild(f[3])) *wild = 1u;
         }
         if (Bhi && b_rm) {
             *reinterpret_cast<uint2 *>(Bhi + o) = make_uint2(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]));
@@ -357,19 +359,20 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
                                                __nv_bfloat16 *__restrict__ Alo, __nv_bfloat16 *__restrict__ Bhi,
                                                __nv_bfloat16 *__restrict__ Blo, int r0, int first, int step,
                                                float sscale, double2 *__restrict__ fix, bool b_rm,
-                                               uint8_t *__restrict__ occ = nullptr) {
+                                               uint8_t *__restrict__ occ = nullptr, unsigned *wild = nullptr) {
     const int nt = d / 64, tid = threadIdx.x;
     int cnt = first < nt ? (nt - 1 - first) / step + 1 : 0;
     // under a tile plan the tiles without a mark (off the diagonal) are zero and stay zero, and so
-    // are their parts: left alone
+    // are their parts: left alone, unless a row's sum may not be finite
     const bool pick = MARKS && cnt <= RN_LIVE;
     if (MARKS && pick) {
         if (tid < 32) {
             int n = 0;
+            const unsigned every = *wild;
             for (int k0 = 0; k0 < cnt; k0 += 32) {
                 const int t = first + (k0 + tid) * step;
                 const bool on = k0 + tid < cnt && (t * 64 == r0 || (occ[(long long)(r0 >> 5) * nt + t] & 2) ||
-                                                   (occ[(long long)((r0 >> 5) + 1) * nt + t] & 2));
+                                                   (occ[(long long)((r0 >> 5) + 1) * nt + t] & 2) || every);
                 const uint32_t m = __ballot_sync(0xffffffffu, on);
                 if (on) sm.live[n + __popc(m & ((1u << tid) - 1u))] = (uint16_t)t;
                 n += __popc(m);
@@ -395,7 +398,8 @@ __device__ __forceinline__ void renorm64_strip(RenormSmem &sm, RenormRing &rg, i
         cp_async_wait<RN_RING - 1>();  // this thread's copies of tile k have landed
         const int sl = k % RN_RING;
         const float4 v[4] = {rg.v[sl][0][tid], rg.v[sl][1][tid], rg.v[sl][2][tid], rg.v[sl][3][tid]};
-        renorm64_apply(sm, d, Xout, mode, Ahi, Alo, Bhi, Blo, r0, col0(k), sscale, v, b_rm, MARKS ? occ : nullptr);
+        renorm64_apply(sm, d, Xout, mode, Ahi, Alo, Bhi, Blo, r0, col0(k), sscale, v, b_rm, MARKS ? occ : nullptr,
+                       wild);
     }
 }
 
@@ -410,14 +414,14 @@ __global__ void __launch_bounds__(256) k_renorm64(int d, float *__restrict__ X, 
                                                   __nv_bfloat16 *__restrict__ Alo, __nv_bfloat16 *__restrict__ Bhi,
                                                   __nv_bfloat16 *__restrict__ Blo, float sscale, int write_x,
                                                   double2 *__restrict__ fix, int b_rm,
-                                                  uint8_t *__restrict__ occ) {
+                                                  uint8_t *__restrict__ occ, unsigned *wild) {
     pdl_begin();
     extern __shared__ __align__(16) uint8_t rn_smem[];
     RenormSmem &sm = *reinterpret_cast<RenormSmem *>(rn_smem);
     RenormRing &rg = *reinterpret_cast<RenormRing *>(rn_smem + sizeof(RenormSmem));
     renorm64_strip<MARKS>(sm, rg, d, X, write_x ? X : nullptr, partial, nparts, mode, Ahi, Alo, Bhi, Blo,
                           (int)blockIdx.y * 64, (int)blockIdx.x, (int)gridDim.x, sscale, blockIdx.x == 0 ? fix : nullptr,
-                          b_rm != 0, occ);
+                          b_rm != 0, occ, wild);
 }
 
 // Column chunks of a k_renorm64 launch: about 8 blocks per SM in total.
@@ -438,7 +442,7 @@ static dim3 renorm64_grid(int d) {
 // row-major A parts as their B operand.
 __global__ void __launch_bounds__(256) k_renorm64_batched(const RenormProblem *__restrict__ probs,
                                                           const uint32_t *__restrict__ work, int parts_div,
-                                                          float sscale, int marks) {
+                                                          float sscale, unsigned *wild) {
     extern __shared__ __align__(16) uint8_t rn_smem[];
     RenormSmem &sm = *reinterpret_cast<RenormSmem *>(rn_smem);
     RenormRing &rg = *reinterpret_cast<RenormRing *>(rn_smem + sizeof(RenormSmem));
@@ -447,10 +451,10 @@ __global__ void __launch_bounds__(256) k_renorm64_batched(const RenormProblem *_
     const int mode = (int)((w >> 14) & 3u);
     const int nparts = parts_div > 0 ? pr.d / parts_div : 0;
     const int r0 = (int)((w >> 7) & 127u) * 64, chunk = (int)(w & 127u);
-    if (marks)
+    if (wild)
         renorm64_strip<true>(sm, rg, pr.d, pr.X, nullptr, pr.partial, nparts, mode, pr.Ahi, pr.Alo,
                    mode == 1 ? pr.Bhi : nullptr, mode == 1 ? pr.Blo : nullptr, r0, chunk, renorm_chunks(pr.d),
-                   sscale, mode == 0 && chunk == 0 ? pr.fix : nullptr, true, pr.occ);
+                   sscale, mode == 0 && chunk == 0 ? pr.fix : nullptr, true, pr.occ, wild);
     else
         renorm64_strip<false>(sm, rg, pr.d, pr.X, nullptr, pr.partial, nparts, mode, pr.Ahi, pr.Alo,
                    mode == 1 ? pr.Bhi : nullptr, mode == 1 ? pr.Blo : nullptr, r0, chunk, renorm_chunks(pr.d),
@@ -479,8 +483,8 @@ static int renorm64_prepare() {
 // Batched ELL scatter into zeroed dense E-form matrices: thread per global ELL slot
 // (rows of all lattices concatenated; row_off[i] = first global row of lattice i).
 __global__ void k_ek_scatter_batched(const BatchLattice *__restrict__ lats, int nlat, long long total_rows, int w,
-                                     const int *__restrict__ cols, const double *__restrict__ vals, int parts,
-                                     float sscale) {
+                                     const int *__restrict__ cols, const double *__restrict__ vals,
+                                     unsigned *wild, float sscale) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= total_rows * w) return;
     const long long grow = t / w;
@@ -495,7 +499,7 @@ __global__ void k_ek_scatter_batched(const BatchLattice *__restrict__ lats, int 
     if (z < 0 || z >= L.d) return;
     const float f = (float)(L.dt * vals[t]);
     L.E[(long long)y * L.d + z] = f;
-    if (parts) e0_parts(E0Parts{L.Ahi, L.Alo, L.occ0, sscale}, y, z, L.d, f);
+    if (wild) e0_parts(E0Parts{L.Ahi, L.Alo, L.occ0, sscale, wild}, y, z, L.d, f);
 }
 
 // Batched payoff splits: G^T[k][z] = (x_z - K_k)^+ for strikes k < nK of lattice i and 0
@@ -792,12 +796,12 @@ int launch_rowsum(int d, const float *X, double *partial, cudaStream_t s) {
 
 int launch_renorm(int d, float *X, const double *partial, int nparts, int eform, __nv_bfloat16 *Ahi,
                   __nv_bfloat16 *Alo, __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale,
-                  int write_x, double2 *fix, uint8_t *occ) {
+                  int write_x, double2 *fix, uint8_t *occ, unsigned *wild) {
     if (d % 64 == 0 && (Ahi != nullptr) == (Alo != nullptr)) {
         if (int r = renorm64_prepare()) return r;
         auto kern = occ ? k_renorm64<true> : k_renorm64<false>;
         launch_pdl(kern, renorm64_grid(d), 256, RN_SMEM, s, d, X, partial, nparts, eform ? 0 : 2, Ahi, Alo, Bhi,
-                   Blo, sscale, write_x, eform ? fix : nullptr, 0, occ);
+                   Blo, sscale, write_x, eform ? fix : nullptr, 0, occ, wild);
         return (int)cudaGetLastError();
     }
     if (!write_x || fix || occ) return OPB_E_UNSUPPORTED;
@@ -810,20 +814,21 @@ int launch_renorm(int d, float *X, const double *partial, int nparts, int eform,
 // (the last squaring level: P1 is the A of the first chain product and of pricing, and
 // the B of every chain product).
 int launch_renorm_to_p(int d, float *X, const double *partial, int nparts, __nv_bfloat16 *Ahi, __nv_bfloat16 *Alo,
-                       __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale, const uint8_t *occ) {
+                       __nv_bfloat16 *Bhi, __nv_bfloat16 *Blo, cudaStream_t s, float sscale, const uint8_t *occ,
+                       unsigned *wild) {
     if (d % 64) return OPB_E_UNSUPPORTED;
     if (int r = renorm64_prepare()) return r;
     auto kern = occ ? k_renorm64<true> : k_renorm64<false>;
     launch_pdl(kern, renorm64_grid(d), 256, RN_SMEM, s, d, X, partial, nparts, 1, Ahi, Alo, Bhi, Blo, sscale, 1,
-               nullptr, 1, const_cast<uint8_t *>(occ));
+               nullptr, 1, const_cast<uint8_t *>(occ), wild);
     return (int)cudaGetLastError();
 }
 
 int launch_renorm_batched(const RenormProblem *probs, const uint32_t *work, int nwork, int parts_div, cudaStream_t s,
-                          float sscale, int marks) {
+                          float sscale, unsigned *wild) {
     if (nwork <= 0) return OPB_OK;
     if (int r = renorm64_prepare()) return r;
-    k_renorm64_batched<<<nwork, 256, RN_SMEM, s>>>(probs, work, parts_div, sscale, marks);
+    k_renorm64_batched<<<nwork, 256, RN_SMEM, s>>>(probs, work, parts_div, sscale, wild);
     return (int)cudaGetLastError();
 }
 
@@ -865,10 +870,10 @@ int launch_pad_batched(const BatchLattice *lats, int nlat, long long total_rows,
 }
 
 int launch_ek_batched(const BatchLattice *lats, int nlat, long long total_rows, int w, const int *cols,
-                      const double *vals, cudaStream_t s, int parts, float sscale) {
+                      const double *vals, cudaStream_t s, unsigned *wild, float sscale) {
     long long n = total_rows * w;
     if (n <= 0) return OPB_OK;
-    k_ek_scatter_batched<<<(int)((n + 255) / 256), 256, 0, s>>>(lats, nlat, total_rows, w, cols, vals, parts, sscale);
+    k_ek_scatter_batched<<<(int)((n + 255) / 256), 256, 0, s>>>(lats, nlat, total_rows, w, cols, vals, wild, sscale);
     return (int)cudaGetLastError();
 }
 
@@ -1201,6 +1206,6 @@ OPB_API int opb_renorm_rows(int d, float *X, const double *partial, int nparts, 
                     nparts, mode, reinterpret_cast<__nv_bfloat16 *>(Ahi), reinterpret_cast<__nv_bfloat16 *>(Alo),
                     mode == 2 ? nullptr : reinterpret_cast<__nv_bfloat16 *>(Bhi),
                     mode == 2 ? nullptr : reinterpret_cast<__nv_bfloat16 *>(Blo), f16 ? 32768.f : 0.f, 1, nullptr, 0,
-                    nullptr);
+                    nullptr, nullptr);
     return opb::launch_check();
 }

@@ -8,7 +8,10 @@
 // 64 blocks that the band leaves, those with both operands non-zero are 3.8 of 9.4 dense
 // products over the 14 squarings of the SV lattice (d = 6144), 0.8 of 4.4 on a 2048-node
 // local-vol lattice.  A left-out block adds +0 products to an accumulator, so the results are
-// the same bits.
+// the same bits -- as long as the other operand is finite.  Whoever stores a value that is NaN or
+// infinite, or at 2 or above, where FP16 parts are, sets TilePlan::wild, and from the next level on
+// a solve's squarings take no notice of their plans (0 x NaN makes the row NaN, as it does in the
+// full product), and its renormalisations leave out no block.
 //
 // Whoever writes the parts marks the blocks (32 rows x 64 columns) that hold a non-zero hi part
 // (lo parts are zero where hi is); before the next squaring one launch of k_tile_plan turns the
@@ -56,6 +59,7 @@ __device__ __forceinline__ void raster_tile(int t, int mtiles, int ntiles, int g
 
 __global__ void __launch_bounds__(TP_THREADS) k_tile_plan(TilePlanArgs a) {
     pdl_begin();
+    const unsigned wild = *a.pl.wild;
     const long long tid = blockIdx.x * (long long)TP_THREADS + threadIdx.x, nth = (long long)gridDim.x * TP_THREADS;
     for (long long i = tid; i < a.clear_bytes / 16; i += nth) reinterpret_cast<uint4 *>(a.clear)[i] = make_uint4(0, 0, 0, 0);
     // ---- row fixes
@@ -172,7 +176,10 @@ __global__ void __launch_bounds__(TP_THREADS) k_tile_plan(TilePlanArgs a) {
                 bucket[b0 + lane] = run + s - v;
                 run += __shfl_sync(0xffffffffu, s, 31);
             }
-            if (lane == 0) *l.nlist = (unsigned)run;
+            if (lane == 0) {
+                l.nlist[0] = (unsigned)run;
+                l.nlist[1] = wild;
+            }
         }
         __syncthreads();
     }

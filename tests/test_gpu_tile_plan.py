@@ -58,3 +58,64 @@ def test_planned_batch_is_bit_identical(cuda, cfg):
     bt.set_config(cfg)
     full, planned = _both(lambda: bt.execute().clone())
     assert torch.equal(full, planned)
+
+
+def _spoiled(lat, how, dt):
+    """The lattice with one node's rates far from the quoted state spoiled, and its band as wide as the
+    matrix (an entry of rate zero in the far corner), so that band skipping leaves nothing out."""
+    from oplib_b200.model import Lattice
+    n, w = lat.d, lat.width
+    cols, vals = lat.cols.view(n, w), lat.vals.view(n, w).clone()
+    cols = torch.cat([cols, torch.full((n, 1), -1, dtype=cols.dtype, device=cols.device)], 1)
+    vals = torch.cat([vals, torch.zeros(n, 1, dtype=vals.dtype, device=vals.device)], 1)
+    cols[0, w] = n - 1
+    row = n - 9
+    if how == "grows":  # BF16 parts hold it, but not its square
+        vals[row] *= 1e18 / (vals[row].abs().max() * dt)
+    elif how == "huge":  # finite, but not in FP16 parts, and not once squared
+        vals[row] *= 1e33
+    else:
+        vals[row, 1] = float(how)
+    return Lattice(n, cols.reshape(-1).contiguous(), vals.reshape(-1).contiguous(), lat.x, lat.y0, lat.rate)
+
+
+@pytest.mark.parametrize("mode", ["bf16x3", "fp16x3"])
+@pytest.mark.parametrize("max_d", [0, 1 << 30])
+@pytest.mark.parametrize("n,how,niter", [(1600, "nan", 4), (2048, "nan", 3), (1600, "inf", 3), (2048, "huge", 3),
+                                         (2048, "grows", 3)])
+def test_values_that_are_not_finite_spread_as_in_the_full_products(cuda, n, how, niter, max_d, mode):
+    """A zero block has products that are not zero where the other operand is NaN or infinite: from the
+    level on at which such a value appears nothing is left out."""
+    from oplib_b200 import _lib
+    from oplib_b200.model import Lattice, Plan
+    lib = _lib.load()
+    clean = Lattice.local_vol(n=n, device=cuda)
+    plan = Plan(niter, clean.plan(0.25, 2.0 ** -12).dt, 0.0)
+    lat = _spoiled(clean, how, plan.dt)
+    assert lib.opb_set_fused_normalisation(max_d) == 0
+    try:
+        full, planned = _both(lambda: lat.solve(STRIKES, 2, 0.01, 0.0, mode=mode, plan=plan, all_states=True)[1])
+        quotes, _ = lat.solve(STRIKES, 2, 0.01, 0.0, mode=mode, plan=plan)
+    finally:
+        lib.opb_set_fused_normalisation(-1)
+    assert how == "grows" or not torch.isfinite(full).all()
+    torch.testing.assert_close(planned, full, rtol=0, atol=0, equal_nan=True)
+    if how == "nan":  # (every state reaches the spoiled one)
+        assert torch.isnan(quotes).all()
+
+
+def test_a_lattice_that_is_not_finite_leaves_the_others_of_a_batch(cuda):
+    from oplib_b200.model import Batch, Lattice
+    lats = [Lattice.local_vol(n=n, level=0.12 + 0.03 * i, device=cuda) for i, n in enumerate([1152, 700, 256])]
+    bt = Batch(lats, STRIKES, 3, 0.25, 2.0 ** -14, autotune=False)
+    clean = bt.execute().clone()
+    at = lats[0].vals.numel() + 3 * 690 + 1  # the second lattice's node 690
+    was = bt.vals[at].clone()
+    bt.vals[at] = float("nan")
+    for cfg in range(8):
+        bt.set_config(cfg)
+        got = bt.execute().clone()
+        assert torch.isnan(got[1]).all()
+        assert torch.equal(got[0], clean[0]) and torch.equal(got[2], clean[2])
+    bt.vals[at] = was
+    assert torch.equal(bt.execute(), clean)
