@@ -480,17 +480,40 @@ static bool sgemm_pipe_ok(const SgemmArgs &a, int batch) {
 //   aligned, whole 128-tiles   512^3: small 22, pipe 58; 1024^3: 79, 112; 1280^3 (100 tiles): 130,
 //                              140; 1408^3 (121): 177, 152; 4096^3: 3272, 2712 -> the pipe from 112 tiles on
 //   aligned, ragged            577 .. 4100: small at every size (4100^3: 3394 against 3576 of k_sgemm_rm)
-//   unaligned rows             1001^3 (64 tiles): small 97, rm 138; 2047^3 (256): 568, 456 -> rm from
-//                              a tile per SM on (the 4-byte copies)
+//   rows off the 16-byte grid  small_tiles_win (the 4-byte copies)
 // and of the small tiles 64 x 64 from 240 of them on (1000^3: 79 against 79), 64 x 32 below.
 constexpr int SG_PIPE_TILES = 112, ST_WIDE_TILES = 240;
+
+// k_sgemm_small against k_sgemm_rm where the rows of A or B are off the 16-byte grid, by their leading
+// dimension or by their base: the first then copies 4 bytes at a time, the second loads that way at
+// any alignment.  Both go by the tiles of the busiest SM, in us per unit of K: 128 x 128 ones in pairs
+// (0.235 a pair, 0.14 alone; a fifth more with A off the grid at a multiple of 128 bytes, where every
+// row's 64 bytes take a further sector), 64 x 64 ones at 0.0333 each with one operand off the grid,
+// 0.038 with both, and 0.02.  Measured, us, small / rm, A off, B off, both:
+//   1500^3  223/203 221/205 250/203     2560^3   958/1340  958/933  1087/1339
+//   1536^3  227/228 226/217 256/228     3000^3  1512/1328 1509/1325 1714/1328
+//   1664^3  300/443 300/407 339/443     4096^3  3777/4275 3773/3577 4293/4275
+//   2048^3  502/544 502/512 568/544     64 x 256^3 68/75    68/72     76/75
+static bool small_tiles_win(const SgemmArgs &a, int batch) {
+    auto off = [&](const float *q, const void *tab, int ld, long long stride) {
+        return ld % 4 || (!tab && (reinterpret_cast<uintptr_t>(q) % 16 || (batch > 1 && stride % 4)));
+    };
+    const bool a4 = off(a.A, a.A_tab, a.lda, a.sA), b4 = off(a.B, a.B_tab, a.ldb, a.sB);
+    if (!a4 && !b4) return true;
+    auto busiest = [&](int t) {
+        const long long n = (long long)((a.M + t - 1) / t) * ((a.N + t - 1) / t) * batch;
+        return (n + num_sms() - 1) / num_sms();
+    };
+    const long long u = busiest(128);
+    const double rm = (0.235 * (u / 2) + 0.14 * (u % 2)) * (a4 && a.lda % 32 == 0 ? 1.2 : 1.0);
+    return (a4 && b4 ? 0.038 : 0.0333) * busiest(64) + 0.02 < rm;
+}
 
 int sgemm_rowmajor(const SgemmArgs &a, int batch, cudaStream_t s, bool ta = false, bool tb = false) {
     if (a.M <= 0 || a.N <= 0 || batch <= 0) return OPB_OK;
     const long long tiles = (long long)((a.M + SG_BM - 1) / SG_BM) * ((a.N + SG_BN - 1) / SG_BN) * batch;
     const bool pipe = !ta && !tb && sgemm_pipe_ok(a, batch) && tiles >= SG_PIPE_TILES;
-    const bool rows16 = a.lda % 4 == 0 && a.ldb % 4 == 0;
-    if (!ta && !tb && !pipe && (rows16 || tiles < num_sms()) && a.M <= 65535 * 64) {  // (grid rows)
+    if (!ta && !tb && !pipe && small_tiles_win(a, batch) && a.M <= 65535 * 64) {  // (grid rows)
         const dim3 g64((a.N + 63) / 64, (a.M + 63) / 64, batch);
         if ((long long)g64.x * g64.y * g64.z >= ST_WIDE_TILES) k_sgemm_small<8, 1, 4><<<g64, 128, 0, s>>>(a);
         else k_sgemm_small<4, 2, 2><<<dim3(g64.x, (a.M + 31) / 32, batch), 128, 0, s>>>(a);

@@ -101,3 +101,32 @@ def test_grouped_products_across_the_table_sizes(cuda, count):
     want[-1, 64:, 14 * 16:] = float("nan")
     assert torch.equal(torch.isnan(got), torch.isnan(want))
     assert torch.equal(got.nan_to_num(), want.nan_to_num())
+
+
+# one 128 x 128 tile an SM, and a second on some; rows on the grid, bases and rows off it
+@pytest.mark.parametrize("M,K,off_a,off_b,kernel", [
+    (1536, 32, 0, 0, "k_sgemm_pipe"), (1536, 32, 1, 0, "k_sgemm_small"), (1536, 32, 0, 1, "k_sgemm_rm"),
+    (1536, 32, 3, 2, "k_sgemm_rm"), (1664, 32, 1, 1, "k_sgemm_small"), (1500, 36, 1, 0, "k_sgemm_rm"),
+    (1501, 33, 0, 0, "k_sgemm_rm"), (1001, 33, 0, 0, "k_sgemm_small")])
+def test_products_off_the_16_byte_grid(cuda, M, K, off_a, off_b, kernel):
+    """The kernel that the measured rule names, and the bits of the product at aligned bases."""
+    from torch.profiler import ProfilerActivity, profile
+    from oplib_b200 import _lib
+    from oplib_b200.model import bind_stream
+    lib = _lib.load()
+    bind_stream(cuda)
+    g = torch.Generator(device=cuda).manual_seed(5)
+    A, B = torch.randn(M, K, device=cuda, generator=g), torch.randn(K, M, device=cuda, generator=g)
+    want = _product(lib, A, B)[0]
+
+    def at(v, o):
+        buf = torch.empty(v.numel() + o, device=cuda)
+        buf[o:] = v.reshape(-1)
+        return buf[o:]
+    a, b, C = at(A, off_a), at(B, off_b), torch.full((M, M), float("nan"), device=cuda)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        assert lib.opb_sgemm_batched_rm(M, M, K, a.data_ptr(), 0, b.data_ptr(), 0, C.data_ptr(), 0, 1) == 0
+        torch.cuda.synchronize()
+    assert torch.equal(C, want)
+    ran = [e.name for e in prof.events() if "k_sgemm" in e.name]
+    assert len(ran) == 1 and kernel in ran[0]
