@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256, ANY_LENGTH ? 4 : 6) k_mc(McArgs a) {
             }
             if (GUIDED || a.guide) {
                 int bkt = (int)__fmul_rn(u, nbf);
-                bkt = bkt < a.nb ? bkt : a.nb - 1;
+                bkt = min(bkt, a.nb - 1);
                 const uint32_t gw = __ldg(a.guide + (uint32_t)(y * a.nb + bkt));
                 lo = (int)(gw & 0xffffu);
                 hi = (int)(gw >> 16);

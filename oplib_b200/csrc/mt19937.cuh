@@ -85,12 +85,12 @@ OPB_MT_FN uint32_t mt19937_cursor_words(uint32_t seed, uint32_t key1, int n, F &
     const uint32_t m1 = mt_init_next(seed, 1u) + key1;
     // cursor A: a1 = mt[i+1]; x0 = mt[i], from phase 2 on with the other cursors' words in it
     uint32_t x0 = seed, a1 = m1, a0 = seed;
-    // cursor B at i + 397
+    // cursor B at i + 397 (its index comes from i: counted in a register of its own, the Monte Carlo
+    // with states spilled)
     uint32_t b = m1;
 #pragma unroll 4
     for (uint32_t j = 2; j <= 397; j++) b = mt_init_next(b, j);
     const uint32_t m397 = b;
-    uint32_t bi = 397;
     int i = 0;
     const int n1 = n < 227 ? n : 227;
 #pragma unroll kMtUnroll
@@ -98,13 +98,13 @@ OPB_MT_FN uint32_t mt19937_cursor_words(uint32_t seed, uint32_t key1, int n, F &
         f(i, mt_tw_xor(x0, a1, b));
         x0 = a0 = a1;
         a1 = mt_init_next(a1, (uint32_t)i + 2u);
-        bi++; b = mt_init_next(b, bi);
+        b = mt_init_next(b, (uint32_t)i + 398u);
     }
     if (i >= n) return a0;
     // phase 2: cursor C (c1 = mt[i-226]) from the seed, cursor B restarted at 397
     uint32_t c1 = m1;
     x0 ^= seed;
-    b = m397; bi = 397;
+    b = m397;
     const int n2 = n < 454 ? n : 454;
 #pragma unroll kMtUnroll
     for (; i < n2; i++) {
@@ -113,13 +113,13 @@ OPB_MT_FN uint32_t mt19937_cursor_words(uint32_t seed, uint32_t key1, int n, F &
         x0 = x1; a0 = a1;
         a1 = mt_init_next(a1, (uint32_t)i + 2u);
         c1 = mt_init_next(c1, (uint32_t)(i - 227) + 2u);
-        bi++; b = mt_init_next(b, bi);
+        b = mt_init_next(b, (uint32_t)(i - 227) + 398u);
     }
     if (i >= n) return a0;
     // phase 3: cursor D (d1 = mt[i-453]) from the seed, B restarted at 397 (= i-57 at i = 454)
     uint32_t d1 = m1;
     x0 ^= seed;
-    b = m397; bi = 397;
+    b = m397;
 #pragma unroll kMtUnroll
     for (; i < n; i++) {
         const uint32_t x1 = a1 ^ c1 ^ d1;
@@ -128,7 +128,7 @@ OPB_MT_FN uint32_t mt19937_cursor_words(uint32_t seed, uint32_t key1, int n, F &
         a1 = mt_init_next(a1, (uint32_t)i + 2u);
         c1 = mt_init_next(c1, (uint32_t)(i - 227) + 2u);
         d1 = mt_init_next(d1, (uint32_t)(i - 454) + 2u);
-        bi++; b = mt_init_next(b, bi);
+        b = mt_init_next(b, (uint32_t)(i - 454) + 398u);
     }
     return a0;
 }

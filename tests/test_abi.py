@@ -207,3 +207,17 @@ def test_mc_scratch_never_falls_as_paths_grow(lib):
     for n, g in zip(sizes, got):
         threads = 64 if n <= 64 * cap else 128 if n <= 128 * cap else 256
         assert g >= min(-(-n // threads), cap)
+
+
+def test_short_monte_carlo_runs_use_no_local_memory(tmp_path):
+    """The kernels of opb_mc_mt19937_noalloc (payoffs, runs of up to 623 steps, with and without a
+    guide and states) have no stack frame, so that no launch makes the driver provision local memory."""
+    from oplib_b200 import build
+    src = build.CSRC / "mc.cu"
+    r = subprocess.run([build.NVCC, *build.ARCH, "-O3", "-std=c++17", "--expt-relaxed-constexpr", "--extended-lambda",
+                        "-Xptxas", "-v", "-cubin", str(src), "-o", str(tmp_path / "mc.cubin")],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    frames = dict(re.findall(r"Function properties for (\S*k_mc\S*)\n\s+(\d+) bytes stack frame", r.stderr))
+    short = {k: int(v) for k, v in frames.items() if re.search(r"k_mcILb0ELb[01]ELb0ELb[01]E", k)}
+    assert len(short) == 4 and not any(short.values()), short
