@@ -79,9 +79,9 @@ struct McArgs {
 // branches for what the launch does not ask for.  Six blocks of 256 an SM (40 registers) hide
 // the step's chain of dependent loads (guide word, row entry, next guide word); the form for
 // longer runs gains more from registers than from warps.  2^20 paths x 504 steps over 512
-// states: 2.51 -> 1.81 ms.
-template <bool ANY_LENGTH, bool GUIDED, bool EVAL, bool STATES>
-__global__ void __launch_bounds__(256, ANY_LENGTH ? 4 : 6) k_mc(McArgs a) {
+// states: 2.51 -> 1.81 ms.  PER_SM: blocks of 256 an SM, see mc_more_resident.
+template <bool ANY_LENGTH, bool GUIDED, bool EVAL, bool STATES, int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM) k_mc(McArgs a) {
     double s_bar = 0.0, s_asi = 0.0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     const float nbf = (float)a.nb;
@@ -231,12 +231,39 @@ static int mc_scratch_blocks(long long npaths) {
 
 // The register-only generator up to 623 steps, the cursor/state-array one beyond; the
 // evaluator form when a cashflow table is given.
+template <bool ANY_LENGTH, bool GUIDED, int PER_SM, bool EVAL>
+static void launch_mc_kernel(int grid, int threads, const McArgs &a) {
+    if (a.ypaths) k_mc<ANY_LENGTH, GUIDED, EVAL, true, PER_SM><<<grid, threads, 0, stream()>>>(a);
+    else k_mc<ANY_LENGTH, GUIDED, EVAL, false, PER_SM><<<grid, threads, 0, stream()>>>(a);
+}
+
+// How many blocks of 256 an SM a form is built for: registers make a path faster, resident paths
+// save waves, and a path is one thread's work from end to end, so a wave costs nearly its whole
+// time however few paths are left for it.  The form with more registers, then, unless the other
+// takes fewer waves.  Measured, us, 700 steps at 4 / 6 blocks: 130,000 paths (one wave either way)
+// 410 / 425; 190,000 (two, one) 697 / 573; 262,144 (two, two) 770 / 842; 454,000 (three, two) 1215 /
+// 1160, unguided the same up to two waves and 8576 / 9066 at 600,000 (four, three), where the searches'
+// loads are the limit.  The evaluator over 252 steps at 6 / 8: 227,000 259 / 261; 262,144 361 / 284;
+// 350,000 (two, two) 390 / 411; 2^20 (five, four) 980 / 908.
+static bool mc_more_resident(long long npaths, int few, int many, int most_waves) {
+    auto waves = [&](int m) { return (npaths + 256LL * m * num_sms() - 1) / (256LL * m * num_sms()); };
+    return waves(many) < waves(few) && waves(many) <= most_waves;
+}
+
 template <bool ANY_LENGTH, bool GUIDED>
 static void launch_mc_form(int grid, int threads, const McArgs &a) {
-    if (a.cf && a.ypaths) k_mc<ANY_LENGTH, GUIDED, true, true><<<grid, threads, 0, stream()>>>(a);
-    else if (a.cf) k_mc<ANY_LENGTH, GUIDED, true, false><<<grid, threads, 0, stream()>>>(a);
-    else if (a.ypaths) k_mc<ANY_LENGTH, GUIDED, false, true><<<grid, threads, 0, stream()>>>(a);
-    else k_mc<ANY_LENGTH, GUIDED, false, false><<<grid, threads, 0, stream()>>>(a);
+    if constexpr (ANY_LENGTH) {
+        const bool more = mc_more_resident(a.npaths, 4, 6, GUIDED ? 1 << 30 : 2);
+        if (a.cf && more) launch_mc_kernel<true, GUIDED, 6, true>(grid, threads, a);
+        else if (a.cf) launch_mc_kernel<true, GUIDED, 4, true>(grid, threads, a);
+        else if (more) launch_mc_kernel<true, GUIDED, 6, false>(grid, threads, a);
+        else launch_mc_kernel<true, GUIDED, 4, false>(grid, threads, a);
+    } else if (a.cf) {
+        if (mc_more_resident(a.npaths, 6, 8, 1 << 30)) launch_mc_kernel<false, GUIDED, 8, true>(grid, threads, a);
+        else launch_mc_kernel<false, GUIDED, 6, true>(grid, threads, a);
+    } else {
+        launch_mc_kernel<false, GUIDED, 6, false>(grid, threads, a);
+    }
 }
 static int launch_mc(McArgs &a) {
     const int grid = mc_grid(a.npaths), threads = mc_threads(a.npaths);
