@@ -726,8 +726,9 @@ OPB_API int opb_batch_execute_bermudan(opb_batch_plan *P, int put, int exercise,
 // keeps the fastest (which K-blocks a tile issues depends on the generators' spread, so a dense
 // product says little: it prefers 256 x 256 tiles where 128 x 256 ones take 15.0 ms to their
 // 15.7 for 256 lattices of the sweep).  A tile plan orders the items by what they issue, whatever
-// order they are listed in, so one run of each tile form is timed and its two orders share it; without
-// plans (band skipping off) every configuration is, reps times.  ms[cfg] (optional,
+// order they are listed in, so a tile form's two orders share one time; without plans (band
+// skipping off) every configuration has its own.  Each is run reps times and the fastest run
+// counts, since a disturbed one would choose for all executions to come.  ms[cfg] (optional,
 // opb_batch_num_configs() entries) receives the times.
 // Blocking; leaves the plan's buffers in an arbitrary state (run execute afterwards).
 OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *best_cfg) {
@@ -738,9 +739,15 @@ OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *
     }
     if (reps < 1) reps = 1;
     cudaStream_t s = opb::stream();
-    cudaEvent_t e0, e1;
-    OPB_TRY(cudaEventCreate(&e0));
-    OPB_TRY(cudaEventCreate(&e1));
+    struct Events {
+        cudaEvent_t e[2] = {nullptr, nullptr};
+        ~Events() {
+            for (cudaEvent_t v : e)
+                if (v) cudaEventDestroy(v);
+        }
+    } ev;
+    OPB_TRY(cudaEventCreate(&ev.e[0]));
+    OPB_TRY(cudaEventCreate(&ev.e[1]));
     float best = 1e30f;
     int bc = 0;
     for (int cfg = 0; cfg < NCFG; cfg++) {
@@ -756,22 +763,20 @@ OPB_API int opb_batch_autotune(opb_batch_plan *P, int reps, float *ms_out, int *
         if (r == 0 && cfg > 0 && planned) r = level_plan(P, cfg, 0, s);
         if (r == 0 && cfg > 0) r = level_gemm(P, cfg, 0, s);
         if (r) return set_status(r);
-        const int n = planned ? 1 : reps;
-        OPB_TRY(cudaEventRecord(e0, s));
-        for (int i = 0; i < n; i++) {
+        float ms = 1e30f;
+        for (int i = 0; i < reps; i++) {
+            OPB_TRY(cudaEventRecord(ev.e[0], s));
             r = batch_square(P, cfg, s);
             if (r) return set_status(r);
+            OPB_TRY(cudaEventRecord(ev.e[1], s));
+            OPB_TRY(cudaEventSynchronize(ev.e[1]));
+            float t = 0.f;
+            OPB_TRY(cudaEventElapsedTime(&t, ev.e[0], ev.e[1]));
+            ms = std::min(ms, t);
         }
-        OPB_TRY(cudaEventRecord(e1, s));
-        OPB_TRY(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        OPB_TRY(cudaEventElapsedTime(&ms, e0, e1));
-        ms /= n;
         if (ms_out) ms_out[cfg] = ms;
         if (ms < best) { best = ms; bc = cfg; }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     P->cfg = bc;
     if (best_cfg) *best_cfg = bc;
     return set_status(OPB_OK);

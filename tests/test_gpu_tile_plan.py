@@ -119,3 +119,24 @@ def test_a_lattice_that_is_not_finite_leaves_the_others_of_a_batch(cuda):
         assert torch.equal(got[0], clean[0]) and torch.equal(got[2], clean[2])
     bt.vals[at] = was
     assert torch.equal(bt.execute(), clean)
+
+
+def test_autotune_runs_every_tile_form_as_often_as_asked(cuda):
+    """One run decides nothing: each of the four tile forms is timed reps times over its squarings."""
+    import ctypes as C
+    from torch.profiler import ProfilerActivity, profile
+    from oplib_b200 import _lib
+    from oplib_b200.model import Batch, Lattice, bind_stream
+    lib = _lib.load()
+    lats = [Lattice.local_vol(n=n, device=cuda) for n in (256, 384)]
+    bt = Batch(lats, STRIKES, 2, 0.25, 2.0 ** -10, autotune=False)
+    levels = max(p.niter for p in bt.plans)
+    ms, best, plans = (C.c_float * 8)(), C.c_int(), []
+    bind_stream(cuda)
+    for reps in (1, 3):
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            assert lib.opb_batch_autotune(bt.plan, reps, ms, C.byref(best)) == 0
+            torch.cuda.synchronize()
+        plans.append(sum("k_tile_plan" in e.name for e in prof.events()))
+        assert ms[best.value] == min(ms) and 0 < min(ms) and max(ms) < 1e3
+    assert plans[1] - plans[0] == 2 * 4 * levels
