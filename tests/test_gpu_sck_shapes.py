@@ -47,3 +47,27 @@ def test_guide_of_a_row_longer_than_the_staged_one(cuda):
         hi = np.searchsorted(got[r], np.arange(1, 257) / 256, side="left").clip(max=d - 1)
         hi[-1] = d - 1
         assert np.array_equal(g[r] & 0xffff, lo) and np.array_equal(g[r] >> 16, np.maximum(lo, hi))
+
+
+# blocks of 32 rows, their last one short; the widest row they take and one past it; in place
+@pytest.mark.parametrize("d,nrows,kernel", [(1, 33, "k_sck_short"), (2, 64, "k_sck_short"), (16, 5000, "k_sck_short"),
+                                            (100, 31, "k_sck_short"), (127, 65, "k_sck_short"),
+                                            (128, 32, "k_sck_short"), (129, 33, "k_sck_rm")])
+def test_short_rows(cuda, d, nrows, kernel):
+    from torch.profiler import ProfilerActivity, profile
+    from oplib_b200 import _lib
+    from oplib_b200.model import bind_stream
+    P, C = rows_for(d, nrows, cuda)
+    acc = np.cumsum(np.where(P > 0, P, np.float32(0)), axis=1, dtype=np.float32)  # sequential FP32 sums
+    with np.errstate(invalid="ignore"):
+        want = acc / acc[:, -1:]
+    want = np.where(want < 1, want, np.float32(1))
+    assert np.array_equal(C.cpu().numpy(), want)
+    same = torch.from_numpy(P).to(cuda)
+    bind_stream(cuda)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        assert _lib.load().opb_sck_rm(d, nrows, same.data_ptr(), same.data_ptr()) == 0
+        torch.cuda.synchronize()
+    assert torch.equal(same, C)
+    ran = [e.name for e in prof.events() if "k_sck" in e.name]
+    assert len(ran) == 1 and kernel in ran[0]
