@@ -146,22 +146,30 @@ __global__ void k_sck_cm(int d, int nm, const float *__restrict__ P, float *__re
     }
 }
 
-// One block per row, a thread per bucket boundary pair; the row is searched in shared memory as
-// long as it fits (GUIDE_STAGED columns), the searches being chains of dependent loads.  512 rows,
-// 1024 buckets: 37 -> 8 us against one warp per row searching in L1.
+// 2^shift threads a row, a thread per bucket boundary pair, 256 >> shift rows a block.  The searches
+// are chains of dependent loads, so a table of few rows gets a block a row, and the row is
+// searched in shared memory as long as it fits (GUIDE_STAGED floats).  512 rows, 1024
+// buckets: 37 -> 8 us against one warp per row searching in L1.  Many rows fill the SMs with a warp
+// each: 50,000 rows of 64, 64 buckets 52 us with a block a row, 25 with a warp; and rows much longer
+// than their buckets are cheaper to probe than to read: 4096 of 4096, 1 bucket 10.9 us staged, 6.7.
 constexpr int GUIDE_THREADS = 256, GUIDE_STAGED = 48 * 1024 / 4;
 
-__global__ void __launch_bounds__(GUIDE_THREADS) k_guide(int d, int nb, const float *__restrict__ C,
-                                                         uint32_t *__restrict__ guide) {
+template <bool STAGED>
+__global__ void __launch_bounds__(GUIDE_THREADS) k_guide(int d, int nrows, int nb, int shift,
+                                                         const float *__restrict__ C, uint32_t *__restrict__ guide) {
     extern __shared__ float staged[];
-    const float *row = C + (long long)blockIdx.x * d;
-    if (d <= GUIDE_STAGED) {
-        for (int c = threadIdx.x; c < d; c += GUIDE_THREADS) staged[c] = row[c];
+    const int per_row = 1 << shift, rows = GUIDE_THREADS >> shift, r0 = blockIdx.x * rows;
+    const int mine = (int)threadIdx.x >> shift;
+    const float *row = C + (long long)(r0 + mine) * d;
+    if constexpr (STAGED) {
+        const int n = min(rows, nrows - r0) * d;
+        for (int c = threadIdx.x; c < n; c += GUIDE_THREADS) staged[c] = C[(long long)r0 * d + c];
         __syncthreads();
-        row = staged;
+        row = staged + mine * d;
     }
+    if (r0 + mine >= nrows) return;
     const float inv = 1.0f / (float)nb;  // exact: nb is a power of two
-    for (int b = threadIdx.x; b < nb; b += GUIDE_THREADS) {
+    for (int b = threadIdx.x & (per_row - 1); b < nb; b += per_row) {
         float lo_t = (float)b * inv, hi_t = (float)(b + 1) * inv;
         // first z with C[z] > lo_t (binary search on the non-decreasing row)
         int lo = 0, hi = d;  // answer in [lo, hi], d = none
@@ -182,7 +190,7 @@ __global__ void __launch_bounds__(GUIDE_THREADS) k_guide(int d, int nb, const fl
             ub = lo < d ? lo : d - 1;
         }
         if (ub < lb) ub = lb;
-        guide[(long long)blockIdx.x * nb + b] = (uint32_t)lb | ((uint32_t)ub << 16);
+        guide[(long long)(r0 + mine) * nb + b] = (uint32_t)lb | ((uint32_t)ub << 16);
     }
 }
 
@@ -193,7 +201,22 @@ int launch_sck_rm(int d, int nrows, const float *P, float *C, cudaStream_t s) {
 }
 
 int launch_guide(int d, int nrows, int nb, const float *C, uint32_t *guide, cudaStream_t s) {
-    k_guide<<<nrows, GUIDE_THREADS, d <= GUIDE_STAGED ? d * sizeof(float) : 0, s>>>(d, nb, C, guide);
+    // tables of few rows: a block a row.  Else a warp a row, twice that and so on while the threads are
+    // fewer than 2^18 and no more than the buckets, or a thread would search 32 buckets or more, or
+    // the block's rows would leave it fewer than three neighbours on its SM
+    int shift = 8;
+    bool staged = d <= GUIDE_STAGED;
+    if (nrows >= 2048) {
+        staged = staged && d < 32 * nb;
+        for (shift = 5; shift < 8; shift++) {
+            const long long per_row = 1LL << shift;
+            if (!((nb > per_row && nrows * per_row < 1 << 18) || nb >= 32 * per_row || (staged && (d << (8 - shift)) > 4096)))
+                break;
+        }
+    }
+    const int rows = GUIDE_THREADS >> shift, grid = (nrows + rows - 1) / rows;
+    if (staged) k_guide<true><<<grid, GUIDE_THREADS, rows * d * sizeof(float), s>>>(d, nrows, nb, shift, C, guide);
+    else k_guide<false><<<grid, GUIDE_THREADS, 0, s>>>(d, nrows, nb, shift, C, guide);
     return (int)cudaGetLastError();
 }
 

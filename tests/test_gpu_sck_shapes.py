@@ -71,3 +71,27 @@ def test_short_rows(cuda, d, nrows, kernel):
     assert torch.equal(same, C)
     ran = [e.name for e in prof.events() if "k_sck" in e.name]
     assert len(ran) == 1 and kernel in ran[0]
+
+
+# tables of many rows: a warp, two, four or eight a row, searched in place or staged; and one of few
+@pytest.mark.parametrize("d,nrows,nb,blocks", [(5, 8195, 8, 1025), (64, 2049, 64, 513), (100, 2050, 256, 1025),
+                                               (512, 2048, 4096, 2048), (1000, 2060, 128, 1030),
+                                               (2100, 2051, 4, 257), (64, 2047, 64, 2047)])
+def test_guides_of_many_rows(cuda, tmp_path, d, nrows, nb, blocks):
+    import json
+    from torch.profiler import ProfilerActivity, profile
+    from oplib_b200.model import guide_table
+    _, C = rows_for(d, nrows, cuda)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        g = guide_table(C, nb)
+        torch.cuda.synchronize()
+    g, got = g.cpu().numpy().view(np.uint32), C.cpu().numpy()
+    for r in list(range(0, nrows, 97)) + [nrows - 2, nrows - 1]:
+        lo = np.searchsorted(got[r], np.arange(nb) / nb, side="right").clip(max=d - 1)
+        hi = np.searchsorted(got[r], np.arange(1, nb + 1) / nb, side="left").clip(max=d - 1)
+        hi[-1] = d - 1
+        assert np.array_equal(g[r] & 0xffff, lo) and np.array_equal(g[r] >> 16, np.maximum(lo, hi))
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+    grids = [e["args"]["grid"][0] for e in events if e.get("cat") == "kernel" and "k_guide" in e["name"]]
+    assert grids == [blocks]
