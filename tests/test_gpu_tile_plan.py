@@ -60,6 +60,75 @@ def test_planned_batch_is_bit_identical(cuda, cfg):
     assert torch.equal(full, planned)
 
 
+
+def test_planned_batch_bermudan_is_bit_identical(cuda):
+    from oplib_b200.model import Batch, Lattice
+    lats = [Lattice.local_vol(n=n, level=0.12 + 0.03 * i, device=cuda) for i, n in enumerate([128, 300, 1024, 1152])]
+    bt = Batch(lats, STRIKES, 3, 0.25, 2.0 ** -14, mode="fp16x3", autotune=False)
+    for cfg in (0, 1, 4, 6):
+        bt.set_config(cfg)
+        full, planned = _both(lambda: bt.execute_bermudan(barrier=0.6).clone())
+        assert torch.equal(full, planned)
+
+
+# what the plan and the kernel have to agree on: the tiles, and the order that a product walks them in
+@pytest.mark.parametrize("knob,value,default", [("opb_set_tile_n", 128, 0), ("opb_set_tile_n", 64, 0),
+                                                ("opb_set_cta_pair", 0, 1), ("opb_set_group_m", 3, 0),
+                                                ("opb_set_group_m", 1, 0), ("opb_set_stage_k", 32, 64)])
+@pytest.mark.parametrize("max_d", [0, 1 << 30])
+def test_planned_squarings_under_the_tuning_knobs(cuda, knob, value, default, max_d):
+    from oplib_b200 import _lib
+    from oplib_b200.model import Lattice
+    lib = _lib.load()
+    lat = Lattice.local_vol(n=2304, device=cuda)
+    assert lib.opb_set_fused_normalisation(max_d) == 0 and getattr(lib, knob)(value) == 0
+    try:
+        full, planned = _both(lambda: lat.solve(STRIKES, 2, 0.25, 2.0 ** -10, mode="bf16x3", all_states=True)[1])
+    finally:
+        getattr(lib, knob)(default)
+        lib.opb_set_fused_normalisation(-1)
+    assert torch.equal(full, planned)
+
+
+@pytest.mark.parametrize("mode", ["bf16x3", "fp16x3"])
+@pytest.mark.parametrize("max_d", [0, 1 << 30])
+@pytest.mark.parametrize("n,banded", [(1536, True), (1600, False), (2048, True)])
+def test_planned_squarings_of_a_dense_generator(cuda, n, banded, max_d, mode):
+    """Given densely, a generator starts with every block marked; banded or not, the results are the full
+    products'."""
+    import ctypes as C
+    from oplib_b200 import _lib
+    from oplib_b200.model import MODES, Lattice, Plan, bind_stream
+    lib = _lib.load()
+    lat = Lattice.local_vol(n=n, device=cuda)
+    L = torch.zeros(n, n, dtype=torch.float64, device=cuda)
+    if banded:
+        cols = lat.cols.view(n, 3).long()
+        L.scatter_add_(1, cols.clamp(min=0), torch.where(cols >= 0, lat.vals.view(n, 3), 0.0))
+    else:
+        L = torch.rand(n, n, dtype=torch.float64, device=cuda, generator=torch.Generator(device=cuda).manual_seed(1))
+        L -= torch.diag(L.sum(1))
+    K = torch.as_tensor(STRIKES, device=cuda)
+    desc = lat.desc(Plan(6, float(0.25 / L.diagonal().abs().max()), 0.0), 0.25, 2, K)
+    desc.ell_width, desc.gen_cols, desc.gen_vals, desc.gen_dense = 0, None, None, L.data_ptr()
+    ws = lat.workspace(len(STRIKES), MODES[mode])
+
+    def run():
+        V = torch.empty(2, n, len(STRIKES), dtype=torch.float64, device=cuda)
+        q = torch.empty(2, len(STRIKES), dtype=torch.float64, device=cuda)
+        bind_stream(cuda)
+        assert lib.opb_lattice_solve(C.byref(desc), MODES[mode], ws.data_ptr(), ws.numel(), q.data_ptr(),
+                                     V.data_ptr()) == 0
+        return V
+
+    assert lib.opb_set_fused_normalisation(max_d) == 0
+    try:
+        full, planned = _both(run)
+    finally:
+        lib.opb_set_fused_normalisation(-1)
+    assert torch.equal(full, planned)
+
+
 def _spoiled(lat, how, dt):
     """The lattice with one node's rates far from the quoted state spoiled, and its band as wide as the
     matrix (an entry of rate zero in the far corner), so that band skipping leaves nothing out."""
