@@ -149,7 +149,9 @@ __global__ void k_bias_gelu(long long total4, float *__restrict__ Z, const float
     if (i >= total4) return;
     const float4 zv = reinterpret_cast<const float4 *>(Z)[i];
     const float *bc = b + 4 * (i % (MLP_H / 4));
-    const float z[4] = {zv.x + bc[0], zv.y + bc[1], zv.z + bc[2], zv.w + bc[3]};
+    const float4 bv = reinterpret_cast<uintptr_t>(b) % 16 == 0 ? *reinterpret_cast<const float4 *>(bc)
+                                                               : make_float4(bc[0], bc[1], bc[2], bc[3]);
+    const float z[4] = {zv.x + bv.x, zv.y + bv.y, zv.z + bv.z, zv.w + bv.w};
     float h[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) h[j] = gelu(z[j]);
