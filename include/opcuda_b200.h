@@ -432,7 +432,7 @@ int opb_mc_mt19937_eval(const float *C, long long row_stride, long long col_stri
  * the device-memory budget, or a loop that cannot afford cudaMalloc's implicit device
  * synchronisation).  The payoff partial sums use a fixed 64 KiB device array inside the
  * library (held by every GPU that loads it until exit); results are bit-identical to
- * opb_mc_mt19937.  Grids above 4096 blocks (devices with more than 512 SMs) return
+ * opb_mc_mt19937.  Grids above 4096 blocks (24 an SM: devices with more than 170 SMs) return
  * OPB_E_UNSUPPORTED, and so do runs longer than 623 steps (they would need the driver's
  * local-memory reservation to grow).  The first call on a device, whatever its arguments, looks up
  * the array's device address (make it before any stream capture); the address is kept for the

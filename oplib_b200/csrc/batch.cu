@@ -6,15 +6,15 @@
 // (oplib/opmodel/models/CModel Common.cs:508-545, CModel Device.cs:216-228).  Here every
 // squaring level of all lattices is ONE persistent tcgen05 launch over a work list of
 // (lattice, m-tile, n-tile) items.  Its epilogue writes the next level's 16-bit parts and
-// applies the previous level's deferred FP64 row normalisation, so between levels only a
-// small row-fix launch runs (plus a renormalisation of the lattices whose last level it
-// was); chaining and pricing are batched the same way.  The plan (tables, tensor maps, work
+// applies the previous level's deferred FP64 row normalisation, so between levels only the
+// next level's tile plan runs, which forms the row fixes (plus a renormalisation of the lattices
+// whose last level it was); chaining and pricing are batched the same way.  The plan (tables, tensor maps, work
 // lists) is built once on the host and uploaded into the caller's workspace; execute()
 // then issues 2-4 launches per level with no host synchronisation and no allocation, so a
 // whole sweep can be captured in a CUDA graph and replayed.
 //
-// Tile shape and work order are chosen by opb_batch_autotune, which times the chain
-// product for each candidate (tile width 64, 128, 256 or 256 on CTA pairs; items ordered
+// Tile shape and work order are chosen by opb_batch_autotune, which times the plan's
+// squarings for each candidate (tile width 64, 128, 256 or 256 on CTA pairs; items ordered
 // longest-K first or by lattice) with CUDA events and keeps the fastest.
 #include <algorithm>
 #include <cmath>
@@ -188,7 +188,6 @@ struct PlanDesc {
     PlanDesc(const opb_batch_desc *b, int mode) : d(plan_sizes(b, mode)), desc(*b) { desc.d = d.data(); }
 };
 
-// Layout of all device buffers and tables; with base == nullptr it only measures.
 // K-blocks of 64 that a squaring tile (rows [m0, m0 + tm), columns [n0, n0 + tn)) issues at
 // `level` when the generator's half-bandwidth is h0 (0: unknown, dense): the host mirror of
 // the kernel's band_kblocks with its 128-wide accumulation chunks, used to order the work.
@@ -203,6 +202,7 @@ int host_band_kblocks(int h0, int level, int m0, int tm, int n0, int tn, int K) 
     return std::min(2 * c_hi, all) - 2 * c_lo;
 }
 
+// Layout of all device buffers and tables; with base == nullptr it only measures.
 // bands: the generators' half-bandwidths (nullptr when only measuring): the squaring levels'
 // work lists of the longest-first configurations are then ordered by the K-blocks each item
 // issues at that level, longest first.

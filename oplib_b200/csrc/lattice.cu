@@ -360,9 +360,10 @@ int solve_tc(const opb_lattice_desc &L, Bufs &b, double *quotes, double *V_all, 
     // Without the all-state values the quotes are one row of each P_m G, and that row of P_m
     // needs the same row of P_{m-1} and P1: one pass over P1 per maturity instead of a d^3
     // product, then one product prices up to kRowSlots maturities' rows together.  The quotes
-    // are the full products' bit for bit (row_chain.cuh).  The rows lie in X (P1's FP32 form,
-    // done with), their parts in the FP32 chain buffer.  Larger lattices than the row kernel's
-    // shared memory takes, and the K-sliced accumulation knob, go through the full products.
+    // are the full products' up to the order of the rows' FP64 sums (row_chain.cuh): 1e-16, unless
+    // that flips an FP32 rounding of the normalised row.  The rows lie in X (P1's FP32 form, done
+    // with), their parts in the FP32 chain buffer.  Larger lattices than the row kernel's shared
+    // memory takes, and the K-sliced accumulation knob, go through the full products.
     if (!V_all && opb::row_chain_fits(d) && g_ksplit <= 1) {
         opb::RowChainLat R{};
         R.d = d;

@@ -73,13 +73,14 @@ struct McArgs {
 // fits 32 bits (McArgs::rs4), which makes a row's address one multiply-add.  STATES: ypaths is
 // given.
 //
-// What bounds it: issue slots, half of them of the integer pipe (one instruction in two cycles
-// a scheduler), so it is the instructions per step that count -- one tw() per output however
+// What bounds it: the gathers (guide word, row entry, node value), of which L1 holds half and L2
+// serves the rest, 26 bytes a step (ncu, 2^20 paths x 504 steps over 512 states: memory pipes 89 %,
+// issue 56 %, integer pipe 57 %), and their latency in the step's chain of dependent loads.  So as
+// few instructions as possible stand between them -- 65 per 32 steps: one tw() per output however
 // many cursors (mt19937.cuh), the barrier as a flag instead of a running FP64 minimum, no
-// branches for what the launch does not ask for.  Six blocks of 256 an SM (40 registers) hide
-// the step's chain of dependent loads (guide word, row entry, next guide word); the form for
-// longer runs gains more from registers than from warps.  2^20 paths x 504 steps over 512
-// states: 2.51 -> 1.81 ms.  PER_SM: blocks of 256 an SM, see mc_more_resident.
+// branches for what the launch does not ask for -- and six blocks of 256 an SM (40 registers) hide
+// it; the form for longer runs gains more from registers than from warps.  That run: 2.51 ms with
+// 110 instructions, 1.50-1.68 now.  PER_SM: blocks of 256 an SM, see mc_more_resident.
 template <bool ANY_LENGTH, bool GUIDED, bool EVAL, bool STATES, int PER_SM>
 __global__ void __launch_bounds__(256, PER_SM) k_mc(McArgs a) {
     double s_bar = 0.0, s_asi = 0.0;
@@ -206,8 +207,8 @@ __global__ void k_mt_raw(uint32_t seed, long long nstreams, int n, uint32_t *__r
 // Paths to blocks.  A path is one thread's work from end to end, so blocks are what the SMs can
 // be evened out with: up to 24 blocks an SM, four times what is resident, each of as few
 // threads as that allows (64 at least) -- a grid of the resident blocks alone walks 3.46 paths
-// a thread at 2^20 paths and waits for the fourth.  100,003 paths of 700 steps: 391 blocks of
-// 256 (three on an SM, or two) 554 us, 1563 of 64 443.
+// a thread at 2^20 paths and waits for the fourth.  100,003 unguided paths of 700 steps: 391
+// blocks of 256 (three on an SM, or two) 1664 us, 1563 of 64 1540.
 constexpr int MC_BLOCKS_PER_SM = 24;
 
 static int mc_threads(long long npaths) {

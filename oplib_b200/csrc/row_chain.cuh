@@ -3,10 +3,13 @@
 //
 // A European solve reads P_m in one row alone, the quoted state's: quotes[m][k] = e^{-rT_m}
 // (P_m G)[y0, k].  Row y0 of P_m is a function of row y0 of P_{m-1} and of P1, and in the
-// tensor cores every output row is formed by itself, so the row comes out of these kernels
-// bit for bit as it does out of the full product: the same operand parts, the same MMAs
+// tensor cores every output row is formed by itself, so from the same row of P_{m-1} these kernels
+// form the product's row bit for bit as the full product does: the same operand parts, the same MMAs
 // (hi.hi, hi.lo, lo.hi per 16 of K) in the same K order into an accumulator that starts from
-// zero every 128 of K, the chunks added in order in FP32, then the epilogue's arithmetic.
+// zero every 128 of K, the chunks added in order in FP32, then the epilogue's arithmetic.  The row's
+// normalisation adds its FP64 sum in another order (256 threads and a shuffle tree, not partials
+// per 128 columns), so from the third maturity on a row agrees to that order's 1e-16, or to an
+// FP32 rounding that it flips.
 // (Callers that ask for the values of every state take the full products.)
 //
 // What bounds it: one pass over P1's parts per maturity (4 d^2 bytes, 151 MB at d = 6144:

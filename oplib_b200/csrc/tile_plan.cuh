@@ -19,8 +19,11 @@
 // stay zero, orders the others by the K-blocks they issue, most first (the persistent CTAs walk
 // the tiles round robin, and the counts now differ by an order of magnitude between the diagonal
 // and the corners), clears the marks that the squaring is going to write, and forms the row
-// fixes of the previous level on the way (it replaces that kernel's launch).  It costs a launch of 4-6 us per level, so single lattices
-// below OPB_PLAN_MIN_D states, whose whole product takes about 16 us, go without.
+// fixes of the previous level on the way (it replaces that kernel's launch).  It costs a launch of
+// 4-6 us per level, so single lattices below OPB_PLAN_MIN_D states, whose whole product takes about 16
+// us, go without.  A dense generator has it too: given densely, a banded one of 2048 states takes
+// 720 us with its plans, 1330 before there were any; one that leaves no block zero pays for them up
+// to there (1017 -> 1065 us) and not from 3072 states on.
 
 struct TilePlanArgs {
     TilePlan pl;
